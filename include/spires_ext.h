@@ -90,7 +90,7 @@ typedef struct {
                          loaded with L2 evict-last priority and younger lags
                          and the ring writes with evict-first, so that part of
                          a ring larger than the L2 stays resident from step to
-                         step; 0 = no cache hints, -1 = automatic (default: 70 %
+                         step; 0 = no cache hints, -1 = automatic (default: 60 %
                          of the L2 when the ring is larger than three quarters
                          of it, else 0) */
 } spires_ext_launch;

@@ -81,15 +81,6 @@ constexpr int kHistC = 8;  // ring values per cp.async group and thread
 // per SM allow, and one CTA per SM halved the sweep's throughput)
 constexpr int kHistS = 4;
 
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem)), "l"(gmem)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 // FLIF_GL history of column `ci` for lags 2..lim in ascending order, with the
 // ring values copied asynchronously into this thread's own shared-memory
 // slots (s_h[(stage * kHistC + j) * kBatchThreads + tid]) kHistS groups ahead,
@@ -179,6 +170,7 @@ __device__ __forceinline__ double rowpass_simple_warp_deep(const long long *__re
 {
     const long long e0 = __ldg(row_ptr + row0);
     const long long e1 = __ldg(row_ptr + row0 + 32);
+    const long long my_start = __ldg(row_ptr + row0 + lane);
     const long long my_end = __ldg(row_ptr + row0 + lane + 1);
     double acc = 0.0;
     int cn[U];
@@ -203,16 +195,8 @@ __device__ __forceinline__ double rowpass_simple_warp_deep(const long long *__re
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const bool sp = c[u] >= 0 && ((s_spk[c[u] >> 5] >> (c[u] & 31)) & 1u);
-            unsigned m = __ballot_sync(kFull, sp);
-            while (m) {
-                const int bpos = __ffs(m) - 1;
-                m &= m - 1;
-                const long long eb = base + 32 * u + bpos;
-                const double wb = __shfl_sync(kFull, wv[u], bpos);
-                const unsigned owner = __ballot_sync(kFull, my_end > eb);
-                if (lane == __ffs(owner) - 1)
-                    acc = add(acc, wb);
-            }
+            const long long cb = base + 32 * u;
+            acc = add_chunk(acc, wv[u], __ballot_sync(kFull, sp), my_start - cb, my_end - cb);
         }
     }
     return acc;

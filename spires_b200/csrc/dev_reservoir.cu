@@ -46,10 +46,30 @@ kfn_t pick_syn(int st)
     return nullptr;
 }
 
+// the cluster kernel: synapses whose exchange is the spike words alone
+template <int ST>
+kfn_t pick_words(int nt)
+{
+    switch (nt) {
+    case SP_LIF_DISCRETE: return k_run<SP_LIF_DISCRETE, ST, 3>;
+    case SP_LIF_BIO: return k_run<SP_LIF_BIO, ST, 3>;
+    case SP_FLIF_CAPUTO: return k_run<SP_FLIF_CAPUTO, ST, 3>;
+    case SP_FLIF_GL: return k_run<SP_FLIF_GL, ST, 3>;
+    case SP_FLIF_DIFFUSIVE: return k_run<SP_FLIF_DIFFUSIVE, ST, 3>;
+    }
+    return nullptr;
+}
+
 kfn_t pick_kernel(int nt, int st, int variant)
 {
     if (variant == 1)
         return nt == SP_FLIF_GL ? pick_syn<SP_FLIF_GL, 1>(st) : nullptr;
+    if (variant == 2)
+        return nt == SP_FLIF_GL       ? pick_syn<SP_FLIF_GL, 2>(st)
+               : nt == SP_FLIF_CAPUTO ? pick_syn<SP_FLIF_CAPUTO, 2>(st)
+                                      : nullptr;
+    if (variant == 3)
+        return st == SP_SYN_SIMPLE ? pick_words<SP_SYN_SIMPLE>(nt) : pick_words<SP_SYN_PSC_HET>(nt);
     switch (nt) {
     case SP_LIF_DISCRETE: return pick_syn<SP_LIF_DISCRETE, 0>(st);
     case SP_LIF_BIO: return pick_syn<SP_LIF_BIO, 0>(st);
@@ -235,12 +255,16 @@ static int dupload(T **p, const T *h, size_t count, cudaStream_t s)
     return SP_OK;
 }
 
+// Zeros before and after the device copy of the coefficients (caputo_sum reads
+// up to three places beyond either end).
+static size_t coef_pad(int ntype) { return ntype == SP_FLIF_CAPUTO ? 4 : 0; }
+
 static int upload_consts(sp_dev *d, const sp_host_model *m)
 {
     d->nc = m->nc;
     if (m->coef && d->coef)
-        SP_CK(cudaMemcpyAsync(d->coef, m->coef, (size_t)m->nc.L * sizeof(double),
-                              cudaMemcpyHostToDevice, d->stream));
+        SP_CK(cudaMemcpyAsync(d->coef + coef_pad(m->neuron_type), m->coef,
+                              (size_t)m->nc.L * sizeof(double), cudaMemcpyHostToDevice, d->stream));
     return SP_OK;
 }
 
@@ -270,57 +294,215 @@ static void box_geometry(const sp_dev *d, const sp_launch &l, int *bw, int *nbx)
     *bw = (w + 1) & ~1;
 }
 
-// SIMPLE synapse: the CTA's CSR slice (position-space row offsets, column
-// positions, weights) is copied to shared memory at the start of a launch
-// when its largest slice has at most kCsrSmemEdges edges, so the row pass
-// after each grid barrier reads no global memory. Returns the edge capacity
-// to reserve (0: rows are walked from global memory).
-constexpr long long kCsrSmemEdges = 2048;
+// SIMPLE synapse, form of the recurrent rows in a launch. A dense matrix keeps
+// column blocks (dense_rows), staged in shared memory when the largest CTA's
+// fit kColSmem* bytes. Other rows are kept as slots and tails (row_slots) and
+// staged when the largest CTA's fit kRowSmem* bytes, else the CSR rows are
+// walked in global memory. Variant 1's ring stages need most of the shared
+// memory, so its limits are lower.
+constexpr size_t kRowSmem0 = 128 * 1024, kRowSmem1 = 48 * 1024;
+constexpr size_t kColSmem0 = 160 * 1024, kColSmem1 = 48 * 1024;
 
-static long long csr_smem_edges(const sp_dev *d, const sp_launch &l)
+struct RowPlan {
+    int ell_cap, tail_cap, col_mode, col_cap;
+    size_t bytes;  // shared memory
+};
+
+static RowPlan row_plan(const sp_dev *d, const sp_launch &l)
 {
-    if (d->stype != SP_SYN_SIMPLE || !d->h_row_ptr || l.ctas < 1 || l.csr_global)
-        return 0;
+    RowPlan r = {0, 0, 0, 0, 0};
+    if (d->stype != SP_SYN_SIMPLE || l.ctas < 1 || l.csr_global)
+        return r;
     const long long nw = (long long)d->nwords;
-    long long mx = 0;
-    for (long long b = 0; b < l.ctas; ++b) {
-        const long long w0 = b * nw / l.ctas, w1 = (b + 1) * nw / l.ctas;
-        const long long e = d->h_row_ptr[32 * w1] - d->h_row_ptr[32 * w0];
-        if (e > mx)
-            mx = e;
+    if (d->col_blk) {
+        int mx = 0;  // most edges of a CTA
+        for (long long b = 0; b < l.ctas; ++b)
+            mx = std::max(mx, d->h_col_off[(b + 1) * nw / l.ctas] - d->h_col_off[b * nw / l.ctas]);
+        const size_t nwn = ((size_t)d->n + 31) / 32;
+        r.col_mode = 1;
+        r.bytes = ((nwn + 3) / 4 * 16 + (size_t)d->n * 2 + 8 + 127) / 128 * 128;
+        const size_t b = ((size_t)mx * 8 + (size_t)l.warps_max * d->n * 8 + 127) / 128 * 128;
+        if (b <= (l.variant == 1 ? kColSmem1 : kColSmem0)) {
+            r.col_mode = 2;
+            r.col_cap = mx;
+            r.bytes += b;
+        }
+    } else if (d->ell_off) {
+        int mg = 1, mt = 0;
+        for (long long b = 0; b < l.ctas; ++b) {
+            const long long w0 = b * nw / l.ctas, w1 = (b + 1) * nw / l.ctas;
+            mg = std::max(mg, d->h_ell_off[w1] - d->h_ell_off[w0]);
+            mt = std::max(mt, d->h_tail_off[w1] - d->h_tail_off[w0]);
+        }
+        mt = (mt + 1) & ~1;
+        const size_t b = (size_t)1280 * mg +
+                         ((size_t)12 * mt + (size_t)132 * l.warps_max + 127) / 128 * 128;
+        if (b <= (l.variant == 1 ? kRowSmem1 : kRowSmem0)) {
+            r.ell_cap = mg;
+            r.tail_cap = mt;
+            r.bytes = b;
+        }
     }
-    return mx <= kCsrSmemEdges ? (mx > 0 ? mx : 1) : 0;
+    return r;
 }
 
-static size_t csr_smem_bytes(long long cap, int warps_max)
+// Slot groups of four per row of one warp, the rest of a longer row becoming its
+// tail: the number with the least estimated cycles (rowpass_lanes: 110 per group
+// beyond two, 200 per 32 tail edges).
+static int row_slots(const long long *rp /* [33] */)
 {
-    if (cap <= 0)
-        return 0;
-    const size_t rows = 32 * (size_t)warps_max + 1;
-    return ((size_t)cap * 8 + 127) / 128 * 128 + ((size_t)cap * 4 + 127) / 128 * 128 +
-           (rows * 4 + 127) / 128 * 128;
+    long long longest = 0;
+    for (int q = 0; q < 32; ++q)
+        longest = std::max(longest, rp[q + 1] - rp[q]);
+    const long long full = (longest + 3) / 4;
+    long long best = 0, best_cost = -1;
+    for (long long g = 1; g <= full; g += g < 8 ? 1 : (g + 7) / 8) {
+        long long cost = 360 + 110 * (g > 2 ? g - 2 : 0);
+        for (int q = 0; q < 32; ++q) {
+            const long long tail = rp[q + 1] - rp[q] - 4 * g;
+            if (tail > 0)
+                cost += 200 * ((tail + 31) / 32);
+        }
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = g;
+        }
+    }
+    return (int)best;
 }
 
-// variant 1 stages the coefficient table in shared memory up to 64 KB
+// Whether the recurrent rows are kept as column blocks: a block of 32 rows has
+// an edge from most spiking neurons (at least one pair in 48), and rows are
+// long enough that walking their edges costs more than listing the spikes (16
+// edges; the list takes about 500 cycles a step and 17 per spiking neuron, the
+// walk 27 per edge of the longest row). The list holds 16-bit neuron numbers
+// and the blocks take n^2 / 4 bytes. (LIF_DISCRETE N=1000, 100 edges per row,
+// 0.5 % of the neurons spiking: 1.6 us per step on 16 CTAs; walking the edges
+// row by row 3.0, and 26.7 edge by edge on one CTA.)
+static bool dense_rows(const sp_host_model *m)
+{
+    return m->syn_type == SP_SYN_SIMPLE && m->n <= 16384 && m->nnz >= 16 * m->n &&
+           (double)m->nnz * 48.0 >= (double)m->n * (double)m->n && m->nnz < ((size_t)1 << 31);
+}
+
+// the coefficient table in shared memory (eight elements of padding), up to 64 KB
 static size_t coef_smem_bytes(const sp_dev *d)
 {
-    const size_t b = ((size_t)d->nc.L * 8 + 127) & ~(size_t)127;
+    const size_t b = ((size_t)d->nc.L * 8 + 64 + 127) & ~(size_t)127;
     return b <= 64 * 1024 ? b : 0;
 }
 
-// dynamic shared memory of a launch shape: spike words, then (variant 1) the
-// ring-row stages and their full/empty mbarriers
-static size_t launch_smem(const sp_dev *d, const sp_launch &l)
+// dynamic shared memory of a launch shape: two buffers of spike words, the
+// recurrent rows, the input weights where they fit, then (variant 1) the
+// coefficients, the ring-row stages and their full/empty mbarriers
+static size_t spk_smem_bytes(const sp_dev *d)
 {
-    size_t spk = (l.variant == 1 ? 2 : 1) * (((d->nwords * 4) + 127) & ~(size_t)127) +
-                 csr_smem_bytes(csr_smem_edges(d, l), l.warps_max);
-    if (l.variant == 1) {
+    return 2 * (((d->nwords * 4) + 127) & ~(size_t)127);
+}
+
+// Kernel variants (the template's VAR). A launch's variant 1 is the bulk-copy
+// pipeline (1). Its variant 0 is, in this order: 2, 4, 8 or 16 CTAs as one
+// cluster that exchanges spike words through shared memory (3); at most
+// kPipeWarps warps per CTA and a gather warp, FLIF_GL with the ring columns of
+// the CTA's neurons in shared memory for the launch (2); the generic kernel
+// (0).
+
+// Whether the launch stages the coefficient table (up to 64 KB): FLIF_GL in
+// every kernel but the generic one, FLIF_CAPUTO in all.
+static bool stages_coef(const sp_dev *d, int kv)
+{
+    return ((kv != 0 && d->ntype == SP_FLIF_GL) || d->ntype == SP_FLIF_CAPUTO) &&
+           coef_smem_bytes(d) > 0;
+}
+
+// Extra warps of a launch: the producer (kernel 1) and the gather warp.
+static int extra_warps(int kv) { return kv == 1 ? 2 : kv == 2 ? 1 : 0; }
+
+struct SmemPlan {
+    int win_smem, u_ring;
+    size_t bytes;
+};
+
+static SmemPlan smem_plan(const sp_dev *d, const sp_launch &l, int kv)
+{
+    SmemPlan pl = {0, 0, 0};
+    size_t b = spk_smem_bytes(d) + row_plan(d, l).bytes;
+    if (kv == 3)
+        b += ((size_t)16 * d->nwords + 127) / 128 * 128;
+    const bool pairs = kv >= 2 && d->ntype == SP_FLIF_GL;  // ring rows in pairs
+    if (stages_coef(d, kv))
+        b += (pairs ? 2 : 1) * coef_smem_bytes(d);
+    if (pairs)
+        b += (size_t)(d->nc.L + 1) / 2 * 64 * l.warps_max * sizeof(double);
+    if (kv == 1) {
         int bw, nbx;
         box_geometry(d, l, &bw, &nbx);
-        return spk + coef_smem_bytes(d) + (size_t)l.stages * nbx * l.rows * bw * sizeof(double) +
-               2 * (size_t)l.stages * sizeof(unsigned long long);
+        b += (size_t)l.stages * nbx * l.rows * bw * sizeof(double) +
+             2 * (size_t)l.stages * sizeof(unsigned long long);
     }
-    return spk;
+    if (d->din > 0 && d->din <= 32) {
+        const size_t u = ((size_t)l.warps_max * kURows * d->din * 8 + 127) / 128 * 128;
+        const size_t win = (size_t)d->din * 32 * l.warps_max * sizeof(double);
+        if (b + u + 1024 <= (size_t)d->smem_max) {
+            pl.u_ring = 1;
+            b += u;
+        }
+        if (b + win + 1024 <= (size_t)d->smem_max) {
+            pl.win_smem = 1;
+            b += win;
+        }
+    }
+    pl.bytes = b;
+    return pl;
+}
+
+static int kernel_variant(const sp_dev *d, const sp_launch &l)
+{
+    if (l.variant != 0)
+        return l.variant;
+    const size_t room = (size_t)d->smem_max - 1024;
+    const bool gl = d->ntype == SP_FLIF_GL;
+    const bool words = d->stype == SP_SYN_SIMPLE || d->stype == SP_SYN_PSC_HET;
+    if (words && l.ctas <= d->cluster_max &&
+        (l.ctas == 2 || l.ctas == 4 || l.ctas == 8 || l.ctas == 16) &&
+        l.warps_max <= kClusterWarps && d->nwords <= (size_t)kClusterWords &&
+        (!gl || coef_smem_bytes(d) > 0) && smem_plan(d, l, 3).bytes <= room)
+        return 3;
+    if ((gl || d->ntype == SP_FLIF_CAPUTO) && l.warps_max <= kPipeWarps &&
+        (!gl || coef_smem_bytes(d) > 0) && smem_plan(d, l, 2).bytes <= room)
+        return 2;
+    return 0;
+}
+
+// Largest cluster (16, 8 or none) that the device schedules with the cluster
+// kernel's largest block and shared memory.
+static int max_cluster(int smem_max)
+{
+    const void *fn = (const void *)k_run<SP_LIF_DISCRETE, SP_SYN_SIMPLE, 3>;
+    if (set_max_dynamic_smem(fn) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    for (int g : {16, 8}) {
+        cudaLaunchConfig_t c;
+        cudaLaunchAttribute a;
+        memset(&c, 0, sizeof(c));
+        memset(&a, 0, sizeof(a));
+        a.id = cudaLaunchAttributeClusterDimension;
+        a.val.clusterDim.x = (unsigned)g;
+        a.val.clusterDim.y = a.val.clusterDim.z = 1;
+        c.gridDim = dim3((unsigned)g);
+        c.blockDim = dim3(32 * kClusterWarps);
+        c.dynamicSmemBytes = (size_t)smem_max - 1024;
+        c.attrs = &a;
+        c.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, fn, &c) == cudaSuccess && n >= 1)
+            return g;
+        cudaGetLastError();
+    }
+    return 0;
 }
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
@@ -366,30 +548,21 @@ static int encode_ring_map(sp_dev *d, int bw, int r)
     return SP_OK;
 }
 
-static int max_smem(const sp_dev *d)
-{
-    int v = 0;
-    cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device);
-    return v > 0 ? v : 48 * 1024;
-}
-
 // Lags kept L2-resident by the variant-1 cache hints when the launch asks for
 // the automatic choice. A ring that does not fit in the L2 would miss on every
 // row under plain replacement (each row is read once per step, in a cycle
-// longer than the cache), so the oldest lags of every step -- 70 % of the L2
+// longer than the cache), so the oldest lags of every step -- 60 % of the L2
 // -- are read with evict-last priority and stay resident, while younger rows
-// stream through with evict-first. (N=20000, L=1024 on one B200: 490 lags,
-// 24.6-24.9 us per step against 29.3 without hints; 600 lags 25.1, 700 lags
-// 27.7 -- the streamed rows then evict resident ones -- and the earlier
-// choice of a fixed set of ring slots at half the L2, 26.0 with a wide
-// spread from launch to launch.)
+// stream through with evict-first. (N=20000, L=1024 on one B200, 256 steps
+// with readouts: 420 lags 6.47 ms, 490 lags -- 70 % -- 6.52, 560 lags 6.60;
+// without hints 7.7.)
 static int auto_l2_pin(const sp_dev *d)
 {
     const double row = (double)d->rs * sizeof(double);
     const double ring = row * d->nc.L;
     if (d->l2_bytes <= 0 || ring <= 0.75 * d->l2_bytes)
         return 0;
-    const int rows = (int)(0.7 * d->l2_bytes / row);
+    const int rows = (int)(0.6 * d->l2_bytes / row);
     return rows < d->nc.L ? rows : d->nc.L;
 }
 
@@ -409,24 +582,48 @@ static void default_launch(sp_dev *d)
     sp_launch l;
     memset(&l, 0, sizeof(l));
     l.l2_pin = -1;
-    if (nw <= 32) {
-        l.ctas = 1;
-        l.warps_max = nw;
-    } else {
-        int G = d->num_sms < nw ? d->num_sms : nw;
-        l.ctas = G;
-        l.warps_max = (nw + G - 1) / G;
-        if (l.warps_max > 32)
-            l.warps_max = 32;
-    }
-    if (d->ntype == SP_FLIF_GL && d->nc.L >= 32 && l.warps_max <= kPipeWarps) {
+    auto shape = [&](int G) {
+        sp_launch v = l;
+        v.ctas = G;
+        v.warps_max = (nw + G - 1) / G;
+        return v;
+    };
+    const bool gl = d->ntype == SP_FLIF_GL;
+    // The fewest warps per CTA that the SMs allow, spread evenly (LIF_DISCRETE
+    // N=20000: 125 CTAs of 5 warps 3.8 us per step, 148 of 4 or 5 4.5); the
+    // balanced layout of FLIF_GL is made for all of them.
+    int W = (nw + d->num_sms - 1) / d->num_sms;
+    W = W > 32 ? 32 : W;
+    const sp_launch wide = d->bal_G > 0 ? shape(d->bal_G) : shape((nw + W - 1) / W);
+    // One cluster, where its exchange through shared memory is what paces a
+    // step: models without a history (N=2000: 1.06 us per step on 16 CTAs of 4
+    // warps, 1.45 on 63 of one; N=8000: 1.37 against 1.53), and a short FLIF_GL
+    // history on many warps (N=4000, L=64: 2.5 us against 3.4; at N=2000, L=256
+    // the history sum hides the slower exchange). Column blocks only where
+    // they fit the 16 CTAs' shared memory.
+    const sp_launch clus = shape(nw >= 16 ? 16 : 8);
+    const bool cluster = nw > 6 && kernel_variant(d, clus) == 3 &&
+                         row_plan(d, clus).col_mode != 1 && d->ntype != SP_FLIF_CAPUTO &&
+                         (!gl || (nw >= 64 && clus.warps_max * d->nc.L <= 768));
+    if (nw <= 4)
+        l = shape(1);  // a warp per scheduler, nothing to exchange
+    else if (cluster)
+        l = clus;
+    else if (nw <= 6 && !gl && d->ntype != SP_FLIF_CAPUTO)
+        l = shape(1);
+    else
+        l = wide;
+    // FLIF_GL: the history in shared memory where it fits (N=2000, L=256: 3.2
+    // us per step, 5.7 through the pipeline; N=20000, L=128: 5.9 and 6.1), else
+    // the pipeline
+    if (gl && d->nc.L >= 32 && l.warps_max <= kPipeWarps && kernel_variant(d, l) == 0) {
         // The ring stream is paced by the bytes in flight per SM (the stages
         // the consumers are not reading): long rings take the stage height of
         // 64 or 48 rows that puts the most rows in flight (ties: taller),
-        // shorter rings 32-row stages. (N=20000, L=1024 on 148 SMs: 3 x 48
-        // rows, 31.7 us per step, against 31.9 for 2 x 64 and 33.0 for 3 x 56,
-        // whose extra bytes in flight slow the serial phase's loads more than
-        // they speed the stream.)
+        // shorter rings 32-row stages. A ring beyond the L2 takes at most 144
+        // KB of them: more slow the serial phase's loads and the resident lags
+        // more than they speed the stream (N=20000, L=1024 on 148 SMs, 256
+        // steps: 2 x 64 rows 6.52 ms, 4 x 32 6.55, 3 x 48 6.69, 4 x 40 6.96).
         sp_launch best = l;
         long long best_rows = 0;
         for (int rows : {64, 48, 32}) {
@@ -438,13 +635,13 @@ static void default_launch(sp_dev *d)
             int bw, nbx;
             box_geometry(d, v, &bw, &nbx);
             const size_t stage = (size_t)v.rows * nbx * bw * sizeof(double);
-            const size_t budget = (size_t)(max_smem(d) - 2 * 1024);
-            const size_t spk = 2 * (((d->nwords * 4) + 127) & ~(size_t)127) +
-                               coef_smem_bytes(d) +
-                               csr_smem_bytes(csr_smem_edges(d, v), v.warps_max);
+            const size_t budget = (size_t)(d->smem_max - 2 * 1024);
+            const size_t spk = spk_smem_bytes(d) + coef_smem_bytes(d) + row_plan(d, v).bytes;
             long long st = budget > spk ? (long long)((budget - spk) / (stage + 16)) : 0;
             if (st > 16)
                 st = 16;
+            if (auto_l2_pin(d) > 0 && st > (long long)(144 * 1024 / stage))
+                st = (long long)(144 * 1024 / stage);
             if (st >= 2 && st * rows > best_rows &&
                 encode_ring_map(d, bw, v.rows < d->nc.L ? v.rows : d->nc.L) == SP_OK) {
                 v.stages = (int)st;
@@ -526,6 +723,10 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
         }
         cudaDeviceGetAttribute(&d->num_sms, cudaDevAttrMultiProcessorCount, d->device);
         cudaDeviceGetAttribute(&d->l2_bytes, cudaDevAttrL2CacheSize, d->device);
+        cudaDeviceGetAttribute(&d->smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device);
+        if (d->smem_max <= 0)
+            d->smem_max = 48 * 1024;
+        d->cluster_max = max_cluster(d->smem_max);
         int coop = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d->device);
         d->coop = coop;
@@ -623,17 +824,100 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
         d->flag_cap = 8 * (d->num_sms > 0 ? d->num_sms : 1);
         TRY(dalloc(&d->flags, (size_t)d->flag_cap * kFlagStride));
         TRY(dalloc(&d->err, 4));
+        TRY(dalloc(&d->ll, 2 * d->nwords));
+        SP_CK(cudaMemsetAsync(d->ll, 0, 2 * d->nwords * sizeof(unsigned long long), s));
+        if (dense_rows(m)) {
+            // blocks (row word q, neuron j); a row's edges are in ascending
+            // neuron order, so filling row by row leaves each block's weights in
+            // row order
+            std::vector<uint2> blk((size_t)d->nw * n, make_uint2(0u, 0u));
+            std::vector<double> cw(m->nnz);
+            int *off = d->h_col_off = (int *)calloc(d->nw + 1, sizeof(int));
+            if (!off)
+                TRY(SP_EALLOC);
+            for (int q = 0; q < d->nw; ++q) {
+                uint2 *bq = blk.data() + (size_t)q * n;
+                off[q] = (int)rp[32 * q];
+                for (int ln = 0; ln < 32; ++ln) {
+                    const int i = nid_of[32 * q + ln];
+                    if (i >= 0)
+                        for (int64_t k = m->row_ptr[i]; k < m->row_ptr[i + 1]; ++k)
+                            bq[m->col[k]].x |= 1u << ln;
+                }
+                unsigned run = 0;
+                for (size_t j = 0; j < n; ++j) {
+                    bq[j].y = run;
+                    run += (unsigned)__builtin_popcount(bq[j].x);
+                }
+                for (int ln = 0; ln < 32; ++ln) {
+                    const int i = nid_of[32 * q + ln];
+                    if (i >= 0)
+                        for (int64_t k = m->row_ptr[i]; k < m->row_ptr[i + 1]; ++k) {
+                            const uint2 b = bq[m->col[k]];
+                            cw[(size_t)off[q] + b.y +
+                               __builtin_popcount(b.x & ((1u << ln) - 1u))] = m->w[k];
+                        }
+                }
+            }
+            off[d->nw] = (int)m->nnz;
+            TRY(dupload(&d->col_blk, blk.data(), blk.size(), s));
+            TRY(dupload(&d->col_off, off, d->nwords + 1, s));
+            TRY(dupload(&d->col_w, cw.data(), cw.size(), s));
+            SP_CK(cudaStreamSynchronize(s));  // the vectors go out of scope
+        } else if (m->syn_type == SP_SYN_SIMPLE && rs <= 65536) {
+            int *eo = d->h_ell_off = (int *)calloc(d->nw + 1, sizeof(int));
+            int *to = d->h_tail_off = (int *)calloc(d->nw + 1, sizeof(int));
+            if (!eo || !to)
+                TRY(SP_EALLOC);
+            size_t cells = 0;
+            for (int q = 0; q < d->nw; ++q) {
+                const int g = row_slots(rp.data() + 32 * q);
+                eo[q + 1] = eo[q] + g;
+                cells += (size_t)128 * g;
+            }
+            std::vector<unsigned short> ec(cells ? cells : 1, 0);
+            std::vector<double> ew(cells ? cells : 1, 0.0), tw(m->nnz ? m->nnz : 1);
+            std::vector<int> trp((size_t)33 * d->nw, 0), tc(m->nnz ? m->nnz : 1);
+            int nt = 0;
+            for (int q = 0; q < d->nw; ++q) {
+                const int slots = 4 * (eo[q + 1] - eo[q]);
+                for (int ln = 0; ln < 32; ++ln) {
+                    trp[(size_t)33 * q + ln] = nt;
+                    const long long k0 = rp[32 * q + ln], k1 = rp[32 * q + ln + 1];
+                    for (long long k = k0; k < k1; ++k) {
+                        const int sl = (int)(k - k0);
+                        if (sl < slots) {
+                            const size_t g = (size_t)eo[q] + sl / 4, u = sl % 4;
+                            ec[(g * 32 + ln) * 4 + u] = (unsigned short)col[k];
+                            ew[(g * 4 + u) * 32 + ln] = w[k];
+                        } else {
+                            tc[nt] = col[k];
+                            tw[nt++] = w[k];
+                        }
+                    }
+                }
+                trp[(size_t)33 * q + 32] = nt;
+                to[q + 1] = nt;
+            }
+            TRY(dupload(&d->ell_off, eo, d->nwords + 1, s));
+            TRY(dupload((unsigned short **)&d->ell_col, ec.data(), ec.size(), s));
+            TRY(dupload(&d->ell_w, ew.data(), ew.size(), s));
+            TRY(dupload(&d->tail_rp, trp.data(), trp.size(), s));
+            TRY(dupload(&d->tail_col, tc.data(), (size_t)nt, s));
+            TRY(dupload(&d->tail_w, tw.data(), (size_t)nt, s));
+            SP_CK(cudaStreamSynchronize(s));  // the vectors go out of scope
+        }
         TRY(dupload(&d->row_ptr, rp.data(), rs + 1, s));
-        d->h_row_ptr = (long long *)malloc((rs + 1) * sizeof(long long));
-        if (!d->h_row_ptr)
-            TRY(SP_EALLOC);
-        memcpy(d->h_row_ptr, rp.data(), (rs + 1) * sizeof(long long));
         TRY(dupload(&d->col, col.data(), m->nnz, s));
         TRY(dupload(&d->w, w.data(), m->nnz, s));
         TRY(dupload(&d->W_in, win.data(), rs * din, s));
         TRY(dupload(&d->W_out, wout.data(), rs * dout, s));
         if (m->neuron_type == SP_FLIF_GL || m->neuron_type == SP_FLIF_CAPUTO) {
-            TRY(dupload(&d->coef, m->coef, (size_t)m->nc.L, s));
+            const size_t pad = coef_pad(m->neuron_type);
+            TRY(dalloc(&d->coef, (size_t)m->nc.L + 2 * pad));
+            SP_CK(cudaMemsetAsync(d->coef, 0, ((size_t)m->nc.L + 2 * pad) * sizeof(double), s));
+            SP_CK(cudaMemcpyAsync(d->coef + pad, m->coef, (size_t)m->nc.L * sizeof(double),
+                                  cudaMemcpyHostToDevice, s));
             // FLIF_GL: [L][rs] time-major rows; Caputo: [rs][D] per-position registers
             d->ring_elems = rs * (size_t)m->nc.L;
             TRY(dalloc(&d->ring, d->ring_elems));
@@ -729,13 +1013,16 @@ extern "C" void sp_dev_destroy(sp_dev *d)
                     d->edge_omd, d->edge_trace, d->scoef, d->Iring, d->mx_decay, d->mx_omd,
                     d->mx_c, d->mx_tr, d->W_in, d->W_out, d->d_u, d->d_phi, d->d_nat, d->d_y,
                     d->d_spkd, d->d_ras, d->d_ras_nat, d->bar, d->err, d->pos_of, d->nid_of,
-                    d->flags};
+                    d->flags, d->ll, d->col_off, d->col_blk, d->col_w, d->ell_off, d->ell_col,
+                    d->ell_w, d->tail_rp, d->tail_col, d->tail_w};
     for (void *b : bufs)
         if (b)
             sp_cuda_free(b);
     if (d->stream)
         cudaStreamDestroy(d->stream);
-    free(d->h_row_ptr);
+    free(d->h_col_off);
+    free(d->h_ell_off);
+    free(d->h_tail_off);
     free(d);
 }
 
@@ -849,7 +1136,6 @@ extern "C" int sp_dev_launch_chunk(sp_dev *d, const double *u, size_t T, double 
         box_geometry(d, l, &p.BW, &p.NBX);
         p.bal = (d->bal_G > 0 && l.ctas == d->bal_G) ? 1 : 0;
         p.RB = p.R < d->nc.L ? p.R : d->nc.L;
-        p.coef_smem = coef_smem_bytes(d) > 0;
         int rc = encode_ring_map(d, p.BW, p.RB);
         if (rc)
             return rc;
@@ -889,20 +1175,62 @@ extern "C" int sp_dev_launch_chunk(sp_dev *d, const double *u, size_t T, double 
     d->hold_cta = -1;
     d->hold_b = -1;
     p.nid_of = d->nid_of;
-    p.csr_cap = (int)csr_smem_edges(d, l);
+    const RowPlan rows = row_plan(d, l);
+    p.ell_cap = rows.ell_cap;
+    p.tail_cap = rows.tail_cap;
+    p.ell_off = d->ell_off;
+    p.ell_col = d->ell_col;
+    p.ell_w = d->ell_w;
+    p.tail_rp = d->tail_rp;
+    p.tail_col = d->tail_col;
+    p.tail_w = d->tail_w;
+    p.col_mode = rows.col_mode;
+    p.col_cap = rows.col_cap;
+    p.col_off = d->col_off;
+    p.col_blk = d->col_blk;
+    p.col_w = d->col_w;
+    // the launch publishes the words of barriers 1 .. steps - 1 with the
+    // numbers ll_base + 1 ..: every number is used once
+    const bool words = d->stype == SP_SYN_SIMPLE || d->stype == SP_SYN_PSC_HET;
+    p.ll = d->ll;
+    p.ll_base = d->ll_seq;
 
-    kfn_t fn = pick_kernel(d->ntype, d->stype, l.variant);
+    const int kv = kernel_variant(d, l);
+    kfn_t fn = pick_kernel(d->ntype, d->stype, kv);
     if (!fn)
         return SP_EINVAL;
-    const size_t smem = launch_smem(d, l);
-    // variant 1: consumer warps, the producer warp and the gather warp
-    dim3 grid(l.ctas), block(32 * (l.warps_max + (l.variant == 1 ? 2 : 0)));
+    const SmemPlan sm = smem_plan(d, l, kv);
+    const size_t smem = sm.bytes;
+    p.win_smem = sm.win_smem;
+    p.u_ring = sm.u_ring && u && d->gamma != 0.0;
+    p.coef_smem = stages_coef(d, kv);
+    // consumer warps, then the producer and gather warps
+    dim3 grid(l.ctas), block(32 * (l.warps_max + extra_warps(kv)));
     if (smem > 48 * 1024)
         SP_CK(set_max_dynamic_smem((const void *)fn));
-    if (l.ctas > 1) {
-        SP_CK(cudaMemsetAsync(d->flags, 0,
-                              (size_t)l.ctas * kFlagStride * sizeof(unsigned long long),
-                              d->stream));
+    if (kv == 3) {
+        SP_CK(cudaFuncSetAttribute((const void *)fn,
+                                   cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        memset(&cfg, 0, sizeof(cfg));
+        memset(&at, 0, sizeof(at));
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)l.ctas;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = d->stream;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        void *args[] = {&p};
+        SP_CK(cudaLaunchKernelExC(&cfg, (const void *)fn, args));
+    } else if (l.ctas > 1) {
+        if (!words)
+            SP_CK(cudaMemsetAsync(d->flags, 0,
+                                  (size_t)l.ctas * kFlagStride * sizeof(unsigned long long),
+                                  d->stream));
         void *args[] = {&p};
         SP_CK(cudaLaunchCooperativeKernel((const void *)fn, grid, block, args, smem, d->stream));
     } else {
@@ -911,6 +1239,7 @@ extern "C" int sp_dev_launch_chunk(sp_dev *d, const double *u, size_t T, double 
     }
     d->launches++;
     const long long micro_total = (long long)T * d->micro;
+    d->ll_seq += (unsigned)(micro_total - 1);
     d->step += micro_total;
     d->syn_step += micro_total;
     d->phase ^= (int)(micro_total & 1);
@@ -1148,17 +1477,18 @@ extern "C" int sp_dev_set_launch(sp_dev *d, const sp_launch *l)
     } else if (l->variant != 0) {
         return SP_EINVAL;
     }
-    const size_t smem = launch_smem(d, *l);
-    if (smem > (size_t)max_smem(d))
+    const int kv = kernel_variant(d, *l);
+    const size_t smem = smem_plan(d, *l, kv).bytes;
+    if (smem > (size_t)d->smem_max)
         return SP_EINVAL;
-    kfn_t fn = pick_kernel(d->ntype, d->stype, l->variant);
+    kfn_t fn = pick_kernel(d->ntype, d->stype, kv);
     if (!fn)
         return SP_EINVAL;
-    if (l->ctas > 1) {
+    if (l->ctas > 1 && kv != 3) {
         if (smem > 48 * 1024)
             SP_CK(set_max_dynamic_smem((const void *)fn));
         int per_sm = 0;
-        const int threads = 32 * (l->warps_max + (l->variant == 1 ? 2 : 0));
+        const int threads = 32 * (l->warps_max + extra_warps(kv));
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, threads,
                                                           smem) != cudaSuccess)
             return SP_EINTERNAL;
@@ -1261,10 +1591,8 @@ extern "C" int sp_dev_autotune(sp_dev *d, size_t steps)
                 int bw, nbx;
                 box_geometry(d, v, &bw, &nbx);
                 const size_t stage = (size_t)rows * nbx * bw * 8;
-                const size_t base = 2 * (((d->nwords * 4) + 127) & ~(size_t)127) +
-                                    coef_smem_bytes(d) +
-                                    csr_smem_bytes(csr_smem_edges(d, v), v.warps_max);
-                const size_t budget = (size_t)(max_smem(d) - 8 * 1024);
+                const size_t base = spk_smem_bytes(d) + coef_smem_bytes(d) + row_plan(d, v).bytes;
+                const size_t budget = (size_t)(d->smem_max - 8 * 1024);
                 long long st = budget > base ? (long long)((budget - base) / (stage + 16)) : 0;
                 if (st > 16)
                     st = 16;

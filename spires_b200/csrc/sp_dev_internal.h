@@ -19,6 +19,8 @@
 struct sp_dev {
     int device, num_sms, coop;
     int l2_bytes;  // device L2 cache size
+    int smem_max;  // opt-in shared memory per CTA
+    int cluster_max;  // largest cluster the device schedules (16, 8 or 0)
     int l2_hinted; // a launch read the ring with evict-last hints (demoted at destroy)
     cudaStream_t stream;
     int n, din, dout, micro;
@@ -51,7 +53,6 @@ struct sp_dev {
     double *scoef, *Iring;
     double *mx_decay, *mx_omd, *mx_c, *mx_tr;
     double *W_in, *W_out;  // rows / columns in position order
-    long long *h_row_ptr;  // host copy of row_ptr [rs + 1] (launch planning)
     int *pos_of;           // [n] position of neuron i
     int *nid_of;           // [rs] neuron at position q, or -1
 
@@ -68,6 +69,19 @@ struct sp_dev {
     unsigned long long *bar;  // grid-barrier arrival counter
     unsigned long long *flags; // per-CTA arrival flags of the step kernel (flag_cap CTAs)
     int flag_cap;
+    unsigned long long *ll;    // spike exchange entries of the step kernel [2][nw]
+    unsigned ll_seq;           // numbers used by the launches so far
+    // SIMPLE synapse, column blocks of a dense matrix (null: not built):
+    // [nw][n] {row bits, weight offset}, first weight of each row word, weights
+    uint2 *col_blk;
+    int *h_col_off, *col_off;
+    double *col_w;
+    // SIMPLE synapse, other matrices: row slots in groups of four per warp --
+    // columns [groups][32][4], weights [groups][4][32] -- and the tails of longer
+    // rows, [nw][33] offsets into tail_col / tail_w (null: not built)
+    int *h_ell_off, *ell_off, *h_tail_off, *tail_rp, *tail_col;
+    uint2 *ell_col;
+    double *ell_w, *tail_w;
     int *err;                 // [0] code, [1]/[2] micro-step low/high word
 
     // bounded waits: limit (ns) of every wait in the step kernel; one-shot

@@ -1,7 +1,7 @@
 // sp_step_kernel.cuh -- the persistent reservoir step kernel (all neuron and
 // synapse models), included by dev_reservoir.cu.
 //
-// Launch: a cooperative grid of G CTAs; CTA b owns the whole warps
+// Launch: a cooperative grid of G CTAs (variant 3: one cluster); CTA b owns the whole warps
 // [b*nw/G, (b+1)*nw/G) of neurons (nw = ceil(n/32)); a consumer thread owns
 // one neuron and keeps its state in registers for the whole launch.
 //
@@ -17,24 +17,50 @@
 //   register, so the producer streams lags 34.. only (3 % fewer ring bytes per
 //   step at L = 1024) and the sum of a step starts as soon as its lag 1 exists.
 //   The grid is sized so that each CTA streams about the same number of ring
-//   columns (balanced layout, dev_reservoir.cu), and the CTA's CSR slice sits
-//   in shared memory for the launch, so the row pass after each grid barrier
-//   reads no global memory but the spike words. A gather warp watches the
-//   other CTAs' arrival flags and copies their spike words into a
-//   double-buffered shared array while the consumers are still summing.
+//   columns (balanced layout, dev_reservoir.cu). A gather warp watches the spike exchange and copies
+//   the words into a double-buffered shared array while the consumers are
+//   still summing.
 //   A ring larger than the L2 is read with cache hints: the oldest l2_pin
 //   lags of a step are loaded with evict-last priority and stay L2-resident
 //   from step to step (each row joins them once, when it reaches lag
 //   L - l2_pin), the younger lags stream through with evict-first, so the
 //   DRAM reads come first in every step and run on through the serial phase.
 //
-// Per micro-step (both variants), with a split-phase grid barrier:
+// Variant 2 (FLIF_GL whose CTAs' ring columns fit in shared memory, and
+//   FLIF_CAPUTO): the history is loaded into shared memory once per launch and
+//   summed there (chain_pairs); the ring in global memory is still written
+//   every step, as the state between launches. A gather warp as in variant 1.
+//   (N=2000, L=256: 3.4 us per step; 5.9 through the pipeline's stages.)
+// Variant 3 (2, 4, 8 or 16 CTAs as one cluster, at most 8192 neurons; SIMPLE and
+//   PSC_HETEROGENEOUS): the exchange below between the CTAs' shared memories.
+//   (LIF_DISCRETE N=2000: 1.1 us per step; 1.5 through the L2.)
+//
+// The recurrent rows of a CTA sit in shared memory for the launch where they
+// fit, so the row pass after each exchange reads no global memory: rows as
+// slots and tails (rowpass_lanes) or, for a dense matrix, column blocks
+// (rowpass_cols).
+//
+// Spike exchange (SIMPLE and PSC_HETEROGENEOUS, whose recurrent input needs
+// nothing of another CTA but its spike bits): a warp publishes its word as one
+// 8-byte store of (sequence number, word), and a reader polls that entry until
+// the number is the step's -- the word comes with its flag, so a step costs one
+// store and one successful poll instead of a fence, a flag store, a flag poll,
+// a fence and a second load, and no CTA-wide barrier before the store. Entries
+// alternate between two buffers: a warp publishes step b + 1 only after it has
+// read every word of step b, so nobody can still be reading the buffer of
+// step b - 1 that it overwrites. (LIF_DISCRETE N=20000: 6.7 us per step with
+// flags and fences, 4.1 with the exchange and the row slots.) A gather warp
+// starts to poll when its own CTA has published: polled all along, the entries'
+// lines slowed the stores and the history stream (FLIF_GL N=20000, L=128: 5.9
+// us per step, 3.6). The other synapses publish a double per neuron as well
+// and keep the flags and fences.
+//
+// Per micro-step, with a split-phase grid barrier:
 //   history sum of step g      (overlaps the barrier wait)
 //   wait barrier g             (spike words / eff of step g-1 visible)
-//   recurrent input            SIMPLE: warp-cooperative walk over the warp's
-//                              CSR edges, ballot of spiking presynaptic bits,
-//                              owner lane adds the weights in ascending edge
-//                              order; others: warp-cooperative walk, one
+//   recurrent input            SIMPLE: the weights of the spiking presynaptic
+//                              neurons, added by the row's lane in ascending
+//                              edge order; others: warp-cooperative walk, one
 //                              term per edge, owner lane adds in edge order
 //   neuron update, ring write, ballot -> spike word of step g
 //   synapse prepare for g+1 (own spike), publish, arrive barrier g+1
@@ -55,8 +81,25 @@ struct KP {
                     // n / G (+1 for b < n % G) of its range, the rest holes
     int RB;         // variant 1: rows per box = min(R, L)
     int coef_smem;  // variant 1: coefficient table staged in shared memory
-    int csr_cap;    // SIMPLE synapse: edges of the CTA's CSR slice kept in shared
-                    // memory for the launch (0: rows are walked in global memory)
+    // SIMPLE synapse, rows in shared memory for the launch (rowpass_lanes): most
+    // slot groups and tail edges of a CTA; ell_cap 0 = the CSR rows are walked in
+    // global memory
+    int ell_cap, tail_cap;
+    const int *ell_off;      // [nwords + 1] first slot group of each warp
+    const uint2 *ell_col;    // [groups][32] four 16-bit column positions
+    const double *ell_w;     // [groups][4][32]
+    const int *tail_rp;      // [nwords][33] tails of a warp's rows, in tail_col / tail_w
+    const int *tail_col;
+    const double *tail_w;
+    // SIMPLE synapse, column blocks of a dense matrix (see rowpass_cols): 0 = not
+    // used by this launch, 1 = read from global memory, 2 = staged in shared
+    // memory (col_cap: most weights of a CTA)
+    int col_mode, col_cap;
+    const int *col_off;      // [nwords + 1] first weight of each row word
+    const uint2 *col_blk;    // [nwords][n] {row bits, weight offset from col_off}
+    const double *col_w;
+    int u_ring;     // input rows prefetched through shared memory, kURows deep per warp
+    int win_smem;   // input weights staged in shared memory, [din][consumer thread]
     const int *nid_of;  // neuron at each position, -1 for an empty lane
     long long step0, syn_step0;
     double a, b, c, d, e, f, g, h, ci, cj, ck, cl, dt;
@@ -91,6 +134,10 @@ struct KP {
     // arrival flags, one per CTA on its own 128-byte line: CTA c stores b + 1
     // once its spike words and drive of micro-step b - 1 are published
     unsigned long long *flags;
+    // spike exchange: [2][nwords] entries (sequence number << 32 | spike word);
+    // the words of barrier b carry the number ll_base + b
+    unsigned long long *ll;
+    unsigned ll_base;
     int *err;                 // [0] error code, [1] / [2] low / high word of the micro-step
     unsigned long long tmo;   // limit of every wait, ns
     // one-shot test hook: CTA hold_cta does not arrive at the barrier that
@@ -192,6 +239,12 @@ __device__ __forceinline__ void st_release_cta(volatile int *ptr, int v)
                  "r"(v)
                  : "memory");
 }
+__device__ __forceinline__ void red_release_cta(volatile int *ptr, int v)
+{
+    asm volatile("red.release.cta.shared::cta.add.s32 [%0], %1;" ::"r"(smem_u32((const void *)ptr)),
+                 "r"(v)
+                 : "memory");
+}
 __device__ __forceinline__ int ld_acquire_cta(volatile int *ptr)
 {
     int v;
@@ -237,6 +290,32 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity
     return true;
 }
 
+// One chunk of 32 consecutive edges, lane l holding the weight of edge l and m
+// the ballot of the spiking ones: every lane adds those of its own row, edges
+// [from, to) of the chunk, in ascending order. A pass serves one edge of every
+// row at once, so a chunk takes as many passes as its busiest row has spiking
+// edges. (One edge a pass, found by its owner with a second ballot, took about
+// 80 cycles per spiking edge.)
+template <typename I>
+__device__ __forceinline__ double add_chunk(double acc, double wv, unsigned m, I from, I to)
+{
+    if (m == 0)
+        return acc;
+    const int a = from <= 0 ? 0 : (from < 32 ? (int)from : 32);
+    const int b = to <= 0 ? 0 : (to < 32 ? (int)to : 32);
+    unsigned mine = 0;
+    if (b > a)
+        mine = m & (0xffffffffu >> (32 - b)) & (0xffffffffu << a);
+    while (__any_sync(kFull, mine != 0)) {
+        const int j = __ffs(mine) - 1;
+        const double w = __shfl_sync(kFull, wv, j & 31);
+        if (mine)
+            acc = add(acc, w);
+        mine &= mine - 1;
+    }
+    return acc;
+}
+
 // SIMPLE synapse, one warp: recurrent input of rows [row0, row0 + nv) for the
 // lane that owns row row0 + lane. Edges are scanned 32 at a time; spiking
 // presynaptic columns are found by a ballot over the spike bits and each
@@ -250,6 +329,7 @@ __device__ __forceinline__ double rowpass_simple_warp(const long long *__restric
 {
     const long long e0 = __ldg(row_ptr + row0);
     const long long e1 = __ldg(row_ptr + row0 + nv);
+    const long long my_start = (lane < nv) ? __ldg(row_ptr + row0 + lane) : e1;
     const long long my_end = (lane < nv) ? __ldg(row_ptr + row0 + lane + 1) : e1;
     double acc = 0.0;
     // next chunk's column index and weight are loaded one chunk ahead
@@ -269,16 +349,7 @@ __device__ __forceinline__ double rowpass_simple_warp(const long long *__restric
             wn = __ldg(w + nx);
         }
         const bool s = c >= 0 && ((s_spk[c >> 5] >> (c & 31)) & 1u);
-        unsigned m = __ballot_sync(kFull, s);
-        while (m) {
-            const int bpos = __ffs(m) - 1;
-            m &= m - 1;
-            const long long eb = base + bpos;
-            const double wb = __shfl_sync(kFull, wv, bpos);
-            const unsigned owner = __ballot_sync(kFull, my_end > eb);
-            if (lane == __ffs(owner) - 1)
-                acc = add(acc, wb);
-        }
+        acc = add_chunk(acc, wv, __ballot_sync(kFull, s), my_start - base, my_end - base);
     }
     return acc;
 }
@@ -359,37 +430,359 @@ __device__ __forceinline__ double rowpass_terms_warp(const KP &p, const double *
     return acc;
 }
 
-// The same walk over the CTA's CSR slice in shared memory: rp = row offsets
-// relative to the slice (rows of the CTA in position order), col = column
-// positions, w = weights. Same terms, same order.
-__device__ __forceinline__ double rowpass_simple_smem(const int *rp, const int *col,
-                                                      const double *w, const unsigned *s_spk,
-                                                      int row0, int lane)
+// SIMPLE synapse, rows in shared memory, one warp, lane r the row of position r.
+// The first slots of every row are stored side by side, four to a group, and
+// lane r walks its own in ascending order; a row shorter than the warp's slots
+// is padded with zero weights, and a slot whose neuron did not spike adds +0.0
+// (which leaves the sum's bits: it starts at +0 and never becomes -0). What a
+// row has beyond the slots -- the hubs of a Barabasi-Albert graph -- follows as
+// a tail that the whole warp tests 32 edges at a time, the row's lane adding
+// the spiking ones in order. A warp issues in order and every addition waits
+// for the one before it, so the tests of one block of eight slots are written
+// between the additions of the other. (About 360 cycles for up to 8 slots and
+// 27 for each more; the edge-parallel walk below takes 300 per 32 edges and 100
+// for each pass that adds one edge of every row.)
+__device__ __forceinline__ double rowpass_lanes(const uint2 *col, const double *w, int groups,
+                                                const int *tail_rp, const int *tail_col,
+                                                const double *tail_w, unsigned tails,
+                                                const unsigned *s_spk, int lane)
 {
-    const int e0 = rp[row0], e1 = rp[row0 + 32];
-    const int my_end = rp[row0 + lane + 1];
     double acc = 0.0;
-    for (int base = e0; base < e1; base += 32) {
-        const int e = base + lane;
-        int c = -1;
-        double wv = 0.0;
-        if (e < e1) {
-            c = col[e];
-            wv = w[e];
+    const uint2 *cp = col + lane;
+    const double *wp = w + lane;
+    const int last = groups - 1;
+    uint2 c[2];
+    auto cols = [&](int q) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            c[e] = cp[(q + e < last ? q + e : last) * 32];
+    };
+    auto block = [&](int q, double (&v)[8]) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const double *wq = wp + (q + e < last ? q + e : last) * 128;
+            const unsigned k[4] = {c[e].x & 0xffffu, c[e].x >> 16, c[e].y & 0xffffu,
+                                   c[e].y >> 16};
+            const unsigned live = q + e <= last ? 1u : 0u;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const double x = wq[32 * u];
+                v[4 * e + u] = ((s_spk[k[u] >> 5] >> (k[u] & 31)) & live) ? x : 0.0;
+            }
         }
-        const bool s = c >= 0 && ((s_spk[c >> 5] >> (c & 31)) & 1u);
-        unsigned m = __ballot_sync(kFull, s);
-        while (m) {
-            const int bpos = __ffs(m) - 1;
-            m &= m - 1;
-            const int eb = base + bpos;
-            const double wb = __shfl_sync(kFull, wv, bpos);
-            const unsigned owner = __ballot_sync(kFull, my_end > eb);
-            if (lane == __ffs(owner) - 1)
-                acc = add(acc, wb);
+    };
+    auto sum = [&](const double (&v)[8]) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            acc = add(acc, v[u]);
+    };
+    if (groups > 0) {
+        double va[8], vb[8];
+        cols(0);
+        block(0, va);
+        cols(2);
+        for (int q = 0; q < groups; q += 4) {
+            if (q + 2 >= groups) {
+                sum(va);
+                break;
+            }
+            block(q + 2, vb);
+            cols(q + 4);
+            sum(va);
+            block(q + 4, va);
+            cols(q + 6);
+            sum(vb);
+        }
+    }
+    for (; tails; tails &= tails - 1) {
+        const int row = __ffs(tails) - 1;
+        const int e1 = tail_rp[row + 1];
+        int base = tail_rp[row];
+        auto test = [&](int at) {  // ballot of the spiking edges at .. at + 31
+            const int e = at + lane < e1 ? at + lane : e1 - 1;
+            const unsigned k = (unsigned)tail_col[e];
+            const unsigned hit = (s_spk[k >> 5] >> (k & 31)) & (at + lane < e1 ? 1u : 0u);
+            return __ballot_sync(kFull, hit != 0);
+        };
+        unsigned m = test(base);
+        for (; base < e1; base += 32) {
+            const unsigned nm = base + 32 < e1 ? test(base + 32) : 0u;
+            // every lane reads the spiking edges' weights, the row's lane keeps the sum
+            while (m) {
+                double x[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    x[u] = m ? tail_w[base + __ffs(m) - 1] : 0.0;
+                    m &= m - 1;
+                }
+                if (lane == row) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        acc = add(acc, x[u]);
+                }
+            }
+            m = nm;
         }
     }
     return acc;
+}
+
+// SIMPLE synapse, column blocks, one warp: for row word q (rows 32q .. 32q + 31)
+// and neuron j, the bits of the rows with an edge from j and where the block's
+// weights, stored in row order, start. The lane of a row walks the list of
+// spiking neurons in ascending order and adds w_ij where its bit is set: the
+// non-zero terms of csr_row_dot (src/sparse.c:68-76) in order, at a cost that
+// follows the spikes of the step and not the edges of the row. Four columns are
+// in flight, the next four's blocks a pass ahead.
+template <bool kShared>
+__device__ __forceinline__ double rowpass_cols(const uint2 *blk, const double *w,
+                                               const unsigned short *s_list, int cnt, int lane)
+{
+    const unsigned below = (1u << lane) - 1u;
+    auto fetch = [&](int t, uint2 (&c)[4]) {
+        const uint2 id = *(const uint2 *)(s_list + t);  // the list is padded to fours
+        const unsigned j[4] = {id.x & 0xffffu, id.x >> 16, id.y & 0xffffu, id.y >> 16};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            c[u] = t + u >= cnt ? make_uint2(0u, 0u) : (kShared ? blk[j[u]] : __ldg(blk + j[u]));
+    };
+    double acc = 0.0;
+    uint2 cur[4], nxt[4];
+    fetch(0, cur);
+    for (int t = 0; t < cnt; t += 4) {
+        double x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const double *a = w + cur[u].y + __popc(cur[u].x & below);
+            x[u] = 0.0;
+            if ((cur[u].x >> lane) & 1u)
+                x[u] = kShared ? *a : __ldg(a);
+        }
+        if (t + 4 < cnt)
+            fetch(t + 4, nxt);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            acc = add(acc, x[u]);  // +0.0 where the row has no such edge
+            cur[u] = nxt[u];
+        }
+    }
+    return acc;
+}
+
+// History in shared memory: ring rows in pairs, [pair][32 lanes][2], so that one
+// 16-byte load brings two lags, and two copies of the coefficients, the second
+// shifted by one, so that a pair of them is a 16-byte load at either parity.
+// hist + the n lags k, k + 1, ... in ascending order, lag k in row r, rows
+// descending (no wrap). (A shared-memory load costs its destination registers'
+// write-back, 4.8 cycles a warp for 8 bytes a lane even when all lanes read one
+// word: 16.8 cycles per lag with 8-byte loads, 10.5 with pairs, against 8.5 for
+// the dependent addition alone.)
+__device__ __forceinline__ double chain_pairs(double hist, const double *ca, const double *cb,
+                                              const double2 *ring, int k, int r, int n)
+{
+    if (n > 0 && !(r & 1)) {
+        hist = add(hist, mul(ca[k], ring[(r >> 1) * 32].x));
+        ++k;
+        --r;
+        --n;
+    }
+    const double2 *c = (const double2 *)((k & 1) ? cb + (k - 1) : ca + k);
+    const double2 *v = ring + (r >> 1) * 32;
+    for (; n >= 16; n -= 16, c += 8, v -= 256) {
+        double x[16];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const double2 cc = c[u], vv = v[-32 * u];
+            x[2 * u] = mul(cc.x, vv.y);
+            x[2 * u + 1] = mul(cc.y, vv.x);
+        }
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            hist = add(hist, x[u]);
+    }
+    for (; n >= 2; n -= 2, ++c, v -= 32) {
+        const double2 cc = *c, vv = *v;
+        hist = add(hist, mul(cc.x, vv.y));
+        hist = add(hist, mul(cc.y, vv.x));
+    }
+    if (n > 0)
+        hist = add(hist, mul(c->x, v->y));
+    return hist;
+}
+
+// hist + sum of cnt products coef[j] * v[-j * stride] in ascending j, U loads
+// at a time, the next U products formed while the chain of dependent additions
+// runs over the current ones. ld(p) reads one value.
+template <int U, typename Ld>
+__device__ __forceinline__ double chain_sum(double hist, const double *coef, const double *v,
+                                            size_t stride, int cnt, Ld ld)
+{
+    double cur[U];
+    int j = 0;
+    if (cnt >= U) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            cur[u] = mul(coef[u], ld(v - (size_t)u * stride));
+        for (; j + 2 * U <= cnt; j += U) {
+            double nxt[U];
+            const double *cn = coef + j + U;
+            const double *vn = v - (size_t)(j + U) * stride;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                nxt[u] = mul(cn[u], ld(vn - (size_t)u * stride));
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                hist = add(hist, cur[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                cur[u] = nxt[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            hist = add(hist, cur[u]);
+        j += U;
+    }
+    for (; j < cnt; ++j)
+        hist = add(hist, mul(coef[j], ld(v - (size_t)j * stride)));
+    return hist;
+}
+
+// History over a time-major ring column: lags k0..lim in ascending order, lag
+// k0 in row r0, rows descending and wrapping at row 0 to row L - 1.
+template <int U, typename Ld>
+__device__ __forceinline__ double ring_sum(double hist, const double *coef, const double *column,
+                                           size_t stride, int L, int r0, int k0, int lim, Ld ld)
+{
+    const int cnt = lim - k0 + 1;
+    if (cnt <= 0)
+        return hist;
+    const int n1 = cnt < r0 + 1 ? cnt : r0 + 1;
+    hist = chain_sum<U>(hist, coef + k0, column + (size_t)r0 * stride, stride, n1, ld);
+    if (cnt > n1)
+        hist = chain_sum<U>(hist, coef + k0 + n1, column + (size_t)(L - 1) * stride, stride,
+                            cnt - n1, ld);
+    return hist;
+}
+
+__device__ __forceinline__ void cp_async8(void *smem, const void *gmem)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Four consecutive doubles from a 32-byte boundary in one load.
+__device__ __forceinline__ void ld_f64x4(const double *p, double (&v)[4])
+{
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                 : "l"(p));
+}
+
+// FLIF_CAPUTO memory sum of one neuron: tab[0] * newest + sum over lags
+// k = 1 .. D-1, ascending, of tab[k] * row[(pos - k) mod D]; tab is readable
+// three places beyond either end. Every neuron's shift register is contiguous
+// with a head of its own, so the 32 lanes of a load touch 32 lines and the load
+// unit's line a cycle bounds the sum (N=20000, D=510, 5 warps an SM: 150 cycles
+// per lag with an 8-byte load each). Lanes therefore walk aligned 32-byte
+// blocks downwards, four lags a load, Q blocks in flight while Q are summed.
+// A block's elements e carry lag c0 - e; those outside the lane's run -- the
+// entries before the head, then from the row's top to behind it -- add +0.0,
+// which leaves the sum's bits (it starts from +0 and never becomes -0).
+template <int Q>
+__device__ __forceinline__ double caputo_sum(double newest, const double *tab, const double *ring,
+                                             long long row, int D, int pos)
+{
+    double mem = add(0.0, mul(tab[0], newest));
+    // element numbers below count from the 32-byte boundary at or under the row
+    const int r0 = (int)(row & 3);
+    const double *base = ring + (row - r0);
+    const int top = r0 + D - 1, stop = r0 + pos + 1;  // the second run: top down to stop
+    int blocks = pos > 0 ? ((r0 + pos - 1) >> 2) + 1 : 0;
+    if (stop <= top)
+        blocks += (top >> 2) - (stop >> 2) + 1;
+    // the block to load next and the block to sum next, with their runs' ends
+    int lat = pos > 0 ? (r0 + pos - 1) & ~3 : top & ~3, llo = pos > 0 ? r0 : stop;
+    int at = lat, lo = llo, hi = pos > 0 ? r0 + pos - 1 : top;
+    int c0 = r0 + pos + (pos > 0 ? 0 : D);
+    auto load = [&](double (&v)[4]) {
+        ld_f64x4(base + (lat > 0 ? lat : 0), v);
+        lat -= 4;
+        if (lat + 3 < llo && llo == r0) {  // the first run is loaded: on from the top
+            lat = top & ~3;
+            llo = stop;
+        }
+    };
+    auto sum = [&](const double (&v)[4]) {
+        const int k3 = c0 - at - 3;  // lag of the block's last element, the first to add
+        const double *t = tab + (k3 < -3 ? -3 : (k3 > D - 1 ? D - 1 : k3));
+        double x[4];
+#pragma unroll
+        for (int u = 3; u >= 0; --u) {
+            const double y = mul(t[3 - u], v[u]);
+            x[u] = (at + u >= lo && at + u <= hi) ? y : 0.0;
+        }
+#pragma unroll
+        for (int u = 3; u >= 0; --u)
+            mem = add(mem, x[u]);
+        at -= 4;
+        if (at + 3 < lo && lo == r0) {
+            at = top & ~3;
+            lo = stop;
+            hi = top;
+            c0 += D;
+        }
+    };
+    double cur[Q][4], nxt[Q][4];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+        load(cur[q]);
+    for (int n = 0; n < blocks; n += 2 * Q) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            load(nxt[q]);
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            sum(cur[q]);
+        if (n + Q >= blocks)
+            break;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            load(cur[q]);
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+            sum(nxt[q]);
+    }
+    return mem;
+}
+
+// Spike exchange between the CTAs of one cluster: the entry is written straight
+// into every CTA's shared memory and polled there (VAR 3).
+__device__ __forceinline__ void st_cluster_u64(const void *local, unsigned rank,
+                                               unsigned long long v)
+{
+    unsigned remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(remote)
+                 : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(v)
+                 : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_cluster_u64(const unsigned long long *local)
+{
+    unsigned long long v;
+    asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];"
+                 : "=l"(v)
+                 : "r"(smem_u32(local))
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;"
+                 ::: "memory");
 }
 
 template <int R>
@@ -412,16 +805,23 @@ __device__ __forceinline__ double stage_sum(double hist, const double *coef_k, c
 // which leaves registers for a stage of lags in flight and the register lags
 // per thread.
 constexpr int kPipeWarps = 8;
+// Variant 3: at most 16 CTAs of 16 warps, 8192 neurons.
+constexpr int kClusterWarps = 16, kClusterWords = 256;
 
 template <int VAR>
 struct Bounds {
-    static constexpr int threads = VAR == 1 ? 32 * (kPipeWarps + 2) : 1024;
+    // variant 2: consumers and the gather warp; variant 3: consumers
+    static constexpr int threads = VAR == 1   ? 32 * (kPipeWarps + 2)
+                                   : VAR == 2 ? 32 * (kPipeWarps + 1)
+                                   : VAR == 3 ? 32 * kClusterWarps
+                                              : 1024;
 };
 
 // Variant 1 keeps lags 2..kRegLags+1 of its own neuron in registers: they are
 // the thread's own last states, so they are neither written to nor read back
 // from the ring for the sum, and the producer streams lags kRegLags+2.. only.
 constexpr int kRegLags = 32;
+constexpr int kURows = 8;  // input rows in flight per warp
 constexpr int kFlagStride = 16;  // u64 per CTA arrival flag (one 128-byte line)
 
 template <int NT, int ST, int VAR>
@@ -433,6 +833,10 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     __shared__ volatile int s_abort;
     __shared__ volatile int s_done;
     __shared__ volatile int s_gather;  // variant 1: barriers whose words are staged
+    __shared__ int s_wsum[32];         // column blocks: spikes per warp of the list scan
+    __shared__ volatile int s_bad[2];  // variant 0: a wait of barrier b (b & 1) ran out
+    // the spike exchange carries everything another CTA needs
+    constexpr bool kWords = ST == SP_SYN_SIMPLE || ST == SP_SYN_PSC_HET;
 
     const int tid = threadIdx.x;
     const int lane = tid & 31;
@@ -443,25 +847,53 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     const int L = p.L;
     const long long B = (long long)p.n_macro * p.micro;
 
-    // spike words of the barrier: one buffer, or two (variant 1: the gather
-    // warp fills barrier b + 1's while the row pass reads barrier b's)
+    // spike words of the barrier, two buffers: barrier b + 1's are filled while
+    // a row pass may still read barrier b's
     const size_t spk_one = (((size_t)p.nwords * 4) + 127) & ~(size_t)127;
     unsigned *s_spkb = (unsigned *)smem;
-    const size_t spk_bytes0 = (VAR == 1 ? 2 : 1) * spk_one;
-    // CSR slice (SIMPLE synapse), between the spike words and the rest
-    double *s_csr_w = (double *)(smem + spk_bytes0);
-    const size_t csr_w_bytes = ((size_t)p.csr_cap * 8 + 127) / 128 * 128;
-    int *s_csr_col = (int *)(smem + spk_bytes0 + csr_w_bytes);
-    const size_t csr_c_bytes = ((size_t)p.csr_cap * 4 + 127) / 128 * 128;
-    int *s_csr_rp = (int *)(smem + spk_bytes0 + csr_w_bytes + csr_c_bytes);
+    const size_t spk_bytes0 = 2 * spk_one;
+    // rows of the CTA (SIMPLE synapse): slot weights and columns, then the tails
+    double *s_ell_w = (double *)(smem + spk_bytes0);
+    uint2 *s_ell_col = (uint2 *)(s_ell_w + (size_t)128 * p.ell_cap);
+    double *s_tail_w = (double *)(s_ell_col + (size_t)32 * p.ell_cap);
+    int *s_tail_col = (int *)(s_tail_w + p.tail_cap);
+    int *s_tail_rp = s_tail_col + p.tail_cap;
     const size_t csr_bytes =
-        p.csr_cap > 0 ? csr_w_bytes + csr_c_bytes +
-                            (((size_t)32 * p.warps + 1) * 4 + 127) / 128 * 128
+        p.ell_cap > 0 ? (size_t)1280 * p.ell_cap +
+                            ((size_t)12 * p.tail_cap + (size_t)132 * p.warps + 127) / 128 * 128
                       : 0;
-    const size_t spk_bytes = spk_bytes0 + csr_bytes;
-    const size_t coef_bytes = p.coef_smem ? (((size_t)L * 8) + 127) & ~(size_t)127 : 0;
-    double *s_coef = (double *)(smem + spk_bytes);
+    // column blocks: spiking neurons as a bitmap in neuron order and as a list,
+    // then (staged) the CTA's weights and blocks; the input weights
+    const int nwn = (p.n + 31) / 32;
+    unsigned *s_bits = (unsigned *)(smem + spk_bytes0 + csr_bytes);
+    unsigned short *s_list = (unsigned short *)(s_bits + (nwn + 3) / 4 * 4);
+    const size_t list_bytes =
+        p.col_mode ? ((size_t)(nwn + 3) / 4 * 16 + (size_t)p.n * 2 + 8 + 127) / 128 * 128 : 0;
+    double *s_col_w = (double *)((char *)s_bits + list_bytes);
+    uint2 *s_col_blk = (uint2 *)(s_col_w + p.col_cap);
+    const size_t col_bytes =
+        list_bytes +
+        (p.col_mode == 2 ? ((size_t)p.col_cap * 8 + (size_t)p.warps * p.n * 8 + 127) / 128 * 128 : 0);
+    double *s_win = (double *)((char *)s_bits + col_bytes);
+    const size_t win_bytes = p.win_smem ? (size_t)p.din * NC * 8 : 0;
+    double *s_u = (double *)((char *)s_win + win_bytes);
+    const size_t u_bytes = p.u_ring ? ((size_t)p.warps * kURows * p.din * 8 + 127) / 128 * 128 : 0;
+    // variant 3: the exchange entries [2][nwords]
+    unsigned long long *s_ll = (unsigned long long *)((char *)s_u + u_bytes);
+    const size_t ll_bytes = VAR == 3 ? ((size_t)16 * p.nwords + 127) / 128 * 128 : 0;
+    const size_t spk_bytes =
+        spk_bytes0 + csr_bytes + col_bytes + win_bytes + u_bytes + ll_bytes;
+    // kernels with the history in shared memory: a second copy, shifted by one
+    constexpr bool kPairs = VAR >= 2 && NT == SP_FLIF_GL;
+    const size_t coef_one = (((size_t)L * 8 + 64) + 127) & ~(size_t)127;
+    const size_t coef_bytes = p.coef_smem ? (kPairs ? 2 : 1) * coef_one : 0;
+    // (FLIF_CAPUTO: four places of padding before and after the table)
+    double *s_coef = (double *)(smem + spk_bytes) + (NT == SP_FLIF_CAPUTO ? 4 : 0);
+    double *s_coef1 = (double *)(smem + spk_bytes + coef_one);
     double *s_stage = (double *)(smem + spk_bytes + coef_bytes);
+    // variants 2 and 3: the thread's column of its warp's ring block (chain_pairs)
+    double2 *s_ring = (double2 *)s_stage + (size_t)warp * ((L + 1) / 2) * 32 + lane;
+    auto ring_at = [&](int r) -> double & { return *((double *)(s_ring + (r >> 1) * 32) + (r & 1)); };
     const size_t STAGE = (size_t)p.NBX * p.R * p.BW;  // doubles per stage
     unsigned long long *full = (unsigned long long *)(smem + spk_bytes + coef_bytes +
                                                       (size_t)p.NST * STAGE * sizeof(double));
@@ -473,20 +905,53 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         s_abort = 0;
         s_done = 0;
         s_gather = 0;
+        s_bad[0] = s_bad[1] = 0;
     }
-    if (VAR == 1 && p.coef_smem)
-        for (int k = tid; k < L; k += blockDim.x)
-            s_coef[k] = p.coef[k];
-    if (ST == SP_SYN_SIMPLE && p.csr_cap > 0) {
-        const long long e_lo = __ldg(p.row_ptr + lo);
-        const int ne = (int)(__ldg(p.row_ptr + lo + S_b) - e_lo);  // <= csr_cap
-        for (int k = tid; k < ne; k += blockDim.x) {
-            s_csr_col[k] = __ldg(p.col + e_lo + k);
-            s_csr_w[k] = __ldg(p.w + e_lo + k);
+    if (p.coef_smem && NT == SP_FLIF_CAPUTO && tid < 8)
+        s_coef[tid < 4 ? tid - 4 : L + tid - 4] = 0.0;
+    if (p.coef_smem)
+        for (int k = tid; k < L; k += blockDim.x) {
+            const double c = p.coef[k + (NT == SP_FLIF_CAPUTO ? 4 : 0)];
+            s_coef[k] = c;
+            if (kPairs && k > 0)
+                s_coef1[k - 1] = c;
         }
-        for (int q = tid; q <= S_b; q += blockDim.x)
-            s_csr_rp[q] = (int)(__ldg(p.row_ptr + lo + q) - e_lo);
+    if (ST == SP_SYN_SIMPLE && p.ell_cap > 0) {
+        const int g0 = __ldg(p.ell_off + wb0), ng = __ldg(p.ell_off + wb1) - g0;  // <= ell_cap
+        for (int k = tid; k < 32 * ng; k += blockDim.x)
+            s_ell_col[k] = __ldg(p.ell_col + (size_t)32 * g0 + k);
+        for (int k = tid; k < 128 * ng; k += blockDim.x)
+            s_ell_w[k] = __ldg(p.ell_w + (size_t)128 * g0 + k);
+        if (wb1 > wb0) {
+            const int t0 = __ldg(p.tail_rp + (size_t)33 * wb0);
+            const int nt = __ldg(p.tail_rp + (size_t)33 * wb1 - 1) - t0;  // <= tail_cap
+            for (int k = tid; k < nt; k += blockDim.x) {
+                s_tail_col[k] = __ldg(p.tail_col + t0 + k);
+                s_tail_w[k] = __ldg(p.tail_w + t0 + k);
+            }
+            for (int k = tid; k < 33 * (wb1 - wb0); k += blockDim.x)
+                s_tail_rp[k] = __ldg(p.tail_rp + (size_t)33 * wb0 + k) - t0;
+        }
     }
+    if (ST == SP_SYN_SIMPLE && p.col_mode) {
+        for (int k = tid; k < nwn; k += blockDim.x)
+            s_bits[k] = 0u;
+        if (p.col_mode == 2) {
+            const int w0 = __ldg(p.col_off + wb0), nwt = __ldg(p.col_off + wb1) - w0;  // <= col_cap
+            for (int k = tid; k < nwt; k += blockDim.x)
+                s_col_w[k] = __ldg(p.col_w + w0 + k);
+            for (int k = tid; k < (wb1 - wb0) * p.n; k += blockDim.x)
+                s_col_blk[k] = __ldg(p.col_blk + (size_t)wb0 * p.n + k);
+        }
+    }
+    if (p.win_smem)
+        for (int k = tid; k < p.din * S_b; k += blockDim.x) {
+            const int q = k / p.din, j = k - q * p.din;
+            s_win[(size_t)j * NC + q] = __ldg(p.W_in + (size_t)(lo + q) * p.din + j);
+        }
+    if (VAR == 3)  // a number that no barrier of this launch carries
+        for (int k = tid; k < 2 * p.nwords; k += blockDim.x)
+            s_ll[k] = (unsigned long long)p.ll_base << 32;
     if (VAR == 1) {
         if (tid == 0) {
             for (int s = 0; s < p.NST; ++s) {
@@ -497,53 +962,114 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         }
     }
     __syncthreads();
+    if (VAR == 3)
+        cluster_sync();  // every CTA's entries are set before anyone writes one
 
-    // ------------------------------------------------------------ producer
+    // Entries first, first + stride, ... of barrier b (b >= 1) into dst, eight
+    // polls in flight; false when the wait ran out or the launch is stopping.
+    auto gather_words = [&](unsigned *dst, long long b, int first, int stride) -> bool {
+        const unsigned long long *src = (VAR == 3 ? s_ll : p.ll) + (size_t)(b & 1) * p.nwords;
+        const unsigned want = p.ll_base + (unsigned)b;
+        unsigned long long t0 = 0;
+        unsigned long long polls = 0;
+        for (int base = first; base < p.nwords; base += 8 * stride) {
+            unsigned pend = 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (base + u * stride < p.nwords)
+                    pend |= 1u << u;
+            while (pend) {
+                unsigned long long v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    v[u] = !((pend >> u) & 1u) ? 0ull
+                           : VAR == 3          ? ld_cluster_u64(src + base + u * stride)
+                                               : ld_volatile_u64(src + base + u * stride);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (((pend >> u) & 1u) && (unsigned)(v[u] >> 32) == want) {
+                        dst[base + u * stride] = (unsigned)v[u];
+                        pend &= ~(1u << u);
+                    }
+                if (VAR < 2 && pend)
+                    __nanosleep(40);  // polls of all CTAs slow the stores they wait for
+                if (pend && (++polls & 63ull) == 0) {
+                    if (s_abort || ld_volatile_i32(p.err) != kErrNone)
+                        return false;
+                    const unsigned long long now = globaltimer_ns();
+                    if (t0 == 0)
+                        t0 = now;
+                    if (now - t0 > p.tmo || polls > kBarrierMaxPolls) {
+                        record_err(p.err, kErrBarrierTimeout, p.step0 + b);
+                        return false;
+                    }
+                }
+            }
+        }
+        return true;
+    };
+
     // ------------------------------------------------------------ gatherer
-    // Variant 1, one warp: for barrier b it watches the arrival flags of all
-    // CTAs (lane l: CTAs l, l + 32, ...), copies each CTA's spike words into
-    // s_spkb[b & 1] as soon as that CTA's flag is up, and announces the
-    // barrier in s_gather -- while the consumers are still summing history.
-    // Buffer b & 1 is free by then: a flag can reach b + 1 only after this
-    // CTA's arrival at barrier b - 1, which follows its row pass of b - 2.
-    if (VAR == 1 && tid >= NC + 32) {
-        constexpr bool kWords = ST == SP_SYN_SIMPLE || ST == SP_SYN_PSC_HET;
+    // Variants 1 and 2, one warp: for barrier b it collects every spike word into
+    // s_spkb[b & 1] as it is published and announces the barrier in s_gather --
+    // while the consumers are still summing history. Buffer b & 1 is free by
+    // then: a word of barrier b is published only after its CTA has seen this
+    // CTA's words of barrier b - 1, which follow the row pass of b - 2. For the
+    // synapses that publish a drive it watches the arrival flags of all CTAs
+    // (lane l: CTAs l, l + 32, ...) instead.
+    constexpr bool kGath = VAR == 1 || VAR == 2;
+    if (kGath && tid >= (VAR == 1 ? NC + 32 : NC)) {
         if (p.G <= 1)
             return;
         for (long long b = 0; b < B; ++b) {
-            const unsigned long long want = (unsigned long long)(b + 1);
-            const int curb = p.phase0 ^ (int)(b & 1);
-            unsigned *dst = s_spkb + (size_t)(b & 1) * (spk_one / 4);
             bool ok = true;
-            for (int c = lane; c < p.G && ok; c += 32) {
-                const unsigned long long *f = p.flags + (size_t)c * kFlagStride;
-                if (ld_volatile_u64(f) < want) {
+            if (kWords) {
+                unsigned *dst = s_spkb + (size_t)(b & 1) * (spk_one / 4);
+                if (b == 0) {  // the previous launch's words
+                    for (int wi = lane; wi < p.nwords; wi += 32)
+                        dst[wi] = __ldcg(p.spk + (size_t)p.phase0 * p.nwords + wi);
+                } else {
+                    // nobody is much ahead of this CTA: no polls of the L2
+                    // while its own warps are still at the step before
+                    const unsigned need = (unsigned)b * (unsigned)(wb1 - wb0);
                     const unsigned long long t0 = globaltimer_ns();
-                    unsigned long long polls = 0;
-                    while (ld_volatile_u64(f) < want) {
-                        if ((++polls & 255ull) == 0) {
-                            if (s_abort || ld_volatile_i32(p.err) != kErrNone) {
-                                ok = false;
-                                break;
-                            }
-                            if (globaltimer_ns() - t0 > p.tmo || polls > kBarrierMaxPolls) {
-                                record_err(p.err, kErrBarrierTimeout, p.step0 + b);
-                                s_abort = 1;
-                                ok = false;
-                                break;
-                            }
-                        }
-                        __nanosleep(32);
+                    unsigned polls = 0;
+                    while ((int)((unsigned)ld_acquire_cta(&s_done) - need) < 0) {
+                        if ((++polls & 63u) == 0 &&
+                            (s_abort || ld_volatile_i32(p.err) != kErrNone ||
+                             globaltimer_ns() - t0 > p.tmo))
+                            break;  // the polls below have their own limit
+                        __nanosleep(20);
                     }
+                    ok = gather_words(dst, b, lane, 32);
+                    if (!ok)
+                        s_abort = 1;
                 }
-                if (!ok)
-                    break;
-                __threadfence();
-                if (kWords) {
-                    const int w0 = (int)(((long long)c * p.nwords) / p.G);
-                    const int w1 = (int)(((long long)(c + 1) * p.nwords) / p.G);
-                    for (int wi = w0; wi < w1; ++wi)
-                        dst[wi] = __ldcg(p.spk + (size_t)curb * p.nwords + wi);
+            } else {
+                const unsigned long long want = (unsigned long long)(b + 1);
+                for (int c = lane; c < p.G && ok; c += 32) {
+                    const unsigned long long *f = p.flags + (size_t)c * kFlagStride;
+                    if (ld_volatile_u64(f) < want) {
+                        const unsigned long long t0 = globaltimer_ns();
+                        unsigned long long polls = 0;
+                        while (ld_volatile_u64(f) < want) {
+                            if ((++polls & 255ull) == 0) {
+                                if (s_abort || ld_volatile_i32(p.err) != kErrNone) {
+                                    ok = false;
+                                    break;
+                                }
+                                if (globaltimer_ns() - t0 > p.tmo || polls > kBarrierMaxPolls) {
+                                    record_err(p.err, kErrBarrierTimeout, p.step0 + b);
+                                    s_abort = 1;
+                                    ok = false;
+                                    break;
+                                }
+                            }
+                            __nanosleep(32);
+                        }
+                    }
+                    if (ok)
+                        __threadfence();
                 }
             }
             if (__any_sync(kFull, !ok))
@@ -555,6 +1081,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         return;
     }
 
+    // ------------------------------------------------------------ producer
     if (VAR == 1 && tid >= NC) {
         if (lane != 0 || S_b == 0)
             return;
@@ -567,7 +1094,8 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         // slots [0, l2_pin) stay L2-resident, the others stream through
         const unsigned long long pol_in = l2_policy(true);
         const unsigned long long pol_out = l2_policy(false);
-        for (long long b = 0; b < B && ok; ++b) {
+        int rh0 = (int)(((p.step0 - 2 - RL) % L + L) % L);  // row of the first streamed lag
+        for (long long b = 0; b < B && ok; ++b, rh0 = rh0 + 1 == L ? 0 : rh0 + 1) {
             const long long g = p.step0 + b;
             const int lim = (int)(g < L ? g : L - 1);
             if (lim < 2 + RL)
@@ -576,7 +1104,9 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                 // rows of step g are states of steps <= g-2
                 unsigned long long t0 = globaltimer_ns();
                 unsigned polls = 0;
-                while (ld_acquire_cta(&s_done) < b - 1) {
+                // (kWords: every consumer warp counts its own steps)
+                const unsigned need = (unsigned)(b - 1) * (unsigned)(kWords ? wb1 - wb0 : 1);
+                while ((int)((unsigned)ld_acquire_cta(&s_done) - need) < 0) {
                     if ((++polls & 63u) == 0) {
                         if (s_abort || ld_volatile_i32(p.err) != kErrNone) {
                             ok = false;
@@ -597,7 +1127,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             // lags k..k+cnt-1 are rows rh down to rh-cnt+1: one contiguous
             // ascending row range per stage (split at the wrap)
             SP_STAMP(true, b, B, 7);
-            int rh = (int)(((g - 2 - RL) % L + L) % L);
+            int rh = rh0;
             for (int k = 2 + RL; k <= lim && ok;) {
                 int cnt = lim - k + 1;
                 if (cnt > p.R)
@@ -685,6 +1215,13 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             hreg[j] = p.ring[(size_t)pr * p.rs + i];
         }
     }
+    const double coef1 = NT == SP_FLIF_GL && L > 1 ? __ldg(p.coef + 1) : 0.0;
+    if (VAR >= 2 && NT == SP_FLIF_GL && wact) {
+        // every thread fills and reads its own column only
+#pragma unroll 16
+        for (int r = 0; r < L; ++r)
+            ring_at(r) = __ldcg(p.ring + (size_t)r * p.rs + i);
+    }
     if (act) {
         if (NT == SP_FLIF_CAPUTO)
             cpos = p.cap_pos[i];
@@ -709,6 +1246,25 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     int cst = 0, cph = 0;  // variant 1: stage consumed next and its phase parity
     double ext = 0.0;
 
+    // FRACTIONAL: history sum of the current of micro-step b, whose row is
+    // shead. It needs the currents up to step b - 1 only, not the spikes of
+    // that step, so it is formed before the barrier, while the other CTAs
+    // finish: with one load in flight after the update it took 60 of the 86 us
+    // per step at N=20000, 512 lags.
+    double fhist = 0.0;
+    int shead = ST == SP_SYN_FRAC ? (int)(p.syn_step0 % p.Ls) : 0;
+    auto frac_history = [&](long long b) {
+        if (!act)
+            return;
+        const long long gs = p.syn_step0 + b;
+        const int lim = (int)(gs < p.Ls ? gs : p.Ls - 1);
+        fhist = 0.0;
+        if (lim >= 1)
+            fhist = add(fhist, mul(__ldg(p.scoef + 1), Ilast));
+        fhist = ring_sum<VAR == 0 ? 4 : 16>(fhist, p.scoef, p.Iring + i, (size_t)p.rs, p.Ls,
+                                            shead >= 2 ? shead - 2 : shead - 2 + p.Ls, 2, lim,
+                                            [](const double *q) { return __ldcg(q); });
+    };
     // synapse prepare for the own neuron before micro-step b (src/synapse.c:145-160)
     auto prepare = [&](long long b, int buf) {
         if (!act)
@@ -717,23 +1273,11 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             ptrace = add(mul(ptrace, p.psc_decay), mul(p.psc_omd, sprev));
             p.eff[(size_t)buf * p.rs + i] = ptrace;
         } else if (ST == SP_SYN_FRAC) {
-            const long long gs = p.syn_step0 + b;
-            const int Ls = p.Ls;
-            const int head = (int)(gs % Ls);
-            const long long lim = gs < Ls ? gs : Ls - 1;
-            double hist = 0.0;
-            if (lim >= 1)
-                hist = add(hist, mul(__ldg(p.scoef + 1), Ilast));
-            int r = head - 2;
-            if (r < 0)
-                r += Ls;
-            for (int k = 2; k <= lim; ++k) {
-                hist = add(hist, mul(__ldg(p.scoef + k), __ldcg(p.Iring + (size_t)r * p.rs + i)));
-                r = (r == 0) ? Ls - 1 : r - 1;
-            }
+            // fhist: the history sum of this step, formed by frac_history
             const double rhs = dvd(add(-Ilast, sprev), p.s_tau);
-            const double In = sub(mul(p.s_dta, rhs), hist);
-            p.Iring[(size_t)head * p.rs + i] = In;
+            const double In = sub(mul(p.s_dta, rhs), fhist);
+            p.Iring[(size_t)shead * p.rs + i] = In;
+            shead = shead + 1 == p.Ls ? 0 : shead + 1;
             Ilast = In;
             p.eff[(size_t)buf * p.rs + i] = In;
         } else if (ST == SP_SYN_FRAC_MEXP) {
@@ -748,13 +1292,31 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         }
     };
 
-    // arrival at the barrier that opens micro-step b
-    // Grid barrier as per-CTA flags: arriving at barrier b publishes b + 1 in
-    // the CTA's own flag (after its spike words); waiting, consumer thread t
-    // watches the flags of CTAs t, t + NC, ... and, as soon as one is up, copies
-    // that CTA's spike words into shared memory -- so the copy of the early
-    // CTAs' words overlaps the wait for the late ones, and no two CTAs write
-    // the same line.
+    // Publication of the words of barrier b (kWords): one entry per warp, or,
+    // when one CTA owns every warp, the word itself in shared memory.
+    auto publish = [&](long long b, unsigned word) {
+        if (VAR == 3) {
+            // lane r writes CTA r's copy
+            if (wact && lane < p.G && !(b == p.hold_b && (int)blockIdx.x == p.hold_cta))
+                st_cluster_u64(s_ll + (size_t)(b & 1) * p.nwords + gw, (unsigned)lane,
+                               ((unsigned long long)(p.ll_base + (unsigned)b) << 32) | word);
+            return;
+        }
+        if (!wact || lane != 0)
+            return;
+        if (p.G > 1) {
+            if (b == p.hold_b && (int)blockIdx.x == p.hold_cta)
+                return;
+            const unsigned long long v =
+                ((unsigned long long)(p.ll_base + (unsigned)b) << 32) | word;
+            *(volatile unsigned long long *)(p.ll + (size_t)(b & 1) * p.nwords + gw) = v;
+        } else {
+            s_spkb[(size_t)(b & 1) * (spk_one / 4) + gw] = word;
+        }
+    };
+    // Drive-publishing synapses: per-CTA arrival flags. Arriving at barrier b
+    // publishes b + 1 in the CTA's own flag after its drive; waiting, consumer
+    // thread t watches the flags of CTAs t, t + NC, ...
     auto barrier_arrive = [&](long long b) {
         named_sync(NC);
         if (tid == 0 && p.G > 1 && !(b == p.hold_b && (int)blockIdx.x == p.hold_cta)) {
@@ -763,33 +1325,78 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                 (unsigned long long)(b + 1);
         }
     };
+    // waits for the gather warp's announcement of barrier b
+    auto gather_wait = [&](long long b) -> bool {
+        if (ld_acquire_cta(&s_gather) >= (int)(b + 1))
+            return true;
+        const unsigned long long t0 = globaltimer_ns();
+        unsigned polls = 0;
+        while (ld_acquire_cta(&s_gather) < (int)(b + 1)) {
+            if ((++polls & 63u) == 0) {
+                if (s_abort || ld_volatile_i32(p.err) != kErrNone)
+                    return false;
+                // the gather warp's own limit comes first
+                if (globaltimer_ns() - t0 > 2 * p.tmo) {
+                    record_err(p.err, kErrBarrierTimeout, p.step0 + b);
+                    s_abort = 1;
+                    return false;
+                }
+            }
+        }
+        return true;
+    };
+    // The warps of a CTA wait by themselves where they share nothing below;
+    // with column blocks they build one spike list, so all must take the same
+    // branch: s_bad[b & 1] is written before the barrier only, and for b + 2
+    // only after everybody has read it.
+    auto verdict = [&](long long b, bool ok) -> bool {
+        ok = __all_sync(kFull, ok);
+        if (ST != SP_SYN_SIMPLE || !p.col_mode)
+            return ok;
+        if (!ok)
+            s_bad[b & 1] = 1;
+        named_sync(NC);
+        return s_bad[b & 1] == 0;
+    };
     // returns false when the launch must stop
     auto barrier_wait = [&](long long b) -> bool {
-        constexpr bool kWords = ST == SP_SYN_SIMPLE || ST == SP_SYN_PSC_HET;
-        const unsigned long long want = (unsigned long long)(b + 1);
-        unsigned *s_spk = s_spkb + (size_t)(VAR == 1 ? (b & 1) : 0) * (spk_one / 4);
-        if (VAR == 1 && p.G > 1) {
-            // the gather warp has the words: wait for its announcement
-            if (tid == 0) {
-                if (ld_acquire_cta(&s_gather) < (int)(b + 1)) {
-                    const unsigned long long t0 = globaltimer_ns();
-                    unsigned polls = 0;
-                    while (ld_acquire_cta(&s_gather) < (int)(b + 1)) {
-                        if ((++polls & 63u) == 0) {
-                            if (s_abort || ld_volatile_i32(p.err) != kErrNone)
-                                break;
-                            if (globaltimer_ns() - t0 > p.tmo) {
-                                record_err(p.err, kErrBarrierTimeout, p.step0 + b);
-                                s_abort = 1;
-                                break;
-                            }
-                        }
-                    }
+        if (kWords) {
+            if (kGath && p.G > 1)
+                return verdict(b, lane != 0 || gather_wait(b));
+            unsigned *dst = s_spkb + (size_t)(b & 1) * (spk_one / 4);
+            if (VAR == 3) {
+                // every warp collects all words, writing the same values into the
+                // CTA's buffer
+                bool ok = true;
+                if (b == 0) {
+                    for (int wi = lane; wi < p.nwords; wi += 32)
+                        dst[wi] = __ldcg(p.spk + (size_t)cur * p.nwords + wi);
+                } else {
+                    ok = gather_words(dst, b, lane, 32);
+                    if (!ok)
+                        s_abort = 1;
                 }
-                if (!kWords)
-                    __threadfence();  // the drive in global memory is read next
+                return verdict(b, ok);
             }
+            if (b == 0) {  // the previous launch's words
+                for (int wi = tid; wi < p.nwords; wi += NC)
+                    dst[wi] = __ldcg(p.spk + (size_t)cur * p.nwords + wi);
+            } else if (p.G > 1) {
+                if (!gather_words(dst, b, tid, NC)) {
+                    s_abort = 1;
+                    s_bad[b & 1] = 1;
+                }
+            }
+            named_sync(NC);
+            if (p.G <= 1)
+                return true;
+            return s_bad[b & 1] == 0;  // as in verdict
+        }
+        if (kGath && p.G > 1) {
+            if (tid == 0 && gather_wait(b))
+                __threadfence();  // the drive in global memory is read next
         } else if (p.G > 1) {
+            const unsigned long long want = (unsigned long long)(b + 1);
             for (int c = tid; c < p.G; c += NC) {
                 const unsigned long long *f = p.flags + (size_t)c * kFlagStride;
                 if (ld_volatile_u64(f) < want) {
@@ -816,16 +1423,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                     }
                 }
                 __threadfence();
-                if (kWords) {
-                    const int w0 = (int)(((long long)c * p.nwords) / p.G);
-                    const int w1 = (int)(((long long)(c + 1) * p.nwords) / p.G);
-                    for (int wi = w0; wi < w1; ++wi)
-                        s_spk[wi] = __ldcg(p.spk + (size_t)cur * p.nwords + wi);
-                }
             }
-        } else if (kWords) {
-            for (int wi = tid; wi < p.nwords; wi += NC)
-                s_spk[wi] = __ldcg(p.spk + (size_t)cur * p.nwords + wi);
         }
         named_sync(NC);
         // one verdict for the whole CTA (another CTA may record an error at any
@@ -836,20 +1434,130 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         return s_flag != 0;
     };
 
-    // prologue: drive of micro-step 0, then arrive at barrier 0
-    if (ST != SP_SYN_SIMPLE && ST != SP_SYN_PSC_HET)
+    // prologue: drive of micro-step 0, then arrive at barrier 0 (whose spike
+    // words are the previous launch's)
+    if (!kWords) {
+        if (ST == SP_SYN_FRAC)
+            frac_history(0);
         prepare(0, cur);
-    barrier_arrive(0);
+        barrier_arrive(0);
+    }
 
+    // Input rows of the next kURows macro steps, in flight to shared memory
+    double *s_ur = s_u + (size_t)warp * kURows * p.din;
+    auto u_issue = [&](int row) {
+        if (lane < p.din && row < p.n_macro)
+            cp_async8(s_ur + (row & (kURows - 1)) * p.din + lane, p.u + (size_t)row * p.din + lane);
+        cp_async_commit();
+    };
+    if (p.u_ring)
+        for (int r = 0; r < kURows; ++r)
+            u_issue(r);
+
+    // step-invariant places and the counters that follow the step (64-bit
+    // divisions cost hundreds of cycles each)
+    const int boff = VAR == 1 ? (tid / p.BW) * p.R * p.BW + (tid % p.BW) : 0;
+    // Column blocks: the spiking neurons of the barrier's words as an ascending
+    // list (all consumers; returns the count). The words are in position order,
+    // so the neurons' bits are collected in neuron order first; every thread then
+    // takes a run of words, and a scan of their counts places its entries.
+    auto spike_list = [&](const unsigned *words) -> int {
+        for (int wi = tid; wi < p.nwords; wi += NC)
+            for (unsigned mw = words[wi]; mw; mw &= mw - 1) {
+                const int nid = __ldg(p.nid_of + wi * 32 + __ffs(mw) - 1);
+                atomicOr(s_bits + (nid >> 5), 1u << (nid & 31));
+            }
+        named_sync(NC);
+        const int per = (nwn + NC - 1) / NC;
+        const int w0 = tid * per < nwn ? tid * per : nwn, w1 = w0 + per < nwn ? w0 + per : nwn;
+        int c = 0;
+        for (int wi = w0; wi < w1; ++wi)
+            c += __popc(s_bits[wi]);
+        int x = c;  // inclusive scan over the warp
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int y = __shfl_up_sync(kFull, x, off);
+            if (lane >= off)
+                x += y;
+        }
+        if (lane == 31)
+            s_wsum[warp] = x;
+        if (p.warps > 1)
+            named_sync(NC);
+        else
+            __syncwarp();
+        int at = x - c, total = 0;
+        for (int q = 0; q < p.warps; ++q) {
+            const int v = s_wsum[q];
+            if (q < warp)
+                at += v;
+            total += v;
+        }
+        for (int wi = w0; wi < w1; ++wi) {
+            for (unsigned mw = s_bits[wi]; mw; mw &= mw - 1)
+                s_list[at++] = (unsigned short)(wi * 32 + __ffs(mw) - 1);
+            s_bits[wi] = 0u;
+        }
+        named_sync(NC);
+        return total;
+    };
+    int colw0 = 0;  // column blocks: the warp's first weight
+    if (ST == SP_SYN_SIMPLE && p.col_mode && wact)
+        colw0 = __ldg(p.col_off + gw) - (p.col_mode == 2 ? __ldg(p.col_off + wb0) : 0);
+    int ell0 = 0, elln = 0;  // the warp's slot groups
+    unsigned tails = 0;      // its rows with a tail
+    if (ST == SP_SYN_SIMPLE && p.ell_cap > 0 && wact) {
+        ell0 = __ldg(p.ell_off + gw) - __ldg(p.ell_off + wb0);
+        elln = __ldg(p.ell_off + gw + 1) - __ldg(p.ell_off + gw);
+        const int *rp = s_tail_rp + 33 * (gw - wb0);
+        tails = __ballot_sync(kFull, rp[lane + 1] > rp[lane]);
+    }
+    int s = 0, m = 0;                   // macro step, micro-step within it
+    int head = (int)(p.step0 % L);      // ring row of the step
     for (long long b = 0; b < B; ++b) {
         const long long g = p.step0 + b;
         SP_STAMP(tid == 0, b, B, 0);
-        const int s = (int)(b / p.micro);
-        const int m = (int)(b % p.micro);
         if (m == 0) {
             // ext = 0 + gamma * sum_j W_in[i][j] u[j] (netlib dgemv order)
             ext = 0.0;
-            if (act && p.din > 0 && p.gamma != 0.0 && p.u) {
+            if (p.u_ring) {
+                cp_async_wait<kURows - 1>();
+                __syncwarp();
+                if (act) {
+                    const double *ur = s_ur + (s & (kURows - 1)) * p.din;
+                    double t = 0.0;
+                    if (p.win_smem) {
+                        const double *wr = s_win + tid;
+                        int j = 0;
+                        for (; j + 4 <= p.din; j += 4) {
+                            double x[4];
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                x[q] = mul(wr[(j + q) * NC], ur[j + q]);
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                t = add(t, x[q]);
+                        }
+                        if (j < p.din) {
+                            const int k1 = j + 1 < p.din ? j + 1 : j, k2 = j + 2 < p.din ? j + 2 : j;
+                            const double x0 = mul(wr[j * NC], ur[j]), x1 = mul(wr[k1 * NC], ur[k1]),
+                                         x2 = mul(wr[k2 * NC], ur[k2]);
+                            t = add(t, x0);
+                            if (k1 > j)
+                                t = add(t, x1);
+                            if (k2 > j)
+                                t = add(t, x2);
+                        }
+                    } else {
+                        const double *wr = p.W_in + (size_t)i * p.din;
+                        for (int j = 0; j < p.din; ++j)
+                            t = add(t, mul(ldg_na(wr + j), ur[j]));
+                    }
+                    ext = add(0.0, mul(p.gamma, t));
+                }
+                __syncwarp();
+                u_issue(s + kURows);
+            } else if (act && p.din > 0 && p.gamma != 0.0 && p.u) {
                 const double *ur = p.u + (size_t)s * p.din;
                 const double *wr = p.W_in + (size_t)i * p.din;
                 double t = 0.0;
@@ -859,30 +1567,33 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             }
         }
 
+        if (ST == SP_SYN_FRAC && b + 1 < B)
+            frac_history(b + 1);
+
         // ---- FLIF_GL history sum of step g
         bool integ = false;
-        double hist = 0.0;
-        int head = 0;
+        double hist = 0.0, leak = 0.0;  // what of the update does not wait for the barrier
         if (NT == SP_FLIF_GL) {
-            head = (int)(g % L);
             integ = tprev > p.f;
+            leak = dvd(-sub(vlast, p.c), p.d);
             const int lim = (int)(g < L ? g : L - 1);
             if (act && integ && lim >= 1)
-                hist = add(hist, mul(__ldg(p.coef + 1), vlast));
+                hist = add(hist, mul(coef1, vlast));
             if (VAR == 0) {
-                if (act && integ) {
-                    int r = head - 2;
-                    if (r < 0)
-                        r += L;
-                    const double *ci = p.ring + i;
-#pragma unroll 8
-                    for (int k = 2; k <= lim; ++k) {
-                        hist = add(hist, mul(__ldg(p.coef + k), __ldcg(ci + (size_t)r * p.rs)));
-                        r = (r == 0) ? L - 1 : r - 1;
-                    }
+                if (act && integ)
+                    hist = ring_sum<4>(hist, p.coef, p.ring + i, (size_t)p.rs, L,
+                                       head >= 2 ? head - 2 : head - 2 + L, 2, lim,
+                                       [](const double *q) { return __ldcg(q); });
+            } else if (VAR >= 2) {
+                // the whole history of the CTA's neurons is in shared memory
+                if (act && integ && lim >= 2) {
+                    const int r = head >= 2 ? head - 2 : head - 2 + L;
+                    const int cnt = lim - 1, n1 = cnt < r + 1 ? cnt : r + 1;
+                    hist = chain_pairs(hist, s_coef, s_coef1, s_ring, 2, r, n1);
+                    if (cnt > n1)
+                        hist = chain_pairs(hist, s_coef, s_coef1, s_ring, 2 + n1, L - 1, cnt - n1);
                 }
             } else {
-                const int boff = (tid / p.BW) * p.R * p.BW + (tid % p.BW);
                 const double *cf = p.coef_smem ? s_coef : p.coef;
                 if (act && integ) {
                     // lags 2 .. RL+1 from registers, in ascending order
@@ -891,7 +1602,9 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                         if (2 + j <= lim)
                             hist = add(hist, mul(cf[2 + j], hreg[j]));
                 }
-                int rh = (int)(((long long)head - 2 - RL) % L + L) % L;
+                int rh = head - 2 - RL;
+                while (rh < 0)
+                    rh += L;
                 for (int k = 2 + RL; k <= lim && S_b > 0;) {
                     int cnt = lim - k + 1;
                     if (cnt > p.R)
@@ -940,22 +1653,44 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             }
         }
 
+        // ---- FLIF_CAPUTO memory sum: the newest entry is V - V_0 of the last
+        // step, so nothing of it waits for this step's input
+        double cmem = 0.0;
+        if (NT == SP_FLIF_CAPUTO) {
+            integ = act && tprev > p.f;
+            if (integ)
+                cmem = caputo_sum<VAR == 0 ? 1 : 8>(sub(V, p.b), p.coef_smem ? s_coef : p.coef + 4,
+                                                    p.ring, (long long)i * L, L, cpos);
+        }
+
         // ---- barrier: spikes / eff of step g-1 are visible
         SP_STAMP(tid == 0, b, B, 1);
-        if (!barrier_wait(b))
+        if (!barrier_wait(b)) {
+            if (VAR == 3)
+                cluster_sync();  // the other CTAs may still write here
             return;
+        }
         SP_STAMP(tid == 0, b, B, 2);
         SP_STAMP(tid == 0, b, B, 3);
-        const unsigned *s_spk = s_spkb + (size_t)(VAR == 1 ? (b & 1) : 0) * (spk_one / 4);
+        const unsigned *s_spk = s_spkb + (size_t)(b & 1) * (spk_one / 4);
 
         // ---- recurrent input
         double rec = 0.0;
         if (ST == SP_SYN_SIMPLE) {
-            if (wact) {
+            if (p.col_mode) {
+                const int cnt = spike_list(s_spk);
+                if (wact && cnt > 0)
+                    rec = p.col_mode == 2
+                              ? rowpass_cols<true>(s_col_blk + (gw - wb0) * p.n, s_col_w + colw0,
+                                                   s_list, cnt, lane)
+                              : rowpass_cols<false>(p.col_blk + (size_t)gw * p.n, p.col_w + colw0,
+                                                    s_list, cnt, lane);
+            } else if (wact) {
                 // CSR rows are in position order; holes are empty rows
-                if (p.csr_cap > 0)
-                    rec = rowpass_simple_smem(s_csr_rp, s_csr_col, s_csr_w, s_spk,
-                                              (gw - wb0) * 32, lane);
+                if (p.ell_cap > 0)
+                    rec = rowpass_lanes(s_ell_col + 32 * ell0, s_ell_w + 128 * ell0, elln,
+                                        s_tail_rp + 33 * (gw - wb0), s_tail_col, s_tail_w, tails,
+                                        s_spk, lane);
                 else
                     rec = rowpass_simple_warp(p.row_ptr, p.col, p.w, s_spk, gw * 32, 32, lane);
             }
@@ -984,7 +1719,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                 }
             } else if (NT == SP_FLIF_GL) {
                 if (integ) {
-                    const double rhs = add(add(dvd(-sub(vlast, p.c), p.d), in), p.e);
+                    const double rhs = add(add(leak, in), p.e);
                     V = sub(mul(p.g, rhs), hist);
                     if (V >= p.a) {
                         V = p.b;
@@ -999,6 +1734,8 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                                 c_pol_out);
                 else
                     p.ring[(size_t)head * p.rs + i] = V;
+                if (VAR >= 2)
+                    ring_at(head) = V;
                 if (RL > 0) {
 #pragma unroll
                     for (int j = (RL > 0 ? RL : 1) - 1; j > 0; --j)
@@ -1008,20 +1745,12 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                 vlast = V;
                 tprev = add(tprev, p.dt);
             } else if (NT == SP_FLIF_CAPUTO) {
-                if (tprev > p.f) {
+                if (integ) {
                     const double dV = dvd(add(mul(-p.c, sub(V, p.d)), in), p.e);
                     const double markov = mul(p.g, dV);
-                    const int D = L;
-                    double *rg = p.ring + (size_t)i * D;
-                    rg[cpos] = sub(V, p.b);
-                    int qq = cpos;
-                    cpos = (cpos + 1 == D) ? 0 : cpos + 1;
-                    double mem = 0.0;
-                    for (int k = 0; k < D; ++k) {
-                        mem = add(mem, mul(__ldg(p.coef + k), rg[qq]));
-                        qq = (qq == 0) ? D - 1 : qq - 1;
-                    }
-                    V = add(V, sub(markov, mem));
+                    p.ring[(size_t)i * L + cpos] = sub(V, p.b);
+                    cpos = (cpos + 1 == L) ? 0 : cpos + 1;
+                    V = add(V, sub(markov, cmem));
                     if (V >= p.a) {
                         V = p.b;
                         fired = true;
@@ -1075,8 +1804,10 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
 
         // ---- spike word of step g
         const unsigned word = __ballot_sync(kFull, fired);
-        if (wact && lane == 0)
-            p.spk[(size_t)(cur ^ 1) * p.nwords + gw] = word;
+        if (kWords && b + 1 < B)
+            publish(b + 1, word);  // first: the other CTAs wait for it
+        if (wact && lane == 0 && (!kWords || b + 1 == B))
+            p.spk[(size_t)(cur ^ 1) * p.nwords + gw] = word;  // read by the next launch
         lastword = word;
         sprev = fired ? 1.0 : 0.0;
         SP_STAMP(tid == 0, b, B, 5);
@@ -1087,16 +1818,28 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                 p.raster[(size_t)s * p.nwords + gw] = lastword;
         }
         if (b + 1 < B) {
-            if (ST != SP_SYN_SIMPLE && ST != SP_SYN_PSC_HET)
+            if (!kWords) {
                 prepare(b + 1, cur ^ 1);
-            barrier_arrive(b + 1);
-            if (VAR == 1 && tid == 0)
-                st_release_cta(&s_done, (int)(b + 1));
+                barrier_arrive(b + 1);
+                if (VAR == 1 && tid == 0)
+                    st_release_cta(&s_done, (int)(b + 1));
+            } else if (kGath) {
+                __syncwarp();
+                if (wact && lane == 0)
+                    red_release_cta(&s_done, 1);
+            }
         }
         SP_STAMP(tid == 0, b, B, 6);
         cur ^= 1;
+        head = head + 1 == L ? 0 : head + 1;
+        if (++m == p.micro) {
+            m = 0;
+            ++s;
+        }
     }
 
+    if (VAR == 3)
+        cluster_sync();
     if (act) {
         p.V[i] = V;
         if (NT == SP_FLIF_GL || NT == SP_FLIF_CAPUTO)

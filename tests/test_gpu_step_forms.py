@@ -1,0 +1,105 @@
+"""The step kernel's forms against the oracle, bit for bit: the cluster launch
+and its spike exchange, the history kept in shared memory, the recurrent rows
+as slots and tails and as column blocks, and FLIF_CAPUTO's 32-byte blocks --
+each at the sizes where it can go wrong, over several launches in a row."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import spires_b200 as sp
+from tests import _oracle as O
+
+pytestmark = pytest.mark.gpu
+
+GL = lambda L: (1.0, 0.0, 0.0, 20.0, 0.7, float(L), 0.1, 2.0)
+
+
+def check(n, neuron, ctas, T, nparams=None, synapse=sp.SYN_SIMPLE, topo=sp.CONN_RANDOM, conn=0.05,
+          dt=1.0):
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=conn, dt=dt, topo=topo,
+                         neuron=neuron, nparams=nparams or O.NEURON_PARAMS[neuron],
+                         synapse=synapse, sparams=O.SYNAPSE_PARAMS[synapse])
+    u = np.random.default_rng(3).uniform(-1.0, 1.5, (T, 2))
+    r = sp.Reservoir(cfg, seed=11)
+    nw = (n + 31) // 32
+    assert r.set_launch(ctas=ctas, warps_max=-(-nw // ctas), variant=0) == sp.SPIRES_OK
+    h = T // 3
+    parts = [r.run_record(x) for x in (u[:h], u[h:h + 1], u[h + 1:])]
+    r.close()
+    phi = np.concatenate([p[0] for p in parts])
+    ras = sp.unpack_raster(np.concatenate([p[1] for p in parts]), n)
+    phi_o, ras_o, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=11)).run(u)
+    assert np.array_equal(ras, ras_o)
+    assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
+
+
+@pytest.mark.parametrize("neuron", [sp.LIF_DISCRETE, sp.LIF_BIO, sp.FLIF_CAPUTO, sp.FLIF_GL,
+                                    sp.FLIF_DIFFUSIVE])
+@pytest.mark.parametrize("synapse", [sp.SYN_SIMPLE, sp.SYN_PSC_HET])
+@pytest.mark.parametrize("ctas", [2, 16, 3])
+def test_exchange(neuron, synapse, ctas):
+    """Clusters of 2 and 16 CTAs, and 3 CTAs exchanging through the L2."""
+    check(600, neuron, ctas, 60, synapse=synapse, dt=0.5 if ctas == 2 else 1.0)
+
+
+def test_largest_cluster():
+    check(8192, sp.LIF_DISCRETE, 16, 16, topo=sp.CONN_SMALL_WORLD, conn=0.001)
+
+
+@pytest.mark.parametrize("L", [1, 2, 3, 33, 64, 201])
+@pytest.mark.parametrize("ctas", [1, 5, 8])
+def test_history_in_shared_memory(L, ctas):
+    """Odd and even ring lengths below and above a block, through ramp-up and wrap."""
+    check(200 if ctas == 1 else 250, sp.FLIF_GL, ctas, 2 * L + 40, nparams=GL(L))
+
+
+@pytest.mark.parametrize("n,conn,ctas", [(250, 0.2, 1), (1000, 0.1, 16), (1000, 0.3, 5),
+                                         (1025, 0.06, 33), (500, 0.9, 4)])
+def test_dense_rows_as_column_blocks(n, conn, ctas):
+    check(n, sp.LIF_DISCRETE, ctas, 40, conn=conn)
+
+
+@pytest.mark.parametrize("topo,conn", [(sp.CONN_SCALE_FREE, 0.003), (sp.CONN_SCALE_FREE, 0.0005),
+                                       (sp.CONN_SMALL_WORLD, 0.004), (sp.CONN_RANDOM, 0.0005)])
+@pytest.mark.parametrize("ctas", [16, 63])
+def test_sparse_rows_as_slots_and_tails(topo, conn, ctas):
+    """Hubs with tails of several 32-edge blocks, even rows, empty rows."""
+    check(2000, sp.LIF_DISCRETE, ctas, 40, topo=topo, conn=conn)
+
+
+@pytest.mark.parametrize("D", [1, 2, 3, 4, 5, 31, 32, 33, 64, 65, 66, 67, 130])
+@pytest.mark.parametrize("ctas", [1, 4])
+def test_caputo_blocks(D, ctas):
+    """Shift registers of every alignment, shorter and longer than the blocks in
+    flight, with each neuron's head at its own place after the first spikes."""
+    check(100, sp.FLIF_CAPUTO, ctas, 2 * D + 40, conn=0.06,
+          nparams=(1.0, 0.2, 0.0, 1.0, 0.0, 1.5, 0.7, 2.0, float(D + 2)))
+
+
+@pytest.mark.parametrize("conn", [0.002, 0.1])
+def test_cluster_wait_runs_out(conn):
+    """A CTA of a cluster that withholds its spike words once: the launch ends
+    with an error naming the micro-step, and the reservoir works after a reset."""
+    cfg = sp.make_config(2000, 2, 2, rho=1.2, ei=0.55, gamma=1.2, conn=conn,
+                         topo=sp.CONN_SCALE_FREE, neuron=sp.LIF_DISCRETE,
+                         nparams=O.NEURON_PARAMS[sp.LIF_DISCRETE])
+    u = np.random.default_rng(0).uniform(-1.0, 1.5, (30, 2))
+    r = sp.Reservoir(cfg, seed=17)
+    assert r.set_launch(ctas=16, warps_max=4, variant=0) == sp.SPIRES_OK
+    assert r.lib.spires_ext_set_wait_limit(r.h, 50.0) == sp.SPIRES_OK
+    r.run_record(u[:12])
+    assert r.lib.spires_ext_test_withhold_arrival(r.h, 1, 5) == sp.SPIRES_OK
+    P = np.empty((10, r.n))
+    st = r.lib.spires_ext_run_record(r.h, sp.dptr(np.ascontiguousarray(u[12:22])), 10, sp.dptr(P),
+                                     None, None)
+    assert st == sp.SPIRES_ERR_INTERNAL
+    code, step = C.c_int(-1), C.c_longlong(-1)
+    assert r.lib.spires_ext_last_device_error(r.h, C.byref(code), C.byref(step)) == sp.SPIRES_OK
+    assert (code.value, step.value) == (1, 17)
+    r.reset()
+    phi, R, _ = r.run_record(u)
+    r.close()
+    phi_o, ras_o, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=17)).run(u)
+    assert np.array_equal(sp.unpack_raster(R, 2000), ras_o)
+    assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
