@@ -17,6 +17,9 @@
 // scaling by GELU'). The network is 18k parameters and the batches are a few
 // thousand rows, so these are latency-sized launches; the layer shapes do
 // not fill a tensor-core tile schedule worth its setup.
+//
+// Training runs a whole epoch in one launch (k_train): one cluster of 16 CTAs
+// keeps the parameters in shared memory and meets twice per minibatch.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cmath>
@@ -126,22 +129,6 @@ __global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float *
     }
 }
 
-// dL/d(out) of the Gaussian NLL for rows [0, B), scaled by 1/B; also the
-// per-row loss terms.
-__global__ void k_nll_grad(const float *__restrict__ out, const float *__restrict__ y, int B,
-                           float *__restrict__ dout, float *__restrict__ row_loss)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= B)
-        return;
-    const float m = out[2 * s], v = out[2 * s + 1];
-    const float r = y[s] - m, iv = expf(-v);
-    const float inv = 1.0f / (float)B;
-    dout[2 * s] = -r * iv * inv;
-    dout[2 * s + 1] = 0.5f * (1.0f - r * r * iv) * inv;
-    row_loss[s] = 0.5f * (v + r * r * iv);
-}
-
 // Column sums (bias gradients): g[j] = sum_s D[s][j], fixed order per column.
 __global__ void k_colsum(const float *__restrict__ D, int B, int N, float *__restrict__ g)
 {
@@ -172,20 +159,423 @@ __global__ void k_mean(const float *__restrict__ x, int B, float *out)
         *out = part[0] / (float)B;
 }
 
+// The rows of a minibatch, gathered by the epoch's row order.
+__global__ void k_take_rows(const float *__restrict__ X, const float *__restrict__ y,
+                            const int *__restrict__ perm, int B, float *__restrict__ xb,
+                            float *__restrict__ yb)
+{
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= B)
+        return;
+    const int r = perm[s];
+    for (int k = 0; k < kIn; ++k)
+        xb[(size_t)s * kIn + k] = X[(size_t)r * kIn + k];
+    yb[s] = y[r];
+}
+
 // Adam (Kingma & Ba 2015) with bias correction; step t >= 1.
+__device__ __forceinline__ void adam_step(float &p, float gi, float &m1, float &m2, float lr,
+                                          float b1, float b2, float eps, float c1, float c2)
+{
+    const float a = b1 * m1 + (1.0f - b1) * gi;
+    const float b = b2 * m2 + (1.0f - b2) * gi * gi;
+    m1 = a;
+    m2 = b;
+    p -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+}
+
 __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m1,
                        float *__restrict__ m2, int n, float lr, float b1, float b2, float eps,
                        float c1, float c2)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    const float gi = g[i];
-    const float a = b1 * m1[i] + (1.0f - b1) * gi;
-    const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
-    m1[i] = a;
-    m2[i] = b;
-    p[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+    if (i < n)
+        adam_step(p[i], g[i], m1[i], m2[i], lr, b1, b2, eps, c1, c2);
+}
+
+// dL/d(out) of one row (out = mean, log-variance), scaled by inv = 1/B, and the
+// row's loss term.
+__device__ __forceinline__ void nll_row(float m, float v, float y, float inv, float &d0, float &d1,
+                                        float &loss)
+{
+    const float r = y - m, iv = expf(-v);
+    d0 = -r * iv * inv;
+    d1 = 0.5f * (1.0f - r * r * iv) * inv;
+    loss = 0.5f * (v + r * r * iv);
+}
+
+// The same for rows [0, B), one thread per row.
+__global__ void k_nll_grad(const float *__restrict__ out, const float *__restrict__ y, int B,
+                           float *__restrict__ dout, float *__restrict__ row_loss)
+{
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < B)
+        nll_row(out[2 * s], out[2 * s + 1], y[s], 1.0f / (float)B, dout[2 * s], dout[2 * s + 1],
+                row_loss[s]);
+}
+
+// ------------------------------------------------------- fused training epoch
+// All minibatches of one epoch in one launch: a cluster of kTC CTAs, each with
+// its own copy of the parameters in shared memory. Per minibatch of B rows
+//   rows     CTA q runs every kTC-th tile of 16 rows forward and back to the
+//            layer gradients, 2 rows x 4 columns of a layer per thread, and
+//            writes H1, H2, dZ1, dZ2 and dL/d(out) to memory
+//   cluster barrier
+//   weights  CTA q sums the gradients it owns over all rows in ascending order
+//            (a 32 x 32 block of W2, 8 rows of W1, 8 columns of W3, the biases
+//            with them) and takes their Adam step
+//   cluster barrier, then every CTA reads the new parameters
+// Every sum runs over the same terms in the same order as the separate kernels
+// above (and so gives the same bits): only the launches between them are gone.
+// What bounds it: the shared-memory reads of the two 128 x 128 products and the
+// two barriers with the parameter reads behind them; 256 rows take about 20 us
+// where 14 launches took 172.
+constexpr int kTC = 16;           // CTAs of the cluster
+constexpr int kTT = 256;          // threads
+constexpr int kTR = 16;           // rows of a tile
+constexpr int kTS = 256;          // rows of a staged block in the weight phase
+constexpr int kW1P = kIn + 1, kHP = kHid + 4;  // padded pitches
+
+struct TrainArgs {
+    float *p, *m1, *m2;
+    const float *X, *y;           // all rows
+    const int *perm;              // row order of the epoch
+    const float2 *corr;           // Adam's bias corrections of each minibatch
+    float *H1, *H2, *dZ1, *dZ2, *dO, *rl;  // [batch][..] activations and gradients
+    int n, batch, steps;
+    float lr, b1, b2, eps;
+};
+
+struct TrainSmem {
+    float W1[kHid * kW1P], b1[kHid], W2[kHid][kHP], b2[kHid], W3[kOut * kHid], b3[4];
+    union {
+        struct {
+            float X[kTR][12], H1[kTR][kHP], H2[kTR][kHP], D2[kTR][kHP], dO[kTR][2];
+        } r;
+        struct {
+            float D2[kTS][32], H1[kTS][32], D1[kTS][8], H2[kTS][8], X[kTS][kIn], dO[kTS][2];
+        } w;
+    };
+};
+
+// Asynchronous copies of 16 and 4 bytes through the L2 (activations and
+// parameters that other CTAs have just written).
+__device__ __forceinline__ void copy16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy4(void *dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_done()
+{
+    asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
+}
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;"
+                 ::: "memory");
+}
+
+// acc[q][c] = sum_k A[q][k] W(lane + 32 c, k), k ascending: W(j, k) is W2[j][k]
+// (the layer forward; 16-byte loads, conflict-free at this pitch) or W2[k][j]
+// (its transpose, for the gradient).
+template <bool kTrans>
+__device__ __forceinline__ void layer_128(float (&acc)[2][4], const float (*A)[kHP],
+                                          const float (*W)[kHP], int lane)
+{
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            acc[q][c] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < kHid; k += 4) {
+        float a[2][4], w[4][4];
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            *(float4 *)a[q] = *(const float4 *)&A[q][k];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (!kTrans) {
+                *(float4 *)w[c] = *(const float4 *)&W[lane + 32 * c][k];
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    w[c][u] = W[k + u][lane + 32 * c];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    acc[q][c] = fmaf(a[q][u], w[c][u], acc[q][c]);
+    }
+}
+
+__global__ void __launch_bounds__(kTT, 1) k_train(TrainArgs t)
+{
+    extern __shared__ __align__(16) unsigned char train_smem[];
+    TrainSmem &S = *(TrainSmem *)train_smem;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cta = blockIdx.x;  // the grid is one cluster
+
+    for (int st = 0; st < t.steps; ++st) {
+        const int s0 = st * t.batch;
+        const int B = s0 + t.batch <= t.n ? t.batch : t.n - s0;
+        const int *perm = t.perm + s0;
+        // ---- the parameters (written by their owners before the last barrier;
+        // read past the L1, which may hold the step before's)
+        {
+            float w1[kP1 / kTT];
+#pragma unroll
+            for (int k = 0; k < kP1 / kTT; ++k)
+                w1[k] = __ldcg(t.p + oW1 + k * kTT + tid);
+            const float b = __ldcg(t.p + (tid < kHid ? ob1 + tid : ob2 + tid - kHid));
+            const float w3 = __ldcg(t.p + oW3 + tid);
+            const float b3 = __ldcg(t.p + ob3 + (tid & 1));
+#pragma unroll
+            for (int k = 0; k < kP2 / 4 / kTT; ++k) {
+                const int e = k * kTT + tid;
+                copy16(&S.W2[e / 32][e % 32 * 4], t.p + oW2 + 4 * e);
+            }
+#pragma unroll
+            for (int k = 0; k < kP1 / kTT; ++k) {
+                const int e = k * kTT + tid;
+                S.W1[e / kIn * kW1P + e % kIn] = w1[k];
+            }
+            (tid < kHid ? S.b1 : S.b2)[tid & (kHid - 1)] = b;
+            S.W3[tid] = w3;
+            if (tid < kOut)
+                S.b3[tid] = b3;
+            copies_done();
+        }
+        // ---- rows: tile g of 16 rows belongs to CTA g % kTC
+        const float inv = 1.0f / (float)B;
+        for (int g = cta; g * kTR < B; g += kTC) {
+            const int base = g * kTR, cnt = B - base < kTR ? B - base : kTR;
+            __syncthreads();
+            for (int k = tid; k < kTR * kIn; k += kTT) {
+                const int r = k / kIn, c = k % kIn;
+                S.r.X[r][c] = r < cnt ? __ldg(t.X + (size_t)__ldg(perm + base + r) * kIn + c) : 0.f;
+            }
+            __syncthreads();
+            // a warp takes two rows from here to their gradients by itself
+            const int r0 = 2 * warp;
+            const bool on[2] = {r0 < cnt, r0 + 1 < cnt};
+            size_t row[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                row[q] = (size_t)(base + r0 + q) * kHid + lane;
+            float z1[2][4], z2[2][4];
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int j = lane + 32 * c;
+                    float acc = 0.f;
+#pragma unroll
+                    for (int k = 0; k < kIn; ++k)
+                        acc = fmaf(S.r.X[r0 + q][k], S.W1[j * kW1P + k], acc);
+                    z1[q][c] = acc + S.b1[j];
+                    const float h = gelu(z1[q][c]);
+                    S.r.H1[r0 + q][j] = h;
+                    if (on[q])
+                        t.H1[row[q] + 32 * c] = h;
+                }
+            __syncwarp();
+            layer_128<false>(z2, S.r.H1 + r0, S.W2, lane);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int j = lane + 32 * c;
+                    z2[q][c] += S.b2[j];
+                    const float h = gelu(z2[q][c]);
+                    S.r.H2[r0 + q][j] = h;
+                    if (on[q])
+                        t.H2[row[q] + 32 * c] = h;
+                }
+            __syncwarp();
+            // output layer and its gradient: lane 2q + o of the warp's rows
+            float o = 0.f;
+            {
+                const float *h = S.r.H2[r0 + ((lane >> 1) & 1)];
+                const float *w = S.W3 + (lane & 1) * kHid;
+#pragma unroll 4
+                for (int k = 0; k < kHid; k += 4) {
+                    const float4 x = *(const float4 *)(h + k), v = *(const float4 *)(w + k);
+                    o = fmaf(x.x, v.x, o);
+                    o = fmaf(x.y, v.y, o);
+                    o = fmaf(x.z, v.z, o);
+                    o = fmaf(x.w, v.w, o);
+                }
+                o += S.b3[lane & 1];
+            }
+            const float v = __shfl_sync(0xffffffffu, o, lane | 1);
+            const int r = r0 + (lane >> 1);
+            if (lane < 4 && !(lane & 1)) {
+                float d0 = 0.f, d1 = 0.f, loss = 0.f;
+                if (r < cnt) {
+                    nll_row(o, v, __ldg(t.y + __ldg(perm + base + r)), inv, d0, d1, loss);
+                    t.dO[2 * (base + r)] = d0;
+                    t.dO[2 * (base + r) + 1] = d1;
+                    t.rl[base + r] = loss;
+                }
+                S.r.dO[r][0] = d0;
+                S.r.dO[r][1] = d1;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int j = lane + 32 * c;
+                    float d = fmaf(S.r.dO[r0 + q][0], S.W3[j], 0.f);
+                    d = fmaf(S.r.dO[r0 + q][1], S.W3[kHid + j], d);
+                    d *= gelu_grad(z2[q][c]);
+                    S.r.D2[r0 + q][j] = d;
+                    if (on[q])
+                        t.dZ2[row[q] + 32 * c] = d;
+                }
+            __syncwarp();
+            layer_128<true>(z2, S.r.D2 + r0, S.W2, lane);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (on[q])
+                        t.dZ1[row[q] + 32 * c] = z2[q][c] * gelu_grad(z1[q][c]);
+        }
+        cluster_barrier();
+        // ---- weights: this CTA's block of W2 is rows 32 bi.., columns 32 bj..
+        const int bi = cta >> 2, bj = cta & 3, c8 = 8 * cta;
+        float gw[4][2] = {}, ga = 0.f, gb = 0.f;
+        // what this thread owns: 8 entries of W2 (at[0] + 128 q + c), or up to two
+        // others; their Adam state is loaded ahead of the sums
+        int at[2] = {-1, -1};
+        if (warp < 4) {
+            at[0] = oW2 + (32 * bi + 4 * (tid >> 4)) * kHid + 32 * bj + 2 * (tid & 15);
+        } else {
+            const int q = tid - 128;
+            at[0] = q < 80 ? oW1 + (c8 + q / kIn) * kIn + q % kIn
+                    : q < 96 ? oW3 + ((q - 80) & 1) * kHid + c8 + ((q - 80) >> 1)
+                    : bj == 0 ? ob2 + 32 * bi + q - 96
+                              : -1;
+            at[1] = q < 8 ? ob1 + c8 + q : (cta == 0 && q < 10 ? ob3 + q - 8 : -1);
+        }
+        float pv[4][2], v1[4][2], v2[4][2];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int i = warp < 4 ? at[0] + q * kHid + c : (q == 0 ? at[c] : -1);
+                const bool own = i >= 0;
+                pv[q][c] = own ? t.p[i] : 0.f;
+                v1[q][c] = own ? t.m1[i] : 0.f;
+                v2[q][c] = own ? t.m2[i] : 0.f;
+            }
+        for (int w0 = 0; w0 < B; w0 += kTS) {
+            const int cnt = B - w0 < kTS ? B - w0 : kTS;
+            __syncthreads();
+            for (int k = tid; k < cnt * 8; k += kTT) {
+                const int r = k >> 3, c = (k & 7) * 4;
+                copy16(&S.w.D2[r][c], t.dZ2 + (size_t)(w0 + r) * kHid + 32 * bi + c);
+                copy16(&S.w.H1[r][c], t.H1 + (size_t)(w0 + r) * kHid + 32 * bj + c);
+            }
+            for (int k = tid; k < cnt * 2; k += kTT) {
+                const int r = k >> 1, c = (k & 1) * 4;
+                copy16(&S.w.D1[r][c], t.dZ1 + (size_t)(w0 + r) * kHid + c8 + c);
+                copy16(&S.w.H2[r][c], t.H2 + (size_t)(w0 + r) * kHid + c8 + c);
+            }
+            for (int k = tid; k < cnt; k += kTT) {
+                const float *x = t.X + (size_t)__ldg(perm + w0 + k) * kIn;
+#pragma unroll
+                for (int c = 0; c < kIn; ++c)
+                    copy4(&S.w.X[k][c], x + c);
+                // written by another CTA: not through the L1
+                const float2 d = __ldcg((const float2 *)t.dO + w0 + k);
+                S.w.dO[k][0] = d.x;
+                S.w.dO[k][1] = d.y;
+            }
+            copies_done();
+            __syncthreads();
+            if (warp < 4) {
+                // 4 rows x 2 columns of the W2 block per thread
+                const int i0 = 4 * (tid >> 4), j0 = 2 * (tid & 15);
+#pragma unroll 4
+                for (int r = 0; r < cnt; ++r) {
+                    const float4 a = *(const float4 *)&S.w.D2[r][i0];
+                    const float2 h = *(const float2 *)&S.w.H1[r][j0];
+                    gw[0][0] = fmaf(a.x, h.x, gw[0][0]);
+                    gw[0][1] = fmaf(a.x, h.y, gw[0][1]);
+                    gw[1][0] = fmaf(a.y, h.x, gw[1][0]);
+                    gw[1][1] = fmaf(a.y, h.y, gw[1][1]);
+                    gw[2][0] = fmaf(a.z, h.x, gw[2][0]);
+                    gw[2][1] = fmaf(a.z, h.y, gw[2][1]);
+                    gw[3][0] = fmaf(a.w, h.x, gw[3][0]);
+                    gw[3][1] = fmaf(a.w, h.y, gw[3][1]);
+                }
+            } else {
+                // 80 entries of W1, 16 of W3 (threads 0..95), then the biases:
+                // 8 of b1, 32 of b2 (CTAs with bj = 0), 2 of b3 (CTA 0)
+                const int q = tid - 128;
+                if (q < 80) {
+                    const int i = q / kIn, c = q % kIn;
+#pragma unroll 8
+                    for (int r = 0; r < cnt; ++r)
+                        ga = fmaf(S.w.D1[r][i], S.w.X[r][c], ga);
+                } else if (q < 96) {
+                    const int o = (q - 80) & 1, c = (q - 80) >> 1;
+#pragma unroll 8
+                    for (int r = 0; r < cnt; ++r)
+                        ga = fmaf(S.w.dO[r][o], S.w.H2[r][c], ga);
+                } else if (bj == 0) {
+#pragma unroll 8
+                    for (int r = 0; r < cnt; ++r)
+                        ga += S.w.D2[r][q - 96];
+                }
+                if (q < 8) {
+#pragma unroll 8
+                    for (int r = 0; r < cnt; ++r)
+                        gb += S.w.D1[r][q];
+                } else if (cta == 0 && q < 10) {
+#pragma unroll 8
+                    for (int r = 0; r < cnt; ++r)
+                        gb += S.w.dO[r][q - 8];
+                }
+            }
+        }
+        // ---- Adam on what this CTA owns
+        const float c1 = __ldg(&t.corr[st].x), c2 = __ldg(&t.corr[st].y);
+        if (warp >= 4) {
+            gw[0][0] = ga;
+            gw[0][1] = gb;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int i = warp < 4 ? at[0] + q * kHid + c : (q == 0 ? at[c] : -1);
+                if (i < 0)
+                    continue;
+                adam_step(pv[q][c], gw[q][c], v1[q][c], v2[q][c], t.lr, t.b1, t.b2, t.eps, c1, c2);
+                t.p[i] = pv[q][c];
+                t.m1[i] = v1[q][c];
+                t.m2[i] = v2[q][c];
+            }
+        cluster_barrier();
+    }
 }
 
 // PCG32 (O'Neill 2014) for the seeded initialisation and batch shuffles.
@@ -211,6 +601,13 @@ struct sp_mlp {
     float *X = nullptr, *y = nullptr, *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr,
           *O = nullptr, *dO = nullptr, *dH2 = nullptr, *dH1 = nullptr, *rl = nullptr,
           *loss = nullptr, *pb = nullptr;
+    // training: all rows, and two epochs' row orders and bias corrections
+    int cap_rows = 0, cap_steps = 0;
+    float *Xall = nullptr, *yall = nullptr;
+    int *d_perm = nullptr, *h_perm = nullptr;        // [2][cap_rows]
+    float2 *d_corr = nullptr, *h_corr = nullptr;     // [2][cap_steps]
+    cudaEvent_t epoch_done[2] = {nullptr, nullptr};
+    int fused = -1;         // the cluster launch is available (-1: not asked yet)
     long long t = 0;        // Adam steps taken
     long long launches = 0; // kernels launched
 };
@@ -309,6 +706,8 @@ static void backward(sp_mlp *m, int B)
 
 extern "C" int sp_mlp_num_params(void) { return kParams; }
 
+static void train_free(sp_mlp *m);
+
 extern "C" void sp_mlp_destroy(sp_mlp *m)
 {
     if (!m)
@@ -316,6 +715,10 @@ extern "C" void sp_mlp_destroy(sp_mlp *m)
     if (m->stream)
         cudaStreamSynchronize(m->stream);
     mlp_free_work(m);
+    train_free(m);
+    for (cudaEvent_t e : m->epoch_done)
+        if (e)
+            cudaEventDestroy(e);
     float *bufs[] = {m->p, m->g, m->m1, m->m2, m->loss, m->pb};
     for (float *b : bufs)
         if (b)
@@ -401,9 +804,96 @@ extern "C" int sp_mlp_loss_grad(sp_mlp *m, const float *X, const float *y, int n
     return SP_OK;
 }
 
+static void train_free(sp_mlp *m)
+{
+    void *dv[] = {m->Xall, m->yall, m->d_perm, m->d_corr};
+    for (void *b : dv)
+        if (b)
+            sp_cuda_free(b);
+    if (m->h_perm)
+        cudaFreeHost(m->h_perm);
+    if (m->h_corr)
+        cudaFreeHost(m->h_corr);
+    m->Xall = m->yall = nullptr;
+    m->d_perm = m->h_perm = nullptr;
+    m->d_corr = m->h_corr = nullptr;
+    m->cap_rows = m->cap_steps = 0;
+}
+
+// Buffers for n rows in `steps` minibatches per epoch, kept by the handle.
+static int train_reserve(sp_mlp *m, int n, int steps)
+{
+    for (cudaEvent_t &e : m->epoch_done)
+        if (!e)
+            MK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (n <= m->cap_rows && steps <= m->cap_steps)
+        return SP_OK;
+    train_free(m);
+    const size_t r = (size_t)n, s = (size_t)steps;
+    MK(sp_cuda_malloc(&m->Xall, r * kIn * 4));
+    MK(sp_cuda_malloc(&m->yall, r * 4));
+    MK(sp_cuda_malloc(&m->d_perm, 2 * r * 4));
+    MK(sp_cuda_malloc(&m->d_corr, 2 * s * sizeof(float2)));
+    MK(cudaMallocHost(&m->h_perm, 2 * r * 4));
+    MK(cudaMallocHost(&m->h_corr, 2 * s * sizeof(float2)));
+    m->cap_rows = n;
+    m->cap_steps = steps;
+    return SP_OK;
+}
+
+// Whether k_train's cluster can be launched on this device.
+static bool train_fused(sp_mlp *m)
+{
+    if (m->fused < 0) {
+        cudaLaunchConfig_t c;
+        cudaLaunchAttribute a;
+        memset(&c, 0, sizeof(c));
+        memset(&a, 0, sizeof(a));
+        a.id = cudaLaunchAttributeClusterDimension;
+        a.val.clusterDim.x = kTC;
+        a.val.clusterDim.y = a.val.clusterDim.z = 1;
+        c.gridDim = dim3(kTC);
+        c.blockDim = dim3(kTT);
+        c.dynamicSmemBytes = sizeof(TrainSmem);
+        c.attrs = &a;
+        c.numAttrs = 1;
+        int n = 0;
+        m->fused = cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(TrainSmem)) == cudaSuccess &&
+                   cudaFuncSetAttribute(k_train, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                        1) == cudaSuccess &&
+                   cudaOccupancyMaxActiveClusters(&n, k_train, &c) == cudaSuccess && n >= 1;
+        cudaGetLastError();
+    }
+    return m->fused == 1;
+}
+
+static int launch_train(sp_mlp *m, const TrainArgs &t)
+{
+    cudaLaunchConfig_t c;
+    cudaLaunchAttribute a;
+    memset(&c, 0, sizeof(c));
+    memset(&a, 0, sizeof(a));
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = kTC;
+    a.val.clusterDim.y = a.val.clusterDim.z = 1;
+    c.gridDim = dim3(kTC);
+    c.blockDim = dim3(kTT);
+    c.dynamicSmemBytes = sizeof(TrainSmem);
+    c.stream = m->stream;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    MK(cudaLaunchKernelEx(&c, k_train, t));
+    m->launches++;
+    return SP_OK;
+}
+
 // Adam on minibatches of a shuffled copy of the n rows, for `epochs` passes.
-// The rows are uploaded once; each step gathers its minibatch on the host
-// order (a permutation of row indices) into the front of the work buffers.
+// The rows are uploaded once; an epoch is one launch that gathers its
+// minibatches by the epoch's row order, which the host draws while the epoch
+// before runs. The separate kernels serve a device that cannot schedule the
+// cluster.
+
 extern "C" int sp_mlp_train(sp_mlp *m, const float *X, const float *y, int n, int epochs,
                             int batch, float lr, uint64_t seed, float *final_loss)
 {
@@ -414,14 +904,18 @@ extern "C" int sp_mlp_train(sp_mlp *m, const float *X, const float *y, int n, in
     int rc = mlp_reserve(m, batch);
     if (rc)
         return rc;
-    const size_t steps_per_epoch = (size_t)((n + batch - 1) / batch);
+    const int steps = (int)(((long long)n + batch - 1) / batch);
+    rc = train_reserve(m, n, steps);
+    if (rc) {
+        train_free(m);
+        return rc;
+    }
     std::vector<int> perm(n);
     for (int i = 0; i < n; ++i)
         perm[i] = i;
-    std::vector<float> xb((size_t)batch * kIn), yb(batch);
-    float *hx = nullptr, *hy = nullptr;
-    MK(cudaMallocHost(&hx, steps_per_epoch * (size_t)batch * kIn * 4));
-    MK(cudaMallocHost(&hy, steps_per_epoch * (size_t)batch * 4));
+    MK(cudaMemcpyAsync(m->Xall, X, (size_t)n * kIn * 4, cudaMemcpyHostToDevice, m->stream));
+    MK(cudaMemcpyAsync(m->yall, y, (size_t)n * 4, cudaMemcpyHostToDevice, m->stream));
+    const bool fused = train_fused(m);
     Pcg r{seed ^ 0x5DEECE66Dull};
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     for (int ep = 0; ep < epochs && !rc; ++ep) {
@@ -432,39 +926,77 @@ extern "C" int sp_mlp_train(sp_mlp *m, const float *X, const float *y, int n, in
             perm[i] = perm[j];
             perm[j] = t;
         }
-        for (size_t st = 0; st < steps_per_epoch; ++st) {
-            const int s0 = (int)(st * batch);
-            const int B = (s0 + batch <= n) ? batch : n - s0;
-            float *px = hx + st * (size_t)batch * kIn, *py = hy + st * (size_t)batch;
-            for (int k = 0; k < B; ++k) {
-                memcpy(px + (size_t)k * kIn, X + (size_t)perm[s0 + k] * kIn, kIn * 4);
-                py[k] = y[perm[s0 + k]];
-            }
-            if (cudaMemcpyAsync(m->X, px, (size_t)B * kIn * 4, cudaMemcpyHostToDevice,
-                                m->stream) != cudaSuccess ||
-                cudaMemcpyAsync(m->y, py, (size_t)B * 4, cudaMemcpyHostToDevice, m->stream) !=
-                    cudaSuccess) {
-                rc = SP_EINTERNAL;
-                break;
-            }
-            forward(m, m->p, B, 0);
-            backward(m, B);
-            m->t++;
-            const float c1 = 1.0f - powf(b1, (float)m->t), c2 = 1.0f - powf(b2, (float)m->t);
-            k_adam<<<(kParams + 255) / 256, 256, 0, m->stream>>>(m->p, m->g, m->m1, m->m2, kParams,
-                                                                 lr, b1, b2, eps, c1, c2);
-            m->launches++;
+        // the staging of the epoch before the last one is free again
+        const int sl = ep & 1;
+        if (ep >= 2 && cudaEventSynchronize(m->epoch_done[sl]) != cudaSuccess) {
+            rc = SP_EINTERNAL;
+            break;
         }
-        // the pinned staging of this epoch is reused by the next one
-        if (cudaStreamSynchronize(m->stream) != cudaSuccess)
+        int *hp = m->h_perm + (size_t)sl * m->cap_rows, *dp = m->d_perm + (size_t)sl * m->cap_rows;
+        float2 *hc = m->h_corr + (size_t)sl * m->cap_steps,
+               *dc = m->d_corr + (size_t)sl * m->cap_steps;
+        memcpy(hp, perm.data(), (size_t)n * 4);
+        for (int st = 0; st < steps; ++st) {
+            m->t++;
+            hc[st] = make_float2(1.0f - powf(b1, (float)m->t), 1.0f - powf(b2, (float)m->t));
+        }
+        if (cudaMemcpyAsync(dp, hp, (size_t)n * 4, cudaMemcpyHostToDevice, m->stream) !=
+                cudaSuccess ||
+            cudaMemcpyAsync(dc, hc, (size_t)steps * sizeof(float2), cudaMemcpyHostToDevice,
+                            m->stream) != cudaSuccess) {
+            rc = SP_EINTERNAL;
+            break;
+        }
+        if (fused) {
+            TrainArgs t;
+            t.p = m->p;
+            t.m1 = m->m1;
+            t.m2 = m->m2;
+            t.X = m->Xall;
+            t.y = m->yall;
+            t.perm = dp;
+            t.corr = dc;
+            t.H1 = m->H1;
+            t.H2 = m->H2;
+            t.dZ1 = m->dH1;
+            t.dZ2 = m->dH2;
+            t.dO = m->dO;
+            t.rl = m->rl;
+            t.n = n;
+            t.batch = batch;
+            t.steps = steps;
+            t.lr = lr;
+            t.b1 = b1;
+            t.b2 = b2;
+            t.eps = eps;
+            rc = launch_train(m, t);
+        } else {
+            for (int st = 0; st < steps; ++st) {
+                const int s0 = st * batch;
+                const int B = s0 + batch <= n ? batch : n - s0;
+                k_take_rows<<<(B + 255) / 256, 256, 0, m->stream>>>(m->Xall, m->yall, dp + s0, B,
+                                                                     m->X, m->y);
+                forward(m, m->p, B, 0);
+                backward(m, B);
+                k_adam<<<(kParams + 255) / 256, 256, 0, m->stream>>>(
+                    m->p, m->g, m->m1, m->m2, kParams, lr, b1, b2, eps, hc[st].x, hc[st].y);
+                m->launches += 2;
+            }
+        }
+        if (!rc && cudaEventRecord(m->epoch_done[sl], m->stream) != cudaSuccess)
             rc = SP_EINTERNAL;
     }
+    if (!rc && fused && epochs > 0) {
+        // the loss of the last minibatch
+        const int last = n - (steps - 1) * batch;
+        k_mean<<<1, 256, 0, m->stream>>>(m->rl, last, m->loss);
+        m->launches++;
+    }
+    if (cudaStreamSynchronize(m->stream) != cudaSuccess)
+        rc = SP_EINTERNAL;
     if (!rc && final_loss &&
         cudaMemcpy(final_loss, m->loss, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = SP_EINTERNAL;
-    cudaStreamSynchronize(m->stream);
-    cudaFreeHost(hx);
-    cudaFreeHost(hy);
     if (cudaGetLastError() != cudaSuccess)
         rc = SP_EINTERNAL;
     return rc;

@@ -91,3 +91,40 @@ def test_training_fits_a_noisy_function():
     # the variance head learns the noise level (std 0.1 -> logvar ~ -4.6)
     assert -6.5 < float(np.median(v)) < -2.5
     assert s.lib.spires_ext_mlp_kernel_launches(s.h) > 0
+
+
+@pytest.mark.parametrize("n,batch", [(1, 1), (37, 64), (300, 16), (300, 17), (600, 257),
+                                     (900, 512)])
+def test_epoch_of_minibatches_matches_oracle(n, batch):
+    """One epoch in one launch: minibatches below, at and above a 16-row tile and
+    a 256-row block, the last one short, against FP64 Adam on the same order.
+    Every step moves a component by at most about lr; a gradient component
+    within FP32 rounding of zero may step the other way."""
+    s = sp.Surrogate(seed=5)
+    p0 = s.params()
+    X, y = data(n, seed=n)
+    s.train(X, y, epochs=1, batch=batch, lr=1e-3, seed=11)
+    # the row order: Fisher-Yates on PCG32, as the library draws it
+    st, M = 11 ^ 0x5DEECE66D, (1 << 64) - 1
+    perm = list(range(n))
+    for i in range(n - 1, 0, -1):
+        old = st
+        st = (old * 6364136223846793005 + 1442695040888963407) & M
+        xs = (((old >> 18) ^ old) >> 27) & 0xFFFFFFFF
+        rot = old >> 59
+        j = (((xs >> rot) | (xs << ((32 - rot) & 31))) & 0xFFFFFFFF) % (i + 1)
+        perm[i], perm[j] = perm[j], perm[i]
+    p = p0.astype(np.float64)
+    m1, m2, t = np.zeros_like(p), np.zeros_like(p), 0
+    b = min(batch, n)
+    for k in range(0, n, b):
+        at = perm[k:k + b]
+        _, g = SO.loss_grad(p, X[at].astype(np.float64), y[at].astype(np.float64))
+        t += 1
+        m1 = 0.9 * m1 + 0.1 * g
+        m2 = 0.999 * m2 + 0.001 * g * g
+        p -= 1e-3 * (m1 / (1 - 0.9 ** t)) / (np.sqrt(m2 / (1 - 0.999 ** t)) + 1e-8)
+    d = np.abs(s.params() - p)
+    assert np.quantile(d, 0.999) <= 1e-5 * max(1, t / 5)
+    assert d.max() <= 1.1e-3 * t
+    assert np.max(np.abs(p - p0)) > 5e-4
