@@ -681,6 +681,203 @@ __global__ void k_diag_init(double *P, int n, double v)
         P[q] = ((q / n) == (q % n)) ? v : 0.0;
 }
 
+// ------------------------------------------------------ fused RLS recursion
+// T steps of the recursion above in one cooperative launch over recorded states
+// X [T][n] (the states do not depend on the readout). CTA c owns a block of rows
+// of P, in shared memory for the launch where it fits, and a step is one pass
+// over them: the rank-one update with the gain of the step before and the
+// product with the new state together. The products travel as the step
+// kernel's spike words do, each double as two 8-byte entries that carry the
+// step's number; every CTA then forms the denominator itself, and output o's
+// weights are kept by CTA o % G while the products of the next step are on
+// their way. Every product and sum is that of the separate kernels in their
+// order, so the bits are theirs. What bounds it: the exchange, about 1 us a
+// step, until P no longer fits the SMs' shared memory (about 1700 neurons)
+// and streams from the L2 or HBM, read and written once a step. (N=800, 400
+// steps: 4.5 us per step beside the 2.4 of the simulation; four launches a step took 47 together.)
+struct RlsArgs {
+    const double *X;           // [T][n] states
+    const double *Y;           // [T][dout] targets
+    double *P;                 // [n][n], or null: in shared memory only
+    double *W;                 // [dout][n]
+    unsigned long long *ll;    // [2][n][2] exchange entries, zero before the launch
+    int *err;
+    size_t T;
+    long long step0;           // steps of earlier launches (error reports)
+    int n, dout, rows;         // rows of P per CTA
+    int resident, first, last; // P in shared memory; first / last launch of the series
+    double p0, lambda;         // initial diagonal of P
+};
+
+constexpr int kRlsThreads = 256;
+
+// the 256-term tree of k_rls_scalars: pairs 128, 64, 32 apart through shared
+// memory, then 16 .. 1 within the first warp; the sum in thread 0's red[0]
+__device__ __forceinline__ double rls_tree(double s, double *red)
+{
+    const int t = threadIdx.x;
+    __syncthreads();  // readers of the last tree's red[] are done
+    red[t] = s;
+    __syncthreads();
+    if (t < 128)
+        red[t] += red[t + 128];
+    __syncthreads();
+    if (t < 64)
+        red[t] += red[t + 64];
+    __syncthreads();
+    if (t < 32) {
+        double v = red[t] + red[t + 32];
+#pragma unroll
+        for (int st = 16; st; st >>= 1)
+            v += __shfl_down_sync(kFull, v, st);
+        if (t == 0)
+            red[0] = v;
+    }
+    __syncthreads();
+    return red[0];
+}
+
+__global__ void __launch_bounds__(kRlsThreads, 1) k_rls(RlsArgs a)
+{
+    extern __shared__ __align__(16) double rls_smem[];
+    const int n = a.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double *s_x = rls_smem;                // [2][n] states of this step and the last
+    double *s_px = s_x + 2 * (size_t)n;    // [2][n] P x of this step and the last
+    double *s_k = s_px + 2 * (size_t)n;    // [n] -denom * gain of the step before
+    double *red = s_k + n;                 // [256]
+    double *s_P = red + kRlsThreads;       // [rows][n]
+    const int r_lo = blockIdx.x * a.rows < n ? blockIdx.x * a.rows : n;
+    const int r_hi = r_lo + a.rows < n ? r_lo + a.rows : n;
+    double *P = a.resident ? s_P : a.P + (size_t)r_lo * n;
+    const double sc = (a.lambda != 1.0) ? 1.0 / a.lambda : 1.0;
+
+    if (a.resident || a.first)
+        for (size_t q = tid; q < (size_t)(r_hi - r_lo) * n; q += kRlsThreads) {
+            const int r = r_lo + (int)(q / n), c = (int)(q % n);
+            P[q] = a.first ? (r == c ? a.p0 : 0.0) : a.P[(size_t)r * n + c];
+        }
+    double denom = 0.0, inv = 0.0;  // of the step before
+    __syncthreads();
+    for (size_t t = 0; t <= a.T; ++t) {
+        double *x = s_x + (t & 1) * (size_t)n, *px = s_px + (t & 1) * (size_t)n;
+        const double *xp = s_x + (~t & 1) * (size_t)n, *pxp = s_px + (~t & 1) * (size_t)n;
+        const bool more = t < a.T;
+        if (!more && a.last && (int)blockIdx.x >= a.dout)
+            break;  // nothing reads P any more, and this CTA keeps no weights
+        for (int i = tid; i < n; i += kRlsThreads) {
+            if (more)
+                x[i] = __ldg(a.X + t * n + i);
+            if (t > 0) {
+                const double kc = inv * pxp[i];
+                s_k[i] = -denom * kc;
+            }
+        }
+        __syncthreads();
+        // rows: a warp each
+        for (int r = r_lo + warp; r < r_hi; r += kRlsThreads / 32) {
+            double *row = P + (size_t)(r - r_lo) * n;
+            double s = 0.0;
+            const double kr = t > 0 ? inv * pxp[r] : 0.0;
+            // eight elements a pass, their loads ahead of the stores
+            for (int c = lane; c < n; c += 256) {
+                double v[8], g[8], y[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const bool in = c + 32 * u < n;
+                    v[u] = in ? row[c + 32 * u] : 0.0;
+                    g[u] = in && t > 0 ? s_k[c + 32 * u] : 0.0;
+                    y[u] = in && more ? x[c + 32 * u] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (c + 32 * u >= n)
+                        break;
+                    if (t > 0) {
+                        v[u] = v[u] + kr * g[u];
+                        v[u] = (a.lambda != 1.0) ? sc * v[u] : v[u];
+                        row[c + 32 * u] = v[u];
+                    }
+                    s = fma(v[u], y[u], s);
+                }
+            }
+            if (!more)
+                continue;
+            for (int off = 16; off; off >>= 1)
+                s += __shfl_xor_sync(kFull, s, off);
+            if (lane < 2) {
+                const unsigned long long bits = (unsigned long long)__double_as_longlong(s);
+                const unsigned half = lane ? (unsigned)(bits >> 32) : (unsigned)bits;
+                *(volatile unsigned long long *)(a.ll + ((t & 1) * (size_t)n + r) * 2 + lane) =
+                    ((unsigned long long)(unsigned)(t + 1) << 32) | half;
+            }
+        }
+        // output weights of the step before
+        if (t > 0)
+            for (int o = blockIdx.x; o < a.dout; o += gridDim.x) {
+                double *w = a.W + (size_t)o * n;
+                double d = 0.0;
+                for (int i = tid; i < n; i += kRlsThreads)
+                    d = fma(w[i], xp[i], d);
+                const double e = __ldg(a.Y + (t - 1) * a.dout + o) - rls_tree(d, red);
+                for (int i = tid; i < n; i += kRlsThreads)
+                    w[i] += (inv * pxp[i]) * e;
+            }
+        if (!more)
+            break;
+        // all products of this step
+        bool ok = true;
+        const unsigned want = (unsigned)(t + 1);
+        const unsigned long long *src = a.ll + (t & 1) * (size_t)n * 2;
+        unsigned long long t0 = 0, polls = 0;
+        for (int base = tid; base < n && ok; base += 4 * kRlsThreads) {
+            unsigned pend = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (base + u * kRlsThreads < n)
+                    pend |= 1u << u;
+            while (pend) {
+                unsigned long long v[4][2];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if ((pend >> u) & 1u) {
+                        const unsigned long long *e = src + 2 * (size_t)(base + u * kRlsThreads);
+                        v[u][0] = ld_volatile_u64(e);
+                        v[u][1] = ld_volatile_u64(e + 1);
+                    }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (((pend >> u) & 1u) && (unsigned)(v[u][0] >> 32) == want &&
+                        (unsigned)(v[u][1] >> 32) == want) {
+                        px[base + u * kRlsThreads] = __longlong_as_double(
+                            (long long)((v[u][1] << 32) | (v[u][0] & 0xffffffffull)));
+                        pend &= ~(1u << u);
+                    }
+                if (pend && (++polls & 63ull) == 0) {
+                    const unsigned long long now = globaltimer_ns();
+                    if (t0 == 0)
+                        t0 = now;
+                    if (ld_volatile_i32(a.err) != kErrNone || now - t0 > kBarrierTimeoutNs) {
+                        if (atomicCAS(a.err, kErrNone, kErrBarrierTimeout) == kErrNone)
+                            a.err[1] = (int)(a.step0 + (long long)t);
+                        ok = false;
+                        break;
+                    }
+                }
+            }
+        }
+        if (__syncthreads_or(!ok))
+            return;
+        double s = 0.0;
+        for (int i = tid; i < n; i += kRlsThreads)
+            s = fma(x[i], px[i], s);
+        denom = a.lambda + rls_tree(s, red);
+        inv = 1.0 / denom;
+    }
+    if (a.resident && !a.last)
+        for (size_t q = tid; q < (size_t)(r_hi - r_lo) * n; q += kRlsThreads)
+            a.P[(size_t)r_lo * n + q] = P[q];
+}
+
 // online delta rule: W_out[o][i] += (lr * (target_o - y_o)) * x_i
 __global__ void k_online(double *W_out, int n, int dout, const double *x, const double *y,
                          const double *target, double lr)
@@ -1430,6 +1627,28 @@ out:
     return rc;
 }
 
+// Launch shape of k_rls for n positions: CTAs, rows of P per CTA, whether P is
+// kept in shared memory. Returns the shared memory, or 0 when the state vectors
+// do not fit (about 5700 positions; the separate kernels then take each step:
+// P is 260 MB and more, and its passes over HBM outweigh the launches).
+static size_t rls_shape(const sp_dev *d, int n, int *ctas, int *rows, int *resident)
+{
+    if (!d->coop)
+        return 0;
+    const size_t room = (size_t)d->smem_max - 1024;
+    const size_t base = (5 * (size_t)n + kRlsThreads) * sizeof(double);
+    if (base > room)
+        return 0;
+    // a row per warp while the SMs last
+    int G = (n + kRlsThreads / 32 - 1) / (kRlsThreads / 32);
+    G = G < d->num_sms ? G : d->num_sms;
+    *rows = (n + G - 1) / G;
+    *ctas = (n + *rows - 1) / *rows;
+    const size_t full = base + (size_t)*rows * n * sizeof(double);
+    *resident = full <= room;
+    return *resident ? full : base;
+}
+
 extern "C" int sp_dev_train_rls(sp_dev *d, const sp_host_model *m, const double *h_u,
                                 const double *h_y, size_t T, double delta, double lambda,
                                 double *h_W_out)
@@ -1439,19 +1658,66 @@ extern "C" int sp_dev_train_rls(sp_dev *d, const sp_host_model *m, const double 
     const int rs = d->rs, n = d->n, dout = d->dout;
     cudaStream_t s = d->stream;
     double *P = nullptr, *Px = nullptr, *scal = nullptr, *Yd = nullptr, *Wn = nullptr;
-    RK(sp_cuda_malloc(&P, (size_t)rs * rs * sizeof(double)));
-    RK(sp_cuda_malloc(&Px, (size_t)rs * sizeof(double)));
-    RK(sp_cuda_malloc(&scal, (size_t)(dout + 1) * sizeof(double)));
+    unsigned long long *ll = nullptr;
+    int ctas = 0, rows = 0, resident = 0;
+    const size_t smem = rls_shape(d, rs, &ctas, &rows, &resident);
     RK(sp_cuda_malloc(&Yd, (T ? T : 1) * (size_t)(dout ? dout : 1) * sizeof(double)));
     RK(sp_cuda_malloc(&Wn, (size_t)(dout ? dout : 1) * n * sizeof(double)));
-    k_diag_init<<<1024, 256, 0, s>>>(P, rs, 1.0 / delta);
+    if (!smem || !resident || T > d->chunk)
+        RK(sp_cuda_malloc(&P, (size_t)rs * rs * sizeof(double)));
+    if (smem) {
+        RK(sp_cuda_malloc(&ll, 4 * (size_t)rs * sizeof(unsigned long long)));
+        RK(set_max_dynamic_smem((const void *)k_rls));
+    } else {
+        RK(sp_cuda_malloc(&Px, (size_t)rs * sizeof(double)));
+        RK(sp_cuda_malloc(&scal, (size_t)(dout + 1) * sizeof(double)));
+        k_diag_init<<<1024, 256, 0, s>>>(P, rs, 1.0 / delta);
+    }
     RK(cudaMemsetAsync(d->W_out, 0, (size_t)rs * dout * sizeof(double), s));
     if (T && dout)
         RK(cudaMemcpyAsync(Yd, h_y, T * dout * sizeof(double), cudaMemcpyHostToDevice, s));
     rc = sp_dev_reset_neurons(d, m);
     if (rc)
         goto out;
-    for (size_t t = 0; t < T; ++t) {
+    for (size_t t = 0; smem && t < T;) {
+        // states of up to a chunk of steps in one launch, then the recursion over
+        // them; the staging is the next chunk's once the stream has passed
+        const size_t tc = T - t < d->chunk ? T - t : d->chunk;
+        const double *u = nullptr;
+        if (t)
+            RK(cudaStreamSynchronize(s));
+        if (h_u && d->din > 0) {
+            RK(cudaMemcpyAsync(d->d_u, h_u + t * d->din, tc * d->din * sizeof(double),
+                               cudaMemcpyHostToDevice, s));
+            u = d->d_u;
+        }
+        rc = sp_dev_launch_chunk(d, u, tc, d->d_phi, nullptr);
+        if (rc)
+            goto out;
+        RK(cudaMemsetAsync(ll, 0, 4 * (size_t)rs * sizeof(unsigned long long), s));
+        RlsArgs a;
+        a.X = d->d_phi;
+        a.Y = Yd + t * dout;
+        a.P = P;
+        a.W = d->W_out;
+        a.ll = ll;
+        a.err = d->err;
+        a.T = tc;
+        a.step0 = (long long)t;
+        a.n = rs;
+        a.dout = dout;
+        a.rows = rows;
+        a.resident = resident;
+        a.first = t == 0;
+        a.last = t + tc == T;
+        a.p0 = 1.0 / delta;
+        a.lambda = lambda;
+        void *args[] = {&a};
+        RK(cudaLaunchCooperativeKernel((const void *)k_rls, dim3(ctas), dim3(kRlsThreads), args,
+                                       smem, s));
+        t += tc;
+    }
+    for (size_t t = 0; !smem && t < T; ++t) {
         sp_run_args a;
         memset(&a, 0, sizeof(a));
         a.u = h_u ? h_u + t * d->din : nullptr;
@@ -1469,7 +1735,9 @@ extern "C" int sp_dev_train_rls(sp_dev *d, const sp_host_model *m, const double 
         goto out;
     RK(cudaMemcpyAsync(h_W_out, Wn, (size_t)n * dout * sizeof(double), cudaMemcpyDeviceToHost,
                        s));
-    RK(cudaStreamSynchronize(s));
+    rc = sp_dev_sync(d);
+    if (rc)
+        goto out;
     RK(cudaGetLastError());
 out:
     cudaStreamSynchronize(s);
@@ -1478,6 +1746,7 @@ out:
     if (scal) sp_cuda_free(scal);
     if (Yd) sp_cuda_free(Yd);
     if (Wn) sp_cuda_free(Wn);
+    if (ll) sp_cuda_free(ll);
     return rc;
 }
 

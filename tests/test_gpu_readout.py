@@ -253,3 +253,27 @@ def test_ridge_more_than_sixteen_outputs():
     assert rel(W, Wo) < 1e-9
     W2, _ = sp.ridge_fit(phi, y, 1e-2)
     assert rel(W2, Wo) < 1e-9
+
+
+@pytest.mark.parametrize("n,T,dout,neuron", [(1, 5, 1, sp.LIF_DISCRETE), (33, 40, 3, sp.FLIF_GL),
+                                             (300, 50, 17, sp.FLIF_GL), (1300, 24, 2, sp.LIF_DISCRETE),
+                                             (1900, 10, 1, sp.LIF_DISCRETE)])
+@pytest.mark.parametrize("lam", [1.0, 0.99])
+def test_rls_in_one_launch_matches_oracle(n, T, dout, neuron, lam):
+    """The fused recursion from one row of P to several rows per warp, with P in
+    shared memory (up to 1300 here) and streamed from memory (1900), more
+    outputs than CTAs or one. Tolerance as in test_rls_matches_oracle."""
+    params = GL if neuron == sp.FLIF_GL else O.NEURON_PARAMS[neuron]
+    cfg = sp.make_config(n, 2, dout, rho=1.2, ei=0.55, gamma=1.2, conn=min(0.5, 6.0 / max(n, 2)),
+                         topo=sp.CONN_SMALL_WORLD, neuron=neuron, nparams=params)
+    u, y = data(T, 2, dout, seed=7)
+    r = sp.Reservoir(cfg, seed=12)
+    r.train_rls(u, y, 1.0, lam)
+    W = r.readout()
+    v = r.state()
+    r.close()
+    orc = O.Oracle(cfg, sp.HostModel(cfg, seed=12))
+    Wo = orc.train_rls(u, y, 1.0, lam)
+    assert rel(W, Wo) < 1e-8
+    phi, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=12)).run(u)
+    assert np.array_equal(v, phi[-1])  # the reservoir is left after the last step
