@@ -19,6 +19,7 @@
 #include <cstdio>
 #include <cmath>
 #include <algorithm>
+#include <atomic>
 #include <numeric>
 #include <vector>
 #include "sp_alloc.h"
@@ -259,6 +260,32 @@ static int dupload(T **p, const T *h, size_t count, cudaStream_t s)
 // up to three places beyond either end).
 static size_t coef_pad(int ntype) { return ntype == SP_FLIF_CAPUTO ? 4 : 0; }
 
+// Several arrays in one allocation and one copy: add() their sizes, fill `host`
+// (sized by the caller) at the returned offsets, upload().
+namespace {
+struct Packed {
+    size_t bytes = 0;
+    std::vector<char> host;
+    size_t add(size_t b)
+    {
+        const size_t at = bytes;
+        bytes += (b + 255) / 256 * 256;
+        return at;
+    }
+    int upload(char **dev, cudaStream_t s)
+    {
+        if (bytes == 0)
+            add(1), host.assign(bytes, 0);
+        int rc = dalloc(dev, bytes);
+        // from pageable memory the copy returns once the bytes are staged
+        if (!rc && cudaMemcpyAsync(*dev, host.data(), bytes, cudaMemcpyHostToDevice, s) !=
+                       cudaSuccess)
+            rc = SP_EINTERNAL;
+        return rc;
+    }
+};
+}  // namespace
+
 static int upload_consts(sp_dev *d, const sp_host_model *m)
 {
     d->nc = m->nc;
@@ -476,7 +503,7 @@ static int kernel_variant(const sp_dev *d, const sp_launch &l)
 
 // Largest cluster (16, 8 or none) that the device schedules with the cluster
 // kernel's largest block and shared memory.
-static int max_cluster(int smem_max)
+static int query_cluster(int smem_max)
 {
     const void *fn = (const void *)k_run<SP_LIF_DISCRETE, SP_SYN_SIMPLE, 3>;
     if (set_max_dynamic_smem(fn) != cudaSuccess ||
@@ -503,6 +530,20 @@ static int max_cluster(int smem_max)
         cudaGetLastError();
     }
     return 0;
+}
+
+// A property of the device, asked once for each.
+static int max_cluster(int device, int smem_max)
+{
+    static std::atomic<int> known[64];  // cluster size + 1
+    if (device < 0 || device >= 64)
+        return query_cluster(smem_max);
+    int v = known[device].load();
+    if (v == 0) {
+        v = query_cluster(smem_max) + 1;
+        known[device].store(v);
+    }
+    return v - 1;
 }
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
@@ -726,7 +767,7 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
         cudaDeviceGetAttribute(&d->smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device);
         if (d->smem_max <= 0)
             d->smem_max = 48 * 1024;
-        d->cluster_max = max_cluster(d->smem_max);
+        d->cluster_max = max_cluster(d->device, d->smem_max);
         int coop = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d->device);
         d->coop = coop;
@@ -822,21 +863,27 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
         TRY(dalloc(&d->spk, 2 * d->nwords));
         TRY(dalloc(&d->bar, 4));
         d->flag_cap = 8 * (d->num_sms > 0 ? d->num_sms : 1);
-        TRY(dalloc(&d->flags, (size_t)d->flag_cap * kFlagStride));
+        // arrival flags, then the spike exchange entries
+        TRY(dalloc(&d->flags, (size_t)d->flag_cap * kFlagStride + 2 * d->nwords));
+        d->ll = d->flags + (size_t)d->flag_cap * kFlagStride;
         TRY(dalloc(&d->err, 4));
-        TRY(dalloc(&d->ll, 2 * d->nwords));
         SP_CK(cudaMemsetAsync(d->ll, 0, 2 * d->nwords * sizeof(unsigned long long), s));
         if (dense_rows(m)) {
             // blocks (row word q, neuron j); a row's edges are in ascending
             // neuron order, so filling row by row leaves each block's weights in
             // row order
-            std::vector<uint2> blk((size_t)d->nw * n, make_uint2(0u, 0u));
-            std::vector<double> cw(m->nnz);
+            Packed pk;
+            const size_t o_blk = pk.add((size_t)d->nw * n * sizeof(uint2)),
+                         o_w = pk.add(m->nnz * sizeof(double)),
+                         o_off = pk.add((d->nwords + 1) * sizeof(int));
+            pk.host.assign(pk.bytes, 0);
+            uint2 *blk = (uint2 *)(pk.host.data() + o_blk);
+            double *cw = (double *)(pk.host.data() + o_w);
             int *off = d->h_col_off = (int *)calloc(d->nw + 1, sizeof(int));
             if (!off)
                 TRY(SP_EALLOC);
             for (int q = 0; q < d->nw; ++q) {
-                uint2 *bq = blk.data() + (size_t)q * n;
+                uint2 *bq = blk + (size_t)q * n;
                 off[q] = (int)rp[32 * q];
                 for (int ln = 0; ln < 32; ++ln) {
                     const int i = nid_of[32 * q + ln];
@@ -860,10 +907,11 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
                 }
             }
             off[d->nw] = (int)m->nnz;
-            TRY(dupload(&d->col_blk, blk.data(), blk.size(), s));
-            TRY(dupload(&d->col_off, off, d->nwords + 1, s));
-            TRY(dupload(&d->col_w, cw.data(), cw.size(), s));
-            SP_CK(cudaStreamSynchronize(s));  // the vectors go out of scope
+            memcpy(pk.host.data() + o_off, off, (d->nwords + 1) * sizeof(int));
+            TRY(pk.upload(&d->rows_buf, s));
+            d->col_blk = (uint2 *)(d->rows_buf + o_blk);
+            d->col_w = (double *)(d->rows_buf + o_w);
+            d->col_off = (int *)(d->rows_buf + o_off);
         } else if (m->syn_type == SP_SYN_SIMPLE && rs <= 65536) {
             int *eo = d->h_ell_off = (int *)calloc(d->nw + 1, sizeof(int));
             int *to = d->h_tail_off = (int *)calloc(d->nw + 1, sizeof(int));
@@ -875,9 +923,16 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
                 eo[q + 1] = eo[q] + g;
                 cells += (size_t)128 * g;
             }
-            std::vector<unsigned short> ec(cells ? cells : 1, 0);
-            std::vector<double> ew(cells ? cells : 1, 0.0), tw(m->nnz ? m->nnz : 1);
-            std::vector<int> trp((size_t)33 * d->nw, 0), tc(m->nnz ? m->nnz : 1);
+            const size_t nnz = m->nnz;
+            Packed pk;
+            const size_t o_c = pk.add(cells * 2), o_w = pk.add(cells * 8), o_tc = pk.add(nnz * 4),
+                         o_tw = pk.add(nnz * 8), o_rp = pk.add((size_t)33 * d->nw * 4),
+                         o_off = pk.add((d->nwords + 1) * 4);
+            pk.host.assign(pk.bytes, 0);
+            char *hb = pk.host.data();
+            unsigned short *ec = (unsigned short *)(hb + o_c);
+            double *ew = (double *)(hb + o_w), *tw = (double *)(hb + o_tw);
+            int *trp = (int *)(hb + o_rp), *tc = (int *)(hb + o_tc);
             int nt = 0;
             for (int q = 0; q < d->nw; ++q) {
                 const int slots = 4 * (eo[q + 1] - eo[q]);
@@ -899,13 +954,14 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
                 trp[(size_t)33 * q + 32] = nt;
                 to[q + 1] = nt;
             }
-            TRY(dupload(&d->ell_off, eo, d->nwords + 1, s));
-            TRY(dupload((unsigned short **)&d->ell_col, ec.data(), ec.size(), s));
-            TRY(dupload(&d->ell_w, ew.data(), ew.size(), s));
-            TRY(dupload(&d->tail_rp, trp.data(), trp.size(), s));
-            TRY(dupload(&d->tail_col, tc.data(), (size_t)nt, s));
-            TRY(dupload(&d->tail_w, tw.data(), (size_t)nt, s));
-            SP_CK(cudaStreamSynchronize(s));  // the vectors go out of scope
+            memcpy(hb + o_off, eo, (d->nwords + 1) * 4);
+            TRY(pk.upload(&d->rows_buf, s));
+            d->ell_col = (uint2 *)(d->rows_buf + o_c);
+            d->ell_w = (double *)(d->rows_buf + o_w);
+            d->tail_col = (int *)(d->rows_buf + o_tc);
+            d->tail_w = (double *)(d->rows_buf + o_tw);
+            d->tail_rp = (int *)(d->rows_buf + o_rp);
+            d->ell_off = (int *)(d->rows_buf + o_off);
         }
         TRY(dupload(&d->row_ptr, rp.data(), rs + 1, s));
         TRY(dupload(&d->col, col.data(), m->nnz, s));
@@ -1013,8 +1069,7 @@ extern "C" void sp_dev_destroy(sp_dev *d)
                     d->edge_omd, d->edge_trace, d->scoef, d->Iring, d->mx_decay, d->mx_omd,
                     d->mx_c, d->mx_tr, d->W_in, d->W_out, d->d_u, d->d_phi, d->d_nat, d->d_y,
                     d->d_spkd, d->d_ras, d->d_ras_nat, d->bar, d->err, d->pos_of, d->nid_of,
-                    d->flags, d->ll, d->col_off, d->col_blk, d->col_w, d->ell_off, d->ell_col,
-                    d->ell_w, d->tail_rp, d->tail_col, d->tail_w};
+                    d->flags, d->rows_buf};
     for (void *b : bufs)
         if (b)
             sp_cuda_free(b);

@@ -71,6 +71,7 @@ struct sp_dev {
     int flag_cap;
     unsigned long long *ll;    // spike exchange entries of the step kernel [2][nw]
     unsigned ll_seq;           // numbers used by the launches so far
+    char *rows_buf;  // the arrays below, one allocation
     // SIMPLE synapse, column blocks of a dense matrix (null: not built):
     // [nw][n] {row bits, weight offset}, first weight of each row word, weights
     uint2 *col_blk;
