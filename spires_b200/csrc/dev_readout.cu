@@ -22,6 +22,7 @@
 #include "sp_kernels.cuh"
 #include "sp_dev_internal.h"
 #include "sp_gram.h"
+#include "sp_solve.h"
 
 using namespace sp;
 
@@ -36,61 +37,6 @@ using namespace sp;
     } while (0)
 
 namespace {
-
-constexpr int NB = 64;  // Cholesky panel width
-
-// ---------------------------------------------------------------- Gram (FP64)
-// C = X^T X over rows [t0, t1) of X (T x n, row-major); lower tiles computed,
-// the upper triangle mirrored. 64x64 tile per CTA, 4x4 per thread.
-__global__ void __launch_bounds__(256) k_syrk_f64(const double *__restrict__ X, int n, size_t t0,
-                                                  size_t t1, double *__restrict__ C, int ldc)
-{
-    // tile index -> (bi, bj) with bi >= bj
-    int b = blockIdx.x;
-    int bi = (int)((sqrt(8.0 * b + 1.0) - 1.0) * 0.5);
-    while ((bi + 1) * (bi + 2) / 2 <= b) ++bi;
-    while (bi * (bi + 1) / 2 > b) --bi;
-    int bj = b - bi * (bi + 1) / 2;
-    const int i0 = bi * 64, j0 = bj * 64;
-    __shared__ double si[16][64 + 1];
-    __shared__ double sj[16][64 + 1];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4] = {};
-    for (size_t t = t0; t < t1; t += 16) {
-        for (int q = threadIdx.x; q < 16 * 64; q += 256) {
-            int r = q >> 6, c = q & 63;
-            size_t tt = t + r;
-            si[r][c] = (tt < t1 && i0 + c < n) ? X[tt * n + i0 + c] : 0.0;
-            sj[r][c] = (tt < t1 && j0 + c < n) ? X[tt * n + j0 + c] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            double a[4], bb[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                a[u] = si[r][ty * 4 + u];
-                bb[u] = sj[r][tx * 4 + u];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    acc[u][v] = fma(a[u], bb[v], acc[u][v]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            int i = i0 + ty * 4 + u, j = j0 + tx * 4 + v;
-            if (i < n && j < n && j <= i) {
-                C[(size_t)i * ldc + j] = acc[u][v];
-                C[(size_t)j * ldc + i] = acc[u][v];
-            }
-        }
-}
 
 // R[i][o] = sum_{t in [t0,t1)} X[t][i] E[t][o] (- lam * W[i][o] when W != 0),
 // split over `parts` contiguous t ranges reduced in a fixed order.
@@ -182,298 +128,6 @@ __global__ void k_add_diag(double *A, int n, int lda, double lam)
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
         A[(size_t)i * lda + i] += lam;
-}
-
-// ------------------------------------------------------- blocked Cholesky
-// A (n x n, row-major, lower triangle used) -> L in place.
-// Diagonal block of panel [k0, k0 + kb), one CTA of 256 threads: thread t
-// owns row t % 64 and the 16 columns t / 64 + 4 m of the trailing update.
-// For column j every thread derives the factor itself from the current
-// values (d = sqrt(a_jj), l_rj = a_rj / d as a_rj * (1 / d)) and updates its
-// entries right of column j; the scaled column is written after the one
-// barrier of the column, when nobody reads it any more.
-__global__ void __launch_bounds__(256) k_potrf_diag(double *A, int n, int lda, int k0, int kb,
-                                                    int *info)
-{
-    __shared__ double s[NB][NB + 1];
-    __shared__ int bad;
-    if (*info)
-        return;
-    for (int q = threadIdx.x; q < kb * kb; q += blockDim.x) {
-        const int r = q / kb, c = q % kb;
-        if (c <= r)
-            s[r][c] = A[(size_t)(k0 + r) * lda + k0 + c];
-    }
-    if (threadIdx.x == 0)
-        bad = 0;
-    __syncthreads();
-    const int r = threadIdx.x & (NB - 1), c0 = threadIdx.x >> 6;
-    for (int j = 0; j < kb; ++j) {
-        const double a = s[j][j];
-        const bool okd = a > 0.0 && isfinite(a);
-        const double d = okd ? sqrt(a) : 1.0;
-        const double inv = 1.0 / d;
-        double lrj = 0.0;
-        if (r > j && r < kb) {
-            lrj = s[r][j] * inv;
-#pragma unroll
-            for (int m = 0; m < NB / 4; ++m) {
-                const int c = c0 + 4 * m;
-                if (c > j && c <= r)
-                    s[r][c] = fma(-lrj, s[c][j] * inv, s[r][c]);
-            }
-        }
-        __syncthreads();  // every read of column j is done
-        if (c0 == 0 && r > j && r < kb)
-            s[r][j] = lrj;
-        if (threadIdx.x == 0) {
-            s[j][j] = d;
-            if (!okd && !bad)
-                bad = k0 + j + 1;
-        }
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < kb * kb; q += blockDim.x) {
-        const int rr = q / kb, cc = q % kb;
-        if (cc <= rr)
-            A[(size_t)(k0 + rr) * lda + k0 + cc] = s[rr][cc];
-    }
-    if (threadIdx.x == 0 && bad)
-        atomicCAS(info, 0, bad);
-}
-
-// Rows r >= k0 + kb: L[r][k0:k0+kb] = A[r][k0:k0+kb] L_kk^-T. A warp solves 4
-// rows side by side (independent chains), lane l holding columns l and l + 32
-// of each; columns are eliminated in order (x_c = a_c * (1 / L_cc), then
-// a_q -= x_c L_qc for q > c). 32 rows per CTA.
-__global__ void __launch_bounds__(256) k_trsm_panel(double *A, int n, int lda, int k0, int kb,
-                                                    const int *info)
-{
-    __shared__ double sL[NB][NB + 1];
-    __shared__ double sInv[NB];
-    if (*info)
-        return;
-    for (int q = threadIdx.x; q < kb * kb; q += blockDim.x) {
-        const int r = q / kb, c = q % kb;
-        sL[r][c] = (c <= r) ? A[(size_t)(k0 + r) * lda + k0 + c] : 0.0;
-    }
-    __syncthreads();
-    if (threadIdx.x < kb)
-        sInv[threadIdx.x] = 1.0 / sL[threadIdx.x][threadIdx.x];
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = k0 + kb + blockIdx.x * 32 + warp * 4;
-    if (r0 >= n)
-        return;
-    double a0[4], a1[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const bool ok = r0 + q < n;
-        const double *row = A + (size_t)(r0 + q) * lda + k0;
-        a0[q] = ok && lane < kb ? row[lane] : 0.0;
-        a1[q] = ok && lane + 32 < kb ? row[lane + 32] : 0.0;
-    }
-    for (int c = 0; c < kb; ++c) {
-        const double ic = sInv[c];
-        const double l0 = (lane > c && lane < kb) ? sL[lane][c] : 0.0;
-        const double l1 = (lane + 32 > c && lane + 32 < kb) ? sL[lane + 32][c] : 0.0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const double xc = __shfl_sync(kFull, c < 32 ? a0[q] : a1[q], c & 31) * ic;
-            if (lane == (c & 31)) {
-                if (c < 32)
-                    a0[q] = xc;
-                else
-                    a1[q] = xc;
-            }
-            if (lane > c && lane < kb)
-                a0[q] = fma(-xc, l0, a0[q]);
-            if (lane + 32 > c && lane + 32 < kb)
-                a1[q] = fma(-xc, l1, a1[q]);
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        if (r0 + q >= n)
-            break;
-        double *row = A + (size_t)(r0 + q) * lda + k0;
-        if (lane < kb)
-            row[lane] = a0[q];
-        if (lane + 32 < kb)
-            row[lane + 32] = a1[q];
-    }
-}
-
-// trailing update A22 -= L21 L21^T on lower tiles of the trailing matrix
-__global__ void __launch_bounds__(256) k_syrk_update(double *A, int n, int lda, int k0, int kb,
-                                                     const int *info)
-{
-    if (*info)
-        return;
-    const int base = k0 + kb;
-    int b = blockIdx.x;
-    int bi = (int)((sqrt(8.0 * b + 1.0) - 1.0) * 0.5);
-    while ((bi + 1) * (bi + 2) / 2 <= b) ++bi;
-    while (bi * (bi + 1) / 2 > b) --bi;
-    int bj = b - bi * (bi + 1) / 2;
-    const int i0 = base + bi * 64, j0 = base + bj * 64;
-    __shared__ double si[64][33];
-    __shared__ double sj[64][33];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4] = {};
-    for (int c0 = 0; c0 < kb; c0 += 32) {
-        const int cw = (kb - c0 < 32) ? kb - c0 : 32;
-        for (int q = threadIdx.x; q < 64 * 32; q += 256) {
-            int r = q >> 5, c = q & 31;
-            si[r][c] = (c < cw && i0 + r < n) ? A[(size_t)(i0 + r) * lda + k0 + c0 + c] : 0.0;
-            sj[r][c] = (c < cw && j0 + r < n) ? A[(size_t)(j0 + r) * lda + k0 + c0 + c] : 0.0;
-        }
-        __syncthreads();
-        for (int c = 0; c < cw; ++c) {
-            double a[4], bb[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                a[u] = si[ty * 4 + u][c];
-                bb[u] = sj[tx * 4 + u][c];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    acc[u][v] = fma(a[u], bb[v], acc[u][v]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            int i = i0 + ty * 4 + u, j = j0 + tx * 4 + v;
-            if (i < n && j < n && j <= i)
-                A[(size_t)i * lda + j] -= acc[u][v];
-        }
-}
-
-// ----------------------------------------------------- triangular solves
-// Forward L Z = B in place on Z (n x dout), panel by panel: the diagonal
-// block by one CTA (warp w takes outputs w, w + 8, ...; lane l holds rows l
-// and l + 32; columns eliminated in order, dividing by the diagonal as a
-// product with its reciprocal), then the rows below it.
-__global__ void __launch_bounds__(256) k_fwd_diag(const double *L, int lda, int k0, int kb,
-                                                  double *Z, int dout)
-{
-    __shared__ double sL[NB][NB + 1];
-    __shared__ double sInv[NB];
-    for (int q = threadIdx.x; q < kb * kb; q += blockDim.x) {
-        const int r = q / kb, c = q % kb;
-        sL[r][c] = (c <= r) ? L[(size_t)(k0 + r) * lda + k0 + c] : 0.0;
-    }
-    __syncthreads();
-    if (threadIdx.x < kb)
-        sInv[threadIdx.x] = 1.0 / sL[threadIdx.x][threadIdx.x];
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int o = warp; o < dout; o += 8) {
-        double z0 = lane < kb ? Z[(size_t)(k0 + lane) * dout + o] : 0.0;
-        double z1 = lane + 32 < kb ? Z[(size_t)(k0 + lane + 32) * dout + o] : 0.0;
-        for (int j = 0; j < kb; ++j) {
-            const double zj = __shfl_sync(kFull, j < 32 ? z0 : z1, j & 31) * sInv[j];
-            if (lane == (j & 31)) {
-                if (j < 32)
-                    z0 = zj;
-                else
-                    z1 = zj;
-            }
-            if (lane > j && lane < kb)
-                z0 = fma(-zj, sL[lane][j], z0);
-            if (lane + 32 > j && lane + 32 < kb)
-                z1 = fma(-zj, sL[lane + 32][j], z1);
-        }
-        if (lane < kb)
-            Z[(size_t)(k0 + lane) * dout + o] = z0;
-        if (lane + 32 < kb)
-            Z[(size_t)(k0 + lane + 32) * dout + o] = z1;
-    }
-}
-
-// Rows r >= k0 + kb: Z[r] -= L[r][k0:k0+kb] Z[k0:k0+kb]; one warp per row.
-__global__ void __launch_bounds__(256) k_fwd_update(const double *L, int n, int lda, int k0,
-                                                    int kb, double *Z, int dout)
-{
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = k0 + kb + blockIdx.x * 8 + warp;
-    if (r >= n)
-        return;
-    const double *Lr = L + (size_t)r * lda + k0;
-    const double l0 = lane < kb ? Lr[lane] : 0.0;
-    const double l1 = lane + 32 < kb ? Lr[lane + 32] : 0.0;
-    for (int o = 0; o < dout; ++o) {
-        double v = 0.0;
-        if (lane < kb)
-            v = l0 * Z[(size_t)(k0 + lane) * dout + o];
-        if (lane + 32 < kb)
-            v = fma(l1, Z[(size_t)(k0 + lane + 32) * dout + o], v);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-            v += __shfl_xor_sync(kFull, v, off);
-        if (lane == 0)
-            Z[(size_t)r * dout + o] -= v;
-    }
-}
-
-// Backward L^T X = Z, panels from the last one: the diagonal block (rows
-// eliminated from the last, x_j = z_j / L_jj, z_r -= L_jr x_j for r < j).
-__global__ void __launch_bounds__(256) k_bwd_diag(const double *L, int lda, int k0, int kb,
-                                                  double *Z, int dout)
-{
-    __shared__ double sL[NB][NB + 1];
-    __shared__ double sInv[NB];
-    for (int q = threadIdx.x; q < kb * kb; q += blockDim.x) {
-        const int r = q / kb, c = q % kb;
-        sL[r][c] = (c <= r) ? L[(size_t)(k0 + r) * lda + k0 + c] : 0.0;
-    }
-    __syncthreads();
-    if (threadIdx.x < kb)
-        sInv[threadIdx.x] = 1.0 / sL[threadIdx.x][threadIdx.x];
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int o = warp; o < dout; o += 8) {
-        double z0 = lane < kb ? Z[(size_t)(k0 + lane) * dout + o] : 0.0;
-        double z1 = lane + 32 < kb ? Z[(size_t)(k0 + lane + 32) * dout + o] : 0.0;
-        for (int j = kb - 1; j >= 0; --j) {
-            const double xj = __shfl_sync(kFull, j < 32 ? z0 : z1, j & 31) * sInv[j];
-            if (lane == (j & 31)) {
-                if (j < 32)
-                    z0 = xj;
-                else
-                    z1 = xj;
-            }
-            if (lane < j)
-                z0 = fma(-xj, sL[j][lane], z0);
-            if (lane + 32 < j)
-                z1 = fma(-xj, sL[j][lane + 32], z1);
-        }
-        if (lane < kb)
-            Z[(size_t)(k0 + lane) * dout + o] = z0;
-        if (lane + 32 < kb)
-            Z[(size_t)(k0 + lane + 32) * dout + o] = z1;
-    }
-}
-
-// Rows i < k0: Z[i] -= L[k0:k0+kb][i]^T X[k0:k0+kb]; one thread per row
-// (coalesced along the rows of L).
-__global__ void __launch_bounds__(256) k_bwd_update(const double *L, int lda, int k0, int kb,
-                                                    double *Z, int dout)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;  // rows i < k0
-    if (i >= k0)
-        return;
-    for (int o = 0; o < dout; ++o) {
-        double v = 0.0;
-        for (int c = 0; c < kb; ++c)
-            v = fma(L[(size_t)(k0 + c) * lda + i], Z[(size_t)(k0 + c) * dout + o], v);
-        Z[(size_t)i * dout + o] -= v;
-    }
 }
 
 // ------------------------------------------------ LU with partial pivoting
@@ -932,11 +586,12 @@ static __global__ void k_col_update(double *__restrict__ Y, const double *__rest
 }
 
 // largest diagonal entry (non-negative doubles compare like their bits)
-static __global__ void k_diag_max(const double *__restrict__ A, int n, unsigned long long *out)
+static __global__ void k_diag_max(const double *__restrict__ A, int n, int lda,
+                                  unsigned long long *out)
 {
     double m = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double v = A[(size_t)i * n + i];
+        const double v = A[(size_t)i * lda + i];
         if (v > m)
             m = v;
     }
@@ -950,58 +605,36 @@ static __global__ void k_diag_max(const double *__restrict__ A, int n, unsigned 
 }
 
 // ------------------------------------------------------------ factor + solve
-// Factor A (n x n) in place; returns 0 or the 1-based failing pivot.
-static int cholesky_inplace(cudaStream_t s, double *A, int n, int *d_info)
+// Factor A (pitch sp_solve_pad(n)) in place and wait; *bad = 0 or the 1-based
+// failing pivot.
+static int cholesky(cudaStream_t s, double *A, int n, void *work, int *d_info, int *bad)
 {
-    for (int k0 = 0; k0 < n; k0 += NB) {
-        const int kb = (n - k0 < NB) ? n - k0 : NB;
-        k_potrf_diag<<<1, 256, 0, s>>>(A, n, n, k0, kb, d_info);
-        const int rest = n - k0 - kb;
-        if (rest > 0) {
-            k_trsm_panel<<<(rest + 31) / 32, 256, 0, s>>>(A, n, n, k0, kb, d_info);
-            const int nt = (rest + 63) / 64;
-            k_syrk_update<<<nt * (nt + 1) / 2, 256, 0, s>>>(A, n, n, k0, kb, d_info);
-        }
-    }
     int h = 0;
-    cudaMemcpyAsync(&h, d_info, sizeof(int), cudaMemcpyDeviceToHost, s);
-    cudaStreamSynchronize(s);
-    return h;
+    if (sp_solve_factor(s, A, n, work, d_info) != cudaSuccess ||
+        cudaMemcpyAsync(&h, d_info, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess) {
+        sp_dev_note_error("ridge factorisation", (int)cudaGetLastError());
+        return SP_EINTERNAL;
+    }
+    *bad = h;
+    return h < 0 ? SP_EINTERNAL : SP_OK;  // < 0: a wait ran out
 }
 
-static void chol_solve(cudaStream_t s, const double *L, int n, double *Z, int dout)
-{
-    for (int k0 = 0; k0 < n; k0 += NB) {
-        const int kb = (n - k0 < NB) ? n - k0 : NB;
-        k_fwd_diag<<<1, 256, 0, s>>>(L, n, k0, kb, Z, dout);
-        const int rest = n - k0 - kb;
-        if (rest > 0)
-            k_fwd_update<<<(rest + 7) / 8, 256, 0, s>>>(L, n, n, k0, kb, Z, dout);
-    }
-    const int last = ((n - 1) / NB) * NB;
-    for (int k0 = last; k0 >= 0; k0 -= NB) {
-        const int kb = (n - k0 < NB) ? n - k0 : NB;
-        k_bwd_diag<<<1, 256, 0, s>>>(L, n, k0, kb, Z, dout);
-        if (k0 > 0)
-            k_bwd_update<<<(k0 + 255) / 256, 256, 0, s>>>(L, n, k0, kb, Z, dout);
-    }
-}
-
-static int lu_factor_solve(cudaStream_t s, double *A, int n, int *d_piv, int *d_info, double *Z,
-                           int dout)
+static int lu_factor_solve(cudaStream_t s, double *A, int n, int lda, int *d_piv, int *d_info,
+                           double *Z, int dout)
 {
     for (int j = 0; j < n; ++j) {
-        k_lu_pivot<<<1, 256, 0, s>>>(A, n, n, j, d_piv, d_info);
+        k_lu_pivot<<<1, 256, 0, s>>>(A, n, lda, j, d_piv, d_info);
         int rows = n - j - 1;
         if (rows > 0)
-            k_lu_update<<<rows < 1024 ? rows : 1024, 256, 0, s>>>(A, n, n, j);
+            k_lu_update<<<rows < 1024 ? rows : 1024, 256, 0, s>>>(A, n, lda, j);
     }
     int h = 0;
     cudaMemcpyAsync(&h, d_info, sizeof(int), cudaMemcpyDeviceToHost, s);
     cudaStreamSynchronize(s);
     if (h)
         return h;
-    k_lu_solve<<<dout, 32, 0, s>>>(A, n, n, d_piv, Z, dout);
+    k_lu_solve<<<dout, 32, 0, s>>>(A, n, lda, d_piv, Z, dout);
     return 0;
 }
 
@@ -1041,17 +674,19 @@ static int ridge_dual(cudaStream_t s, const double *Phi, int n, size_t T, size_t
     const size_t tw = T - w0;
     const int m = (int)tw;
     double *Pt = nullptr, *K = nullptr;
+    void *work = nullptr;
+    const int mp = sp_solve_pad(m);
     const size_t tot = (size_t)n * dout;
     const dim3 gp((n + 127) / 128, parts);
     auto tg = std::chrono::steady_clock::now();
-    RK(sp_cuda_malloc(&Pt, (size_t)n * tw * sizeof(double)));
-    RK(sp_cuda_malloc(&K, tw * tw * sizeof(double)));
+    RK(sp_cuda_malloc_async(&Pt, (size_t)n * tw * sizeof(double), s));
+    RK(sp_cuda_malloc_async(&K, (size_t)mp * mp * sizeof(double), s));
+    RK(sp_cuda_malloc_async((char **)&work, sp_solve_work_bytes(m), s));
     {
         dim3 g((n + 31) / 32, (unsigned)((tw + 31) / 32));
         k_rows_to_cols<<<g, dim3(32, 8), 0, s>>>(Phi, n, w0, T, Pt);
-        const int nt = (m + 63) / 64;
-        k_syrk_f64<<<nt * (nt + 1) / 2, 256, 0, s>>>(Pt, m, 0, (size_t)n, K, m);
-        k_add_diag<<<(m + 255) / 256, 256, 0, s>>>(K, m, m, lambda);
+        RK(sp_solve_gram(s, Pt, m, 0, (size_t)n, K, mp));
+        RK(sp_solve_diag(s, K, m, lambda));
         k_xt_e_part<<<gp, 128, 0, s>>>(Phi, n, w0, T, Y, dout, parts, part);
         k_reduce_parts<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(part, parts, n, dout, nullptr,
                                                                      0.0, B);
@@ -1063,19 +698,22 @@ static int ridge_dual(cudaStream_t s, const double *Phi, int n, size_t T, size_t
     {
         auto tf = std::chrono::steady_clock::now();
         double *Z = E + w0 * dout;
-        if (cholesky_inplace(s, K, m, info)) {
+        int bad = 0;
+        rc = cholesky(s, K, m, work, info, &bad);
+        if (rc)
+            goto out;
+        if (bad) {
             rep->factor_failed = 1;
             rep->lu_fallback = 1;
             RK(cudaMemsetAsync(info, 0, sizeof(int), s));
-            const int nt = (m + 63) / 64;
-            k_syrk_f64<<<nt * (nt + 1) / 2, 256, 0, s>>>(Pt, m, 0, (size_t)n, K, m);
-            k_add_diag<<<(m + 255) / 256, 256, 0, s>>>(K, m, m, lambda);
-            if (lu_factor_solve(s, K, m, piv, info, Z, dout)) {
+            RK(sp_solve_gram(s, Pt, m, 0, (size_t)n, K, mp));
+            k_add_diag<<<(m + 255) / 256, 256, 0, s>>>(K, m, mp, lambda);
+            if (lu_factor_solve(s, K, m, mp, piv, info, Z, dout)) {
                 rc = SP_RIDGE_SINGULAR;
                 goto out;
             }
         } else {
-            chol_solve(s, K, m, Z, dout);
+            RK(sp_solve_apply(s, K, m, work, Z, dout, info));
         }
         k_xt_e_part<<<gp, 128, 0, s>>>(Phi, n, w0, T, E, dout, parts, part);
         k_reduce_parts<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(part, parts, n, dout, nullptr,
@@ -1085,11 +723,13 @@ static int ridge_dual(cudaStream_t s, const double *Phi, int n, size_t T, size_t
         rep->factor_ms = ms_since(tf);
     }
 out:
-    cudaStreamSynchronize(s);
     if (Pt)
-        sp_cuda_free(Pt);
+        sp_cuda_free_async(Pt, s);
     if (K)
-        sp_cuda_free(K);
+        sp_cuda_free_async(K, s);
+    if (work)
+        sp_cuda_free_async(work, s);
+    cudaStreamSynchronize(s);
     return rc;
 }
 
@@ -1106,10 +746,11 @@ static int ridge_mixed(cudaStream_t s, const double *Phi, int n, size_t T, size_
                        const double *Y, int dout, double lambda, int mode,
                        const sp_ridge_opts *o, sp_ridge_report *rep, double *A, double *B,
                        double *W, double *R, double *E, double *part, int parts, double *tmp,
-                       int *info)
+                       void *work, int *info)
 {
     int rc = SP_OK;
-    const size_t nn = (size_t)n * n, tot = (size_t)n * dout;
+    const int lda = sp_solve_pad(n);
+    const size_t nn = (size_t)lda * lda, tot = (size_t)n * dout;
     const unsigned gb = (unsigned)((tot + 255) / 256 < 4096 ? (tot + 255) / 256 : 4096);
     double *A0 = nullptr, *Z = nullptr, *P = nullptr, *Q = nullptr, *Yz = nullptr, *c = nullptr,
            *dots = nullptr;
@@ -1126,7 +767,7 @@ static int ridge_mixed(cudaStream_t s, const double *Phi, int n, size_t T, size_
     RK(cudaMemcpyAsync(A0, A, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
     {
         RK(cudaMemsetAsync(tmp, 0, sizeof(double), s));
-        k_diag_max<<<(n + 255) / 256, 256, 0, s>>>(A, n, (unsigned long long *)tmp);
+        k_diag_max<<<(n + 255) / 256, 256, 0, s>>>(A, n, lda, (unsigned long long *)tmp);
         double dmax = 0.0;
         RK(cudaMemcpyAsync(&dmax, tmp, sizeof(double), cudaMemcpyDeviceToHost, s));
         RK(cudaStreamSynchronize(s));
@@ -1138,8 +779,12 @@ static int ridge_mixed(cudaStream_t s, const double *Phi, int n, size_t T, size_
                 RK(cudaMemcpyAsync(A, A0, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
                 RK(cudaMemsetAsync(info, 0, sizeof(int), s));
             }
-            k_add_diag<<<(n + 255) / 256, 256, 0, s>>>(A, n, n, delta);
-            ok = cholesky_inplace(s, A, n, info) == 0;
+            RK(sp_solve_diag(s, A, n, delta));
+            int bad = 0;
+            rc = cholesky(s, A, n, work, info, &bad);
+            if (rc)
+                goto out;
+            ok = bad == 0;
         }
         if (!ok) {
             rc = SP_RIDGE_SINGULAR;
@@ -1153,10 +798,10 @@ static int ridge_mixed(cudaStream_t s, const double *Phi, int n, size_t T, size_
         const double bden = bnorm > 0 ? bnorm : 1.0;
         // W = M^-1 B, R = B - A W (FP64 from Phi), Z = M^-1 R, P = Z
         RK(cudaMemcpyAsync(W, B, tot * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        chol_solve(s, A, n, W, dout);
+        RK(sp_solve_apply(s, A, n, work, W, dout, info));
         ridge_residual(s, Phi, n, w0, T, Y, W, dout, lambda, E, part, parts, R);
         RK(cudaMemcpyAsync(Z, R, tot * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        chol_solve(s, A, n, Z, dout);
+        RK(sp_solve_apply(s, A, n, work, Z, dout, info));
         RK(cudaMemcpyAsync(P, Z, tot * sizeof(double), cudaMemcpyDeviceToDevice, s));
         k_coldot<<<dout, 256, 0, s>>>(R, Z, n, dout, dots);
         RK(cudaMemcpyAsync(h_rz, dots, dout * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1174,7 +819,7 @@ static int ridge_mixed(cudaStream_t s, const double *Phi, int n, size_t T, size_
             k_col_update<<<gb, 256, 0, s>>>(W, P, c, n, dout, 0);  // W += alpha P
             k_col_update<<<gb, 256, 0, s>>>(R, Q, c, n, dout, 0);  // R -= alpha A P
             RK(cudaMemcpyAsync(Z, R, tot * sizeof(double), cudaMemcpyDeviceToDevice, s));
-            chol_solve(s, A, n, Z, dout);
+            RK(sp_solve_apply(s, A, n, work, Z, dout, info));
             k_coldot<<<dout, 256, 0, s>>>(R, Z, n, dout, dots);
             double h_rz2[16];
             RK(cudaMemcpyAsync(h_rz2, dots, dout * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1210,6 +855,7 @@ out:
 struct sp_ridge_ws {
     double *A = nullptr, *B = nullptr, *W = nullptr, *R = nullptr, *E = nullptr,
            *part = nullptr, *tmp = nullptr;
+    char *work = nullptr;
     int *info = nullptr, *piv = nullptr;
     size_t cap_nn = 0, cap_nd = 0, cap_td = 0, cap_n = 0;
 };
@@ -1218,7 +864,7 @@ extern "C" sp_ridge_ws *sp_ridge_ws_new(void) { return new sp_ridge_ws(); }
 
 static void ws_release(sp_ridge_ws *w)
 {
-    void *bufs[] = {w->A, w->B, w->W, w->R, w->E, w->part, w->tmp, w->info, w->piv};
+    void *bufs[] = {w->A, w->B, w->W, w->R, w->E, w->part, w->tmp, w->work, w->info, w->piv};
     for (void *b : bufs)
         if (b)
             sp_cuda_free(b);
@@ -1238,7 +884,8 @@ extern "C" void sp_ridge_ws_free(sp_ridge_ws *w)
 // each instance before the next).
 static int ws_ensure(sp_ridge_ws *w, int n, size_t T, int dout, int parts)
 {
-    const size_t nn = (size_t)n * n, nd = (size_t)n * dout, td = (T ? T : 1) * (size_t)dout;
+    const size_t np = (size_t)sp_solve_pad(n), nn = np * np, nd = (size_t)n * dout,
+                 td = (T ? T : 1) * (size_t)dout;
     if (nn <= w->cap_nn && nd <= w->cap_nd && td <= w->cap_td && (size_t)n <= w->cap_n)
         return SP_OK;
     const size_t cnn = nn > w->cap_nn ? nn : w->cap_nn, cnd = nd > w->cap_nd ? nd : w->cap_nd,
@@ -1255,6 +902,7 @@ static int ws_ensure(sp_ridge_ws *w, int n, size_t T, int dout, int parts)
     RK(sp_cuda_malloc(&w->tmp, 4 * sizeof(double)));
     RK(sp_cuda_malloc(&w->info, sizeof(int)));
     RK(sp_cuda_malloc(&w->piv, cn * sizeof(int)));
+    RK(sp_cuda_malloc(&w->work, sp_solve_work_bytes((int)cn)));
     w->cap_nn = cnn;
     w->cap_nd = cnd;
     w->cap_td = ctd;
@@ -1272,10 +920,11 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
                            sp_ridge_report *rep, double *d_W_out, sp_ridge_ws *ws)
 {
     int rc = SP_OK;
-    double *A = nullptr, *Aw = nullptr, *B = nullptr, *W = nullptr, *R = nullptr, *E = nullptr,
+    double *A = nullptr, *B = nullptr, *W = nullptr, *R = nullptr, *E = nullptr,
            *part = nullptr, *tmp = nullptr;
+    char *work = nullptr;
     int *info = nullptr, *piv = nullptr;
-    const int parts = 64;
+    const int parts = 64, lda = sp_solve_pad(n);
     const size_t w0 = o->washout;
     if (dout == 0)
         return SP_OK;
@@ -1292,18 +941,20 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
         E = ws->E;
         part = ws->part;
         tmp = ws->tmp;
+        work = ws->work;
         info = ws->info;
         piv = ws->piv;
     } else {
-        RK(sp_cuda_malloc(&A, (size_t)n * n * sizeof(double)));
-        RK(sp_cuda_malloc(&B, (size_t)n * dout * sizeof(double)));
-        RK(sp_cuda_malloc(&W, (size_t)n * dout * sizeof(double)));
-        RK(sp_cuda_malloc(&R, (size_t)n * dout * sizeof(double)));
-        RK(sp_cuda_malloc(&E, (T ? T : 1) * (size_t)dout * sizeof(double)));
-        RK(sp_cuda_malloc(&part, (size_t)parts * n * dout * sizeof(double)));
-        RK(sp_cuda_malloc(&tmp, 4 * sizeof(double)));
-        RK(sp_cuda_malloc(&info, sizeof(int)));
-        RK(sp_cuda_malloc(&piv, (size_t)n * sizeof(int)));
+        RK(sp_cuda_malloc_async(&A, (size_t)lda * lda * sizeof(double), s));
+        RK(sp_cuda_malloc_async(&B, (size_t)n * dout * sizeof(double), s));
+        RK(sp_cuda_malloc_async(&W, (size_t)n * dout * sizeof(double), s));
+        RK(sp_cuda_malloc_async(&R, (size_t)n * dout * sizeof(double), s));
+        RK(sp_cuda_malloc_async(&E, (T ? T : 1) * (size_t)dout * sizeof(double), s));
+        RK(sp_cuda_malloc_async(&part, (size_t)parts * n * dout * sizeof(double), s));
+        RK(sp_cuda_malloc_async(&tmp, 4 * sizeof(double), s));
+        RK(sp_cuda_malloc_async(&work, sp_solve_work_bytes(n), s));
+        RK(sp_cuda_malloc_async(&info, sizeof(int), s));
+        RK(sp_cuda_malloc_async(&piv, (size_t)n * sizeof(int), s));
     }
     RK(cudaMemsetAsync(info, 0, sizeof(int), s));
 
@@ -1335,20 +986,18 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
         const int slices = o->gram_slices > 0 ? o->gram_slices : SP_GRAM_INT8_SLICES;
         if ((mode == SP_GRAM_BF16X3 || mode == SP_GRAM_TF32X3 || mode == SP_GRAM_INT8) &&
             sp_gram_tc_available()) {
-            rc = sp_gram_tc(s, mode, slices, Phi, n, w0, T, A, n);
+            rc = sp_gram_tc(s, mode, slices, Phi, n, w0, T, A, lda);
             if (rc == SP_EINVAL && mode == SP_GRAM_INT8) {
                 // a state that is not finite: the FP64 Gram, as the reference
                 rc = SP_OK;
                 mode = 0;
-                const int nt = (n + 63) / 64;
-                k_syrk_f64<<<nt * (nt + 1) / 2, 256, 0, s>>>(Phi, n, w0, T, A, n);
+                RK(sp_solve_gram(s, Phi, n, w0, T, A, lda));
             }
             if (rc)
                 goto out;
         } else {
             mode = 0;
-            const int nt = (n + 63) / 64;
-            k_syrk_f64<<<nt * (nt + 1) / 2, 256, 0, s>>>(Phi, n, w0, T, A, n);
+            RK(sp_solve_gram(s, Phi, n, w0, T, A, lda));
         }
         rep->gram_mode_used = mode;
         dim3 g((n + 127) / 128, parts);
@@ -1356,7 +1005,7 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
         const size_t tot = (size_t)n * dout;
         k_reduce_parts<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(part, parts, n, dout, nullptr,
                                                                      0.0, B);
-        k_add_diag<<<(n + 255) / 256, 256, 0, s>>>(A, n, n, lambda);
+        RK(sp_solve_diag(s, A, n, lambda));
         RK(cudaStreamSynchronize(s));
         RK(cudaGetLastError());
         rep->gram_ms = ms_since(tg);
@@ -1366,7 +1015,7 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
         // an FP32-accumulated Gram is too coarse to factor directly at small
         // lambda: Cholesky-preconditioned CG on the FP64 operator
         rc = ridge_mixed(s, Phi, n, T, w0, Y, dout, lambda, rep->gram_mode_used, o, rep, A, B, W,
-                         R, E, part, parts, tmp, info);
+                         R, E, part, parts, tmp, work, info);
         if (rc)
             goto out;
         const size_t tot = (size_t)n * dout;
@@ -1379,7 +1028,10 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
     {
         auto tf = std::chrono::steady_clock::now();
         RK(cudaMemcpyAsync(W, B, (size_t)n * dout * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        int bad = cholesky_inplace(s, A, n, info);
+        int bad = 0;
+        rc = cholesky(s, A, n, work, info, &bad);
+        if (rc)
+            goto out;
         if (bad) {
             // dgesv semantics: LU with partial pivoting on the original matrix
             rep->factor_failed = 1;
@@ -1388,25 +1040,24 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
             if (rep->gram_mode_used != 0) {
                 rc = sp_gram_tc(s, rep->gram_mode_used,
                                 o->gram_slices > 0 ? o->gram_slices : SP_GRAM_INT8_SLICES, Phi,
-                                n, w0, T, A, n);
+                                n, w0, T, A, lda);
                 if (rc)
                     goto out;
             } else {
-                const int nt = (n + 63) / 64;
-                k_syrk_f64<<<nt * (nt + 1) / 2, 256, 0, s>>>(Phi, n, w0, T, A, n);
+                RK(sp_solve_gram(s, Phi, n, w0, T, A, lda));
             }
-            k_add_diag<<<(n + 255) / 256, 256, 0, s>>>(A, n, n, lambda);
-            int lbad = lu_factor_solve(s, A, n, piv, info, W, dout);
+            k_add_diag<<<(n + 255) / 256, 256, 0, s>>>(A, n, lda, lambda);
+            int lbad = lu_factor_solve(s, A, n, lda, piv, info, W, dout);
             if (lbad) {
                 rc = SP_RIDGE_SINGULAR;
                 goto out;
             }
             rep->factor_ms = ms_since(tf);
         } else {
-            // cholesky_inplace has waited for the factorisation
+            // cholesky() has waited for the factorisation
             rep->factor_ms = ms_since(tf);
             auto ts = std::chrono::steady_clock::now();
-            chol_solve(s, A, n, W, dout);
+            RK(sp_solve_apply(s, A, n, work, W, dout, info));
             RK(cudaStreamSynchronize(s));
             rep->solve_ms = ms_since(ts);
         }
@@ -1426,7 +1077,7 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
             rel = device_norm(s, R, (size_t)n * dout, tmp) / (bnorm > 0 ? bnorm : 1.0);
             if (rel <= o->refine_tol || it >= maxit)
                 break;
-            chol_solve(s, A, n, R, dout);
+            RK(sp_solve_apply(s, A, n, work, R, dout, info));
             const size_t tot = (size_t)n * dout;
             k_axpy<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(W, R, tot);
             ++it;
@@ -1440,28 +1091,28 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
         const size_t tot = (size_t)n * dout;
         // W (n x dout) -> W_out (dout x n)
         k_transpose_w<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(W, n, dout, d_W_out);
+        int h = 0;
+        RK(cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, s));
         RK(cudaStreamSynchronize(s));
         RK(cudaGetLastError());
+        if (h < 0)
+            rc = SP_EINTERNAL;  // a wait of a solve ran out
     }
 out:
-    cudaStreamSynchronize(s);
     if (!ws) {
-        void *bufs[] = {A, Aw, B, W, R, E, part, tmp, info, piv};
+        void *bufs[] = {A, B, W, R, E, part, tmp, work, info, piv};
         for (void *b : bufs)
             if (b)
-                sp_cuda_free(b);
-    } else if (Aw) {
-        sp_cuda_free(Aw);
+                sp_cuda_free_async(b, s);
     }
+    cudaStreamSynchronize(s);
     return rc;
 }
 
 extern "C" int sp_gram_fp64(cudaStream_t s, const double *X, int n, size_t t0, size_t t1,
                             double *C, int ldc)
 {
-    const int nt = (n + 63) / 64;
-    k_syrk_f64<<<nt * (nt + 1) / 2, 256, 0, s>>>(X, n, t0, t1, C, ldc);
-    return cudaGetLastError() == cudaSuccess ? SP_OK : SP_EINTERNAL;
+    return sp_solve_gram(s, X, n, t0, t1, C, ldc) == cudaSuccess ? SP_OK : SP_EINTERNAL;
 }
 
 // Ridge on states already on the device: Phi [T x n] row-major (neuron order),
@@ -1547,9 +1198,9 @@ extern "C" int sp_ridge_host(const double *h_phi, size_t T, int n, const double 
         return SP_EINVAL;
     auto t0 = std::chrono::steady_clock::now();
     RK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    RK(sp_cuda_malloc(&Phi, T * (size_t)n * sizeof(double)));
-    RK(sp_cuda_malloc(&Y, T * (size_t)dout * sizeof(double)));
-    RK(sp_cuda_malloc(&Wt, (size_t)n * dout * sizeof(double)));
+    RK(sp_cuda_malloc_async(&Phi, T * (size_t)n * sizeof(double), s));
+    RK(sp_cuda_malloc_async(&Y, T * (size_t)dout * sizeof(double), s));
+    RK(sp_cuda_malloc_async(&Wt, (size_t)n * dout * sizeof(double), s));
     RK(cudaMemcpyAsync(Phi, h_phi, T * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, s));
     RK(cudaMemcpyAsync(Y, h_y, T * (size_t)dout * sizeof(double), cudaMemcpyHostToDevice, s));
     RK(cudaStreamSynchronize(s));
@@ -1560,14 +1211,14 @@ extern "C" int sp_ridge_host(const double *h_phi, size_t T, int n, const double 
     RK(cudaMemcpyAsync(h_w_out, Wt, (size_t)n * dout * sizeof(double), cudaMemcpyDeviceToHost, s));
     RK(cudaStreamSynchronize(s));
 out:
-    if (s)
-        cudaStreamSynchronize(s);
     void *bufs[] = {Phi, Y, Wt};
     for (void *b : bufs)
         if (b)
-            sp_cuda_free(b);
-    if (s)
+            sp_cuda_free_async(b, s);
+    if (s) {
+        cudaStreamSynchronize(s);
         cudaStreamDestroy(s);
+    }
     return rc;
 }
 
@@ -1587,9 +1238,9 @@ extern "C" int sp_dev_train_ridge(sp_dev *d, const sp_host_model *m, const doubl
     rc = sp_dev_reset_neurons(d, m);
     if (rc)
         return rc;
-    RK(sp_cuda_malloc(&Phi, (T ? T : 1) * (size_t)n * sizeof(double)));
-    RK(sp_cuda_malloc(&Y, (T ? T : 1) * (size_t)dout * sizeof(double)));
-    RK(sp_cuda_malloc(&Wt, (size_t)n * dout * sizeof(double)));
+    RK(sp_cuda_malloc_async(&Phi, (T ? T : 1) * (size_t)n * sizeof(double), s));
+    RK(sp_cuda_malloc_async(&Y, (T ? T : 1) * (size_t)dout * sizeof(double), s));
+    RK(sp_cuda_malloc_async(&Wt, (size_t)n * dout * sizeof(double), s));
     RK(cudaMemcpyAsync(Y, h_y, T * dout * sizeof(double), cudaMemcpyHostToDevice, s));
     {
         sp_run_args a;
@@ -1619,11 +1270,11 @@ extern "C" int sp_dev_train_ridge(sp_dev *d, const sp_host_model *m, const doubl
     RK(cudaStreamSynchronize(s));
     RK(cudaGetLastError());
 out:
-    cudaStreamSynchronize(s);
     void *bufs[] = {Phi, Y, Wt};
     for (void *b : bufs)
         if (b)
-            sp_cuda_free(b);
+            sp_cuda_free_async(b, s);
+    cudaStreamSynchronize(s);
     return rc;
 }
 
@@ -1795,10 +1446,12 @@ out:
 #define SP_NA_MAX_DOUT 16
 #define SP_NA_MAX_T 16384
 #define SP_NA_PARTS 64
+/* the solver's inverted blocks and flags: sp_solve_work_bytes(512) in doubles */
+#define SP_NA_WORK (8 * 4 * 256 + (8 * 8 + 2 * 8 + 4 + 1) / 2)
 #define SP_NA_DOUBLES                                                                  \
     ((size_t)SP_NA_MAX_N * SP_NA_MAX_N + 3 * (size_t)SP_NA_MAX_N * SP_NA_MAX_DOUT +    \
      (size_t)SP_NA_MAX_T * SP_NA_MAX_DOUT +                                            \
-     (size_t)SP_NA_PARTS * SP_NA_MAX_N * SP_NA_MAX_DOUT + 8)
+     (size_t)SP_NA_PARTS * SP_NA_MAX_N * SP_NA_MAX_DOUT + 8 + SP_NA_WORK)
 
 static __device__ __align__(256) double g_na_scratch[SP_NA_DOUBLES];
 static __device__ __align__(256) int g_na_iscratch[SP_NA_MAX_N + 8];
@@ -1853,6 +1506,8 @@ spires_ext_ridge_solve_noalloc(const double *d_states, const double *d_targets, 
     double *E = R + (size_t)SP_NA_MAX_N * SP_NA_MAX_DOUT;
     double *part = E + (size_t)SP_NA_MAX_T * SP_NA_MAX_DOUT;
     double *tmp = part + (size_t)SP_NA_PARTS * SP_NA_MAX_N * SP_NA_MAX_DOUT;
+    void *work = tmp + 8;
+    const int lda = sp_solve_pad((int)n_);
     int *info = g_na_iptr[dev];
     int *piv = info + 8;
     const int parts = SP_NA_PARTS;
@@ -1864,31 +1519,34 @@ spires_ext_ridge_solve_noalloc(const double *d_states, const double *d_targets, 
     // must start at zero; every other region is fully rewritten below
     if (cudaMemsetAsync(info, 0, sizeof(int), s) != cudaSuccess)
         return SP_EINTERNAL;
-    const int nt = (n + 63) / 64;
-    k_syrk_f64<<<nt * (nt + 1) / 2, 256, 0, s>>>(d_states, n, washout, T, A, n);
+    if (sp_solve_gram(s, d_states, n, washout, T, A, lda) != cudaSuccess)
+        return SP_EINTERNAL;
     {
         dim3 g((n + 127) / 128, parts);
         k_xt_e_part<<<g, 128, 0, s>>>(d_states, n, washout, T, d_targets, dout, parts, part);
         k_reduce_parts<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(part, parts, n, dout,
                                                                      nullptr, 0.0, B);
     }
-    k_add_diag<<<(n + 255) / 256, 256, 0, s>>>(A, n, n, lambda);
-    if (cudaMemcpyAsync(W, B, tot * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+    if (sp_solve_diag(s, A, n, lambda) != cudaSuccess ||
+        cudaMemcpyAsync(W, B, tot * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
         return SP_EINTERNAL;
-    int bad = cholesky_inplace(s, A, n, info);
+    int bad = 0;
+    if (cholesky(s, A, n, work, info, &bad) != SP_OK)
+        return SP_EINTERNAL;
     bool lu = false;
     if (bad) {
         lu = true;
         cudaMemsetAsync(info, 0, sizeof(int), s);
-        k_syrk_f64<<<nt * (nt + 1) / 2, 256, 0, s>>>(d_states, n, washout, T, A, n);
-        k_add_diag<<<(n + 255) / 256, 256, 0, s>>>(A, n, n, lambda);
-        if (lu_factor_solve(s, A, n, piv, info, W, dout) != 0) {
+        if (sp_solve_gram(s, d_states, n, washout, T, A, lda) != cudaSuccess)
+            return SP_EINTERNAL;
+        k_add_diag<<<(n + 255) / 256, 256, 0, s>>>(A, n, lda, lambda);
+        if (lu_factor_solve(s, A, n, lda, piv, info, W, dout) != 0) {
             // singular system: d_w_out is not written, and the caller is told
             cudaStreamSynchronize(s);
             return SP_EINTERNAL;
         }
-    } else {
-        chol_solve(s, A, n, W, dout);
+    } else if (sp_solve_apply(s, A, n, work, W, dout, info) != cudaSuccess) {
+        return SP_EINTERNAL;
     }
     const double bnorm = device_norm(s, B, tot, tmp);
     for (int it = 0;; ++it) {
@@ -1896,9 +1554,14 @@ spires_ext_ridge_solve_noalloc(const double *d_states, const double *d_targets, 
         const double rel = device_norm(s, R, tot, tmp) / (bnorm > 0 ? bnorm : 1.0);
         if (rel <= tol || it >= (lu ? 0 : maxit))
             break;
-        chol_solve(s, A, n, R, dout);
+        if (sp_solve_apply(s, A, n, work, R, dout, info) != cudaSuccess)
+            return SP_EINTERNAL;
         k_axpy<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(W, R, tot);
     }
+    int h = 0;
+    if (cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess || h < 0)
+        return SP_EINTERNAL;  // h < 0: a wait of the solver ran out
     k_transpose_w<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(W, n, dout, d_w_out);
     if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
         return SP_EINTERNAL;

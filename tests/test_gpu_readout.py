@@ -277,3 +277,25 @@ def test_rls_in_one_launch_matches_oracle(n, T, dout, neuron, lam):
     assert rel(W, Wo) < 1e-8
     phi, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=12)).run(u)
     assert np.array_equal(v, phi[-1])  # the reservoir is left after the last step
+
+
+# One 64-wide tile and its edges, several tiles, odd widths, tile pairs split over
+# row parts or not, the 128-wide Gram tiles, and the dual form (few rows).
+@pytest.mark.parametrize("n,T,dout", [(1, 3, 1), (63, 200, 2), (64, 130, 1), (65, 1000, 16),
+                                      (129, 4099, 3), (577, 700, 5), (1000, 90, 2),
+                                      (2050, 2304, 1)])
+def test_ridge_solver_at_tile_edges(n, T, dout):
+    """The direct solve (no refinement) against float64 LAPACK. With lambda = T the
+    condition number of X^T X + lambda I is at most 1 + (1 + sqrt(n / T))^2 for
+    entries in [-1, 1), and both sides' forward error is below
+    2 (T + n) eps times it."""
+    rng = np.random.default_rng(n)
+    X = rng.uniform(-1, 1, (T, n))
+    Y = rng.uniform(-1, 1, (T, dout))
+    W, rep = sp.ridge_fit(X, Y, float(T), max_refine=0)
+    ref = np.linalg.solve(X.T @ X + T * np.eye(n), X.T @ Y).T
+    cond = 1 + (1 + np.sqrt(n / T)) ** 2
+    assert rep.factor_failed == 0
+    assert rel(W, ref) < 4 * (T + n) * np.finfo(float).eps * cond
+    # the same bits again: the sums' order is fixed
+    assert np.array_equal(W, sp.ridge_fit(X, Y, float(T), max_refine=0)[0])
