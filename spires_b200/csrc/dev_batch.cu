@@ -7,12 +7,26 @@
 //
 // Work table. The host plans a static schedule: the cooperative grid of P CTAs
 // (256 threads each) is cut into groups of consecutive CTAs; each group runs a
-// list of instances one after another, all its CTAs on one instance at a time
-// with a group-local grid barrier (a counter per group). An instance needs at
-// least ceil(nw / 8) CTAs (one neuron per thread); instances are placed
-// heaviest first on the group that finishes them earliest (list scheduling on
-// an estimated time that takes both the history stream and the per-step
-// latency floor into account).
+// list of instances one after another, all its CTAs on one instance at a time,
+// its CTAs exchanging spike words after every step. An instance needs at least
+// ceil(nw / 8) CTAs (one neuron per thread).
+//
+// A batch that fits one CTA per SM with every instance running at once is spread
+// over the SMs: the slowest instance gets more CTAs until no more are free, and
+// with few warps each CTA holds its neurons' FLIF_GL rings and its column blocks
+// in shared memory (plan_spread; FLIF_GL N=1366, L=256: 18.2 us per step streamed
+// on 8 CTAs, 5.8 on 43; 20 such instances 21.5 -> 6.9 ms). Larger batches run two CTAs per SM in
+// size-class groups, the rings streamed from L2 and DRAM through asynchronous
+// copies; instances are placed heaviest first on the group that finishes them
+// earliest (list scheduling on an estimated time that takes both the history
+// stream and the per-step latency floor into account).
+//
+// Spike exchange: a warp publishes its word as one 8-byte (step, word) entry in
+// one of two alternating buffers, and readers poll the entries themselves, so a
+// step costs one store and one successful poll. A warp publishes step b + 1 only
+// after its CTA has read every word of step b, so nobody still reads the entries
+// it overwrites. (LIF N=930 on 4 CTAs: 3.8 us per step with a counter
+// barrier, 1.4 with the entries read by every warp.)
 //
 // The launch sequence of a run (input upload, state reset, barrier reset, the
 // cooperative kernel, the raster gather and download) is captured once into a
@@ -27,6 +41,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 #include "sp_alloc.h"
 #include "sp_dev.h"
@@ -46,10 +61,13 @@ struct BInst {
     int dense;      // recurrent input from column blocks (see rowpass_columns)
     const uint2 *cmo;   // [n][nw] {row bits, weight offset} per (column, row word)
     const double *cw;   // [nnz] weights in column order
+    int wcap;           // most weights of a row word's column blocks
+    int mode;           // kRingSmem | kRowsSmem: what a CTA keeps in shared memory; kAlone
+    int region;         // bytes of it per warp
     long long T;  // macro steps of the current run
     double a, b, c, d, e, f, g, dt, gamma, v_init, tprev_init;
     double *V, *tprev, *ring;
-    unsigned *spk;  // [2][nw]
+    unsigned long long *ll;  // [2][nw] spike exchange: step << 32 | word
     const long long *row_ptr;
     const int *col;
     const double *w, *W_in, *coef;
@@ -67,12 +85,24 @@ struct BInst {
 struct BParams {
     const BInst *inst;
     const int *cta_group, *group_start, *group_size, *job_off, *jobs;
-    unsigned long long *bar;  // one arrival counter per group
     int *err;
     int lmax;                 // longest FLIF_GL ring of the batch (coefficients in smem)
     int max_nw;               // most spike words of an instance
+    int spk_bufs;             // spike word arrays: two, or one when they are long
     int list_cap;             // largest column-block instance (spike list in smem)
 };
+
+// kAlone: every warp reads all spike words of a step itself, into arrays of its
+// own, and the warps of a CTA never wait for one another.
+constexpr int kRingSmem = 1, kRowsSmem = 2, kAlone = 4;
+
+// One warp's FLIF_GL ring in shared memory: rows in pairs, [pair][32 lanes][2].
+__host__ __device__ constexpr size_t ring_bytes(int L) { return (size_t)((L + 1) / 2) * 512; }
+// One row word's column blocks: {row bits, weight offset} per column, weights.
+__host__ __device__ constexpr size_t rows_bytes(int n, int wcap)
+{
+    return (size_t)((n + 1) / 2) * 16 + (size_t)((wcap + 1) / 2) * 16;
+}
 
 constexpr int kHistChunk = 32;  // ring values in flight per thread (cost model)
 
@@ -80,6 +110,7 @@ constexpr int kHistC = 8;  // ring values per cp.async group and thread
 // groups in flight per thread (6 or 8 need more shared memory than two CTAs
 // per SM allow, and one CTA per SM halved the sweep's throughput)
 constexpr int kHistS = 4;
+constexpr size_t kStageBytes = (size_t)kHistS * kHistC * kBatchThreads * 8;
 
 // FLIF_GL history of column `ci` for lags 2..lim in ascending order, with the
 // ring values copied asynchronously into this thread's own shared-memory
@@ -212,8 +243,8 @@ __device__ __forceinline__ double rowpass_simple_warp_deep(const long long *__re
 // stored edge. Blocks are fetched C columns ahead.
 __device__ __forceinline__ double rowpass_columns(const uint2 *__restrict__ cmo,
                                                   const double *__restrict__ cw,
-                                                  const int *s_list, int cnt, int nw, int q,
-                                                  int lane)
+                                                  const unsigned short *s_list, int cnt, int nw,
+                                                  int q, int lane)
 {
     constexpr int C = 8;
     const unsigned below = (1u << lane) - 1u;
@@ -246,7 +277,7 @@ __device__ __forceinline__ double rowpass_columns(const uint2 *__restrict__ cmo,
 // Ascending list of the spiking positions from the CTA's spike words: each
 // thread takes a contiguous range of words, a block scan of their bit counts
 // gives its write offset. Returns the count (all threads).
-__device__ __forceinline__ int spike_list(const unsigned *s_spk, int nw, int *s_list,
+__device__ __forceinline__ int spike_list(const unsigned *s_spk, int nw, unsigned short *s_list,
                                           int *s_warp)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -275,7 +306,7 @@ __device__ __forceinline__ int spike_list(const unsigned *s_spk, int nw, int *s_
     for (int wi = w0; wi < w1; ++wi) {
         unsigned m = s_spk[wi];
         while (m) {
-            s_list[base++] = wi * 32 + __ffs(m) - 1;
+            s_list[base++] = (unsigned short)(wi * 32 + __ffs(m) - 1);
             m &= m - 1;
         }
     }
@@ -283,10 +314,96 @@ __device__ __forceinline__ int spike_list(const unsigned *s_spk, int nw, int *s_
     return total;
 }
 
+// Arrays of one warp that reads the spike words itself: the words, and for column
+// blocks the list of spiking positions in whole eights.
+__host__ __device__ constexpr size_t alone_bytes(int nw, int dense)
+{
+    return (size_t)(nw + 3) / 4 * 16 + (dense ? (size_t)nw * 64 + 16 : 0);
+}
+
+// The spike word of an entry once it carries step `seq`; false when the wait ran
+// out or another CTA's did.
+__device__ __forceinline__ bool batch_poll(const unsigned long long *e, unsigned seq, int *err,
+                                           long long step, unsigned &word)
+{
+    unsigned long long v = ld_volatile_u64(e), t0 = 0, polls = 0;
+    while ((unsigned)(v >> 32) != seq) {
+        if ((++polls & 255ull) == 0) {
+            const unsigned long long now = globaltimer_ns();
+            if (t0 == 0)
+                t0 = now;
+            if (ld_volatile_i32(err) != kErrNone)
+                return false;
+            if (now - t0 > kBarrierTimeoutNs || polls > kBarrierMaxPolls) {
+                if (atomicCAS(err, kErrNone, kErrBarrierTimeout) == kErrNone)
+                    err[1] = (int)step;
+                return false;
+            }
+        }
+        v = ld_volatile_u64(e);
+    }
+    word = (unsigned)v;
+    return true;
+}
+
+// One warp reads the nw spike words of step `seq` (none before the first step)
+// and, when `list` is given, lists the spiking positions in ascending order.
+// Four entries per lane are in flight. Returns the list's length, or -1.
+__device__ __forceinline__ int batch_words(const unsigned long long *e, int nw, unsigned seq,
+                                           int *err, long long step, unsigned *words,
+                                           unsigned short *list, int lane)
+{
+    int total = 0;
+    for (int w0 = 0; w0 < nw; w0 += 128) {
+        unsigned word[4] = {0u, 0u, 0u, 0u};
+        if (seq > 0) {
+            unsigned long long v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                v[u] = w0 + 32 * u + lane < nw ? ld_volatile_u64(e + w0 + 32 * u + lane) : 0ull;
+            int late = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (w0 + 32 * u + lane < nw) {
+                    word[u] = (unsigned)v[u];
+                    if ((unsigned)(v[u] >> 32) != seq)
+                        late |= !batch_poll(e + w0 + 32 * u + lane, seq, err, step, word[u]);
+                }
+            if (__any_sync(kFull, late))
+                return -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int wi = w0 + 32 * u + lane;
+            if (w0 + 32 * u >= nw)
+                break;
+            if (!list) {
+                if (wi < nw)
+                    words[wi] = word[u];
+                continue;
+            }
+            const int c = __popc(word[u]);
+            int x = c;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const int y = __shfl_up_sync(kFull, x, off);
+                if (lane >= off)
+                    x += y;
+            }
+            int at = total + x - c;
+            for (unsigned m = word[u]; m; m &= m - 1)
+                list[at++] = (unsigned short)(wi * 32 + __ffs(m) - 1);
+            total += __shfl_sync(kFull, x, 31);
+        }
+    }
+    __syncwarp();
+    return total;
+}
+
 // One persistent cooperative launch over the whole batch. CTA c belongs to
 // group cta_group[c] (or to none, then it returns at once); a group runs its
-// job list in order, splitting each instance's warps evenly over its CTAs,
-// and meets at its own counter between micro-steps. The per-neuron arithmetic
+// job list in order, splitting each instance's warps evenly over its CTAs, which
+// exchange their spike words between micro-steps. The per-neuron arithmetic
 // is that of the single-reservoir kernel for LIF_DISCRETE / FLIF_GL with
 // SIMPLE synapses (src/neurons/lif_discrete.c:22-34, src/neurons/flif_gl.c:50-100,
 // src/synapses/simple.c:59-64, src/reservoir.c:113-165).
@@ -298,71 +415,32 @@ constexpr int kJobStampCap = 4096;
 __device__ unsigned long long g_sp_jobstamps[kJobStampCap * 5];
 #endif
 
-__global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BParams p)
+// kSpread: the launch of plan_spread, one CTA per SM and one instance per group.
+template <bool kSpread>
+__global__ void __launch_bounds__(kBatchThreads, kSpread ? 1 : 2) k_batch(BParams p)
 {
     extern __shared__ __align__(16) unsigned char s_dyn[];
     double *s_coef = (double *)s_dyn;                    // [lmax]
-    unsigned *s_spk = (unsigned *)(s_coef + p.lmax);     // [max_nw]
-    int *s_list = (int *)(s_spk + p.max_nw);             // [list_cap]
-    // per-thread ring staging (FLIF_GL batches), 16-byte aligned
-    double *s_h = (double *)(((uintptr_t)(s_list + p.list_cap) + 15) & ~(uintptr_t)15);
-    __shared__ int s_flag, s_abort;
+    unsigned *s_spkb = (unsigned *)(s_coef + p.lmax);    // [spk_bufs][max_nw]
+    // offsets, not cast pointers: the compiler has to see shared memory here
+    const int list_at = (p.lmax * 8 + p.spk_bufs * p.max_nw * 4 + 7) / 8 * 8;
+    unsigned short *s_list = (unsigned short *)(s_dyn + list_at);  // [list_cap], whole fours
+    // ring staging of the streamed FLIF_GL history, and / or what the plan keeps
+    // here
+    unsigned char *s_pool = s_dyn + (list_at + (p.list_cap + 3) / 4 * 8 + 15) / 16 * 16;
     __shared__ int s_warp[kBatchThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int grp = p.cta_group[blockIdx.x];
     if (grp < 0)
-        return;  // CTA outside every group: takes part in no barrier
+        return;  // CTA outside every group: takes part in no exchange
     const int rank = blockIdx.x - p.group_start[grp];
     const int gsize = p.group_size[grp];
-    unsigned long long *bar = p.bar + grp;
-    unsigned long long nbar = 0;
-    if (tid == 0)
-        s_abort = 0;
-
-    auto arrive = [&]() {
-        __syncthreads();
-        if (tid == 0 && gsize > 1) {
-            __threadfence();
-            atomicAdd(bar, 1ull);
-        }
-    };
-    auto wait = [&](long long step) -> bool {
-        ++nbar;
-        if (tid == 0) {
-            int ok = !s_abort;
-            if (ok && gsize > 1) {
-                const unsigned long long target = nbar * (unsigned long long)gsize;
-                unsigned long long t0 = globaltimer_ns(), polls = 0;
-                while (ld_volatile_u64(bar) < target) {
-                    if ((++polls & 255ull) == 0) {
-                        if (ld_volatile_i32(p.err) != kErrNone) {
-                            ok = 0;
-                            break;
-                        }
-                        if (globaltimer_ns() - t0 > kBarrierTimeoutNs || polls > kBarrierMaxPolls) {
-                            if (atomicCAS(p.err, kErrNone, kErrBarrierTimeout) == kErrNone)
-                                p.err[1] = (int)step;
-                            ok = 0;
-                            break;
-                        }
-                    }
-                    __nanosleep(32);
-                }
-                __threadfence();
-            }
-            s_flag = ok;
-            if (!ok)
-                s_abort = 1;
-        }
-        __syncthreads();
-        return s_flag != 0;
-    };
 
     for (int j = p.job_off[grp]; j < p.job_off[grp + 1]; ++j) {
-        const BInst &I = p.inst[p.jobs[j]];
+        std::conditional_t<kSpread, const BInst, const BInst &> I = p.inst[p.jobs[j]];
         const long long B = I.T * I.micro;
         if (B == 0)
-            continue;  // no steps: no arrival either, the counts stay matched
+            continue;
 #ifdef SP_PHASE_STAMPS
         if (rank == 0 && tid == 0 && j < kJobStampCap) {
             g_sp_jobstamps[j * 5 + 0] = globaltimer_ns();
@@ -380,19 +458,61 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BParams p)
         const int i = gw * 32 + lane;
         const int nid = wact ? I.nid_of[i] : -1;
         const bool act = nid >= 0;
-        __syncthreads();  // previous job's readers of s_coef are done
+        const bool ring_smem = kSpread && (I.mode & kRingSmem);
+        const bool rows_smem = kSpread && (I.mode & kRowsSmem);
+        const bool alone = kSpread && (I.mode & kAlone);
+        double *s_h = (double *)s_pool;
+        // coefficients shifted by one (see chain_pairs)
+        double *s_coef1 = (double *)s_pool;
+        unsigned char *mine = s_pool + (ring_smem ? (size_t)((L + 1) / 2) * 16
+                                        : gl      ? kStageBytes
+                                                  : 0) +
+                              (size_t)warp * I.region;
+        double2 *s_ring = (double2 *)mine + lane;
+        uint2 *s_blk = (uint2 *)(mine + (ring_smem ? ring_bytes(L) : 0));
+        double *s_w = (double *)(s_blk + (I.n + 1) / 2 * 2);
+        unsigned *my_words =
+            (unsigned *)((unsigned char *)s_blk + (rows_smem ? rows_bytes(I.n, I.wcap) : 0));
+        unsigned short *my_list = (unsigned short *)(my_words + (nw + 3) / 4 * 4);
+        __syncthreads();  // previous job's readers are done
         if (gl)
-            for (int k = tid; k < L; k += kBatchThreads)
-                s_coef[k] = I.coef[k];
+            for (int k = tid; k < L; k += kBatchThreads) {
+                const double c = I.coef[k];
+                s_coef[k] = c;
+                if (ring_smem && k > 0)
+                    s_coef1[k - 1] = c;
+            }
+        if (rows_smem && wact) {
+            // this word's column blocks, weights in column order
+            unsigned run = 0;
+            for (int j0 = 0; j0 < I.n; j0 += 32) {
+                const int cj = j0 + lane;
+                const uint2 c = cj < I.n ? __ldg(I.cmo + (size_t)cj * nw + gw) : make_uint2(0u, 0u);
+                const unsigned cnt = __popc(c.x);
+                unsigned x = cnt;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const unsigned y = __shfl_up_sync(kFull, x, off);
+                    if (lane >= off)
+                        x += y;
+                }
+                if (cj < I.n)
+                    s_blk[cj] = make_uint2(c.x, run + x - cnt);
+                for (unsigned e = 0; e < cnt; ++e)
+                    s_w[run + x - cnt + e] = __ldg(I.cw + c.y + e);
+                run += __shfl_sync(kFull, x, 31);
+            }
+        }
         double V = act ? I.V[i] : 0.0;
         double tprev = (act && gl) ? I.tprev[i] : 0.0;
-        double vlast = (act && gl) ? I.ring[(size_t)(L - 1) * rs + i] : 0.0;
-        int cur = 0;
+        double vlast = (act && gl) ? I.v_init : 0.0;
         double ext = 0.0;
-        arrive();  // also publishes s_coef to the CTA
+        __syncthreads();
+        if (alone && !wact)
+            continue;  // to the next job's first barrier
+        long long s = 0;        // macro step of b, micro-step in it, ring row
+        int m = 0, head = 0;
         for (long long b = 0; b < B; ++b) {
-            const long long s = b / I.micro;
-            const int m = (int)(b % I.micro);
             if (m == 0) {
                 // ext = 0 + gamma * sum_k W_in[i][k] u[k] (netlib dgemv order)
                 ext = 0.0;
@@ -401,34 +521,67 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BParams p)
                     const double *wr = I.W_in + (size_t)i * I.din;
                     double t = 0.0;
                     for (int k = 0; k < I.din; ++k)
-                        t = add(t, mul(ldg_na(wr + k), ldg_na(ur + k)));
+                        t = add(t, mul(__ldg(wr + k), __ldg(ur + k)));
                     ext = add(0.0, mul(I.gamma, t));
                 }
             }
             bool integ = false;
-            double hist = 0.0;
-            int head = 0;
+            double hist = 0.0, leak = 0.0;
             if (gl) {
-                head = (int)(b % L);
                 integ = tprev > I.f;
+                leak = dvd(-sub(vlast, I.c), I.d);
                 const int lim = (int)(b < L ? b : L - 1);
                 if (act && integ) {
                     if (lim >= 1)
                         hist = add(hist, mul(s_coef[1], vlast));
-                    hist = batch_history_async(hist, s_coef, I.ring + i, rs, L, head, lim,
-                                               s_h, tid);
+                    if (ring_smem) {
+                        const int r = head >= 2 ? head - 2 : head - 2 + L;
+                        const int cnt = lim - 1, n1 = cnt < r + 1 ? cnt : r + 1;
+                        if (cnt > 0)
+                            hist = chain_pairs(hist, s_coef, s_coef1, s_ring, 2, r, n1);
+                        if (cnt > n1)
+                            hist = chain_pairs(hist, s_coef, s_coef1, s_ring, 2 + n1, L - 1,
+                                               cnt - n1);
+                    } else {
+                        hist = batch_history_async(hist, s_coef, I.ring + i, rs, L, head, lim,
+                                                   s_h, tid);
+                    }
                 }
             }
-            if (!wait(b))
-                return;
-            for (int wi = tid; wi < nw; wi += kBatchThreads)
-                s_spk[wi] = __ldcg(I.spk + (size_t)cur * nw + wi);
-            __syncthreads();
+            // every spike word of the step before
+            const unsigned long long *entries = I.ll + (size_t)(b & 1) * nw;
+            const unsigned *s_spk;
+            int cnt = 0;  // spikes, of column blocks
+            if (alone) {
+                cnt = batch_words(entries, nw, (unsigned)b, p.err, b, my_words,
+                                  I.dense ? my_list : nullptr, lane);
+                if (cnt < 0)
+                    return;
+                s_spk = my_words;
+            } else {
+                unsigned *words = s_spkb + (p.spk_bufs > 1 && (b & 1) ? p.max_nw : 0);
+                if (p.spk_bufs == 1)
+                    __syncthreads();  // its readers of the step before are done
+                int late = 0;
+                for (int wi = tid; wi < nw; wi += kBatchThreads) {
+                    unsigned word = 0;
+                    if (b > 0)
+                        late |= !batch_poll(entries + wi, (unsigned)b, p.err, b, word);
+                    words[wi] = word;
+                }
+                if (__syncthreads_or(late))
+                    return;
+                s_spk = words;
+                if (I.dense)
+                    cnt = spike_list(words, nw, s_list, s_warp);
+            }
             double rec = 0.0;
             if (I.dense) {
-                const int cnt = spike_list(s_spk, nw, s_list, s_warp);
-                if (wact)
-                    rec = rowpass_columns(I.cmo, I.cw, s_list, cnt, nw, gw, lane);
+                if (wact && cnt > 0)
+                    rec = !rows_smem ? rowpass_columns(I.cmo, I.cw, alone ? my_list : s_list, cnt,
+                                                       nw, gw, lane)
+                          : alone ? rowpass_cols<true, 8>(s_blk, s_w, my_list, cnt, lane)
+                                  : rowpass_cols<true>(s_blk, s_w, s_list, cnt, lane);
             } else if (wact) {
                 // warp-uniform choice: long edge ranges take the deep pipeline
                 const long long span = __ldg(I.row_ptr + gw * 32 + 32) - __ldg(I.row_ptr + gw * 32);
@@ -448,7 +601,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BParams p)
                     }
                 } else {
                     if (integ) {
-                        const double rhs = add(add(dvd(-sub(vlast, I.c), I.d), in), I.e);
+                        const double rhs = add(add(leak, in), I.e);
                         V = sub(mul(I.g, rhs), hist);
                         if (V >= I.a) {
                             V = I.b;
@@ -458,23 +611,31 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BParams p)
                     } else {
                         V = I.b;
                     }
-                    I.ring[(size_t)head * rs + i] = V;
+                    if (ring_smem)
+                        *((double *)(s_ring + (head >> 1) * 32) + (head & 1)) = V;
+                    else
+                        I.ring[(size_t)head * rs + i] = V;
                     vlast = V;
                     tprev = add(tprev, I.dt);
                 }
             }
             const unsigned word = __ballot_sync(kFull, fired);
             if (wact && lane == 0)
-                I.spk[(size_t)(cur ^ 1) * nw + gw] = word;
+                *(volatile unsigned long long *)(I.ll + (size_t)((b + 1) & 1) * nw + gw) =
+                    (unsigned long long)(unsigned)(b + 1) << 32 | word;
             if (m == I.micro - 1) {
                 if (act && I.phi)
                     I.phi[(size_t)s * rs + i] = V;
                 if (wact && lane == 0)
                     I.raster[(size_t)s * nw + gw] = word;
             }
-            if (b + 1 < B)
-                arrive();
-            cur ^= 1;
+            if (++m == I.micro) {
+                m = 0;
+                ++s;
+            }
+            if (++head == L)
+                head = 0;
+            __syncwarp();  // a lane's next words or ring row after every lane's reads
         }
         if (act) {
             I.V[i] = V;
@@ -501,10 +662,7 @@ __global__ void k_batch_reset(const BInst *inst)
             I.tprev[q] = I.tprev_init;
     }
     for (size_t q = start; q < 2 * (size_t)I.nw; q += stride)
-        I.spk[q] = 0u;
-    if (I.ntype == SP_FLIF_GL)
-        for (size_t k = start; k < (size_t)I.L * I.rs; k += stride)
-            I.ring[k] = I.v_init;
+        I.ll[q] = 0ull;
 }
 
 // out[t][q] = in[t][nid[q]] (0 at holes): states of a column-block instance
@@ -555,9 +713,13 @@ struct sp_batch {
     int device = 0, num_sms = 0, P = 0;
     int P_max = 0;      // CTAs of the grid at full occupancy (P <= P_max)
     int plan_mode = 0;  // schedule family (plan()): set by sp_batch_autotune
-    size_t smem = 0;
+    size_t smem = 0;    // of the grid at full occupancy
+    size_t fixed = 0;   // coefficients, spike words and list
     int lmax = 0;
-    int max_nw = 1, list_cap = 0;
+    int max_nw = 1, spk_bufs = 2, list_cap = 0;
+    bool spread = false;    // the planned launch: plan_spread's, its CTAs, its
+    int grid = 0;           // shared memory
+    size_t grid_smem = 0;
     cudaStream_t stream = nullptr;
     std::vector<sp_host_model> models;
     std::vector<BInst> inst;
@@ -565,7 +727,6 @@ struct sp_batch {
     char *arena = nullptr;
     BInst *d_inst = nullptr;
     int *d_sched = nullptr;  // cta_group | group_start | group_size | job_off | jobs
-    unsigned long long *d_bar = nullptr;
     int *d_err = nullptr;
     int ngroups = 0;
     std::vector<int> cta_group, group_start, group_size, job_off, jobs;
@@ -618,7 +779,7 @@ extern "C" void sp_batch_destroy(sp_batch *b)
     if (b->stream)
         cudaStreamSynchronize(b->stream);
     batch_free_run(b);
-    void *d[] = {b->arena, b->d_inst, b->d_sched, b->d_bar, b->d_err};
+    void *d[] = {b->arena, b->d_inst, b->d_sched, b->d_err};
     for (void *p : d)
         if (p)
             sp_cuda_free(p);
@@ -832,13 +993,130 @@ static bool plan_classes(sp_batch *b, const std::vector<long long> &T, int widen
     return true;
 }
 
-// Schedule families (b->plan_mode): 0 size classes of power-of-two widths,
+// Seconds of one step of instance I with `warps` of its warps per CTA, one CTA per
+// SM, and what each CTA then keeps in `pool` bytes of shared memory: the rings
+// before the column blocks. The figures are step times measured on one B200: the
+// exchange and the update 1.6 us; a ring in shared memory 5.5 ns per lag and warp
+// (10.5 cycles, its loads), streamed 30 ns per lag; the column blocks' walk.
+static double spread_step(const BInst &I, int warps, size_t pool, int *mode, int *region,
+                          size_t *bytes)
+{
+    const bool gl = I.ntype == SP_FLIF_GL;
+    const size_t ring = gl ? ring_bytes(I.L) : 0, coef1 = gl ? (size_t)((I.L + 1) / 2) * 16 : 0;
+    const size_t rows = I.dense ? rows_bytes(I.n, I.wcap) : 0;
+    // up to four warps read the spike words themselves: more of them would poll
+    // the same lines for longer than the CTA barriers take
+    const size_t own = warps <= 4 ? alone_bytes(I.nw, I.dense) : 0;
+    *mode = own ? kAlone : 0;
+    *region = (int)own;
+    *bytes = (gl ? kStageBytes : 0) + warps * own;
+    if (*bytes > pool) {
+        *mode = *region = 0;
+        *bytes = gl ? kStageBytes : 0;
+    }
+    if (gl && coef1 + warps * (*region + ring) <= pool) {
+        *mode |= kRingSmem;
+        *region += (int)ring;
+        *bytes = coef1 + (size_t)warps * *region;
+    }
+    if (I.dense && *bytes + warps * rows <= pool) {
+        *mode |= kRowsSmem;
+        *region += (int)rows;
+        *bytes += warps * rows;
+    }
+    double s = 1.6e-6;
+    if (gl)
+        s += (*mode & kRingSmem) ? 5.5e-9 * I.L * warps : 30e-9 * I.L;
+    if (I.dense)
+        s += ((*mode & kRowsSmem) ? 0.4e-9 : 1.3e-9) * I.n;
+    return s * I.micro;
+}
+
+// One group per instance, all running at once with one CTA per SM: from the
+// fewest CTAs each can have, the instance that would finish last gets more until
+// that gains nothing or no SM is left. false when they do not all fit; they then
+// run in turns, and two CTAs per SM hide more latency than shared memory saves.
+static bool plan_spread(sp_batch *b, const std::vector<long long> &T)
+{
+    const size_t cnt = b->inst.size();
+    const size_t limit = 220 * 1024;
+    if (b->P < b->num_sms || b->fixed + 128 * 1024 > limit)
+        return false;
+    const size_t pool = limit - b->fixed;
+    struct Share {
+        int warps, ctas, mode, region;
+        size_t bytes;
+        double time;
+    };
+    auto share = [&](size_t k, int warps) {
+        const BInst &I = b->inst[k];
+        Share x;
+        x.warps = warps;
+        x.ctas = (I.nw + warps - 1) / warps;
+        x.time = (double)T[k] * spread_step(I, warps, pool, &x.mode, &x.region, &x.bytes);
+        return x;
+    };
+    std::vector<Share> cur(cnt);
+    int used = 0;
+    for (size_t k = 0; k < cnt; ++k) {
+        const int g = min_ctas(b->inst[k]);
+        cur[k] = share(k, (b->inst[k].nw + g - 1) / g);
+        used += cur[k].ctas;
+        if (used > b->num_sms)
+            return false;
+    }
+    for (;;) {
+        size_t last = 0;
+        for (size_t k = 1; k < cnt; ++k)
+            if (cur[k].time > cur[last].time)
+                last = k;
+        // the next narrower share that is faster
+        Share next = cur[last];
+        for (int w = cur[last].warps - 1; w >= 1 && next.time >= cur[last].time; --w)
+            next = share(last, w);
+        if (next.time >= cur[last].time || used - cur[last].ctas + next.ctas > b->num_sms)
+            break;
+        used += next.ctas - cur[last].ctas;
+        cur[last] = next;
+    }
+    b->ngroups = (int)cnt;
+    b->grid = used;
+    b->spread = true;
+    b->grid_smem = 0;
+    b->cta_group.clear();
+    b->group_start.clear();
+    b->group_size.clear();
+    b->job_off.assign(1, 0);
+    b->jobs.clear();
+    for (size_t k = 0; k < cnt; ++k) {
+        BInst &I = b->inst[k];
+        I.mode = cur[k].mode;
+        I.region = cur[k].region;
+        b->group_start.push_back((int)b->cta_group.size());
+        b->group_size.push_back(cur[k].ctas);
+        b->cta_group.insert(b->cta_group.end(), cur[k].ctas, (int)k);
+        b->jobs.push_back((int)k);
+        b->job_off.push_back((int)b->jobs.size());
+        b->grid_smem = std::max(b->grid_smem, b->fixed + cur[k].bytes);
+    }
+    return true;
+}
+
+// Schedule families (b->plan_mode): 0 one group per instance where that fits one
+// CTA per SM, else size classes of power-of-two widths,
 // 1 size classes of the exact minimum widths, 2 size classes of twice the
 // power-of-two widths (fewer, wider groups), 3 list scheduling heaviest first.
 // Each falls back to list scheduling when its classes do not fit the grid.
 static void plan(sp_batch *b, const std::vector<long long> &T)
 {
     const int mode = b->plan_mode;
+    b->grid = b->P;
+    b->grid_smem = b->smem;
+    b->spread = false;
+    for (BInst &I : b->inst)
+        I.mode = I.region = 0;
+    if (mode == 0 && plan_spread(b, T))
+        return;
     if (mode == 0 && plan_classes(b, T, 1, true))
         return;
     if (mode == 1 && plan_classes(b, T, 1, false))
@@ -891,7 +1169,7 @@ extern "C" int sp_batch_create(sp_host_model *models, size_t count, sp_batch **o
     b->inst.resize(count);
     b->w_pos.resize(count);
     struct Off {
-        size_t V, tp, ring, spk, rp, col, w, win, coef, nid, pos, wout, cmo, cw, nro, pro;
+        size_t V, tp, ring, ll, rp, col, w, win, coef, nid, pos, wout, cmo, cw, nro, pro;
     };
     std::vector<Off> off(count);
     std::vector<std::vector<int>> pos(count), nid(count);
@@ -932,7 +1210,7 @@ extern "C" int sp_batch_create(sp_host_model *models, size_t count, sp_batch **o
         o.V = take(rs * 8);
         o.tp = take(rs * 8);
         o.ring = take(I.ntype == SP_FLIF_GL ? rs * (size_t)I.L * 8 : 8);
-        o.spk = take(2 * (size_t)I.nw * 4);
+        o.ll = take(2 * (size_t)I.nw * 8);
         o.rp = take((rs + 1) * 8);
         o.col = take((I.dense || !m.nnz ? 1 : m.nnz) * 4);
         o.w = take((I.dense || !m.nnz ? 1 : m.nnz) * 8);
@@ -950,16 +1228,21 @@ extern "C" int sp_batch_create(sp_host_model *models, size_t count, sp_batch **o
     }
     b->max_nw = (int)max_nw;
     b->list_cap = list_cap;
-    b->smem = (size_t)b->lmax * 8 + max_nw * 4 + (size_t)list_cap * 4 + 16 +
-              (b->lmax > 0 ? (size_t)kHistS * kHistC * kBatchThreads * 8 : 0);
+    const size_t stage = b->lmax > 0 ? kStageBytes : 0;
+    b->fixed = (size_t)b->lmax * 8 + max_nw * 4 + ((size_t)list_cap + 3) * 2 + 32;
+    // a second array of spike words saves a barrier per step
+    b->spk_bufs = b->fixed + max_nw * 4 + stage <= 100 * 1024 ? 2 : 1;
+    b->fixed += (b->spk_bufs - 1) * max_nw * 4;
+    b->smem = b->fixed + stage;
     int rc = SP_OK;
     int per_sm = 0;
-    if (b->smem > 200 * 1024)
+    if ((size_t)b->lmax * 8 + max_nw * 4 + (size_t)list_cap * 4 + 16 + stage > 200 * 1024)
         rc = SP_EINVAL;
-    if (!rc && b->smem > 48 * 1024 && set_max_dynamic_smem((const void *)k_batch) != cudaSuccess)
+    if (!rc && (set_max_dynamic_smem((const void *)k_batch<false>) != cudaSuccess ||
+                set_max_dynamic_smem((const void *)k_batch<true>) != cudaSuccess))
         rc = SP_EINVAL;
     if (!rc) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch, kBatchThreads, b->smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<false>, kBatchThreads, b->smem);
         per_sm = std::min(per_sm, 2);
         if (per_sm < 1)
             rc = SP_EINVAL;
@@ -1036,6 +1319,12 @@ extern "C" int sp_batch_create(sp_host_model *models, size_t count, sp_batch **o
                     run += __builtin_popcount(cmo[(size_t)j * I.nw + q].x);
                 }
             }
+            for (int q = 0; q < I.nw; ++q) {
+                int cnt = 0;
+                for (size_t j = 0; j < m.n; ++j)
+                    cnt += __builtin_popcount(cmo[j * I.nw + q].x);
+                I.wcap = std::max(I.wcap, cnt);
+            }
         }
         size_t e = 0;
         for (size_t q = 0; q < rs; ++q) {
@@ -1058,7 +1347,7 @@ extern "C" int sp_batch_create(sp_host_model *models, size_t count, sp_batch **o
         I.V = (double *)(A + o.V);
         I.tprev = (double *)(A + o.tp);
         I.ring = (double *)(A + o.ring);
-        I.spk = (unsigned *)(A + o.spk);
+        I.ll = (unsigned long long *)(A + o.ll);
         I.row_ptr = (const long long *)(A + o.rp);
         I.col = (const int *)(A + o.col);
         I.w = (const double *)(A + o.w);
@@ -1115,8 +1404,7 @@ extern "C" int sp_batch_create(sp_host_model *models, size_t count, sp_batch **o
         sp_batch_destroy(b);
         return SP_EINTERNAL;
     }
-    if (sp_cuda_malloc(&b->d_bar, (size_t)b->P * sizeof(unsigned long long)) != cudaSuccess ||
-        sp_cuda_malloc(&b->d_err, 4 * sizeof(int)) != cudaSuccess ||
+    if (sp_cuda_malloc(&b->d_err, 4 * sizeof(int)) != cudaSuccess ||
         sp_cuda_malloc(&b->d_inst, count * sizeof(BInst)) != cudaSuccess ||
         cudaMemset(b->d_err, 0, 4 * sizeof(int)) != cudaSuccess) {
         sp_batch_destroy(b);
@@ -1198,23 +1486,23 @@ static int batch_enqueue(sp_batch *b)
     const dim3 rg(64, cnt);
     k_batch_reset<<<rg, 256, 0, b->stream>>>(b->d_inst);
     BK(cudaGetLastError());
-    BK(cudaMemsetAsync(b->d_bar, 0, (size_t)b->P * sizeof(unsigned long long), b->stream));
     BParams p;
-    const int P = b->P, G = b->ngroups;
+    const int P = b->grid, G = b->ngroups;
     p.inst = b->d_inst;
     p.cta_group = b->d_sched;
     p.group_start = b->d_sched + P;
     p.group_size = b->d_sched + P + G;
     p.job_off = b->d_sched + P + 2 * G;
     p.jobs = b->d_sched + P + 3 * G + 1;
-    p.bar = b->d_bar;
     p.err = b->d_err;
     p.lmax = b->lmax;
     p.max_nw = b->max_nw;
+    p.spk_bufs = b->spk_bufs;
     p.list_cap = b->list_cap;
     void *args[] = {&p};
-    BK(cudaLaunchCooperativeKernel((const void *)k_batch, dim3(P), dim3(kBatchThreads), args,
-                                   b->smem, b->stream));
+    BK(cudaLaunchCooperativeKernel(b->spread ? (const void *)k_batch<true>
+                                             : (const void *)k_batch<false>, dim3(P), dim3(kBatchThreads), args,
+                                   b->grid_smem, b->stream));
     k_batch_gather<<<rg, 256, 0, b->stream>>>(b->d_inst);
     BK(cudaGetLastError());
     BK(cudaMemcpyAsync(b->h_ras, b->d_ras_nat, (b->ras_total ? b->ras_total : 1) * 4,

@@ -532,36 +532,44 @@ __device__ __forceinline__ double rowpass_lanes(const uint2 *col, const double *
 // weights, stored in row order, start. The lane of a row walks the list of
 // spiking neurons in ascending order and adds w_ij where its bit is set: the
 // non-zero terms of csr_row_dot (src/sparse.c:68-76) in order, at a cost that
-// follows the spikes of the step and not the edges of the row. Four columns are
-// in flight, the next four's blocks a pass ahead.
-template <bool kShared>
+// follows the spikes of the step and not the edges of the row. C columns are in
+// flight, the next C's blocks a pass ahead: four where other warps fill the gaps,
+// eight for a warp that runs alone.
+template <bool kShared, int C = 4>
 __device__ __forceinline__ double rowpass_cols(const uint2 *blk, const double *w,
                                                const unsigned short *s_list, int cnt, int lane)
 {
     const unsigned below = (1u << lane) - 1u;
-    auto fetch = [&](int t, uint2 (&c)[4]) {
-        const uint2 id = *(const uint2 *)(s_list + t);  // the list is padded to fours
-        const unsigned j[4] = {id.x & 0xffffu, id.x >> 16, id.y & 0xffffu, id.y >> 16};
+    auto fetch = [&](int t, uint2 (&c)[C]) {  // the list is padded to a multiple of C
+        unsigned j[C];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < C; u += 4) {
+            const uint2 id = *(const uint2 *)(s_list + t + u);
+            j[u] = id.x & 0xffffu;
+            j[u + 1] = id.x >> 16;
+            j[u + 2] = id.y & 0xffffu;
+            j[u + 3] = id.y >> 16;
+        }
+#pragma unroll
+        for (int u = 0; u < C; ++u)
             c[u] = t + u >= cnt ? make_uint2(0u, 0u) : (kShared ? blk[j[u]] : __ldg(blk + j[u]));
     };
     double acc = 0.0;
-    uint2 cur[4], nxt[4];
+    uint2 cur[C], nxt[C];
     fetch(0, cur);
-    for (int t = 0; t < cnt; t += 4) {
-        double x[4];
+    for (int t = 0; t < cnt; t += C) {
+        double x[C];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < C; ++u) {
             const double *a = w + cur[u].y + __popc(cur[u].x & below);
             x[u] = 0.0;
             if ((cur[u].x >> lane) & 1u)
                 x[u] = kShared ? *a : __ldg(a);
         }
-        if (t + 4 < cnt)
-            fetch(t + 4, nxt);
+        if (t + C < cnt)
+            fetch(t + C, nxt);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < C; ++u) {
             acc = add(acc, x[u]);  // +0.0 where the row has no such edge
             cur[u] = nxt[u];
         }

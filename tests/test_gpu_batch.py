@@ -217,3 +217,38 @@ def test_batch_runs_after_a_smaller_batch_was_built():
     finally:
         big.close()
         small.close()
+
+
+# (neurons, ring, connectivity) per instance: the smallest rings and sizes, odd
+# ring lengths, rings that fit shared memory beside the column blocks, alone, and
+# not at all, edges walked as column blocks (dense) or CSR rows.
+@pytest.mark.parametrize("shapes", [
+    [(1, 1, 0.5), (2, 2, 0.5), (33, 3, 0.3), (64, 17, 0.1)],
+    [(300, 0, 0.2), (700, 0, 0.002), (257, 0, 0.0)],
+    [(300, 129, 0.1), (1100, 64, 0.15), (500, 300, 0.003)],
+    [(4200, 40, 0.02), (96, 1500, 0.1)],
+    [(60, 0 if k % 3 else 20 + k, 0.2) for k in range(160)],
+])
+def test_batch_forms_match_single_reservoirs(shapes):
+    """Bit for bit, for batches spread one instance per group and, with more
+    instances than SMs, in turns."""
+    rng = np.random.default_rng(len(shapes))
+    cfgs, seeds, us = [], [], []
+    for n, L, conn in shapes:
+        neuron = dict(neuron=sp.FLIF_GL, nparams=gl_params(0.6, L)) if L else \
+            dict(neuron=sp.LIF_DISCRETE, nparams=(0.0, 1.0, 0.1, 0.05))
+        cfgs.append(sp.make_config(n, 2, 1, rho=1.2, ei=0.5, gamma=1.5, conn=conn,
+                                   topo=sp.CONN_RANDOM, **neuron))
+        seeds.append(int(rng.integers(1, 2**31 - 1)))
+        us.append(rng.uniform(-1.0, 2.0, size=(int(rng.integers(20, 90)), 2)))
+    b = sp.Batch(cfgs, seeds)
+    R, V, _ = b.run(us)
+    fired = 0
+    for k in range(0, len(cfgs), 1 if len(cfgs) < 20 else 16):
+        R1, V1 = solo(cfgs[k], seeds[k], us[k])
+        assert np.array_equal(R[k], R1), f"instance {k}: raster differs"
+        assert same_bits(V[k], V1), f"instance {k}: final states differ"
+        fired += int(R1.any())
+    assert fired > 0
+    assert b.info()["groups"] == len(cfgs) or len(cfgs) > 148
+    b.close()
