@@ -18,6 +18,7 @@
 #include <cmath>
 #include <chrono>
 #include "sp_alloc.h"
+#include "sp_stage.h"
 #include "sp_dev.h"
 #include "sp_kernels.cuh"
 #include "sp_dev_internal.h"
@@ -1201,8 +1202,8 @@ extern "C" int sp_ridge_host(const double *h_phi, size_t T, int n, const double 
     RK(sp_cuda_malloc_async(&Phi, T * (size_t)n * sizeof(double), s));
     RK(sp_cuda_malloc_async(&Y, T * (size_t)dout * sizeof(double), s));
     RK(sp_cuda_malloc_async(&Wt, (size_t)n * dout * sizeof(double), s));
-    RK(cudaMemcpyAsync(Phi, h_phi, T * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, s));
-    RK(cudaMemcpyAsync(Y, h_y, T * (size_t)dout * sizeof(double), cudaMemcpyHostToDevice, s));
+    RK(sp_copy_in(Phi, h_phi, T * (size_t)n * sizeof(double), s));
+    RK(sp_copy_in(Y, h_y, T * (size_t)dout * sizeof(double), s));
     RK(cudaStreamSynchronize(s));
     rep->collect_ms = ms_since(t0);
     rc = sp_ridge_phi(s, Phi, n, T, Y, dout, lambda, o, rep, Wt);

@@ -23,6 +23,7 @@
 #include <numeric>
 #include <vector>
 #include "sp_alloc.h"
+#include "sp_stage.h"
 #include "sp_dev.h"
 #include "sp_kernels.cuh"
 #include "sp_dev_internal.h"
@@ -1377,8 +1378,8 @@ extern "C" int sp_dev_run(sp_dev *d, const sp_run_args *a)
             if (a->u_on_device) {
                 u = a->u + t0 * d->din;
             } else if (d->din > 0) {
-                SP_CK(cudaMemcpyAsync(d->d_u, a->u + t0 * d->din, tc * d->din * sizeof(double),
-                                      cudaMemcpyHostToDevice, d->stream));
+                SP_CK(sp_copy_in(d->d_u, a->u + t0 * d->din, tc * d->din * sizeof(double),
+                                 d->stream));
                 u = d->d_u;
             }
         }
@@ -1402,8 +1403,7 @@ extern "C" int sp_dev_run(sp_dev *d, const sp_run_args *a)
             if (rc)
                 return rc;
             if (a->h_phi)
-                SP_CK(cudaMemcpyAsync(a->h_phi + t0 * n, dst, tc * n * sizeof(double),
-                                      cudaMemcpyDeviceToHost, d->stream));
+                SP_CK(sp_copy_out(a->h_phi + t0 * n, dst, tc * n * sizeof(double), d->stream));
         }
         if (want_y) {
             double *Y = a->d_y ? a->d_y + t0 * d->dout : d->d_y;
@@ -1756,7 +1756,7 @@ extern "C" int sp_dev_state_save(sp_dev *d, void *buf)
     for (const auto &it : items) {
         if (!it.ptr || !it.bytes)
             continue;
-        SP_CK(cudaMemcpyAsync(p, it.ptr, it.bytes, cudaMemcpyDeviceToHost, d->stream));
+        SP_CK(sp_copy_out(p, it.ptr, it.bytes, d->stream));
         p += it.bytes;
     }
     SP_CK(cudaStreamSynchronize(d->stream));
@@ -1791,7 +1791,7 @@ extern "C" int sp_dev_state_load(sp_dev *d, const void *buf)
     for (const auto &it : items) {
         if (!it.ptr || !it.bytes)
             continue;
-        SP_CK(cudaMemcpyAsync(it.ptr, p, it.bytes, cudaMemcpyHostToDevice, d->stream));
+        SP_CK(sp_copy_in(it.ptr, p, it.bytes, d->stream));
         p += it.bytes;
     }
     SP_CK(cudaStreamSynchronize(d->stream)); // the caller's buffer may go away

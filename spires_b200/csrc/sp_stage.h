@@ -1,0 +1,11 @@
+// sp_stage.h -- copies between the caller's host memory and the device.
+//
+// Same meaning as cudaMemcpyAsync from or to pageable memory: sp_copy_in returns
+// when the source has been read (the device copy may still run on the stream),
+// sp_copy_out when the destination holds the data.
+#pragma once
+#include <cuda_runtime.h>
+#include <cstddef>
+
+cudaError_t sp_copy_in(void *dev, const void *host, size_t bytes, cudaStream_t s);
+cudaError_t sp_copy_out(void *host, const void *dev, size_t bytes, cudaStream_t s);
