@@ -681,6 +681,27 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// A CTA's copy of n 8-byte words into shared memory, asynchronous, in 16-byte
+// pieces where both sides are aligned; commit and wait by the caller. The start of
+// a launch is these copies (67 KB of column blocks per CTA for LIF_DISCRETE N=1000,
+// conn 0.1): loaded and stored, a few at a time by the CTA's few threads, they
+// took most of a one-step launch (33.6 us; now 13.0, N=4000 conn 0.05 83 -> 15).
+__device__ __forceinline__ void stage_words(void *dst, const void *src, int n)
+{
+    const bool wide = ((smem_u32(dst) | (unsigned)(uintptr_t)src) & 15u) == 0;
+    int k = threadIdx.x;
+    if (wide) {
+        for (; k < n / 2; k += blockDim.x)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             smem_u32((char *)dst + 16 * (size_t)k)),
+                         "l"((const char *)src + 16 * (size_t)k)
+                         : "memory");
+        k = (n & ~1) + threadIdx.x;
+    }
+    for (; k < n; k += blockDim.x)
+        cp_async8((char *)dst + 8 * (size_t)k, (const char *)src + 8 * (size_t)k);
+}
+
 // Four consecutive doubles from a 32-byte boundary in one load.
 __device__ __forceinline__ void ld_f64x4(const double *p, double (&v)[4])
 {
@@ -917,26 +938,24 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     }
     if (p.coef_smem && NT == SP_FLIF_CAPUTO && tid < 8)
         s_coef[tid < 4 ? tid - 4 : L + tid - 4] = 0.0;
-    if (p.coef_smem)
-        for (int k = tid; k < L; k += blockDim.x) {
-            const double c = p.coef[k + (NT == SP_FLIF_CAPUTO ? 4 : 0)];
-            s_coef[k] = c;
-            if (kPairs && k > 0)
-                s_coef1[k - 1] = c;
-        }
+    if (p.coef_smem) {
+        stage_words(s_coef, p.coef + (NT == SP_FLIF_CAPUTO ? 4 : 0), L);
+        if (kPairs && L > 1)
+            stage_words(s_coef1, p.coef + 1, L - 1);
+    }
     if (ST == SP_SYN_SIMPLE && p.ell_cap > 0) {
         const int g0 = __ldg(p.ell_off + wb0), ng = __ldg(p.ell_off + wb1) - g0;  // <= ell_cap
-        for (int k = tid; k < 32 * ng; k += blockDim.x)
-            s_ell_col[k] = __ldg(p.ell_col + (size_t)32 * g0 + k);
-        for (int k = tid; k < 128 * ng; k += blockDim.x)
-            s_ell_w[k] = __ldg(p.ell_w + (size_t)128 * g0 + k);
+        stage_words(s_ell_col, p.ell_col + (size_t)32 * g0, 32 * ng);
+        stage_words(s_ell_w, p.ell_w + (size_t)128 * g0, 128 * ng);
         if (wb1 > wb0) {
             const int t0 = __ldg(p.tail_rp + (size_t)33 * wb0);
             const int nt = __ldg(p.tail_rp + (size_t)33 * wb1 - 1) - t0;  // <= tail_cap
-            for (int k = tid; k < nt; k += blockDim.x) {
-                s_tail_col[k] = __ldg(p.tail_col + t0 + k);
-                s_tail_w[k] = __ldg(p.tail_w + t0 + k);
-            }
+            stage_words(s_tail_w, p.tail_w + t0, nt);
+            for (int k = tid; k < nt; k += blockDim.x)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                 smem_u32(s_tail_col + k)),
+                             "l"(p.tail_col + t0 + k)
+                             : "memory");
             for (int k = tid; k < 33 * (wb1 - wb0); k += blockDim.x)
                 s_tail_rp[k] = __ldg(p.tail_rp + (size_t)33 * wb0 + k) - t0;
         }
@@ -946,16 +965,14 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             s_bits[k] = 0u;
         if (p.col_mode == 2) {
             const int w0 = __ldg(p.col_off + wb0), nwt = __ldg(p.col_off + wb1) - w0;  // <= col_cap
-            for (int k = tid; k < nwt; k += blockDim.x)
-                s_col_w[k] = __ldg(p.col_w + w0 + k);
-            for (int k = tid; k < (wb1 - wb0) * p.n; k += blockDim.x)
-                s_col_blk[k] = __ldg(p.col_blk + (size_t)wb0 * p.n + k);
+            stage_words(s_col_w, p.col_w + w0, nwt);
+            stage_words(s_col_blk, p.col_blk + (size_t)wb0 * p.n, (wb1 - wb0) * p.n);
         }
     }
     if (p.win_smem)
         for (int k = tid; k < p.din * S_b; k += blockDim.x) {
             const int q = k / p.din, j = k - q * p.din;
-            s_win[(size_t)j * NC + q] = __ldg(p.W_in + (size_t)(lo + q) * p.din + j);
+            cp_async8(s_win + (size_t)j * NC + q, p.W_in + (size_t)(lo + q) * p.din + j);
         }
     if (VAR == 3)  // a number that no barrier of this launch carries
         for (int k = tid; k < 2 * p.nwords; k += blockDim.x)
@@ -969,6 +986,8 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
     }
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
     if (VAR == 3)
         cluster_sync();  // every CTA's entries are set before anyone writes one
@@ -1225,10 +1244,12 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     }
     const double coef1 = NT == SP_FLIF_GL && L > 1 ? __ldg(p.coef + 1) : 0.0;
     if (VAR >= 2 && NT == SP_FLIF_GL && wact) {
-        // every thread fills and reads its own column only
-#pragma unroll 16
+        // every thread fills and reads its own column only, the whole of it in flight
+#pragma unroll 8
         for (int r = 0; r < L; ++r)
-            ring_at(r) = __ldcg(p.ring + (size_t)r * p.rs + i);
+            cp_async8(&ring_at(r), p.ring + (size_t)r * p.rs + i);
+        cp_async_commit();
+        cp_async_wait<0>();
     }
     if (act) {
         if (NT == SP_FLIF_CAPUTO)
