@@ -22,6 +22,7 @@ struct sp_dev {
     int smem_max;  // opt-in shared memory per CTA
     int cluster_max;  // largest cluster the device schedules (16, 8 or 0)
     int l2_hinted; // a launch read the ring with evict-last hints (demoted at destroy)
+    int *h_mail;   // pinned, device-visible: error words [4], then one output row [dout]
     cudaStream_t stream;
     int n, din, dout, micro;
     int nw;              // warps of positions (= spike words in position space)

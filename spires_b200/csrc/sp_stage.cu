@@ -148,3 +148,54 @@ cudaError_t sp_copy_out(void *host, const void *dev, size_t bytes, cudaStream_t 
         cudaStreamSynchronize(s);
     return e;
 }
+
+// 256 slots of 256 bytes, made by the first that is taken (a cudaHostAlloc of its
+// own per reservoir would cost each one 2.5 ms) and given back when the library is
+// unloaded.
+namespace {
+
+constexpr int kMailSlots = 256;
+constexpr size_t kMailBytes = 256;
+
+struct Mail {
+    std::mutex m;
+    char *p = nullptr;
+    bool refused = false;
+    bool used[kMailSlots] = {};
+    ~Mail()
+    {
+        if (p)
+            cudaFreeHost(p);
+    }
+};
+Mail g_mail;
+
+}  // namespace
+
+void *sp_mail_take(size_t bytes)
+{
+    if (bytes > kMailBytes)
+        return nullptr;
+    std::lock_guard<std::mutex> lock(g_mail.m);
+    if (!g_mail.p && !g_mail.refused &&
+        cudaHostAlloc((void **)&g_mail.p, kMailSlots * kMailBytes,
+                      cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        g_mail.p = nullptr;
+        g_mail.refused = true;
+    }
+    for (int k = 0; g_mail.p && k < kMailSlots; ++k)
+        if (!g_mail.used[k]) {
+            g_mail.used[k] = true;
+            return g_mail.p + k * kMailBytes;
+        }
+    return nullptr;
+}
+
+void sp_mail_give(void *slot)
+{
+    if (!slot)
+        return;
+    std::lock_guard<std::mutex> lock(g_mail.m);
+    g_mail.used[((char *)slot - g_mail.p) / kMailBytes] = false;
+}

@@ -9,3 +9,9 @@
 
 cudaError_t sp_copy_in(void *dev, const void *host, size_t bytes, cudaStream_t s);
 cudaError_t sp_copy_out(void *host, const void *dev, size_t bytes, cudaStream_t s);
+
+// A little host memory that the device can write, from a pool of the process; null
+// when none is left or `bytes` is more than a slot's. Give it back when nothing on
+// the device can still write it.
+void *sp_mail_take(size_t bytes);
+void sp_mail_give(void *slot);

@@ -51,3 +51,28 @@ def test_fits_from_several_threads():
         t.join()
     for a, b in out:
         assert np.array_equal(a, ref) and np.array_equal(b, small)
+
+
+@pytest.mark.parametrize("dout", [1, 30, 31])
+def test_outputs_of_many_reservoirs(dout):
+    """The largest output row of a mail slot and one more, more reservoirs than
+    slots, and slots taken again: the outputs of a run."""
+    cfg = sp.make_config(40, 1, dout, rho=0.9, conn=0.2, topo=sp.CONN_RANDOM,
+                         neuron=sp.LIF_DISCRETE, nparams=(0.0, 1.0, 0.1, 0.05))
+    u = np.random.default_rng(3).uniform(0, 2, (6, 1))
+    one = sp.Reservoir(cfg, seed=9)
+    y = one.run(u)
+    rs = [sp.Reservoir(cfg, seed=9) for _ in range(260 if dout == 1 else 3)]
+    for k in range(2):
+        for r in rs:
+            r.reset()
+            for t in range(len(u)):
+                r.step(u[t])
+            assert np.array_equal(r.output(), y[-1])
+        if k == 0:
+            for r in rs[::2]:
+                r.close()
+            rs = rs[1::2] + [sp.Reservoir(cfg, seed=9) for _ in range(3)]
+    for r in rs:
+        r.close()
+    one.close()
