@@ -423,6 +423,16 @@ static size_t coef_smem_bytes(const sp_dev *d)
     return b <= 64 * 1024 ? b : 0;
 }
 
+// FRACTIONAL synapse coefficients in shared memory, up to 32 KB: the synapse's
+// history then passes through the ring's stages
+static size_t scoef_smem_bytes(const sp_dev *d)
+{
+    if (d->stype != SP_SYN_FRAC)
+        return 0;
+    const size_t b = ((size_t)d->sc.frac_L * 8 + 127) & ~(size_t)127;
+    return b <= 32 * 1024 ? b : 0;
+}
+
 // dynamic shared memory of a launch shape: two buffers of spike words, the
 // recurrent rows, the input weights where they fit, then (variant 1) the
 // coefficients, the ring-row stages and their full/empty mbarriers
@@ -450,13 +460,13 @@ static bool stages_coef(const sp_dev *d, int kv)
 static int extra_warps(int kv) { return kv == 1 ? 2 : kv == 2 ? 1 : 0; }
 
 struct SmemPlan {
-    int win_smem, u_ring;
+    int win_smem, u_ring, frac_stage;
     size_t bytes;
 };
 
 static SmemPlan smem_plan(const sp_dev *d, const sp_launch &l, int kv)
 {
-    SmemPlan pl = {0, 0, 0};
+    SmemPlan pl = {0, 0, 0, 0};
     size_t b = spk_smem_bytes(d) + row_plan(d, l).bytes;
     if (kv == 3)
         b += ((size_t)16 * d->nwords + 127) / 128 * 128;
@@ -470,6 +480,12 @@ static SmemPlan smem_plan(const sp_dev *d, const sp_launch &l, int kv)
         box_geometry(d, l, &bw, &nbx);
         b += (size_t)l.stages * nbx * l.rows * bw * sizeof(double) +
              2 * (size_t)l.stages * sizeof(unsigned long long);
+        const size_t sc = scoef_smem_bytes(d);
+        if (sc > 0 && d->sc.frac_L >= (l.rows < d->nc.L ? l.rows : d->nc.L) &&
+            b + sc + 1024 <= (size_t)d->smem_max) {
+            pl.frac_stage = 1;
+            b += sc;
+        }
     }
     if (d->din > 0 && d->din <= 32) {
         const size_t u = ((size_t)l.warps_max * kURows * d->din * 8 + 127) / 128 * 128;
@@ -555,7 +571,7 @@ typedef CUresult (*encode_tiled_fn)(CUtensorMap *, CUtensorMapDataType, cuuint32
                                     const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// Tiled map of the FLIF_GL ring: dims {rs, L}, row pitch rs*8 bytes, box
+// Tiled maps of the FLIF_GL ring and of the FRACTIONAL synapse's: dims {rs, L}, row pitch rs*8 bytes, box
 // {bw, r}; out-of-range rows/columns of a box read as zero.
 static int encode_ring_map(sp_dev *d, int bw, int r)
 {
@@ -586,6 +602,12 @@ static int encode_ring_map(sp_dev *d, int bw, int r)
     CUresult res = enc(&d->tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, d->ring, dims, strides, box,
                        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, promo,
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (res == CUDA_SUCCESS && d->Iring && d->sc.frac_L >= r) {
+        dims[1] = (cuuint64_t)d->sc.frac_L;
+        res = enc(&d->tmap_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, d->Iring, dims, strides, box,
+                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, promo,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
     if (res != CUDA_SUCCESS)
         return SP_EINTERNAL;
     d->tmap_bw = bw;
@@ -681,7 +703,8 @@ static void default_launch(sp_dev *d)
             box_geometry(d, v, &bw, &nbx);
             const size_t stage = (size_t)v.rows * nbx * bw * sizeof(double);
             const size_t budget = (size_t)(d->smem_max - 2 * 1024);
-            const size_t spk = spk_smem_bytes(d) + coef_smem_bytes(d) + row_plan(d, v).bytes;
+            const size_t spk = spk_smem_bytes(d) + coef_smem_bytes(d) + scoef_smem_bytes(d) +
+                               row_plan(d, v).bytes;
             long long st = budget > spk ? (long long)((budget - spk) / (stage + 16)) : 0;
             if (st > 16)
                 st = 16;
@@ -1276,6 +1299,9 @@ extern "C" int sp_dev_launch_chunk(sp_dev *d, const double *u, size_t T, double 
     p.win_smem = sm.win_smem;
     p.u_ring = sm.u_ring && u && d->gamma != 0.0;
     p.coef_smem = stages_coef(d, kv);
+    p.frac_stage = sm.frac_stage;
+    if (sm.frac_stage)
+        p.tmap_s = d->tmap_s;
     // consumer warps, then the producer and gather warps
     dim3 grid(l.ctas), block(32 * (l.warps_max + extra_warps(kv)));
     if (smem > 48 * 1024)

@@ -96,7 +96,7 @@ struct sp_dev {
     long long last_err_step;
 
     // 2-D tiled tensor map over the FLIF_GL ring (variant 1), box BW x R
-    CUtensorMap tmap;
+    CUtensorMap tmap, tmap_s;  // FLIF_GL ring, FRACTIONAL synapse's ring
     int tmap_bw, tmap_r;
 };
 

@@ -151,6 +151,10 @@ struct KP {
     // variant 1: 2-D tiled map of the ring [L rows][rs columns] of doubles,
     // box = BW columns x R rows
     alignas(64) CUtensorMap tmap;
+    // variant 1, FRACTIONAL: the synapse's history passes through the same stages,
+    // its coefficients staged in shared memory
+    alignas(64) CUtensorMap tmap_s;
+    int frac_stage;
 };
 
 // ------------------------------------------------------------ PTX helpers
@@ -919,12 +923,15 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     // (FLIF_CAPUTO: four places of padding before and after the table)
     double *s_coef = (double *)(smem + spk_bytes) + (NT == SP_FLIF_CAPUTO ? 4 : 0);
     double *s_coef1 = (double *)(smem + spk_bytes + coef_one);
-    double *s_stage = (double *)(smem + spk_bytes + coef_bytes);
+    double *s_scoef = (double *)(smem + spk_bytes + coef_bytes);
+    const size_t scoef_bytes =
+        ST == SP_SYN_FRAC && p.frac_stage ? ((size_t)p.Ls * 8 + 127) / 128 * 128 : 0;
+    double *s_stage = (double *)(smem + spk_bytes + coef_bytes + scoef_bytes);
     // variants 2 and 3: the thread's column of its warp's ring block (chain_pairs)
     double2 *s_ring = (double2 *)s_stage + (size_t)warp * ((L + 1) / 2) * 32 + lane;
     auto ring_at = [&](int r) -> double & { return *((double *)(s_ring + (r >> 1) * 32) + (r & 1)); };
     const size_t STAGE = (size_t)p.NBX * p.R * p.BW;  // doubles per stage
-    unsigned long long *full = (unsigned long long *)(smem + spk_bytes + coef_bytes +
+    unsigned long long *full = (unsigned long long *)(smem + spk_bytes + coef_bytes + scoef_bytes +
                                                       (size_t)p.NST * STAGE * sizeof(double));
     unsigned long long *empty = full + p.NST;
     const int lo = wb0 * 32;
@@ -943,6 +950,8 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         if (kPairs && L > 1)
             stage_words(s_coef1, p.coef + 1, L - 1);
     }
+    if (scoef_bytes > 0)
+        stage_words(s_scoef, p.scoef, p.Ls);
     if (ST == SP_SYN_SIMPLE && p.ell_cap > 0) {
         const int g0 = __ldg(p.ell_off + wb0), ng = __ldg(p.ell_off + wb1) - g0;  // <= ell_cap
         stage_words(s_ell_col, p.ell_col + (size_t)32 * g0, 32 * ng);
@@ -1122,17 +1131,68 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         const unsigned long long pol_in = l2_policy(true);
         const unsigned long long pol_out = l2_policy(false);
         int rh0 = (int)(((p.step0 - 2 - RL) % L + L) % L);  // row of the first streamed lag
+        // lags k .. lim of a ring of `len` rows, lag k in row rh: a stage holds one
+        // contiguous ascending row range (split at the wrap)
+        auto issue = [&](const CUtensorMap *map, int k, int lim, int rh, int len, int pin,
+                         long long g) {
+            while (k <= lim && ok) {
+                int cnt = lim - k + 1;
+                if (cnt > p.R)
+                    cnt = p.R;
+                if (cnt > rh + 1)
+                    cnt = rh + 1;
+                const int y0 = rh - cnt + 1;
+                if (rounds > 0 &&
+                    !mbar_wait(&empty[st], (unsigned)((rounds - 1) & 1), &s_abort, p.err,
+                               p.tmo, g)) {
+                    ok = false;
+                    break;
+                }
+                mbar_expect_tx(&full[st], (unsigned)(nbox * p.RB * p.BW * 8));
+                double *dst = s_stage + (size_t)st * STAGE;
+                if (p.l2_pin > 0) {
+                    // the oldest `pin` lags stay resident: a row is read
+                    // evict-first while young and turns evict-last when it
+                    // reaches lag len - pin (one row per step comes back from
+                    // DRAM for that)
+                    const unsigned long long pol = k + cnt > len - pin ? pol_in : pol_out;
+                    for (int c = 0; c < nbox; ++c)
+                        tma_load_2d_hint(dst + (size_t)c * p.R * p.BW, map, lo + c * p.BW, y0,
+                                         &full[st], pol);
+                } else {
+                    for (int c = 0; c < nbox; ++c)
+                        tma_load_2d(dst + (size_t)c * p.R * p.BW, map, lo + c * p.BW, y0,
+                                    &full[st]);
+                }
+                ++q;
+                if (++st == p.NST) {
+                    st = 0;
+                    ++rounds;
+                }
+                k += cnt;
+                rh -= cnt;
+                if (rh < 0)
+                    rh += len;
+            }
+        };
         for (long long b = 0; b < B && ok; ++b, rh0 = rh0 + 1 == L ? 0 : rh0 + 1) {
             const long long g = p.step0 + b;
             const int lim = (int)(g < L ? g : L - 1);
-            if (lim < 2 + RL)
+            const long long gs = p.syn_step0 + b + 1;  // FRACTIONAL: the current formed in step b
+            const int slim = ST == SP_SYN_FRAC && p.frac_stage && b + 1 < B
+                                 ? (int)(gs < p.Ls ? gs : p.Ls - 1)
+                                 : 0;
+            if (lim < 2 + RL && slim < 2)
                 continue;
-            if (b >= 2) {
-                // rows of step g are states of steps <= g-2
+            if (b >= 2 || (b == 1 && slim >= 2)) {
+                // rows of step g are states of steps <= g-2; the synapse's newest
+                // row is the current of step b-1, formed at the end of step b-2
+                // or (b = 1) before step 0
                 unsigned long long t0 = globaltimer_ns();
                 unsigned polls = 0;
                 // (kWords: every consumer warp counts its own steps)
-                const unsigned need = (unsigned)(b - 1) * (unsigned)(kWords ? wb1 - wb0 : 1);
+                const unsigned need =
+                    (unsigned)(b >= 2 ? b - 1 : 1) * (unsigned)(kWords ? wb1 - wb0 : 1);
                 while ((int)((unsigned)ld_acquire_cta(&s_done) - need) < 0) {
                     if ((++polls & 63u) == 0) {
                         if (s_abort || ld_volatile_i32(p.err) != kErrNone) {
@@ -1151,49 +1211,10 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                 if (!ok)
                     break;
             }
-            // lags k..k+cnt-1 are rows rh down to rh-cnt+1: one contiguous
-            // ascending row range per stage (split at the wrap)
             SP_STAMP(true, b, B, 7);
-            int rh = rh0;
-            for (int k = 2 + RL; k <= lim && ok;) {
-                int cnt = lim - k + 1;
-                if (cnt > p.R)
-                    cnt = p.R;
-                if (cnt > rh + 1)
-                    cnt = rh + 1;
-                const int y0 = rh - cnt + 1;
-                if (rounds > 0 &&
-                    !mbar_wait(&empty[st], (unsigned)((rounds - 1) & 1), &s_abort, p.err,
-                               p.tmo, g)) {
-                    ok = false;
-                    break;
-                }
-                mbar_expect_tx(&full[st], (unsigned)(nbox * p.RB * p.BW * 8));
-                double *dst = s_stage + (size_t)st * STAGE;
-                if (p.l2_pin > 0) {
-                    // the oldest l2_pin lags stay resident: a row is read
-                    // evict-first while young and turns evict-last when it
-                    // reaches lag L - l2_pin (one row per step comes back
-                    // from DRAM for that)
-                    const unsigned long long pol = k + cnt > L - p.l2_pin ? pol_in : pol_out;
-                    for (int c = 0; c < nbox; ++c)
-                        tma_load_2d_hint(dst + (size_t)c * p.R * p.BW, &p.tmap, lo + c * p.BW,
-                                         y0, &full[st], pol);
-                } else {
-                    for (int c = 0; c < nbox; ++c)
-                        tma_load_2d(dst + (size_t)c * p.R * p.BW, &p.tmap, lo + c * p.BW, y0,
-                                    &full[st]);
-                }
-                ++q;
-                if (++st == p.NST) {
-                    st = 0;
-                    ++rounds;
-                }
-                k += cnt;
-                rh -= cnt;
-                if (rh < 0)
-                    rh += L;
-            }
+            if (slim >= 2)
+                issue(&p.tmap_s, 2, slim, (int)((gs - 2) % p.Ls), p.Ls, 0, g);
+            issue(&p.tmap, 2 + RL, lim, rh0, L, p.l2_pin, g);
         }
         // every issued copy must land before the CTA may exit
         const unsigned long long t0 = globaltimer_ns();
@@ -1275,14 +1296,82 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     int cst = 0, cph = 0;  // variant 1: stage consumed next and its phase parity
     double ext = 0.0;
 
+    // this thread's column in a stage
+    const int boff = VAR == 1 ? (tid / p.BW) * p.R * p.BW + (tid % p.BW) : 0;
+    // Variant 1: sum + lags k .. lim of a ring of `len` rows (lag k in row rh) from
+    // the stages, in ascending order; `use` false only passes the stages on.
+    auto stage_hist = [&](double hist, const double *cf, int k, int lim, int rh, int len, bool use,
+                          long long g) -> double {
+        while (k <= lim && S_b > 0) {
+            int cnt = lim - k + 1;
+            if (cnt > p.R)
+                cnt = p.R;
+            if (cnt > rh + 1)
+                cnt = rh + 1;
+            // on a failed wait the launch aborts at the next barrier_wait;
+            // every consumer keeps the same control flow until then
+            const bool landed = mbar_wait(&full[cst], (unsigned)cph, &s_abort, p.err, p.tmo, g);
+            const double *buf = s_stage + (size_t)cst * STAGE + boff;
+            if (landed && use) {
+                if ((cnt & 15) == 0) {
+                    // full stages of 16, 32 or 64 rows: 16 lags at a time
+                    // with their loads batched, still in ascending lag
+                    // order (lag k + jr sits at row offset cnt-1-jr)
+                    for (int h = 0; h < cnt; h += 16)
+                        hist = stage_sum<16>(hist, cf + k + h,
+                                             buf + (size_t)(cnt - 16 - h) * p.BW, p.BW);
+                } else if ((cnt & 7) == 0) {
+                    // stages of 24, 40, 48 or 56 rows: 16 at a time, then 8
+                    int h = 0;
+                    for (; h + 16 <= cnt; h += 16)
+                        hist = stage_sum<16>(hist, cf + k + h,
+                                             buf + (size_t)(cnt - 16 - h) * p.BW, p.BW);
+                    for (; h < cnt; h += 8)
+                        hist = stage_sum<8>(hist, cf + k + h,
+                                            buf + (size_t)(cnt - 8 - h) * p.BW, p.BW);
+                } else {
+                    for (int jr = 0; jr < cnt; ++jr)
+                        hist = add(hist, mul(cf[k + jr], buf[(size_t)(cnt - 1 - jr) * p.BW]));
+                }
+            }
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&empty[cst]);
+            if (++cst == p.NST) {
+                cst = 0;
+                cph ^= 1;
+            }
+            k += cnt;
+            rh -= cnt;
+            if (rh < 0)
+                rh += len;
+        }
+        return hist;
+    };
+
     // FRACTIONAL: history sum of the current of micro-step b, whose row is
     // shead. It needs the currents up to step b - 1 only, not the spikes of
     // that step, so it is formed before the barrier, while the other CTAs
-    // finish: with one load in flight after the update it took 60 of the 86 us
-    // per step at N=20000, 512 lags.
+    // finish. Variant 1 takes it from the ring's stages where its coefficients
+    // fit shared memory: the bulk copies keep more bytes in flight than the
+    // threads' loads, sixteen each. (N=20000, 512 lags beside a ring of 1024: 86
+    // us per step with one load in flight after the update, 69 with sixteen
+    // before the barrier, 46 through the stages; the two histories are 245 MB.)
     double fhist = 0.0;
     int shead = ST == SP_SYN_FRAC ? (int)(p.syn_step0 % p.Ls) : 0;
+    int srow = shead;  // its row, counted by empty lanes too
     auto frac_history = [&](long long b) {
+        if (VAR == 1 && p.frac_stage && b > 0) {
+            const long long gs = p.syn_step0 + b;
+            const int lim = (int)(gs < p.Ls ? gs : p.Ls - 1);
+            srow = srow + 1 == p.Ls ? 0 : srow + 1;
+            fhist = 0.0;
+            if (lim >= 1)
+                fhist = add(fhist, mul(s_scoef[1], Ilast));
+            fhist = stage_hist(fhist, s_scoef, 2, lim, srow >= 2 ? srow - 2 : srow - 2 + p.Ls, p.Ls,
+                               act, p.step0 + b - 1);
+            return;
+        }
         if (!act)
             return;
         const long long gs = p.syn_step0 + b;
@@ -1485,7 +1574,6 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
 
     // step-invariant places and the counters that follow the step (64-bit
     // divisions cost hundreds of cycles each)
-    const int boff = VAR == 1 ? (tid / p.BW) * p.R * p.BW + (tid % p.BW) : 0;
     // Column blocks: the spiking neurons of the barrier's words as an ascending
     // list (all consumers; returns the count). The words are in position order,
     // so the neurons' bits are collected in neuron order first; every thread then
@@ -1634,51 +1722,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                 int rh = head - 2 - RL;
                 while (rh < 0)
                     rh += L;
-                for (int k = 2 + RL; k <= lim && S_b > 0;) {
-                    int cnt = lim - k + 1;
-                    if (cnt > p.R)
-                        cnt = p.R;
-                    if (cnt > rh + 1)
-                        cnt = rh + 1;
-                    // on a failed wait the launch aborts at the next barrier_wait;
-                    // every consumer keeps the same control flow until then
-                    const bool landed = mbar_wait(&full[cst], (unsigned)cph, &s_abort, p.err, p.tmo, g);
-                    const double *buf = s_stage + (size_t)cst * STAGE + boff;
-                    if (landed && act && integ) {
-                        if ((cnt & 15) == 0) {
-                            // full stages of 16, 32 or 64 rows: 16 lags at a time
-                            // with their loads batched, still in ascending lag
-                            // order (lag k + jr sits at row offset cnt-1-jr)
-                            for (int h = 0; h < cnt; h += 16)
-                                hist = stage_sum<16>(hist, cf + k + h,
-                                                     buf + (size_t)(cnt - 16 - h) * p.BW, p.BW);
-                        } else if ((cnt & 7) == 0) {
-                            // stages of 24, 40, 48 or 56 rows: 16 at a time, then 8
-                            int h = 0;
-                            for (; h + 16 <= cnt; h += 16)
-                                hist = stage_sum<16>(hist, cf + k + h,
-                                                     buf + (size_t)(cnt - 16 - h) * p.BW, p.BW);
-                            for (; h < cnt; h += 8)
-                                hist = stage_sum<8>(hist, cf + k + h,
-                                                    buf + (size_t)(cnt - 8 - h) * p.BW, p.BW);
-                        } else {
-                            for (int jr = 0; jr < cnt; ++jr)
-                                hist = add(hist, mul(cf[k + jr],
-                                                     buf[(size_t)(cnt - 1 - jr) * p.BW]));
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0)
-                        mbar_arrive(&empty[cst]);
-                    if (++cst == p.NST) {
-                        cst = 0;
-                        cph ^= 1;
-                    }
-                    k += cnt;
-                    rh -= cnt;
-                    if (rh < 0)
-                        rh += L;
-                }
+                hist = stage_hist(hist, cf, 2 + RL, lim, rh, L, act && integ, g);
             }
         }
 
@@ -1849,6 +1893,8 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         if (b + 1 < B) {
             if (!kWords) {
                 prepare(b + 1, cur ^ 1);
+                if (VAR == 1 && ST == SP_SYN_FRAC && p.frac_stage)
+                    fence_proxy_async();  // the current just written is lag 2 of a bulk copy
                 barrier_arrive(b + 1);
                 if (VAR == 1 && tid == 0)
                     st_release_cta(&s_done, (int)(b + 1));

@@ -103,3 +103,25 @@ def test_cluster_wait_runs_out(conn):
     phi_o, ras_o, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=17)).run(u)
     assert np.array_equal(sp.unpack_raster(R, 2000), ras_o)
     assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
+
+
+# synapse lags: fewer than a stage holds (read by the consumers), a stage, one more,
+# several with a ragged last one; the neuron's ring shorter and longer than that
+@pytest.mark.parametrize("Ls", [3, 16, 17, 40, 75])
+@pytest.mark.parametrize("L", [16, 90])
+@pytest.mark.parametrize("rows,stages", [(16, 2), (8, 5)])
+def test_fractional_history_through_the_pipeline(Ls, L, rows, stages):
+    """FLIF_GL with the FRACTIONAL synapse, both rings in the pipeline's stages,
+    through ramp-up and wrap and over several launches."""
+    n, T = 230, 2 * max(L, Ls) + 30
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=0.05, dt=1.0,
+                         topo=sp.CONN_RANDOM, neuron=sp.FLIF_GL, nparams=GL(L),
+                         synapse=sp.SYN_FRAC, sparams=(0.6, 4.0, float(Ls)))
+    u = np.random.default_rng(3).uniform(-1.0, 1.5, (T, 2))
+    r = sp.Reservoir(cfg, seed=11)
+    assert r.set_launch(ctas=4, warps_max=2, variant=1, rows=rows, stages=stages) == sp.SPIRES_OK
+    parts = [r.run_record(x) for x in (u[:7], u[7:8], u[8:10], u[10:])]
+    r.close()
+    phi = np.concatenate([p[0] for p in parts])
+    phi_o, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=11)).run(u)
+    assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
