@@ -1619,6 +1619,89 @@ static int batch_readout(sp_batch *b, const BInst &I, const double *phi, size_t 
     return rc;
 }
 
+// Ridge fits of every instance's recorded states, rows [washout, T_fit[k]), in
+// parts of at most 1 GB of states and working memory (an instance beyond that by
+// itself): the fits of a part share launches and waits (sp_ridge_phi_many). After
+// a part, done(k, states, status, W) for each of its instances, W [dout][n] on the
+// device: the solution, or work space when the system was singular.
+template <typename Done>
+static int batch_fit(sp_batch *b, const double *const *y, const size_t *T_fit,
+                     const double *lambda, const sp_ridge_opts *o, Done done)
+{
+    const size_t cnt = b->inst.size();
+    auto pad = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    std::vector<size_t> po(cnt);
+    for (size_t k = 0, at = 0; k < cnt; ++k) {
+        po[k] = at;
+        at += (size_t)b->T[k] * b->inst[k].rs;
+    }
+    int rc = SP_OK;
+    sp_ridge_ws *ws = sp_ridge_ws_new();  // one set of solver buffers for fits that go alone
+    size_t limit = (size_t)1 << 30;
+    for (size_t k0 = 0; k0 < cnt && !rc;) {
+        // instances k0 .. k1 - 1
+        std::vector<size_t> off(1, 0);
+        size_t k1 = k0, work = 0;
+        for (; k1 < cnt; ++k1) {
+            const size_t n = b->inst[k1].n, dout = b->models[k1].dout, t = T_fit[k1];
+            const size_t own = dout ? pad(t * n * 8) + pad(t * dout * 8) + pad(n * dout * 8) : 0;
+            work += dout ? sp_ridge_item_bytes((int)n, t, (int)dout) : 0;
+            if (k1 > k0 && off.back() + own + work > limit)
+                break;
+            off.push_back(off.back() + own);
+        }
+        char *slab = nullptr;
+        if (sp_cuda_malloc_async(&slab, off.back() ? off.back() : 256, b->stream) != cudaSuccess) {
+            cudaGetLastError();
+            if (k1 - k0 > 1) {
+                limit = 0;  // no room for a part: one instance at a time
+                continue;
+            }
+            rc = SP_EALLOC;
+        }
+        std::vector<sp_ridge_item> items;
+        std::vector<size_t> which;
+        for (size_t k = k0; k < k1 && !rc; ++k) {
+            const BInst &I = b->inst[k];
+            const size_t n = I.n, dout = b->models[k].dout, t = T_fit[k];
+            if (dout == 0)
+                continue;
+            double *nat = (double *)(slab + off[k - k0]);
+            double *Y = (double *)((char *)nat + pad(t * n * 8));
+            double *W = (double *)((char *)Y + pad(t * dout * 8));
+            if (cudaMemcpyAsync(Y, y[k], t * dout * 8, cudaMemcpyHostToDevice, b->stream) !=
+                cudaSuccess)
+                rc = SP_EINTERNAL;
+            if (!rc)
+                rc = sp_launch_gather_rows(b->stream, b->d_phi + po[k], I.rs, I.pos_of, I.n, t, nat);
+            items.push_back({nat, Y, W, t, lambda[k], I.n, (int)dout, SP_OK});
+            which.push_back(k);
+        }
+        int many = rc ? rc : sp_ridge_phi_many(b->stream, items.data(), items.size(), o, ws);
+        if (!rc && many == SP_EALLOC && k1 - k0 > 1) {
+            limit = 0;
+            cudaGetLastError();
+            sp_cuda_free_async(slab, b->stream);
+            cudaStreamSynchronize(b->stream);
+            continue;
+        }
+        rc = many;
+        for (size_t q = 0; q < items.size() && !rc; ++q)
+            rc = done(which[q], (const double *)(b->d_phi + po[which[q]]), items[q].rc,
+                      items[q].d_W_out);
+        if (rc && getenv("SPIRES_DEBUG"))
+            fprintf(stderr, "spires: batch fit of instances %zu to %zu (washout %zu) failed: %d\n",
+                    k0, k1 - 1, o->washout, rc);
+        if (slab)
+            sp_cuda_free_async(slab, b->stream);
+        if (cudaStreamSynchronize(b->stream) != cudaSuccess && !rc)
+            rc = SP_EINTERNAL;
+        k0 = k1;
+    }
+    sp_ridge_ws_free(ws);
+    return rc;
+}
+
 // Ridge readouts of every instance from one batched simulation: states of
 // all instances recorded in one launch, then per instance the FP64 ridge of
 // the single-reservoir path (Gram + Cholesky + refinement) on its states.
@@ -1634,72 +1717,25 @@ extern "C" int sp_batch_train_ridge(sp_batch *b, const double *const *u, const d
     rc = batch_simulate(b, u, nullptr);
     if (rc)
         return rc;
-    size_t max_tn = 1, max_ty = 1, max_wn = 1;
-    for (size_t k = 0; k < b->inst.size(); ++k) {
-        max_tn = std::max(max_tn, T[k] * (size_t)b->inst[k].n);
-        max_ty = std::max(max_ty, T[k] * b->models[k].dout);
-        max_wn = std::max(max_wn, (size_t)b->inst[k].n * b->models[k].dout);
-    }
-    double *nat = nullptr, *Y = nullptr, *W = nullptr;
-    sp_ridge_ws *ws = sp_ridge_ws_new();  // one set of solver buffers for every instance
-    auto cleanup = [&]() {
-        cudaStreamSynchronize(b->stream);
-        sp_ridge_ws_free(ws);
-        if (nat)
-            sp_cuda_free(nat);
-        if (Y)
-            sp_cuda_free(Y);
-        if (W)
-            sp_cuda_free(W);
-    };
-    if (sp_cuda_malloc(&nat, max_tn * 8) != cudaSuccess || sp_cuda_malloc(&Y, max_ty * 8) != cudaSuccess ||
-        sp_cuda_malloc(&W, max_wn * 8) != cudaSuccess) {
-        cudaGetLastError();
-        cleanup();
-        return SP_EALLOC;
-    }
-    size_t po = 0;
-    for (size_t k = 0; k < b->inst.size() && !rc; ++k) {
+    rc = batch_fit(b, y, T, lambda, o, [&](size_t k, const double *phi, int fit_rc, double *W) {
         const BInst &I = b->inst[k];
         const int dout = (int)b->models[k].dout;
-        const double *phi = b->d_phi + po;
-        po += T[k] * I.rs;
-        if (dout == 0)
-            continue;
-        if (cudaMemcpyAsync(Y, y[k], T[k] * dout * 8, cudaMemcpyHostToDevice, b->stream) !=
-            cudaSuccess) {
-            rc = SP_EINTERNAL;
-            break;
-        }
-        rc = sp_launch_gather_rows(b->stream, phi, I.rs, I.pos_of, I.n, T[k], nat);
-        if (rc)
-            break;
-        sp_ridge_report rep;
-        memset(&rep, 0, sizeof(rep));
-        rc = sp_ridge_phi_ws(b->stream, nat, I.n, T[k], Y, dout, lambda[k], o, &rep, W, ws);
-        if (rc == SP_RIDGE_SINGULAR) {
+        (void)phi;
+        int r = SP_OK;
+        if (fit_rc == SP_RIDGE_SINGULAR) {
             // singular: W_out of this instance stays as it was (dgesv failure)
-            rc = SP_OK;
-            if (w_out && w_out[k]) {
-                rc = sp_launch_gather_rows(b->stream, b->w_pos[k], I.rs, I.pos_ro, I.n,
-                                           (size_t)dout, W);
-                if (!rc && cudaMemcpy(w_out[k], W, (size_t)dout * I.n * 8,
-                                      cudaMemcpyDeviceToHost) != cudaSuccess)
-                    rc = SP_EINTERNAL;
-            }
-            continue;
+            if (!w_out || !w_out[k])
+                return r;
+            r = sp_launch_gather_rows(b->stream, b->w_pos[k], I.rs, I.pos_ro, I.n, (size_t)dout, W);
+        } else {
+            r = sp_launch_wout_to_pos(b->stream, W, I.nid_ro, I.n, I.rs, dout, b->w_pos[k]);
         }
-        if (rc)
-            break;
-        rc = sp_launch_wout_to_pos(b->stream, W, I.nid_ro, I.n, I.rs, dout, b->w_pos[k]);
-        if (!rc && w_out && w_out[k] &&
+        if (!r && w_out && w_out[k] &&
             cudaMemcpyAsync(w_out[k], W, (size_t)dout * I.n * 8, cudaMemcpyDeviceToHost,
                             b->stream) != cudaSuccess)
-            rc = SP_EINTERNAL;
-        if (!rc && cudaStreamSynchronize(b->stream) != cudaSuccess)
-            rc = SP_EINTERNAL;
-    }
-    cleanup();
+            r = SP_EINTERNAL;
+        return r;
+    });
     if (elapsed_ms)
         *elapsed_ms =
             std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -1761,69 +1797,36 @@ extern "C" int sp_batch_fit_predict(sp_batch *b, const double *const *u, const d
     rc = batch_simulate(b, u, nullptr);
     if (rc)
         return rc;
-    size_t max_tn = 1, max_ty = 1, max_wn = 1;
-    for (size_t k = 0; k < b->inst.size(); ++k) {
-        max_tn = std::max(max_tn, T_fit[k] * (size_t)b->inst[k].n);
+    size_t max_ty = 1;
+    for (size_t k = 0; k < b->inst.size(); ++k)
         max_ty = std::max(max_ty, T[k] * b->models[k].dout);
-        max_wn = std::max(max_wn, (size_t)b->inst[k].n * b->models[k].dout);
-    }
-    double *nat = nullptr, *Y = nullptr, *W = nullptr;
-    if (sp_cuda_malloc(&nat, max_tn * 8) != cudaSuccess || sp_cuda_malloc(&Y, max_ty * 8) != cudaSuccess ||
-        sp_cuda_malloc(&W, max_wn * 8) != cudaSuccess) {
+    double *Y = nullptr;
+    if (sp_cuda_malloc_async(&Y, max_ty * 8, b->stream) != cudaSuccess) {
         cudaGetLastError();
-        if (nat)
-            sp_cuda_free(nat);
-        if (Y)
-            sp_cuda_free(Y);
         return SP_EALLOC;
     }
-    size_t po = 0;
-    sp_ridge_ws *ws = sp_ridge_ws_new();  // one set of solver buffers for every instance
-    for (size_t k = 0; k < b->inst.size() && !rc; ++k) {
+    rc = batch_fit(b, y, T_fit, lambda, o, [&](size_t k, const double *phi, int fit_rc, double *W) {
         const BInst &I = b->inst[k];
         const int dout = (int)b->models[k].dout;
-        const double *phi = b->d_phi + po;
-        po += T[k] * I.rs;
-        if (dout == 0)
-            continue;
-        if (cudaMemcpyAsync(Y, y[k], T_fit[k] * dout * 8, cudaMemcpyHostToDevice, b->stream) !=
-            cudaSuccess) {
-            rc = SP_EINTERNAL;
-            break;
-        }
-        rc = sp_launch_gather_rows(b->stream, phi, I.rs, I.pos_of, I.n, T_fit[k], nat);
-        if (rc)
-            break;
-        sp_ridge_report rep;
-        memset(&rep, 0, sizeof(rep));
-        rc = sp_ridge_phi_ws(b->stream, nat, I.n, T_fit[k], Y, dout, lambda[k], o, &rep, W, ws);
-        if (rc == SP_RIDGE_SINGULAR) {
-            rc = SP_OK; /* this instance keeps its previous W_out */
-        } else if (!rc) {
-            rc = sp_launch_wout_to_pos(b->stream, W, I.nid_ro, I.n, I.rs, dout, b->w_pos[k]);
-            if (!rc && w_out && w_out[k] &&
+        int r = SP_OK;
+        if (fit_rc != SP_RIDGE_SINGULAR) {  // else this instance keeps its previous W_out
+            r = sp_launch_wout_to_pos(b->stream, W, I.nid_ro, I.n, I.rs, dout, b->w_pos[k]);
+            if (!r && w_out && w_out[k] &&
                 cudaMemcpyAsync(w_out[k], W, (size_t)dout * I.n * 8, cudaMemcpyDeviceToHost,
                                 b->stream) != cudaSuccess)
-                rc = SP_EINTERNAL;
+                r = SP_EINTERNAL;
         }
-        if (rc)
-            break;
-        rc = batch_readout(b, I, phi, T[k], dout, Y);
-        if (!rc && y_out && y_out[k] &&
+        if (!r)
+            r = batch_readout(b, I, phi, T[k], dout, Y);
+        if (!r && y_out && y_out[k] &&
             cudaMemcpyAsync(y_out[k], Y, T[k] * dout * 8, cudaMemcpyDeviceToHost, b->stream) !=
                 cudaSuccess)
-            rc = SP_EINTERNAL;
-        if (!rc && cudaStreamSynchronize(b->stream) != cudaSuccess)
-            rc = SP_EINTERNAL;
-        if (rc && getenv("SPIRES_DEBUG"))
-            fprintf(stderr, "spires: batch fit of instance %zu (n %d, rows %zu, washout %zu) failed: %d\n",
-                    k, I.n, T_fit[k], o->washout, rc);
-    }
-    cudaStreamSynchronize(b->stream);
-    sp_ridge_ws_free(ws);
-    sp_cuda_free(nat);
-    sp_cuda_free(Y);
-    sp_cuda_free(W);
+            r = SP_EINTERNAL;
+        return r;
+    });
+    sp_cuda_free_async(Y, b->stream);
+    if (cudaStreamSynchronize(b->stream) != cudaSuccess && !rc)
+        rc = SP_EINTERNAL;
     if (elapsed_ms)
         *elapsed_ms =
             std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

@@ -225,12 +225,21 @@ __global__ void k_diag_pad(double *A, int n, int np, double lam)
 // tile solve, one product, two flags) is what bounds the smaller matrices, the
 // FP64 pipe the larger. (N=4000: 7.05 ms with 189 launches, now 1.49; N=1000: 1.18
 // -> 0.35 ms, 22 us a panel.)
-struct FactorArgs {
+// Several matrices share a launch, column j of every one before column j + 1 of
+// any: one matrix's chain leaves most of the device idle (20 of N 300 to 1600: 4.0
+// ms one after the other, 0.8 together).
+struct FactorItem {
     double *A;
     int np, nb;
     double *dinv;   // [nb][4][16][16] inverses of the diagonal blocks
-    int *flags;     // [nb][nb] tile ready; then the hand-out counter
-    int *counter, *info;
+    int *flags;     // [nb][nb] tile ready
+    int *info;
+};
+constexpr int kItems = 32;  // matrices of a launch
+struct FactorArgs {
+    FactorItem item[kItems];
+    int count, ntiles;
+    int *counter;   // the hand-out
 };
 
 constexpr size_t kTile = (size_t)NB * kPitch;  // doubles
@@ -359,32 +368,49 @@ __device__ __forceinline__ void factor_tile(double *T, double *s_inv, int *s_bad
     }
 }
 
-__global__ void __launch_bounds__(kThreads, 1) k_factor(FactorArgs f)
+__global__ void __launch_bounds__(kThreads, 1) k_factor(const __grid_constant__ FactorArgs args)
 {
     extern __shared__ __align__(16) double sm[];
     double *sA[2] = {sm, sm + kTile}, *sB[2] = {sm + 2 * kTile, sm + 3 * kTile};
     double *s_d = sm + 4 * kTile;          // [4][16][20] inverses of L_jj's blocks
     double *s_inv = s_d + 4 * 16 * 20;     // [64]
-    __shared__ int s_task, s_ready, s_bad;
+    __shared__ int s_item, s_i, s_j, s_ready, s_bad;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nb = f.nb, np = f.np, ntiles = nb * (nb + 1) / 2;
     const int wm = 16 * (warp >> 1), wn = 32 * (warp & 1);
+    int col = 0, first = 0;  // thread 0: the column of the last tile, its first tile
     for (;;) {
-        if (tid == 0)
-            s_task = atomicAdd(f.counter, 1);
-        __syncthreads();
-        const int t = s_task;
-        if (t >= ntiles)
-            return;
-        // column j holds tiles (j, j) .. (nb - 1, j)
-        int j = 0;
-        {
-            const double b = 2.0 * nb + 1.0;
-            j = (int)((b - sqrt(b * b - 8.0 * t)) * 0.5);
-            while (j > 0 && j * nb - j * (j - 1) / 2 > t) --j;
-            while ((j + 1) * nb - (j + 1) * j / 2 <= t) ++j;
+        if (tid == 0) {
+            // column `col` holds tiles (col, col) .. (nb - 1, col) of every matrix
+            int t = atomicAdd(args.counter, 1);
+            s_item = -1;
+            if (t < args.ntiles) {
+                for (;;) {
+                    int tiles = 0;
+                    for (int k = 0; k < args.count; ++k)
+                        tiles += args.item[k].nb > col ? args.item[k].nb - col : 0;
+                    if (t < first + tiles)
+                        break;
+                    first += tiles;
+                    ++col;
+                }
+                t -= first;
+                int k = 0;
+                for (;; ++k) {
+                    const int tiles = args.item[k].nb > col ? args.item[k].nb - col : 0;
+                    if (t < tiles)
+                        break;
+                    t -= tiles;
+                }
+                s_item = k;
+                s_i = col + t;
+                s_j = col;
+            }
         }
-        const int i = j + t - (j * nb - j * (j - 1) / 2);
+        __syncthreads();
+        if (s_item < 0)
+            return;
+        const FactorItem &f = args.item[s_item];
+        const int i = s_i, j = s_j, nb = f.nb, np = f.np;
         const bool diag = i == j;
         const double *Li = f.A + (size_t)i * NB * np, *Lj = f.A + (size_t)j * NB * np;
         // A_ij, minus one product after the other: each is summed by itself first,
@@ -587,12 +613,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_factor(FactorArgs f)
 // block through the inverted 16 x 16 blocks. A block's chain -- a flag, a 64 x 64
 // product, the diagonal solve -- is what bounds it. (N=4000, one output: 1.70 ms
 // with 250 launches, now 0.57; N=1000: 0.37 -> 0.14 ms.)
-struct SolveArgs {
+struct SolveItem {
     const double *L;
     int np, nb, n, dout;
     const double *dinv;
     double *Z;          // [n][dout]
     int *flags, *info;  // [2][nb]
+    int cta0, ctas;     // the launch's CTAs that work on it
+};
+struct SolveArgs {
+    SolveItem item[kItems];
+    int count;
 };
 
 constexpr int kSolveStages = 4;
@@ -600,7 +631,7 @@ constexpr size_t kSolveSmem = (kSolveStages * kTile + 4 * 16 * 20 + 3 * NB * 16)
 
 // DO: outputs held per thread (dout <= DO).
 template <bool kBack, int DO>
-__device__ __forceinline__ bool solve_block(const SolveArgs &a, double *sm, int i)
+__device__ __forceinline__ bool solve_block(const SolveItem &a, double *sm, int i)
 {
     double *s_d = sm + kSolveStages * kTile;
     double *s_z = s_d + 4 * 16 * 20;   // [64][dout] a block of the solution
@@ -748,14 +779,19 @@ __device__ __forceinline__ bool solve_block(const SolveArgs &a, double *sm, int 
 }
 
 template <int DO>
-__global__ void __launch_bounds__(kThreads, 1) k_solve(SolveArgs a)
+__global__ void __launch_bounds__(kThreads, 1) k_solve(const __grid_constant__ SolveArgs args)
 {
     extern __shared__ __align__(16) double sm[];
-    for (int i = blockIdx.x; i < a.nb; i += gridDim.x)
+    int k = 0;
+    while (k + 1 < args.count && (int)blockIdx.x >= args.item[k + 1].cta0)
+        ++k;
+    const SolveItem &a = args.item[k];
+    const int rank = blockIdx.x - a.cta0;
+    for (int i = rank; i < a.nb; i += a.ctas)
         if (!solve_block<false, DO>(a, sm, i))
             return;
     // the last blocks first, each on the CTA that has the same number of blocks
-    for (int c = blockIdx.x; c < a.nb; c += gridDim.x) {
+    for (int c = rank; c < a.nb; c += a.ctas) {
         __syncthreads();
         if (!solve_block<true, DO>(a, sm, a.nb - 1 - c))
             return;
@@ -834,50 +870,80 @@ cudaError_t sp_solve_diag(cudaStream_t s, double *A, int n, double lambda)
     return cudaGetLastError();
 }
 
-cudaError_t sp_solve_factor(cudaStream_t s, double *A, int n, void *work, int *info)
+cudaError_t sp_solve_factor(cudaStream_t s, const sp_solve_item *items, int count)
 {
-    FactorArgs f;
-    f.A = A;
-    f.np = sp_solve_pad(n);
-    f.nb = f.np / NB;
-    f.dinv = (double *)work;
-    f.flags = (int *)(f.dinv + (size_t)f.nb * 4 * 256);
-    f.counter = f.flags + (size_t)f.nb * f.nb + 2 * f.nb;
-    f.info = info;
     cudaError_t e = set_max_dynamic_smem((const void *)k_factor);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(f.flags, 0, ((size_t)f.nb * f.nb + 2 * f.nb + 4) * sizeof(int), s);
-    if (e != cudaSuccess)
-        return e;
-    const int tiles = f.nb * (f.nb + 1) / 2, sms = sm_count();
-    void *args[] = {&f};
-    return cudaLaunchCooperativeKernel((const void *)k_factor, dim3(tiles < sms ? tiles : sms),
-                                       dim3(kThreads), args, kFactorSmem, s);
+    for (int k0 = 0; k0 < count && e == cudaSuccess; k0 += kItems) {
+        FactorArgs a;
+        a.count = count - k0 < kItems ? count - k0 : kItems;
+        a.ntiles = 0;
+        a.counter = nullptr;
+        for (int k = 0; k < a.count; ++k) {
+            const sp_solve_item &it = items[k0 + k];
+            FactorItem &f = a.item[k];
+            f.A = it.A;
+            f.np = sp_solve_pad(it.n);
+            f.nb = f.np / NB;
+            f.dinv = (double *)it.work;
+            f.flags = (int *)(f.dinv + (size_t)f.nb * 4 * 256);
+            f.info = it.info;
+            a.ntiles += f.nb * (f.nb + 1) / 2;
+            if (!a.counter)
+                a.counter = f.flags + (size_t)f.nb * f.nb + 2 * f.nb;
+            e = cudaMemsetAsync(f.flags, 0, ((size_t)f.nb * f.nb + 2 * f.nb + 4) * sizeof(int), s);
+            if (e != cudaSuccess)
+                return e;
+        }
+        const int sms = sm_count();
+        void *args[] = {&a};
+        e = cudaLaunchCooperativeKernel((const void *)k_factor,
+                                        dim3(a.ntiles < sms ? a.ntiles : sms), dim3(kThreads), args,
+                                        kFactorSmem, s);
+    }
+    return e;
 }
 
-cudaError_t sp_solve_apply(cudaStream_t s, const double *L, int n, void *work, double *Z, int dout,
-                           int *info)
+cudaError_t sp_solve_apply(cudaStream_t s, const sp_solve_item *items, int count)
 {
-    SolveArgs a;
-    a.L = L;
-    a.np = sp_solve_pad(n);
-    a.nb = a.np / NB;
-    a.n = n;
-    a.dout = dout;
-    a.dinv = (const double *)work;
-    a.Z = Z;
-    a.flags = (int *)((double *)work + (size_t)a.nb * 4 * 256) + (size_t)a.nb * a.nb;
-    a.info = info;
-    const void *fn = dout == 1  ? (const void *)k_solve<1>
-                     : dout <= 4 ? (const void *)k_solve<4>
-                                 : (const void *)k_solve<16>;
-    cudaError_t e = set_max_dynamic_smem(fn);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(a.flags, 0, 2 * (size_t)a.nb * sizeof(int), s);
-    if (e != cudaSuccess)
-        return e;
     const int sms = sm_count();
-    void *args[] = {&a};
-    return cudaLaunchCooperativeKernel(fn, dim3(a.nb < sms ? a.nb : sms),
-                                       dim3(kThreads), args, kSolveSmem, s);
+    cudaError_t e = cudaSuccess;
+    // a matrix has a CTA per row block; as many matrices as the SMs hold at once
+    for (int k0 = 0; k0 < count && e == cudaSuccess;) {
+        SolveArgs a;
+        a.count = 0;
+        int grid = 0, dout = 1;
+        while (k0 + a.count < count && a.count < kItems) {
+            const sp_solve_item &it = items[k0 + a.count];
+            SolveItem &f = a.item[a.count];
+            f.L = it.A;
+            f.np = sp_solve_pad(it.n);
+            f.nb = f.np / NB;
+            f.n = it.n;
+            f.dout = it.dout;
+            f.dinv = (const double *)it.work;
+            f.Z = it.Z;
+            f.flags = (int *)((double *)it.work + (size_t)f.nb * 4 * 256) + (size_t)f.nb * f.nb;
+            f.info = it.info;
+            f.cta0 = grid;
+            f.ctas = f.nb < sms ? f.nb : sms;
+            if (grid + f.ctas > sms)
+                break;
+            grid += f.ctas;
+            dout = it.dout > dout ? it.dout : dout;
+            ++a.count;
+            e = cudaMemsetAsync(f.flags, 0, 2 * (size_t)f.nb * sizeof(int), s);
+            if (e != cudaSuccess)
+                return e;
+        }
+        const void *fn = dout == 1  ? (const void *)k_solve<1>
+                         : dout <= 4 ? (const void *)k_solve<4>
+                                     : (const void *)k_solve<16>;
+        e = set_max_dynamic_smem(fn);
+        if (e != cudaSuccess)
+            return e;
+        void *args[] = {&a};
+        e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, kSolveSmem, s);
+        k0 += a.count;
+    }
+    return e;
 }

@@ -119,7 +119,23 @@ extern "C" int sp_ridge_phi(cudaStream_t s, const double *Phi, int n, size_t T,
                             const double *Y, int dout, double lambda, const sp_ridge_opts *o,
                             sp_ridge_report *rep, double *d_W_out);
 // The same with reusable work buffers (primal solves of up to 16 outputs).
+// One fit of sp_ridge_phi_many: states Phi [T x n] and targets Y [T x dout] on the
+// device, d_W_out [dout x n] written on success; rc as sp_ridge_phi returns it.
+struct sp_ridge_item {
+    const double *Phi, *Y;
+    double *d_W_out;
+    size_t T;
+    double lambda;
+    int n, dout, rc;
+};
 struct sp_ridge_ws;
+// Bytes of working memory that an item adds to a call of sp_ridge_phi_many.
+extern "C" size_t sp_ridge_item_bytes(int n, size_t T, int dout);
+// Fits of one set of options: those that take the direct FP64 way share the
+// factorisation's and the solves' launches and the host's waits, the others go
+// through sp_ridge_phi_ws. Returns an error of the call; each fit's own is its rc.
+extern "C" int sp_ridge_phi_many(cudaStream_t s, sp_ridge_item *items, size_t count,
+                                 const sp_ridge_opts *o, sp_ridge_ws *ws);
 extern "C" sp_ridge_ws *sp_ridge_ws_new(void);
 extern "C" void sp_ridge_ws_free(sp_ridge_ws *w);
 extern "C" int sp_ridge_phi_ws(cudaStream_t s, const double *Phi, int n, size_t T,

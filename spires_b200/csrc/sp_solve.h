@@ -27,9 +27,30 @@ cudaError_t sp_solve_gram(cudaStream_t s, const double *X, int n, size_t t0, siz
                           int ldc);
 // A += lambda I, and the identity in rows and columns n .. pad(n) - 1.
 cudaError_t sp_solve_diag(cudaStream_t s, double *A, int n, double lambda);
-// A = L L^T in place (lower triangle). *info (zero before) becomes the 1-based
-// index of a pivot that is not positive, or -1 when a wait ran out.
-cudaError_t sp_solve_factor(cudaStream_t s, double *A, int n, void *work, int *info);
-// L L^T Z = Z in place for Z (n x dout, dout <= 16).
-cudaError_t sp_solve_apply(cudaStream_t s, const double *L, int n, void *work, double *Z, int dout,
-                           int *info);
+// One system: A (then its factor), its work area, right-hand sides Z (n x dout,
+// dout <= 16) and an error word.
+struct sp_solve_item {
+    double *A;
+    int n;
+    void *work;
+    double *Z;
+    int dout;
+    int *info;
+};
+// A = L L^T in place (lower triangle) of every item. *info (zero before) becomes
+// the 1-based index of a pivot that is not positive, or -1 when a wait ran out.
+cudaError_t sp_solve_factor(cudaStream_t s, const sp_solve_item *items, int count);
+// L L^T Z = Z in place of every item.
+cudaError_t sp_solve_apply(cudaStream_t s, const sp_solve_item *items, int count);
+
+inline cudaError_t sp_solve_factor(cudaStream_t s, double *A, int n, void *work, int *info)
+{
+    const sp_solve_item it = {A, n, work, nullptr, 0, info};
+    return sp_solve_factor(s, &it, 1);
+}
+inline cudaError_t sp_solve_apply(cudaStream_t s, double *L, int n, void *work, double *Z,
+                                  int dout, int *info)
+{
+    const sp_solve_item it = {L, n, work, Z, dout, info};
+    return sp_solve_apply(s, &it, 1);
+}

@@ -4,6 +4,8 @@ reproduce, bit for bit, the spike raster and final states of the same
 reservoir created and run on its own -- and through it the oracle.
 
 All calls go through the C ABI of libspires.so."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -251,4 +253,39 @@ def test_batch_forms_match_single_reservoirs(shapes):
         fired += int(R1.any())
     assert fired > 0
     assert b.info()["groups"] == len(cfgs) or len(cfgs) > 148
+    b.close()
+
+
+def test_fits_of_a_batch_share_their_launches():
+    """More fits than one factorisation takes (32): sizes around the solver's tiles,
+    a fit in the dual form, systems that are singular -- each the single
+    reservoir's W_out."""
+    rng = np.random.default_rng(4)
+    ns = [1, 2, 63, 64, 65, 128, 129, 200, 700, 500] + [40 + k for k in range(26)]
+    cfgs = [sp.make_config(n, 1, 1 + k % 3, rho=1.2, ei=0.5, gamma=1.5, conn=0.2,
+                           topo=sp.CONN_RANDOM, neuron=sp.LIF_DISCRETE,
+                           nparams=(0.0, 1.0, 0.3, 0.05)) for k, n in enumerate(ns)]
+    seeds = [int(s) for s in rng.integers(1, 2**31 - 1, len(ns))]
+    Ts = [90 if n == 500 else 260 + n for n in ns]  # 500: the dual form
+    us = [rng.uniform(-1.0, 2.0, size=(T, 1)) for T in Ts]
+    ys = [rng.standard_normal((T, 1 + k % 3)) for k, T in enumerate(Ts)]
+    b = sp.Batch(cfgs, seeds)
+    b.run(us)
+    W, _ = b.train_ridge(us, ys, 1e-2, washout=20)
+    for k, n in enumerate(ns):
+        r = sp.Reservoir(cfgs[k], seed=seeds[k])
+        o = sp.RidgeOpts(0, 30, 1e-13, 20)
+        rep = sp.RidgeReport()
+        assert r.lib.spires_ext_train_ridge(r.h, sp.dptr(us[k]), sp.dptr(ys[k]), Ts[k], 1e-2,
+                                            C.byref(o), C.byref(rep)) == sp.SPIRES_OK
+        assert np.allclose(W[k], r.readout(), rtol=1e-9, atol=1e-12), f"instance {k} (n={n})"
+        assert rep.dual == (n == 500)
+        r.close()
+    # the same fits beside singular ones (no rows to tell 700 neurons apart)
+    lam = np.array([0.0 if n == 700 else 1e-2 for n in ns])
+    short = [u[:300] if n == 700 else u for n, u in zip(ns, us)]
+    W2, _ = b.train_ridge(short, [y[:len(u)] for y, u in zip(ys, short)], lam, washout=20)
+    for k, n in enumerate(ns):
+        if n != 700:
+            assert np.array_equal(W2[k], W[k]), f"instance {k} (n={n})"
     b.close()
