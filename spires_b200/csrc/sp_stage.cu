@@ -1,12 +1,13 @@
 // sp_stage.cu -- large copies of pageable host memory through pinned buffers.
 //
 // The driver moves pageable memory with one thread (11 GB/s in, 17 out, measured
-// at 288 MB), a fifth of the link. Here up to eight threads copy 2 MB pieces
-// between the caller's memory and four pinned buffers while the pieces before
-// are on the link: 49 GB/s with two, 50 GB/s with eight buffers, 55 GB/s for
-// memory that is pinned already.
+// at 288 MB), a fifth of the link. Here up to eight threads copy pieces between the
+// caller's memory and 16 MB of pinned buffers while the pieces before are on the
+// link: 51 GB/s with four of 4 MB, 49 with eight of 2 MB, 32 with half as many of
+// either; 55 for memory that is pinned already. Copies below 32 MB take the smaller
+// pieces: their first and last are not overlapped.
 //
-// The four buffers (8 MB) are made by the first copy that is large enough and
+// The buffers are made by the first copy that is large enough and
 // given back when the library is unloaded. One copy uses them at a time; one that
 // finds them taken, a small one, and one whose memory the driver knows (pinned,
 // managed or device memory) goes to cudaMemcpyAsync as it is.
@@ -19,11 +20,13 @@
 
 namespace {
 
-constexpr size_t kPiece = 2u << 20;
-constexpr int kSlots = 4;
+constexpr size_t kPool = 16u << 20;
+constexpr int kMaxSlots = 8;
 constexpr int kThreads = 8;
 // below, the threads' start costs what they save (4 MB in: 0.36 ms as it is)
 constexpr size_t kLeast = 4u << 20;
+
+size_t piece_of(size_t bytes) { return bytes < (32u << 20) ? 2u << 20 : 4u << 20; }
 
 struct Buffers {
     std::mutex m;
@@ -64,7 +67,7 @@ int take(const void *host, size_t bytes, std::unique_lock<std::mutex> &lock)
     if (at.type != cudaMemoryTypeUnregistered || !lock.try_lock() || g_buf.refused)
         return 0;
     if (!g_buf.p &&
-        cudaHostAlloc((void **)&g_buf.p, kSlots * kPiece, cudaHostAllocPortable) != cudaSuccess) {
+        cudaHostAlloc((void **)&g_buf.p, kPool, cudaHostAllocPortable) != cudaSuccess) {
         cudaGetLastError();
         g_buf.p = nullptr;
         g_buf.refused = true;
@@ -74,7 +77,7 @@ int take(const void *host, size_t bytes, std::unique_lock<std::mutex> &lock)
 }
 
 struct Events {
-    cudaEvent_t e[kSlots] = {};
+    cudaEvent_t e[kMaxSlots] = {};
     bool make()
     {
         for (auto &x : e)
@@ -100,18 +103,19 @@ cudaError_t sp_copy_in(void *dev, const void *host, size_t bytes, cudaStream_t s
     if (threads == 0 || !ev.make())
         return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s);
     cudaError_t e = cudaSuccess;
-    const size_t pieces = (bytes + kPiece - 1) / kPiece;
+    const size_t piece = piece_of(bytes), slots = kPool / piece;
+    const size_t pieces = (bytes + piece - 1) / piece;
     for (size_t k = 0; k < pieces && e == cudaSuccess; ++k) {
-        const size_t at = k * kPiece, n = std::min(kPiece, bytes - at);
-        char *slot = g_buf.p + k % kSlots * kPiece;
-        if (k >= kSlots)
-            e = cudaEventSynchronize(ev.e[k % kSlots]);
+        const size_t at = k * piece, n = std::min(piece, bytes - at);
+        char *slot = g_buf.p + k % slots * piece;
+        if (k >= slots)
+            e = cudaEventSynchronize(ev.e[k % slots]);
         if (e != cudaSuccess)
             break;
         copy_threads(slot, (const char *)host + at, n, threads);
         e = cudaMemcpyAsync((char *)dev + at, slot, n, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess)
-            e = cudaEventRecord(ev.e[k % kSlots], s);
+            e = cudaEventRecord(ev.e[k % slots], s);
     }
     // the buffers go to the next copy: nothing may still read them
     const cudaError_t done = cudaStreamSynchronize(s);
@@ -126,23 +130,24 @@ cudaError_t sp_copy_out(void *host, const void *dev, size_t bytes, cudaStream_t 
     if (threads == 0 || !ev.make())
         return cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaSuccess;
-    const size_t pieces = (bytes + kPiece - 1) / kPiece;
+    const size_t piece = piece_of(bytes), slots = kPool / piece;
+    const size_t pieces = (bytes + piece - 1) / piece;
     auto start = [&](size_t k) {
-        const size_t at = k * kPiece, n = std::min(kPiece, bytes - at);
-        cudaError_t r = cudaMemcpyAsync(g_buf.p + k % kSlots * kPiece, (const char *)dev + at, n,
+        const size_t at = k * piece, n = std::min(piece, bytes - at);
+        cudaError_t r = cudaMemcpyAsync(g_buf.p + k % slots * piece, (const char *)dev + at, n,
                                         cudaMemcpyDeviceToHost, s);
-        return r == cudaSuccess ? cudaEventRecord(ev.e[k % kSlots], s) : r;
+        return r == cudaSuccess ? cudaEventRecord(ev.e[k % slots], s) : r;
     };
-    for (size_t k = 0; k < pieces && k < kSlots && e == cudaSuccess; ++k)
+    for (size_t k = 0; k < pieces && k < slots && e == cudaSuccess; ++k)
         e = start(k);
     for (size_t k = 0; k < pieces && e == cudaSuccess; ++k) {
-        const size_t at = k * kPiece, n = std::min(kPiece, bytes - at);
-        e = cudaEventSynchronize(ev.e[k % kSlots]);
+        const size_t at = k * piece, n = std::min(piece, bytes - at);
+        e = cudaEventSynchronize(ev.e[k % slots]);
         if (e != cudaSuccess)
             break;
-        copy_threads((char *)host + at, g_buf.p + k % kSlots * kPiece, n, threads);
-        if (k + kSlots < pieces)
-            e = start(k + kSlots);
+        copy_threads((char *)host + at, g_buf.p + k % slots * piece, n, threads);
+        if (k + slots < pieces)
+            e = start(k + slots);
     }
     if (e != cudaSuccess)
         cudaStreamSynchronize(s);

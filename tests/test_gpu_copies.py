@@ -1,5 +1,5 @@
 """Large copies of the caller's host memory (staged through pinned buffers in 2 MB
-pieces from 4 MB on) against the small ones, which the driver moves as they are."""
+pieces from 4 MB on, 4 MB from 32 MB on) against the small ones, which the driver moves as they are."""
 import threading
 
 import numpy as np
@@ -20,7 +20,8 @@ def reservoir(n):
 
 # around the first staged size, whole pieces and one double more, more than the buffers
 @pytest.mark.parametrize("doubles", [4 * MB // 8 - 1, 4 * MB // 8, 6 * MB // 8 + 1,
-                                     10 * MB // 8, 21 * MB // 8 + 77])
+                                     10 * MB // 8, 21 * MB // 8 + 77,
+                                     34 * MB // 8 + 5])
 def test_states_of_a_long_run_match_short_runs(doubles):
     n = 1009
     T = -(-doubles // n)
