@@ -77,7 +77,7 @@ struct GramTile {
 template <int BT>
 __global__ void __launch_bounds__(kThreads, 1) k_gram(const double *__restrict__ X, int n,
                                                       size_t t0, size_t t1, double *__restrict__ C,
-                                                      int ldc, int S, int wide)
+                                                      int ldc, int S, int wide, int more)
 {
     using G = GramTile<BT>;
     extern __shared__ __align__(16) double sm[];
@@ -121,6 +121,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_gram(const double *__restrict__
     double acc[G::MT][G::NT][2] = {};
     load(0);
     load(1);
+    if (more) {  // the sums over the rows before (S = 1)
+#pragma unroll
+        for (int m = 0; m < G::MT; ++m)
+#pragma unroll
+            for (int q = 0; q < G::NT; ++q)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int i = i0 + wm + 8 * m + (lane >> 2);
+                    const int j = j0 + wn + 8 * q + 2 * (lane & 3) + e;
+                    if (i < n && j <= i)
+                        acc[m][q][e] = C[(size_t)i * ldc + j];
+                }
+    }
     for (int st = 0; st < steps; ++st) {
         copy_wait<1>();
         __syncthreads();
@@ -809,7 +822,7 @@ int sm_count()
 
 template <int BT>
 cudaError_t launch_gram(cudaStream_t s, const double *X, int n, size_t t0, size_t t1, double *C,
-                        int ldc, int S)
+                        int ldc, int S, bool more)
 {
     using G = GramTile<BT>;
     const int nt = (n + BT - 1) / BT, tiles = nt * (nt + 1) / 2;
@@ -829,13 +842,13 @@ cudaError_t launch_gram(cudaStream_t s, const double *X, int n, size_t t0, size_
     c.numAttrs = 1;
     // 16-byte copies need even row lengths and an aligned base
     const int wide = n % 2 == 0 && ((uintptr_t)X & 15) == 0;
-    return cudaLaunchKernelEx(&c, k_gram<BT>, X, n, t0, t1, C, ldc, S, wide);
+    return cudaLaunchKernelEx(&c, k_gram<BT>, X, n, t0, t1, C, ldc, S, wide, more ? 1 : 0);
 }
 
 }  // namespace
 
-cudaError_t sp_solve_gram(cudaStream_t s, const double *X, int n, size_t t0, size_t t1, double *C,
-                          int ldc)
+// The tile width for n neurons and the parts of `rows` rows.
+static int gram_shape(int n, size_t rows, int *parts)
 {
     // The widest tile that still fills the SMs; 32-wide ones split their rows over
     // up to 8 CTAs until they do, at least 4096 rows each (a part then takes
@@ -845,18 +858,38 @@ cudaError_t sp_solve_gram(cudaStream_t s, const double *X, int n, size_t t0, siz
         const long long t = (n + bt - 1) / bt;
         return t * (t + 1) / 2;
     };
-    cudaError_t e;
-    if (tiles(128) >= sms * 9 / 10) {
-        e = launch_gram<128>(s, X, n, t0, t1, C, ldc, 1);
-    } else if (tiles(64) >= sms * 3 / 5) {
-        e = launch_gram<64>(s, X, n, t0, t1, C, ldc, 1);
-    } else {
-        int S = 1;
-        while (S < 8 && tiles(32) * S < sms && (t1 - t0) >= (size_t)8192 * S)
-            S *= 2;
-        e = launch_gram<32>(s, X, n, t0, t1, C, ldc, S);
-    }
-    if (e != cudaSuccess)
+    *parts = 1;
+    if (tiles(128) >= sms * 9 / 10)
+        return 128;
+    if (tiles(64) >= sms * 3 / 5)
+        return 64;
+    while (*parts < 8 && tiles(32) * *parts < sms && rows >= (size_t)8192 * *parts)
+        *parts *= 2;
+    return 32;
+}
+
+bool sp_solve_gram_in_ranges(int n, size_t rows)
+{
+    int parts;
+    gram_shape(n, rows, &parts);
+    return parts == 1;
+}
+
+cudaError_t sp_solve_gram(cudaStream_t s, const double *X, int n, size_t t0, size_t t1, double *C,
+                          int ldc)
+{
+    return sp_solve_gram_range(s, X, n, t0, t1, C, ldc, false, true);
+}
+
+cudaError_t sp_solve_gram_range(cudaStream_t s, const double *X, int n, size_t t0, size_t t1,
+                                double *C, int ldc, bool more, bool last)
+{
+    int S;
+    const int bt = gram_shape(n, t1 - t0, &S);
+    const cudaError_t e = bt == 128  ? launch_gram<128>(s, X, n, t0, t1, C, ldc, S, more)
+                          : bt == 64 ? launch_gram<64>(s, X, n, t0, t1, C, ldc, S, more)
+                                     : launch_gram<32>(s, X, n, t0, t1, C, ldc, S, more);
+    if (e != cudaSuccess || !last)
         return e;
     const unsigned g = (unsigned)((n + 31) / 32);
     k_mirror_upper<<<dim3(g, g), 256, 0, s>>>(C, n, ldc);

@@ -25,6 +25,13 @@ inline size_t sp_solve_work_bytes(int n)
 // full matrix is written.
 cudaError_t sp_solve_gram(cudaStream_t s, const double *X, int n, size_t t0, size_t t1, double *C,
                           int ldc);
+// The same row range by row range, in order: `more` continues the sums in C's lower
+// triangle where the rows so far (a multiple of four) ended, with the same bits as
+// one call over all rows; the upper triangle comes with `last`. Only for the n and
+// rows in all that sp_solve_gram sums in one part.
+bool sp_solve_gram_in_ranges(int n, size_t rows);
+cudaError_t sp_solve_gram_range(cudaStream_t s, const double *X, int n, size_t t0, size_t t1,
+                                double *C, int ldc, bool more, bool last);
 // A += lambda I, and the identity in rows and columns n .. pad(n) - 1.
 cudaError_t sp_solve_diag(cudaStream_t s, double *A, int n, double lambda);
 // One system: A (then its factor), its work area, right-hand sides Z (n x dout,

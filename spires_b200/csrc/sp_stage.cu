@@ -95,13 +95,16 @@ struct Events {
 
 }  // namespace
 
-cudaError_t sp_copy_in(void *dev, const void *host, size_t bytes, cudaStream_t s)
+cudaError_t sp_copy_in(void *dev, const void *host, size_t bytes, cudaStream_t s,
+                       const std::function<cudaError_t(size_t)> &enqueued)
 {
     std::unique_lock<std::mutex> lock(g_buf.m, std::defer_lock);
     const int threads = take(host, bytes, lock);
     Events ev;
-    if (threads == 0 || !ev.make())
-        return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s);
+    if (threads == 0 || !ev.make()) {
+        const cudaError_t r = cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s);
+        return r == cudaSuccess && enqueued ? enqueued(bytes) : r;
+    }
     cudaError_t e = cudaSuccess;
     const size_t piece = piece_of(bytes), slots = kPool / piece;
     const size_t pieces = (bytes + piece - 1) / piece;
@@ -116,6 +119,8 @@ cudaError_t sp_copy_in(void *dev, const void *host, size_t bytes, cudaStream_t s
         e = cudaMemcpyAsync((char *)dev + at, slot, n, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess)
             e = cudaEventRecord(ev.e[k % slots], s);
+        if (e == cudaSuccess && enqueued)
+            e = enqueued(at + n);
     }
     // the buffers go to the next copy: nothing may still read them
     const cudaError_t done = cudaStreamSynchronize(s);

@@ -6,8 +6,12 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>
+#include <functional>
 
-cudaError_t sp_copy_in(void *dev, const void *host, size_t bytes, cudaStream_t s);
+// `enqueued`, when given, is called with the number of bytes whose copies are on
+// the stream, each time it grows and at last with `bytes`.
+cudaError_t sp_copy_in(void *dev, const void *host, size_t bytes, cudaStream_t s,
+                       const std::function<cudaError_t(size_t)> &enqueued = nullptr);
 cudaError_t sp_copy_out(void *host, const void *dev, size_t bytes, cudaStream_t s);
 
 // A little host memory that the device can write, from a pool of the process; null

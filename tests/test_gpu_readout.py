@@ -299,3 +299,18 @@ def test_ridge_solver_at_tile_edges(n, T, dout):
     assert rel(W, ref) < 4 * (T + n) * np.finfo(float).eps * cond
     # the same bits again: the sums' order is fixed
     assert np.array_equal(W, sp.ridge_fit(X, Y, float(T), max_refine=0)[0])
+
+
+# states large enough that the Gram starts on the rows that have arrived: whole and
+# ragged ranges, 128-, 64- and 32-wide tiles, a washout beyond the first range
+@pytest.mark.parametrize("n,T,washout", [(2050, 3001, 0), (1300, 5000, 3), (1001, 6007, 2500)])
+def test_ridge_fit_overlapped_with_its_copy(n, T, washout):
+    """Sixteen outputs and fewer take the overlapped way, seventeen copy first: the
+    same sums, so the same bits for the outputs they share."""
+    rng = np.random.default_rng(n)
+    X = rng.uniform(-1, 1, (T, n))
+    Y = rng.uniform(-1, 1, (T, 17))
+    W, rep = sp.ridge_fit(X, Y[:, :2], float(T), washout=washout, max_refine=0)
+    W17, _ = sp.ridge_fit(X, Y, float(T), washout=washout, max_refine=0)
+    assert rep.factor_failed == 0 and rep.dual == 0
+    assert np.array_equal(W, W17[:2])
