@@ -303,7 +303,7 @@ spires_status spires_ext_agile_batch_best(const spires_ext_agile_batch *b, int c
  * layout). FP64 Gram, Cholesky and iterative refinement: the same kernels, in
  * the same order, as spires_ext_train_ridge with SPIRES_EXT_GRAM_FP64.
  * It calls no cudaMalloc/cudaFree: its working memory is one fixed array of
- * this library (8.6 MB, held on every GPU that loads the library until the
+ * this library (8.7 MB, held on every GPU that loads the library until the
  * process exits), which bounds the sizes: n <= 512, dout <= 16, T <= 16384;
  * larger requests return SPIRES_ERR_INVALID_ARG. A singular system (the
  * Cholesky factorisation fails and so does LU with partial pivoting) returns

@@ -1691,7 +1691,7 @@ out:
 // control loop that cannot afford the implicit device-wide synchronisation of
 // cudaMalloc/cudaFree. All working memory is the file-scope array below,
 // sized for at most SP_NA_MAX_N neurons, SP_NA_MAX_DOUT outputs and
-// SP_NA_MAX_T rows (8.6 MB); every GPU that loads this library holds it until
+// SP_NA_MAX_T rows (8.7 MB); every GPU that loads this library holds it until
 // the process exits. The same kernels as spires_ext_train_ridge with the FP64
 // Gram run in the same order, so the two agree given the same states.
 #define SP_NA_MAX_N 512
