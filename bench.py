@@ -974,9 +974,12 @@ def main():
         dist.init_process_group("nccl", timeout=datetime.timedelta(seconds=120))
     line = run_gpu_arm(args, rank, world)
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        v, sample, cores = cpu_reference_sample(args.cpu_fill, args.cpu_timed)
-        line["cpu_baseline"] = {"value": v, "unit": "neuron-steps/s", "cores": cores,
-                                "kind": "reference", "sample": sample}
+        try:
+            v, sample, cores = cpu_reference_sample(args.cpu_fill, args.cpu_timed)
+            line["cpu_baseline"] = {"value": v, "unit": "neuron-steps/s", "cores": cores,
+                                    "kind": "reference", "sample": sample}
+        except OSError as e:  # no build of the reference and no sources to make one
+            line["cpu_baseline"] = {"unavailable": str(e)}
     if world > 1:
         import torch.distributed as dist
 
