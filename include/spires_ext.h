@@ -128,6 +128,9 @@ spires_status spires_ext_set_seed(spires_reservoir *r, uint64_t seed);
  * test_fail_device_alloc: test hook, process-wide. After `after` more device
  * allocations by this library the next one fails (as an out-of-memory
  * cudaMalloc would), then allocations succeed again; -1 clears it.
+ * test_fill_device_allocs: test hook, process-wide. Every later device
+ * allocation by this library is filled with `byte` (0 to 255), so that memory
+ * read before it is written shows in the results; -1 ends it.
  * test_live_device_allocs: device allocations of this library not yet freed
  * (process-wide), to check that failed calls release what they allocated. */
 spires_status spires_ext_set_wait_limit(spires_reservoir *r, double ms);
@@ -136,6 +139,7 @@ spires_status spires_ext_last_device_error(const spires_reservoir *r, int *code,
 spires_status spires_ext_test_withhold_arrival(spires_reservoir *r, int cta,
                                                long long micro_step);
 void          spires_ext_test_fail_device_alloc(long long after);
+void          spires_ext_test_fill_device_allocs(int byte);
 long long     spires_ext_test_live_device_allocs(void);
 
 /* ---- state checkpoint -------------------------------------------------------

@@ -171,6 +171,7 @@ EXT_SIGNATURES = {
                                               C.POINTER(C.c_longlong)]),
     "spires_ext_test_withhold_arrival": (C.c_int, [_VP, C.c_int, C.c_longlong]),
     "spires_ext_test_fail_device_alloc": (None, [C.c_longlong]),
+    "spires_ext_test_fill_device_allocs": (None, [C.c_int]),
     "spires_ext_test_live_device_allocs": (C.c_longlong, []),
     "spires_ext_state_bytes": (C.c_size_t, [_VP]),
     "spires_ext_state_save": (C.c_int, [_VP, _VP, C.c_size_t]),

@@ -530,6 +530,7 @@ SPIRES_EXPORT spires_status spires_ext_set_seed(spires_reservoir *r, uint64_t se
 /* bounded waits and failure-path test hooks */
 long long sp_alloc_live(void);
 void      sp_alloc_fail_after(long long count);
+void      sp_alloc_fill(int byte);
 
 SPIRES_EXPORT spires_status spires_ext_set_wait_limit(spires_reservoir *r, double ms)
 {
@@ -557,6 +558,11 @@ SPIRES_EXPORT spires_status spires_ext_last_device_error(const spires_reservoir 
 SPIRES_EXPORT void spires_ext_test_fail_device_alloc(long long after)
 {
     sp_alloc_fail_after(after);
+}
+
+SPIRES_EXPORT void spires_ext_test_fill_device_allocs(int byte)
+{
+    sp_alloc_fill(byte);
 }
 
 SPIRES_EXPORT long long spires_ext_test_live_device_allocs(void)

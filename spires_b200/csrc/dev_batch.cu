@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(kBatchThreads, kSpread ? 1 : 2) k_batch(BParam
                 *(volatile unsigned long long *)(I.ll + (size_t)((b + 1) & 1) * nw + gw) =
                     (unsigned long long)(unsigned)(b + 1) << 32 | word;
             if (m == I.micro - 1) {
-                if (act && I.phi)
+                if (wact && I.phi)  // empty lanes too: the readout reads whole rows
                     I.phi[(size_t)s * rs + i] = V;
                 if (wact && lane == 0)
                     I.raster[(size_t)s * nw + gw] = word;

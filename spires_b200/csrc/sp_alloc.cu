@@ -1,5 +1,5 @@
-// sp_alloc.cu -- counted device allocations and the allocation-failure test
-// hook (sp_alloc.h).
+// sp_alloc.cu -- counted device allocations and the test hooks that make one
+// fail or fill it (sp_alloc.h).
 #include <atomic>
 #include "sp_alloc.h"
 
@@ -7,6 +7,7 @@ namespace {
 std::atomic<long long> g_live{0};
 // allocations still allowed before the injected failure; -1 = no failure
 std::atomic<long long> g_fail_after{-1};
+std::atomic<int> g_fill{-1};  // byte that fills new allocations; -1 = left as they come
 
 bool injected_failure()
 {
@@ -50,9 +51,14 @@ extern "C" cudaError_t sp_cuda_malloc_bytes(void **p, size_t bytes)
         return cudaErrorMemoryAllocation;
     }
     cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaSuccess)
-        ++g_live;
-    return e;
+    if (e != cudaSuccess)
+        return e;
+    ++g_live;
+    const int fill = g_fill.load();
+    if (fill < 0)
+        return e;
+    e = cudaMemset(*p, fill, bytes);  // the caller's stream does not wait for this one
+    return e == cudaSuccess ? cudaDeviceSynchronize() : e;
 }
 
 extern "C" cudaError_t sp_cuda_malloc_async_bytes(void **p, size_t bytes, cudaStream_t s)
@@ -63,9 +69,11 @@ extern "C" cudaError_t sp_cuda_malloc_async_bytes(void **p, size_t bytes, cudaSt
     }
     keep_pool();
     cudaError_t e = cudaMallocAsync(p, bytes, s);
-    if (e == cudaSuccess)
-        ++g_live;
-    return e;
+    if (e != cudaSuccess)
+        return e;
+    ++g_live;
+    const int fill = g_fill.load();
+    return fill < 0 ? e : cudaMemsetAsync(*p, fill, bytes, s);
 }
 
 extern "C" cudaError_t sp_cuda_free(void *p)
@@ -85,5 +93,7 @@ extern "C" cudaError_t sp_cuda_free_async(void *p, cudaStream_t s)
 }
 
 extern "C" void sp_alloc_fail_after(long long count) { g_fail_after.store(count < 0 ? -1 : count); }
+
+extern "C" void sp_alloc_fill(int byte) { g_fill.store(byte < 0 ? -1 : byte & 0xff); }
 
 extern "C" long long sp_alloc_live(void) { return g_live.load(); }

@@ -2,6 +2,8 @@
 // calls. They count the allocations that are live, and a test hook can make
 // an allocation fail, so the failure paths of create, ridge and the other
 // entry points can be exercised on the host side without touching the GPU.
+// Another fills every new allocation, so that memory which is read before it is
+// written shows in the results.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstddef>

@@ -314,3 +314,56 @@ def test_ridge_fit_overlapped_with_its_copy(n, T, washout):
     W17, _ = sp.ridge_fit(X, Y, float(T), washout=washout, max_refine=0)
     assert rep.factor_failed == 0 and rep.dual == 0
     assert np.array_equal(W, W17[:2])
+
+
+@pytest.fixture
+def filled_allocations(request):
+    """New device memory holds 32.5 (0x40 in every byte) or NaN (0xff) in every
+    double, as after another use of it."""
+    lib = sp.load()
+    lib.spires_ext_test_fill_device_allocs(request.param)
+    yield
+    lib.spires_ext_test_fill_device_allocs(-1)
+
+
+@pytest.mark.parametrize("n,T,dout,neuron", [(1, 5, 1, sp.LIF_DISCRETE), (33, 40, 3, sp.FLIF_GL),
+                                             (300, 50, 2, sp.FLIF_GL), (1900, 10, 1, sp.LIF_DISCRETE)])
+@pytest.mark.parametrize("filled_allocations", [0x40], indirect=True)
+def test_rls_reads_only_recorded_states(filled_allocations, n, T, dout, neuron):
+    """Sizes that leave lanes of the last warp without a neuron: whatever memory held
+    before, the recursion and the readout see a state of 0 there. Tolerance of the
+    weights as in test_rls_matches_oracle; an output is a dot product of n terms."""
+    params = GL if neuron == sp.FLIF_GL else O.NEURON_PARAMS[neuron]
+    cfg = sp.make_config(n, 2, dout, rho=1.2, ei=0.55, gamma=1.2, conn=min(0.5, 6.0 / max(n, 2)),
+                         topo=sp.CONN_SMALL_WORLD, neuron=neuron, nparams=params)
+    u, y = data(T, 2, dout, seed=7)
+    r = sp.Reservoir(cfg, seed=12)
+    r.train_rls(u, y, 1.0, 1.0)
+    W = r.readout()
+    r.reset()
+    phi, _, Y = r.run_record(u, y=True)
+    r.close()
+    Wo = O.Oracle(cfg, sp.HostModel(cfg, seed=12)).train_rls(u, y, 1.0, 1.0)
+    assert rel(W, Wo) < 1e-8
+    bound = 2 * n * np.finfo(float).eps * (np.abs(phi) @ np.abs(W).T)
+    assert (np.abs(Y - phi @ W.T) <= bound).all()
+
+
+@pytest.mark.parametrize("filled_allocations", [0xff], indirect=True)
+@pytest.mark.parametrize("n,conn", [(33, 0.2), (300, 0.002)])
+def test_outputs_of_recorded_rows_ignore_empty_lanes(filled_allocations, n, conn):
+    """Outputs from recorded rows, of one reservoir and of a batch with and without
+    column blocks. Bound of a dot product of n terms."""
+    cfg = sp.make_config(n, 2, 2, rho=1.2, ei=0.55, gamma=1.2, conn=conn, topo=sp.CONN_RANDOM,
+                         neuron=sp.LIF_DISCRETE, nparams=O.NEURON_PARAMS[sp.LIF_DISCRETE])
+    u, _ = data(30, 2, 2, seed=4)
+    r = sp.Reservoir(cfg, seed=8)
+    phi, _, Y = r.run_record(u, y=True)
+    W = r.readout()
+    r.close()
+    bound = 2 * n * np.finfo(float).eps * (np.abs(phi) @ np.abs(W).T)
+    assert (np.abs(Y - phi @ W.T) <= bound).all()
+    b = sp.Batch([cfg], [8])
+    Yb = b.predict([u])[0][0]
+    b.close()
+    assert np.array_equal(Yb, Y)
