@@ -1137,8 +1137,8 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                          long long g) {
             while (k <= lim && ok) {
                 int cnt = lim - k + 1;
-                if (cnt > p.R)
-                    cnt = p.R;
+                if (cnt > p.RB)  // what a box holds: fewer than R when the ring is short
+                    cnt = p.RB;
                 if (cnt > rh + 1)
                     cnt = rh + 1;
                 const int y0 = rh - cnt + 1;
@@ -1304,8 +1304,8 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                           long long g) -> double {
         while (k <= lim && S_b > 0) {
             int cnt = lim - k + 1;
-            if (cnt > p.R)
-                cnt = p.R;
+            if (cnt > p.RB)
+                cnt = p.RB;
             if (cnt > rh + 1)
                 cnt = rh + 1;
             // on a failed wait the launch aborts at the next barrier_wait;

@@ -125,3 +125,22 @@ def test_fractional_history_through_the_pipeline(Ls, L, rows, stages):
     phi = np.concatenate([p[0] for p in parts])
     phi_o, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=11)).run(u)
     assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
+
+
+@pytest.mark.parametrize("L,rows", [(16, 32), (40, 64), (64, 256)])
+@pytest.mark.parametrize("Ls", [64, 75, 300])
+def test_fractional_history_with_stages_taller_than_the_ring(L, rows, Ls):
+    """A stage holds as many rows as the neuron's ring has, also for the synapse's
+    longer ring."""
+    n, T = 230, 2 * Ls + 30
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=0.05, dt=1.0,
+                         topo=sp.CONN_RANDOM, neuron=sp.FLIF_GL, nparams=GL(L),
+                         synapse=sp.SYN_FRAC, sparams=(0.6, 4.0, float(Ls)))
+    u = np.random.default_rng(3).uniform(-1.0, 1.5, (T, 2))
+    r = sp.Reservoir(cfg, seed=11)
+    assert r.set_launch(ctas=8, warps_max=1, variant=1, rows=rows, stages=2) == sp.SPIRES_OK
+    parts = [r.run_record(x) for x in (u[:7], u[7:8], u[8:])]
+    r.close()
+    phi = np.concatenate([p[0] for p in parts])
+    phi_o, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=11)).run(u)
+    assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
