@@ -453,6 +453,11 @@ __global__ void __launch_bounds__(kBatchThreads, kSpread ? 1 : 2) k_batch(BParam
         const bool gl = I.ntype == SP_FLIF_GL;
         const int wb0 = (int)((long long)rank * nw / gsize);
         const int wb1 = (int)((long long)(rank + 1) * nw / gsize);
+        // A CTA without neurons (a group wider than the instance) publishes nothing, so
+        // nobody waits for its reads and the entries could be overwritten before
+        // it has seen them: it takes no part.
+        if (wb0 == wb1)
+            continue;
         const int gw = wb0 + warp;
         const bool wact = gw < wb1;
         const int i = gw * 32 + lane;

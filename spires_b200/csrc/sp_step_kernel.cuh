@@ -48,7 +48,9 @@
 // a fence and a second load, and no CTA-wide barrier before the store. Entries
 // alternate between two buffers: a warp publishes step b + 1 only after it has
 // read every word of step b, so nobody can still be reading the buffer of
-// step b - 1 that it overwrites. (LIF_DISCRETE N=20000: 6.7 us per step with
+// step b - 1 that it overwrites. That holds for a reader only if a warp that
+// publishes waits for it: a CTA without neurons (more CTAs than warps), and in
+// variant 3 a warp without, read no words and skip the steps. (LIF_DISCRETE N=20000: 6.7 us per step with
 // flags and fences, 4.1 with the exchange and the row slots.) A gather warp
 // starts to poll when its own CTA has published: polled all along, the entries'
 // lines slowed the stores and the history stream (FLIF_GL N=20000, L=128: 5.9
@@ -1055,7 +1057,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     // (lane l: CTAs l, l + 32, ...) instead.
     constexpr bool kGath = VAR == 1 || VAR == 2;
     if (kGath && tid >= (VAR == 1 ? NC + 32 : NC)) {
-        if (p.G <= 1)
+        if (p.G <= 1 || (kWords && wb0 == wb1))
             return;
         for (long long b = 0; b < B; ++b) {
             bool ok = true;
@@ -1288,6 +1290,10 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             pr += p.Ls;
         Ilast = p.Iring[(size_t)pr * p.rs + i];
     }
+    // Nothing here publishes, so no other CTA waits for this one's reads of the words
+    // and their entries could be overwritten before they are seen. With column
+    // blocks (variant 3) a CTA's warps share one spike list: verdict() couples them.
+    const bool idle = kWords && (wb0 == wb1 || (VAR == 3 && !wact && !p.col_mode));
     int cur = p.phase0;
     double sprev = 0.0;
     if (act)
@@ -1486,7 +1492,9 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
                 // every warp collects all words, writing the same values into the
                 // CTA's buffer
                 bool ok = true;
-                if (b == 0) {
+                if (!wact) {
+                    // column blocks: the others' words, after verdict()
+                } else if (b == 0) {
                     for (int wi = lane; wi < p.nwords; wi += 32)
                         dst[wi] = __ldcg(p.spk + (size_t)cur * p.nwords + wi);
                 } else {
@@ -1568,7 +1576,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
             cp_async8(s_ur + (row & (kURows - 1)) * p.din + lane, p.u + (size_t)row * p.din + lane);
         cp_async_commit();
     };
-    if (p.u_ring)
+    if (p.u_ring && !idle)
         for (int r = 0; r < kURows; ++r)
             u_issue(r);
 
@@ -1631,7 +1639,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     }
     int s = 0, m = 0;                   // macro step, micro-step within it
     int head = (int)(p.step0 % L);      // ring row of the step
-    for (long long b = 0; b < B; ++b) {
+    for (long long b = idle ? B : 0; b < B; ++b) {
         const long long g = p.step0 + b;
         SP_STAMP(tid == 0, b, B, 0);
         if (m == 0) {

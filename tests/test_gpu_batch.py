@@ -289,3 +289,22 @@ def test_fits_of_a_batch_share_their_launches():
         if n != 700:
             assert np.array_equal(W2[k], W[k]), f"instance {k} (n={n})"
     b.close()
+
+
+def test_groups_wider_than_an_instance():
+    """Instances of one warp beside wide ones: the schedules that autotune times put
+    them on groups with CTAs that have no neurons of theirs, several in turn."""
+    rng = np.random.default_rng(6)
+    ns = [20, 32, 7, 1] * 40 + [2300, 1200, 600]
+    cfgs = [sp.make_config(n, 2, 1, rho=1.2, ei=0.5, gamma=1.5, conn=0.1, topo=sp.CONN_RANDOM,
+                           neuron=sp.LIF_DISCRETE, nparams=(0.0, 1.0, 0.1, 0.05)) for n in ns]
+    seeds = [int(s) for s in rng.integers(1, 2**31 - 1, len(ns))]
+    us = [rng.uniform(-1.0, 2.0, size=(200, 2)) for _ in ns]
+    b = sp.Batch(cfgs, seeds)
+    b.autotune(us)
+    R, V, _ = b.run(us)
+    b.close()
+    for k in list(range(0, len(ns), 23)) + [160, 161, 162]:
+        Rs, Vs = solo(cfgs[k], seeds[k], us[k])
+        assert np.array_equal(R[k], Rs), f"instance {k} (n={ns[k]})"
+        assert same_bits(V[k], Vs), f"instance {k} (n={ns[k]})"

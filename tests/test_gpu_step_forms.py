@@ -144,3 +144,31 @@ def test_fractional_history_with_stages_taller_than_the_ring(L, rows, Ls):
     phi = np.concatenate([p[0] for p in parts])
     phi_o, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=11)).run(u)
     assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
+
+
+# 7 warps of neurons: more CTAs than warps (clusters of 8 and 16, the L2's exchange on
+# 12); 25 warps on 16 CTAs and 19 on 4: CTAs with a warp less than the others
+@pytest.mark.parametrize("n,ctas", [(200, 8), (200, 16), (200, 12), (800, 16), (600, 4)])
+@pytest.mark.parametrize("neuron,synapse", [(sp.LIF_DISCRETE, sp.SYN_SIMPLE),
+                                            (sp.LIF_DISCRETE, sp.SYN_PSC_HET),
+                                            (sp.FLIF_GL, sp.SYN_SIMPLE),
+                                            (sp.FLIF_CAPUTO, sp.SYN_SIMPLE)])
+@pytest.mark.parametrize("conn", [0.005, 0.1])
+def test_ctas_and_warps_without_neurons(n, ctas, neuron, synapse, conn):
+    """They publish no spike words and read none; rows as slots and as column blocks."""
+    check(n, neuron, ctas, 300, synapse=synapse, conn=conn)
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+def test_more_ctas_than_warps_with_a_gather_warp(variant):
+    """FLIF_GL with its history in shared memory and through the stages."""
+    n, T = 200, 120
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=0.05,
+                         topo=sp.CONN_RANDOM, neuron=sp.FLIF_GL, nparams=GL(64))
+    u = np.random.default_rng(3).uniform(-1.0, 1.5, (T, 2))
+    r = sp.Reservoir(cfg, seed=11)
+    assert r.set_launch(ctas=40, warps_max=1, variant=variant, rows=16, stages=2) == sp.SPIRES_OK
+    phi, _, _ = r.run_record(u)
+    r.close()
+    phi_o, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=11)).run(u)
+    assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
