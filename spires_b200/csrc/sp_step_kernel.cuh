@@ -731,6 +731,9 @@ __device__ __forceinline__ double caputo_sum(double newest, const double *tab, c
                                              long long row, int D, int pos)
 {
     double mem = add(0.0, mul(tab[0], newest));
+    // the loads below stay between the stores of the steps around (ld_f64x4 does not
+    // say that it reads memory, so that the sums' other loads may move past it)
+    asm volatile("" ::: "memory");
     // element numbers below count from the 32-byte boundary at or under the row
     const int r0 = (int)(row & 3);
     const double *base = ring + (row - r0);
@@ -790,6 +793,7 @@ __device__ __forceinline__ double caputo_sum(double newest, const double *tab, c
         for (int q = 0; q < Q; ++q)
             sum(nxt[q]);
     }
+    asm volatile("" ::: "memory");
     return mem;
 }
 
@@ -1475,6 +1479,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     // only after everybody has read it.
     auto verdict = [&](long long b, bool ok) -> bool {
         ok = __all_sync(kFull, ok);
+        __syncwarp();  // the vote orders no memory: the lanes' (lane 0's) words before all reads
         if (ST != SP_SYN_SIMPLE || !p.col_mode)
             return ok;
         if (!ok)
@@ -1747,6 +1752,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         // ---- barrier: spikes / eff of step g-1 are visible
         SP_STAMP(tid == 0, b, B, 1);
         if (!barrier_wait(b)) {
+            cp_async_wait<0>();  // input rows still on their way
             if (VAR == 3)
                 cluster_sync();  // the other CTAs may still write here
             return;
