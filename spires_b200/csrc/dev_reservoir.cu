@@ -339,10 +339,15 @@ struct RowPlan {
     size_t bytes;  // shared memory
 };
 
-static RowPlan row_plan(const sp_dev *d, const sp_launch &l)
+// Forms, from the one that takes most shared memory: the rows staged; a dense
+// matrix's column blocks in global memory, with the spike list only; none, the
+// edges walked in global memory.
+constexpr int kRowForms = 3;
+
+static RowPlan row_plan(const sp_dev *d, const sp_launch &l, int form = 0)
 {
     RowPlan r = {0, 0, 0, 0, 0};
-    if (d->stype != SP_SYN_SIMPLE || l.ctas < 1 || l.csr_global)
+    if (d->stype != SP_SYN_SIMPLE || l.ctas < 1 || l.csr_global || form == kRowForms - 1)
         return r;
     const long long nw = (long long)d->nwords;
     if (d->col_blk) {
@@ -353,12 +358,12 @@ static RowPlan row_plan(const sp_dev *d, const sp_launch &l)
         r.col_mode = 1;
         r.bytes = ((nwn + 3) / 4 * 16 + (size_t)d->n * 2 + 8 + 127) / 128 * 128;
         const size_t b = ((size_t)mx * 8 + (size_t)l.warps_max * d->n * 8 + 127) / 128 * 128;
-        if (b <= (l.variant == 1 ? kColSmem1 : kColSmem0)) {
+        if (form == 0 && b <= (l.variant == 1 ? kColSmem1 : kColSmem0)) {
             r.col_mode = 2;
             r.col_cap = mx;
             r.bytes += b;
         }
-    } else if (d->ell_off) {
+    } else if (form == 0 && d->ell_off) {
         int mg = 1, mt = 0;
         for (long long b = 0; b < l.ctas; ++b) {
             const long long w0 = b * nw / l.ctas, w1 = (b + 1) * nw / l.ctas;
@@ -460,18 +465,20 @@ static bool stages_coef(const sp_dev *d, int kv)
 static int extra_warps(int kv) { return kv == 1 ? 2 : kv == 2 ? 1 : 0; }
 
 struct SmemPlan {
-    int win_smem, u_ring, frac_stage;
+    RowPlan rows;
+    int coef_smem, win_smem, u_ring, frac_stage;
     size_t bytes;
 };
 
 static SmemPlan smem_plan(const sp_dev *d, const sp_launch &l, int kv)
 {
-    SmemPlan pl = {0, 0, 0, 0};
-    size_t b = spk_smem_bytes(d) + row_plan(d, l).bytes;
+    SmemPlan pl = {};
+    size_t b = spk_smem_bytes(d);
     if (kv == 3)
         b += ((size_t)16 * d->nwords + 127) / 128 * 128;
     const bool pairs = kv >= 2 && d->ntype == SP_FLIF_GL;  // ring rows in pairs
-    if (stages_coef(d, kv))
+    pl.coef_smem = stages_coef(d, kv);
+    if (pl.coef_smem)
         b += (pairs ? 2 : 1) * coef_smem_bytes(d);
     if (pairs)
         b += (size_t)(d->nc.L + 1) / 2 * 64 * l.warps_max * sizeof(double);
@@ -480,6 +487,19 @@ static SmemPlan smem_plan(const sp_dev *d, const sp_launch &l, int kv)
         box_geometry(d, l, &bw, &nbx);
         b += (size_t)l.stages * nbx * l.rows * bw * sizeof(double) +
              2 * (size_t)l.stages * sizeof(unsigned long long);
+    }
+    // The rows take the largest form that the rest leaves room for, in the kernels
+    // that a launch cannot do without: the generic one, the pipeline asked for,
+    // FLIF_CAPUTO's. (A FLIF_GL history or a cluster's exchange in shared memory that
+    // leaves the rows no room is not taken: kernel_variant.) Without staged rows the
+    // generic kernel always fits: 38 KB of words, 35 of a spike list, 64 of
+    // coefficients at most.
+    pl.rows = row_plan(d, l);
+    if (kv < 2 || (kv == 2 && d->ntype == SP_FLIF_CAPUTO))
+        for (int form = 1; form < kRowForms && b + pl.rows.bytes + 1024 > (size_t)d->smem_max; ++form)
+            pl.rows = row_plan(d, l, form);
+    b += pl.rows.bytes;
+    if (kv == 1) {
         const size_t sc = scoef_smem_bytes(d);
         if (sc > 0 && d->sc.frac_L >= (l.rows < d->nc.L ? l.rows : d->nc.L) &&
             b + sc + 1024 <= (size_t)d->smem_max) {
@@ -501,6 +521,20 @@ static SmemPlan smem_plan(const sp_dev *d, const sp_launch &l, int kv)
     }
     pl.bytes = b;
     return pl;
+}
+
+// Stages of `stage` bytes (at most 16) that a pipeline launch has room for with
+// `spare` bytes left over: beside the largest form of the rows that leaves two.
+static long long pipe_stages(const sp_dev *d, const sp_launch &l, size_t stage, size_t spare)
+{
+    const size_t budget = (size_t)d->smem_max - spare;
+    long long st = 0;
+    for (int form = 0; form < kRowForms && st < 2; ++form) {
+        const size_t base = spk_smem_bytes(d) + coef_smem_bytes(d) + scoef_smem_bytes(d) +
+                            row_plan(d, l, form).bytes;
+        st = budget > base ? (long long)((budget - base) / (stage + 16)) : 0;
+    }
+    return st < 16 ? st : 16;
 }
 
 static int kernel_variant(const sp_dev *d, const sp_launch &l)
@@ -702,12 +736,7 @@ static void default_launch(sp_dev *d)
             int bw, nbx;
             box_geometry(d, v, &bw, &nbx);
             const size_t stage = (size_t)v.rows * nbx * bw * sizeof(double);
-            const size_t budget = (size_t)(d->smem_max - 2 * 1024);
-            const size_t spk = spk_smem_bytes(d) + coef_smem_bytes(d) + scoef_smem_bytes(d) +
-                               row_plan(d, v).bytes;
-            long long st = budget > spk ? (long long)((budget - spk) / (stage + 16)) : 0;
-            if (st > 16)
-                st = 16;
+            long long st = pipe_stages(d, v, stage, 2 * 1024);
             if (auto_l2_pin(d) > 0 && st > (long long)(144 * 1024 / stage))
                 st = (long long)(144 * 1024 / stage);
             if (st >= 2 && st * rows > best_rows &&
@@ -1270,7 +1299,9 @@ extern "C" int sp_dev_launch_chunk(sp_dev *d, const double *u, size_t T, double 
     d->hold_cta = -1;
     d->hold_b = -1;
     p.nid_of = d->nid_of;
-    const RowPlan rows = row_plan(d, l);
+    const int kv = kernel_variant(d, l);
+    const SmemPlan sm = smem_plan(d, l, kv);
+    const RowPlan &rows = sm.rows;
     p.ell_cap = rows.ell_cap;
     p.tail_cap = rows.tail_cap;
     p.ell_off = d->ell_off;
@@ -1290,15 +1321,13 @@ extern "C" int sp_dev_launch_chunk(sp_dev *d, const double *u, size_t T, double 
     p.ll = d->ll;
     p.ll_base = d->ll_seq;
 
-    const int kv = kernel_variant(d, l);
     kfn_t fn = pick_kernel(d->ntype, d->stype, kv);
     if (!fn)
         return SP_EINVAL;
-    const SmemPlan sm = smem_plan(d, l, kv);
     const size_t smem = sm.bytes;
     p.win_smem = sm.win_smem;
     p.u_ring = sm.u_ring && u && d->gamma != 0.0;
-    p.coef_smem = stages_coef(d, kv);
+    p.coef_smem = sm.coef_smem;
     p.frac_stage = sm.frac_stage;
     if (sm.frac_stage)
         p.tmap_s = d->tmap_s;
@@ -1700,11 +1729,7 @@ extern "C" int sp_dev_autotune(sp_dev *d, size_t steps)
                 int bw, nbx;
                 box_geometry(d, v, &bw, &nbx);
                 const size_t stage = (size_t)rows * nbx * bw * 8;
-                const size_t base = spk_smem_bytes(d) + coef_smem_bytes(d) + row_plan(d, v).bytes;
-                const size_t budget = (size_t)(d->smem_max - 8 * 1024);
-                long long st = budget > base ? (long long)((budget - base) / (stage + 16)) : 0;
-                if (st > 16)
-                    st = 16;
+                const long long st = pipe_stages(d, v, stage, 8 * 1024);
                 if (st < 2)
                     continue;
                 v.stages = (int)st;

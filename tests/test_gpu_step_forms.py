@@ -172,3 +172,33 @@ def test_more_ctas_than_warps_with_a_gather_warp(variant):
     r.close()
     phi_o, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=11)).run(u)
     assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
+
+
+def run_against_oracle(r, cfg, T, seed):
+    u = np.random.default_rng(3).uniform(-1.0, 1.5, (T, 2))
+    phi, _, _ = r.run_record(u)
+    r.close()
+    phi_o, _, _ = O.Oracle(cfg, sp.HostModel(cfg, seed=seed)).run(u)
+    assert np.array_equal(phi.view(np.uint64), phi_o.view(np.uint64))
+
+
+@pytest.mark.parametrize("n,edges,D", [(6000, 128, 7400), (4000, 505, 8180)])
+def test_caputo_table_beside_dense_rows(n, edges, D):
+    """Column blocks and memory coefficients that fit a CTA's shared memory one by one
+    and not together: the default launch keeps what fits."""
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=edges / n, dt=1.0,
+                         topo=sp.CONN_RANDOM, neuron=sp.FLIF_CAPUTO,
+                         nparams=(1.0, 0.2, 0.0, 1.0, 0.0, 1.5, 0.7, 2.0, float(D + 2)))
+    run_against_oracle(sp.Reservoir(cfg, seed=11), cfg, 24, 11)
+
+
+@pytest.mark.parametrize("n,conn,stages", [(1000, 0.1, 13), (2000, 0.004, 13)])
+def test_stages_that_leave_the_rows_no_room(n, conn, stages):
+    """A pipeline that takes all the shared memory: the rows are read from global
+    memory, as column blocks or edge by edge."""
+    nw = (n + 31) // 32
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=conn, dt=1.0,
+                         topo=sp.CONN_RANDOM, neuron=sp.FLIF_GL, nparams=GL(64))
+    r = sp.Reservoir(cfg, seed=11)
+    assert r.set_launch(ctas=nw, warps_max=1, variant=1, rows=64, stages=stages) == sp.SPIRES_OK
+    run_against_oracle(r, cfg, 150, 11)
