@@ -202,3 +202,14 @@ def test_stages_that_leave_the_rows_no_room(n, conn, stages):
     r = sp.Reservoir(cfg, seed=11)
     assert r.set_launch(ctas=nw, warps_max=1, variant=1, rows=64, stages=stages) == sp.SPIRES_OK
     run_against_oracle(r, cfg, 150, 11)
+
+
+def test_pipeline_with_coefficients_in_global_memory():
+    """More coefficients than the launch stages (8192), a chain of stages and a
+    ragged one by the end."""
+    n = 70
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=0.2, dt=1.0,
+                         topo=sp.CONN_RANDOM, neuron=sp.FLIF_GL, nparams=GL(8300))
+    r = sp.Reservoir(cfg, seed=11)
+    assert r.set_launch(ctas=3, warps_max=1, variant=1, rows=16, stages=3) == sp.SPIRES_OK
+    run_against_oracle(r, cfg, 90, 11)
