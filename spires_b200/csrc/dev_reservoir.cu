@@ -654,9 +654,9 @@ static int encode_ring_map(sp_dev *d, int bw, int r)
 // row under plain replacement (each row is read once per step, in a cycle
 // longer than the cache), so the oldest lags of every step -- 60 % of the L2
 // -- are read with evict-last priority and stay resident, while younger rows
-// stream through with evict-first. (N=20000, L=1024 on one B200, 256 steps
-// with readouts: 420 lags 6.47 ms, 490 lags -- 70 % -- 6.52, 560 lags 6.60;
-// without hints 7.7.)
+// stream through with evict-first. (N=20000, L=1024 on one B200, scale-free
+// graph, 256 steps with readouts: 350 lags 22.9 us per step, 420 23.0, 490 -- 70 %
+// -- 23.4, 560 24.5; without hints 28.2.)
 static int auto_l2_pin(const sp_dev *d)
 {
     const double row = (double)d->rs * sizeof(double);
@@ -721,10 +721,11 @@ static void default_launch(sp_dev *d)
         // The ring stream is paced by the bytes in flight per SM (the stages
         // the consumers are not reading): long rings take the stage height of
         // 64 or 48 rows that puts the most rows in flight (ties: taller),
-        // shorter rings 32-row stages. A ring beyond the L2 takes at most 144
-        // KB of them: more slow the serial phase's loads and the resident lags
-        // more than they speed the stream (N=20000, L=1024 on 148 SMs, 256
-        // steps: 2 x 64 rows 6.52 ms, 4 x 32 6.55, 3 x 48 6.69, 4 x 40 6.96).
+        // shorter rings 32-row stages. (128 steps on 148 SMs, us per step on a
+        // scale-free graph and on a small world: N=20000, L=1024 3 x 48 rows 22.8
+        // and 19.6, 2 x 64 23.5 and 21.1, 2 x 48 25.3 and 22.8; N=12000, L=2000 4 x
+        // 64 28.2 and 28.3, 3 x 64 29.2 and 28.8; N=32000, L=1024, where only 2 x
+        // 48 fit, 35.3 and 36.1, and 162 in the generic kernel.)
         sp_launch best = l;
         long long best_rows = 0;
         for (int rows : {64, 48, 32}) {
@@ -737,8 +738,6 @@ static void default_launch(sp_dev *d)
             box_geometry(d, v, &bw, &nbx);
             const size_t stage = (size_t)v.rows * nbx * bw * sizeof(double);
             long long st = pipe_stages(d, v, stage, 2 * 1024);
-            if (auto_l2_pin(d) > 0 && st > (long long)(144 * 1024 / stage))
-                st = (long long)(144 * 1024 / stage);
             if (st >= 2 && st * rows > best_rows &&
                 encode_ring_map(d, bw, v.rows < d->nc.L ? v.rows : d->nc.L) == SP_OK) {
                 v.stages = (int)st;

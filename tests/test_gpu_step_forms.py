@@ -213,3 +213,15 @@ def test_pipeline_with_coefficients_in_global_memory():
     r = sp.Reservoir(cfg, seed=11)
     assert r.set_launch(ctas=3, warps_max=1, variant=1, rows=16, stages=3) == sp.SPIRES_OK
     run_against_oracle(r, cfg, 90, 11)
+
+
+@pytest.mark.parametrize("n,L", [(30000, 1024), (37500, 600)])
+def test_wide_ctas_keep_the_pipeline(n, L):
+    """Rings beyond the L2 on CTAs of seven and eight warps, where two stages take more
+    than the share that narrower CTAs keep to."""
+    cfg = sp.make_config(n, 1, 1, rho=0.0, conn=2.0 / n, topo=sp.CONN_SMALL_WORLD,
+                         neuron=sp.FLIF_GL, nparams=GL(L))
+    r = sp.Reservoir(cfg, seed=1)
+    l = r.launch()
+    r.close()
+    assert l.variant == 1 and l.stages >= 2
