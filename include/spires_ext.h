@@ -313,8 +313,8 @@ spires_status spires_ext_agile_batch_best(const spires_ext_agile_batch *b, int c
  * Cholesky factorisation fails and so does LU with partial pivoting) returns
  * SPIRES_ERR_INTERNAL with d_w_out left as it was. The first call on a device
  * looks up the array's device address, so make that first call before any
- * stream capture. Every call shares the one array, so calls that overlap on
- * the GPU (other streams, other host threads) race; serialise them. `stream`
+ * stream capture. Every call on a device shares the one array: calls from
+ * several host threads wait for one another, whatever their streams. `stream`
  * is a cudaStream_t (NULL = default stream). Each call waits on the host for
  * its work on that stream: the refinement reads a residual norm back after
  * every sweep, and the call returns after the last kernel has finished. */

@@ -16,6 +16,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <vector>
+#include <mutex>
 #include <cmath>
 #include <chrono>
 #include "sp_alloc.h"
@@ -1709,14 +1710,16 @@ static __device__ __align__(256) double g_na_scratch[SP_NA_DOUBLES];
 static __device__ __align__(256) int g_na_iscratch[SP_NA_MAX_N + 8];
 
 // Device addresses of the two arrays, looked up once per device (with that
-// device current) on the first call made on it.
+// device current) on the first call made on it, and the lock that a call holds
+// until its work on them has ended: the solver's flags and hand-out counter are
+// in them too, and a second call that zeroed those under a running factorisation
+// would have its tiles taken before they are ready.
 static double *g_na_dptr[64];
 static int *g_na_iptr[64];
+static std::mutex g_na_lock[64];
 
 static int na_setup(int dev)
 {
-    if (dev < 0 || dev >= 64)
-        return SP_EINTERNAL;
     if (g_na_dptr[dev] && g_na_iptr[dev])
         return SP_OK;
     void *pd = nullptr, *pi = nullptr;
@@ -1729,28 +1732,13 @@ static int na_setup(int dev)
     return SP_OK;
 }
 
-extern "C" __attribute__((visibility("default"))) int
-spires_ext_ridge_solve_noalloc(const double *d_states, const double *d_targets, size_t T,
-                               size_t n_, size_t dout_, size_t washout, double lambda,
-                               double *d_w_out, void *stream)
+// The solve, with the device's lock held.
+static int na_solve(int dev, const double *d_states, const double *d_targets, size_t T, int n,
+                    int dout, size_t washout, double lambda, double *d_w_out, cudaStream_t s)
 {
-    if (!d_states || !d_targets || !d_w_out || T == 0 || n_ == 0 || dout_ == 0 || washout >= T)
-        return SP_EINVAL;
-    if (n_ > SP_NA_MAX_N || dout_ > SP_NA_MAX_DOUT || T > SP_NA_MAX_T) {
-        fprintf(stderr,
-                "spires_ext_ridge_solve_noalloc: size beyond the fixed work area "
-                "(N=%zu > %d, outputs=%zu > %d or rows=%zu > %d)\n",
-                n_, SP_NA_MAX_N, dout_, SP_NA_MAX_DOUT, T, SP_NA_MAX_T);
-        return SP_EINVAL;
-    }
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess)
-        return SP_EINTERNAL;
     int rc = na_setup(dev);
     if (rc)
         return rc;
-    const int n = (int)n_, dout = (int)dout_;
-    cudaStream_t s = (cudaStream_t)stream;
     double *A = g_na_dptr[dev];
     double *B = A + (size_t)SP_NA_MAX_N * SP_NA_MAX_N;
     double *W = B + (size_t)SP_NA_MAX_N * SP_NA_MAX_DOUT;
@@ -1759,7 +1747,7 @@ spires_ext_ridge_solve_noalloc(const double *d_states, const double *d_targets, 
     double *part = E + (size_t)SP_NA_MAX_T * SP_NA_MAX_DOUT;
     double *tmp = part + (size_t)SP_NA_PARTS * SP_NA_MAX_N * SP_NA_MAX_DOUT;
     void *work = tmp + 8;
-    const int lda = sp_solve_pad((int)n_);
+    const int lda = sp_solve_pad(n);
     int *info = g_na_iptr[dev];
     int *piv = info + 8;
     const int parts = SP_NA_PARTS;
@@ -1818,4 +1806,31 @@ spires_ext_ridge_solve_noalloc(const double *d_states, const double *d_targets, 
     if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
         return SP_EINTERNAL;
     return SP_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int
+spires_ext_ridge_solve_noalloc(const double *d_states, const double *d_targets, size_t T,
+                               size_t n_, size_t dout_, size_t washout, double lambda,
+                               double *d_w_out, void *stream)
+{
+    if (!d_states || !d_targets || !d_w_out || T == 0 || n_ == 0 || dout_ == 0 || washout >= T)
+        return SP_EINVAL;
+    if (n_ > SP_NA_MAX_N || dout_ > SP_NA_MAX_DOUT || T > SP_NA_MAX_T) {
+        fprintf(stderr,
+                "spires_ext_ridge_solve_noalloc: size beyond the fixed work area "
+                "(N=%zu > %d, outputs=%zu > %d or rows=%zu > %d)\n",
+                n_, SP_NA_MAX_N, dout_, SP_NA_MAX_DOUT, T, SP_NA_MAX_T);
+        return SP_EINVAL;
+    }
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess)
+        return SP_EINTERNAL;
+    if (dev < 0 || dev >= 64)
+        return SP_EINTERNAL;
+    std::lock_guard<std::mutex> lock(g_na_lock[dev]);
+    const int rc = na_solve(dev, d_states, d_targets, T, (int)n_, (int)dout_, washout, lambda,
+                            d_w_out, (cudaStream_t)stream);
+    if (rc)
+        cudaStreamSynchronize((cudaStream_t)stream);  // nothing of it is left on the work area
+    return rc;
 }

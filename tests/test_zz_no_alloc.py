@@ -129,3 +129,45 @@ def test_noalloc_ridge_singular_and_sizes():
                  (0, n, dout, 0)):
         assert lib.spires_ext_ridge_solve_noalloc(p(dev.phi), p(dev.y), *args, 1e-3, p(dev.w),
                                                   s) == sp.SPIRES_ERR_INVALID_ARG
+
+
+def test_noalloc_ridge_from_two_threads():
+    """Two host threads, each with its own stream and system: the calls share the work
+    area one after the other, so each result is the bits of a call made alone."""
+    import threading
+
+    import torch
+
+    lib = sp.load()
+    rng = np.random.default_rng(3)
+    devs, alone = [], []
+    shapes = [(500, 2, 700), (310, 5, 900)]
+    for n, dout, T in shapes:
+        dev = _Dev(rng.standard_normal((T, n)), rng.standard_normal((T, dout)), dout, n)
+        st, W = dev.solve(lib, T, n, dout, 10, 1e-3)
+        assert st == sp.SPIRES_OK
+        devs.append(dev)
+        alone.append(W)
+    got = [[], []]
+
+    def work(k):
+        n, dout, T = shapes[k]
+        stream = torch.cuda.Stream()
+        w = [torch.empty_like(devs[k].w) for _ in range(20)]
+        torch.cuda.synchronize()
+        for out in w:
+            st = lib.spires_ext_ridge_solve_noalloc(
+                _Dev.ptr(devs[k].phi), _Dev.ptr(devs[k].y), T, n, dout, 10, 1e-3, _Dev.ptr(out),
+                C.c_void_p(stream.cuda_stream))
+            got[k].append((st, out))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(2):
+        assert len(got[k]) == 20
+        for st, out in got[k]:
+            assert st == sp.SPIRES_OK
+            assert np.array_equal(out.cpu().numpy(), alone[k])
