@@ -1642,7 +1642,9 @@ extern "C" long long sp_dev_kernel_launches(const sp_dev *d) { return d->launche
 // ------------------------------------------------------------- autotuner --
 // Candidate launch shapes are timed from one saved state (every mutable device
 // buffer and the step counters are snapshotted, and restored after each
-// candidate and at the end), with zero input, `steps` macro steps each.
+// candidate and at the end), with zero input, `steps` macro steps each. The launch
+// in force is the first of them and the default one the second; another has to
+// be 1 % faster than the first, so that two timings of one shape do not swap it.
 
 struct sp_snap_item {
     void *ptr;
@@ -1699,7 +1701,10 @@ extern "C" int sp_dev_autotune(sp_dev *d, size_t steps)
     const long long step0 = d->step, syn0 = d->syn_step;
     const int phase0 = d->phase;
     int rc = snapshot(d, items, true);
-    std::vector<sp_launch> cand;
+    const sp_launch keep = d->launch;
+    default_launch(d);
+    std::vector<sp_launch> cand = {keep, d->launch};
+    d->launch = keep;
     const int nw = d->nw;
     std::vector<int> Gs;
     auto addG = [&](int g) {
@@ -1740,30 +1745,35 @@ extern "C" int sp_dev_autotune(sp_dev *d, size_t steps)
             }
         }
     }
-    const sp_launch keep = d->launch;
     sp_launch best = keep;
     float best_ms = 1e30f;
+    float keep_ms = 1e30f;  // of candidate 0, less 1 %
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (!rc && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
         rc = SP_EINTERNAL;
     for (size_t c = 0; c < cand.size() && !rc; ++c) {
         if (sp_dev_set_launch(d, &cand[c]) != SP_OK)
             continue;
-        cudaEventRecord(e0, d->stream);
-        int r2 = sp_dev_launch_chunk(d, nullptr, steps, nullptr, nullptr);
-        cudaEventRecord(e1, d->stream);
-        int r3 = sp_dev_sync(d);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (!r2 && !r3 && ms < best_ms) {
-            best_ms = ms;
-            best = cand[c];
+        // the faster of two launches: the first may load the kernel
+        for (int pass = 0; pass < 2; ++pass) {
+            cudaEventRecord(e0, d->stream);
+            int r2 = sp_dev_launch_chunk(d, nullptr, steps, nullptr, nullptr);
+            cudaEventRecord(e1, d->stream);
+            int r3 = sp_dev_sync(d);
+            float ms = 0.f;
+            cudaEventElapsedTime(&ms, e0, e1);
+            if (!r2 && !r3 && c == 0)
+                keep_ms = std::min(keep_ms, 0.99f * ms);
+            if (!r2 && !r3 && ms < best_ms && (c == 0 || ms < keep_ms)) {
+                best_ms = ms;
+                best = cand[c];
+            }
+            // back to the saved state
+            snapshot(d, items, false);
+            d->step = step0;
+            d->syn_step = syn0;
+            d->phase = phase0;
         }
-        // back to the saved state
-        snapshot(d, items, false);
-        d->step = step0;
-        d->syn_step = syn0;
-        d->phase = phase0;
     }
     if (e0)
         cudaEventDestroy(e0);

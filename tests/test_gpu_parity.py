@@ -237,3 +237,36 @@ def test_autotune_keeps_state_and_results(neuron, L):
     pb, _, _ = b.run_record(u)
     b.close()
     assert same_bits(np.concatenate([pa1, pa2]), pb)
+
+
+def step_time(r, T, passes=6):
+    """Seconds of T steps without input, the fastest of several passes."""
+    import time
+
+    best = 1e9
+    for _ in range(passes):
+        t0 = time.perf_counter()
+        assert r.lib.spires_ext_run_device(r.h, None, T, None, None, None) == sp.SPIRES_OK
+        assert r.lib.spires_ext_sync(r.h) == sp.SPIRES_OK
+        best = min(best, time.perf_counter() - t0)
+    return best
+
+
+@pytest.mark.parametrize("n,neuron,L", [(20000, sp.LIF_DISCRETE, 0), (2000, sp.LIF_DISCRETE, 0),
+                                        (12000, sp.FLIF_GL, 2000)])
+def test_autotune_is_no_slower_than_the_launch_it_found(n, neuron, L):
+    """The launch in force is timed with the others: 125 CTAs, one cluster, and tall
+    stages, none of which the list of shapes holds. A tenth is far above what two
+    timings of one shape differ by, and below what the next shape costs."""
+    params = (1.0, 0.0, 0.0, 20.0, 0.6, float(L), 0.1, 2.0) if L else (0.0, 1.0, 0.3, 0.05)
+    cfg = sp.make_config(n, 1, 1, rho=0.0, ei=0.5, gamma=0.5, conn=8.0 / n,
+                         topo=sp.CONN_SMALL_WORLD, neuron=neuron, nparams=params)
+    r = sp.Reservoir(cfg, seed=4)
+    T = 200 if L else 2000
+    for _ in range(L // T + 1):
+        step_time(r, T, 1)
+    before = step_time(r, T)
+    assert r.lib.spires_ext_autotune(r.h, 64) == sp.SPIRES_OK
+    after = step_time(r, T)
+    r.close()
+    assert after <= 1.1 * before
