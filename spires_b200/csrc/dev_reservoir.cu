@@ -363,7 +363,7 @@ static RowPlan row_plan(const sp_dev *d, const sp_launch &l, int form = 0)
             r.col_cap = mx;
             r.bytes += b;
         }
-    } else if (form == 0 && d->ell_off) {
+    } else if (form == 0 && d->h_ell_off) {
         int mg = 1, mt = 0;
         for (long long b = 0; b < l.ctas; ++b) {
             const long long w0 = b * nw / l.ctas, w1 = (b + 1) * nw / l.ctas;
@@ -967,21 +967,35 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
             d->col_blk = (uint2 *)(d->rows_buf + o_blk);
             d->col_w = (double *)(d->rows_buf + o_w);
             d->col_off = (int *)(d->rows_buf + o_off);
-        } else if (m->syn_type == SP_SYN_SIMPLE && rs <= 65536) {
+        } else if (m->syn_type == SP_SYN_SIMPLE && rs <= 65536 && m->nnz < ((size_t)1 << 31)) {
             int *eo = d->h_ell_off = (int *)calloc(d->nw + 1, sizeof(int));
             int *to = d->h_tail_off = (int *)calloc(d->nw + 1, sizeof(int));
             if (!eo || !to)
                 TRY(SP_EALLOC);
-            size_t cells = 0;
             for (int q = 0; q < d->nw; ++q) {
                 const int g = row_slots(rp.data() + 32 * q);
                 eo[q + 1] = eo[q] + g;
-                cells += (size_t)128 * g;
+                to[q + 1] = to[q];
+                for (int r = 32 * q; r < 32 * q + 32; ++r)
+                    to[q + 1] += (int)std::max(0ll, rp[r + 1] - rp[r] - 4 * g);
             }
-            const size_t nnz = m->nnz;
+            // built where a launch has room for them: the widest takes two CTAs per SM
+            sp_launch wide;
+            memset(&wide, 0, sizeof(wide));
+            wide.ctas = std::min(d->nw, 2 * std::max(d->num_sms, 1));
+            wide.warps_max = (d->nw + wide.ctas - 1) / wide.ctas;
+            if (row_plan(d, wide).ell_cap == 0) {
+                free(d->h_ell_off);
+                free(d->h_tail_off);
+                d->h_ell_off = d->h_tail_off = nullptr;
+            }
+        }
+        if (d->h_ell_off) {
+            const int *eo = d->h_ell_off;
+            const size_t cells = (size_t)128 * eo[d->nw], tails = (size_t)d->h_tail_off[d->nw];
             Packed pk;
-            const size_t o_c = pk.add(cells * 2), o_w = pk.add(cells * 8), o_tc = pk.add(nnz * 4),
-                         o_tw = pk.add(nnz * 8), o_rp = pk.add((size_t)33 * d->nw * 4),
+            const size_t o_c = pk.add(cells * 2), o_w = pk.add(cells * 8), o_tc = pk.add(tails * 4),
+                         o_tw = pk.add(tails * 8), o_rp = pk.add((size_t)33 * d->nw * 4),
                          o_off = pk.add((d->nwords + 1) * 4);
             pk.host.assign(pk.bytes, 0);
             char *hb = pk.host.data();
@@ -1007,7 +1021,6 @@ extern "C" int sp_dev_create(const sp_host_model *m, sp_dev **out)
                     }
                 }
                 trp[(size_t)33 * q + 32] = nt;
-                to[q + 1] = nt;
             }
             memcpy(hb + o_off, eo, (d->nwords + 1) * 4);
             TRY(pk.upload(&d->rows_buf, s));

@@ -53,3 +53,22 @@ def test_created_reservoir_keeps_weight_parity():
     m = sp.HostModel(cfg, seed=99)
     assert m.info.nnz >= 1 << 15
     assert np.array_equal(W.view(np.uint64), m.dense().view(np.uint64))
+
+
+def test_rows_too_long_for_shared_memory_are_kept_once():
+    """20000 rows of 400 edges fit no CTA's shared memory: the device holds the plain
+    rows (12 bytes an edge) and nothing else per edge."""
+    import torch
+
+    n, edges = 20000, 400
+    held = []
+    for deg in (2, edges):
+        cfg = sp.make_config(n, 1, 1, rho=0.0, conn=deg / n, topo=sp.CONN_SMALL_WORLD,
+                             neuron=sp.LIF_DISCRETE, nparams=(0.0, 1.0, 0.3, 0.05))
+        sp.Reservoir(cfg, seed=1).close()  # kernels loaded, pools made
+        free = torch.cuda.mem_get_info()[0]
+        r = sp.Reservoir(cfg, seed=1)
+        held.append(free - torch.cuda.mem_get_info()[0])
+        r.close()
+    m = sp.HostModel(cfg, seed=1)
+    assert held[1] - held[0] < 1.1 * 12 * int(m.info.nnz)
