@@ -316,9 +316,11 @@ __device__ __forceinline__ void factor_tile(double *T, double *s_inv, int *s_bad
                 const bool ok = a > 0.0 && isfinite(a);
                 if (!ok && !bad)
                     bad = c0 + j + 1;
+                // sqrt(a) as a * rsqrt(a) and one Newton step for d^2 = a, d + (a - d^2)
+                // / (2 d) with inv / 2 for 1 / (2 d)
                 const double inv = ok ? rsqrt(a) : 1.0;
                 double d = a * inv;
-                d = ok ? fma(0.5 * inv, fma(-d, d, a), d) : 1.0;  // sqrt(a), corrected
+                d = ok ? fma(0.5 * inv, fma(-d, d, a), d) : 1.0;
                 if (r == j)
                     my_inv = inv;
                 v[j] = r == j ? d : v[j] * inv;

@@ -308,3 +308,39 @@ def test_groups_wider_than_an_instance():
         Rs, Vs = solo(cfgs[k], seeds[k], us[k])
         assert np.array_equal(R[k], Rs), f"instance {k} (n={ns[k]})"
         assert same_bits(V[k], Vs), f"instance {k} (n={ns[k]})"
+
+
+def test_singular_fits_in_a_batch():
+    """Fits without a ridge term whose Cholesky fails, beside one that is solved: an
+    exactly singular system (every state 0) keeps the instance's W_out, one with
+    fewer rows than neurons takes the way that the single reservoir takes."""
+    rng = np.random.default_rng(8)
+    lif = lambda bias: dict(neuron=sp.LIF_DISCRETE, nparams=(0.0, 1.0, 0.3, bias))
+    cfgs = [sp.make_config(40, 1, 2, conn=0.2, gamma=0.0, topo=sp.CONN_RANDOM, **lif(0.0)),
+            sp.make_config(700, 1, 1, rho=1.2, gamma=1.5, conn=0.2, topo=sp.CONN_RANDOM, **lif(0.05)),
+            sp.make_config(90, 1, 3, rho=1.2, gamma=1.5, conn=0.2, topo=sp.CONN_RANDOM, **lif(0.05)),
+            sp.make_config(64, 1, 2, conn=0.2, gamma=0.0, topo=sp.CONN_RANDOM, **lif(0.0))]
+    seeds = [5, 6, 7, 8]
+    us = [rng.uniform(-1.0, 2.0, size=(300, 1)) for _ in cfgs]
+    ys = [rng.standard_normal((300, int(c.num_outputs))) for c in cfgs]
+    b = sp.Batch(cfgs, seeds)
+    W, _ = b.train_ridge(us, ys, np.array([0.0, 0.0, 1e-2, 0.0]), washout=20)
+    Y, _ = b.predict(us)
+    b.close()
+    for k, cfg in enumerate(cfgs):
+        r = sp.Reservoir(cfg, seed=seeds[k])
+        before = r.readout()
+        o, rep = sp.RidgeOpts(0, 30, 1e-13, 20), sp.RidgeReport()
+        st = r.lib.spires_ext_train_ridge(r.h, sp.dptr(us[k]), sp.dptr(ys[k]), 300,
+                                          1e-2 if k == 2 else 0.0, C.byref(o), C.byref(rep))
+        after = r.readout()
+        r.reset()
+        Y1 = r.run(us[k])
+        r.close()
+        assert st == sp.SPIRES_OK
+        if k != 1:
+            assert rep.factor_failed == (k != 2)
+        if k in (0, 3):
+            assert np.array_equal(after, before) and np.count_nonzero(before) == before.size
+        assert np.allclose(W[k], after, rtol=1e-9, atol=1e-12), f"instance {k}"
+        assert np.allclose(Y[k], Y1, rtol=1e-9, atol=1e-9), f"instance {k}"

@@ -367,3 +367,17 @@ def test_outputs_of_recorded_rows_ignore_empty_lanes(filled_allocations, n, conn
     Yb = b.predict([u])[0][0]
     b.close()
     assert np.array_equal(Yb, Y)
+
+
+def test_ridge_pivots_over_the_exponent_range():
+    """One neuron, one row: w = x y / x^2, through the reciprocal root of the pivot
+    twice. rsqrt is good to 1 ulp (2 eps / 2 at most, relative), the four roundings
+    around it to eps / 2 each: 4 eps in all."""
+    rng = np.random.default_rng(0)
+    for e in range(-500, 505, 5):
+        x = np.ldexp(rng.uniform(1.0, 2.0), e)
+        y = rng.uniform(1.0, 2.0)
+        W, rep = sp.ridge_fit(np.array([[x]]), np.array([[y]]), 0.0, max_refine=0)
+        assert rep.factor_failed == 0
+        exact = np.longdouble(y) / np.longdouble(x)
+        assert abs(np.longdouble(W[0, 0]) - exact) <= 4 * np.finfo(float).eps * exact, e
