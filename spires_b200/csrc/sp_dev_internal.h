@@ -60,7 +60,7 @@ struct sp_dev {
     // staging for host-driven runs
     size_t chunk;        // macro steps per chunk
     double *d_u;         // [chunk][din]
-    double *d_phi;       // [chunk][rs] position-space states
+    double *d_phi;       // [chunk][rs] position-space states; empty lanes 0
     double *d_nat;       // [chunk][n] neuron-order states
     double *d_y;         // [chunk][dout]
     unsigned *d_ras;     // [chunk][nw] position-space spike words

@@ -1908,7 +1908,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
         sprev = fired ? 1.0 : 0.0;
         SP_STAMP(tid == 0, b, B, 5);
         if (m == p.micro - 1) {
-            if (wact && p.phi)  // empty lanes too: a recorded row is read whole, 0 there
+            if (act && p.phi)  // empty lanes stay 0: a recorded row is read whole
                 p.phi[(size_t)s * p.rs + i] = V;
             if (wact && lane == 0 && p.raster)
                 p.raster[(size_t)s * p.nwords + gw] = lastword;
