@@ -641,6 +641,17 @@ static int lu_factor_solve(cudaStream_t s, double *A, int n, int lda, int *d_piv
     return 0;
 }
 
+// Waits for the stream; SP_EINTERNAL when a wait of a factorisation or solve on it
+// ran out (their results are then not the system's).
+static int solves_done(cudaStream_t s, const int *d_info)
+{
+    int h = 0;
+    if (cudaMemcpyAsync(&h, d_info, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
+        return SP_EINTERNAL;
+    return h < 0 ? SP_EINTERNAL : SP_OK;
+}
+
 // Residual R = Phi^T (Y - Phi W) - lambda W for rows [t0, t1).
 static void ridge_residual(cudaStream_t s, const double *Phi, int n, size_t t0, size_t t1,
                            const double *Y, const double *W, int dout, double lambda, double *E,
@@ -721,8 +732,9 @@ static int ridge_dual(cudaStream_t s, const double *Phi, int n, size_t T, size_t
         k_xt_e_part<<<gp, 128, 0, s>>>(Phi, n, w0, T, E, dout, parts, part);
         k_reduce_parts<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(part, parts, n, dout, nullptr,
                                                                      0.0, W);
-        RK(cudaStreamSynchronize(s));
-        RK(cudaGetLastError());
+        rc = solves_done(s, info);
+        if (rc)
+            goto out;
         rep->factor_ms = ms_since(tf);
     }
 out:
@@ -841,7 +853,7 @@ static int ridge_mixed(cudaStream_t s, const double *Phi, int n, size_t T, size_
         rep->rel_residual = device_norm(s, R, tot, tmp) / bden;
         rep->refine_iters = it;
         rep->refine_ms = ms_since(tr);
-        RK(cudaGetLastError());
+        rc = solves_done(s, info);
     }
 out:
     cudaStreamSynchronize(s);
@@ -1154,12 +1166,7 @@ static int ridge_phi_group(cudaStream_t s, const double *Phi, int n, size_t T,
         const size_t tot = (size_t)n * dout;
         // W (n x dout) -> W_out (dout x n)
         k_transpose_w<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(W, n, dout, d_W_out);
-        int h = 0;
-        RK(cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, s));
-        RK(cudaStreamSynchronize(s));
-        RK(cudaGetLastError());
-        if (h < 0)
-            rc = SP_EINTERNAL;  // a wait of a solve ran out
+        rc = solves_done(s, info);
     }
 out:
     if (!ws) {
@@ -1798,10 +1805,8 @@ static int na_solve(int dev, const double *d_states, const double *d_targets, si
             return SP_EINTERNAL;
         k_axpy<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(W, R, tot);
     }
-    int h = 0;
-    if (cudaMemcpyAsync(&h, info, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess || h < 0)
-        return SP_EINTERNAL;  // h < 0: a wait of the solver ran out
+    if (solves_done(s, info) != SP_OK)
+        return SP_EINTERNAL;
     k_transpose_w<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(W, n, dout, d_w_out);
     if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
         return SP_EINTERNAL;
