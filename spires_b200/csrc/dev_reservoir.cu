@@ -726,25 +726,35 @@ static void default_launch(sp_dev *d)
         // and 19.6, 2 x 64 23.5 and 21.1, 2 x 48 25.3 and 22.8; N=12000, L=2000 4 x
         // 64 28.2 and 28.3, 3 x 64 29.2 and 28.8; N=32000, L=1024, where only 2 x
         // 48 fit, 35.3 and 36.1, and 162 in the generic kernel.)
+        // The other synapses read their drive or traces in the serial phase, which a
+        // fuller stream slows: beside a ring beyond the L2 they take at most three
+        // stages in 160 KB, where that leaves two (scale-free graph, PSC_HOMOGENEOUS,
+        // PSC_HETEROGENEOUS, FRACTIONAL_MULTIEXP: N=20000, L=1024 3 x 48 31.9, 27.7 and
+        // 33.0, 3 x 64 34.5, 31.5 and 36.0, 2 x 64 32.2, 29.6 and 34.0; N=12000, L=2000
+        // 3 x 64 19.0, 17.5 and 20.0, 5 x 64 20.8, 19.9 and 21.7).
         sp_launch best = l;
         long long best_rows = 0;
-        for (int rows : {64, 48, 32}) {
-            if ((rows > 32) != (d->nc.L >= 512))
-                continue;
-            sp_launch v = l;
-            v.variant = 1;
-            v.rows = rows;
-            int bw, nbx;
-            box_geometry(d, v, &bw, &nbx);
-            const size_t stage = (size_t)v.rows * nbx * bw * sizeof(double);
-            long long st = pipe_stages(d, v, stage, 2 * 1024);
-            if (st >= 2 && st * rows > best_rows &&
-                encode_ring_map(d, bw, v.rows < d->nc.L ? v.rows : d->nc.L) == SP_OK) {
-                v.stages = (int)st;
-                best = v;
-                best_rows = st * rows;
+        const bool few = d->stype != SP_SYN_SIMPLE && auto_l2_pin(d) > 0;
+        for (int pass = few ? 0 : 1; pass < 2 && best_rows == 0; ++pass)
+            for (int rows : {64, 48, 32}) {
+                if ((rows > 32) != (d->nc.L >= 512))
+                    continue;
+                sp_launch v = l;
+                v.variant = 1;
+                v.rows = rows;
+                int bw, nbx;
+                box_geometry(d, v, &bw, &nbx);
+                const size_t stage = (size_t)v.rows * nbx * bw * sizeof(double);
+                long long st = pipe_stages(d, v, stage, 2 * 1024);
+                if (pass == 0)
+                    st = std::min({st, 3ll, (long long)(160 * 1024 / stage)});
+                if (st >= 2 && st * rows > best_rows &&
+                    encode_ring_map(d, bw, v.rows < d->nc.L ? v.rows : d->nc.L) == SP_OK) {
+                    v.stages = (int)st;
+                    best = v;
+                    best_rows = st * rows;
+                }
             }
-        }
         if (best_rows > 0) {
             l = best;
             int bw, nbx;

@@ -225,3 +225,20 @@ def test_wide_ctas_keep_the_pipeline(n, L):
     l = r.launch()
     r.close()
     assert l.variant == 1 and l.stages >= 2
+
+
+@pytest.mark.parametrize("n,L,syn,prm", [(20000, 1024, sp.SYN_PSC_HOM, (3.0,)),
+                                         (12000, 2000, sp.SYN_FRAC, (0.6, 4.0, 100.0)),
+                                         (30000, 700, sp.SYN_PSC_HET, (1.0, 10.0))])
+def test_stages_beside_a_drive_are_few(n, L, syn, prm):
+    """The synapses that read memory in the serial phase: at most three stages in 160 KB
+    beside a ring beyond the L2, and the pipeline all the same where two take more."""
+    cfg = sp.make_config(n, 1, 1, rho=0.0, conn=2.0 / n, topo=sp.CONN_SMALL_WORLD,
+                         neuron=sp.FLIF_GL, nparams=GL(L), synapse=syn, sparams=prm)
+    r = sp.Reservoir(cfg, seed=1)
+    l = r.launch()
+    r.close()
+    width = (n + l.ctas - 1) // l.ctas
+    assert l.variant == 1 and l.stages >= 2
+    if 2 * 48 * width * 8 <= 160 * 1024:
+        assert l.stages <= 3 and l.stages * l.rows * width * 8 <= 160 * 1024
