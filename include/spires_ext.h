@@ -215,6 +215,10 @@ typedef struct {
     int    refine_iters;
     double rel_residual;     /* ||Phi^T Y - (Phi^T Phi + lambda I) W|| / ||Phi^T Y|| */
     double collect_ms, gram_ms, factor_ms, refine_ms;
+                             /* collect: simulation, or the copies of host states
+                                that the Gram waits for; the FP64 Gram of host
+                                states of up to 16 outputs runs beside their copy
+                                and gram_ms is then both */
     int    factor_failed;
     int    lu_fallback;
     int    dual;             /* 1: fewer fitted rows than N/2, solved as

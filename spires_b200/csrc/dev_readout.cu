@@ -351,7 +351,8 @@ __global__ void k_diag_init(double *P, int n, double v)
 // order, so the bits are theirs. What bounds it: the exchange, about 1 us a
 // step, until P no longer fits the SMs' shared memory (about 1700 neurons)
 // and streams from the L2 or HBM, read and written once a step. (N=800, 400
-// steps: 4.5 us per step beside the 2.4 of the simulation; four launches a step took 47 together.)
+// steps: 4.4 us per step beside the 3.1 of a FLIF_GL, L=64 simulation; four
+// launches a step took 47 together.)
 struct RlsArgs {
     const double *X;           // [T][n] states
     const double *Y;           // [T][dout] targets

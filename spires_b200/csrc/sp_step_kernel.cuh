@@ -1,9 +1,9 @@
 // sp_step_kernel.cuh -- the persistent reservoir step kernel (all neuron and
 // synapse models), included by dev_reservoir.cu.
 //
-// Launch: a cooperative grid of G CTAs (variant 3: one cluster); CTA b owns the whole warps
-// [b*nw/G, (b+1)*nw/G) of neurons (nw = ceil(n/32)); a consumer thread owns
-// one neuron and keeps its state in registers for the whole launch.
+// Launch: a cooperative grid of G CTAs (variant 3: one cluster); CTA b owns the
+// whole warps [b*nw/G, (b+1)*nw/G) of neurons (nw = ceil(n/32)); a consumer
+// thread owns one neuron and keeps its state in registers for the whole launch.
 //
 // Variant 0: the FLIF_GL history is summed with direct loads from the
 //   time-major ring (each lag is one coalesced row segment).
@@ -17,9 +17,9 @@
 //   register, so the producer streams lags 34.. only (3 % fewer ring bytes per
 //   step at L = 1024) and the sum of a step starts as soon as its lag 1 exists.
 //   The grid is sized so that each CTA streams about the same number of ring
-//   columns (balanced layout, dev_reservoir.cu). A gather warp watches the spike exchange and copies
-//   the words into a double-buffered shared array while the consumers are
-//   still summing.
+//   columns (balanced layout, dev_reservoir.cu). A gather warp watches the
+//   spike exchange and copies the words into a double-buffered shared array
+//   while the consumers are still summing.
 //   A ring larger than the L2 is read with cache hints: the oldest l2_pin
 //   lags of a step are loaded with evict-last priority and stay L2-resident
 //   from step to step (each row joins them once, when it reaches lag
@@ -27,10 +27,12 @@
 //   DRAM reads come first in every step and run on through the serial phase.
 //
 // Variant 2 (FLIF_GL whose CTAs' ring columns fit in shared memory, and
-//   FLIF_CAPUTO): the history is loaded into shared memory once per launch and
-//   summed there (chain_pairs); the ring in global memory is still written
-//   every step, as the state between launches. A gather warp as in variant 1.
-//   (N=2000, L=256: 3.4 us per step; 5.9 through the pipeline's stages.)
+//   FLIF_CAPUTO): FLIF_GL's history is loaded into shared memory once per launch
+//   and summed there (chain_pairs); the ring in global memory is still written
+//   every step, as the state between launches. (N=2000, L=256: 3.4 us per step;
+//   5.9 through the pipeline's stages.) FLIF_CAPUTO's registers stay in global
+//   memory, read as 32-byte blocks (caputo_sum), eight in flight. A gather warp
+//   as in variant 1.
 // Variant 3 (2, 4, 8 or 16 CTAs as one cluster, at most 8192 neurons; SIMPLE and
 //   PSC_HETEROGENEOUS): the exchange below between the CTAs' shared memories.
 //   (LIF_DISCRETE N=2000: 1.1 us per step; 1.5 through the L2.)
@@ -50,12 +52,12 @@
 // read every word of step b, so nobody can still be reading the buffer of
 // step b - 1 that it overwrites. That holds for a reader only if a warp that
 // publishes waits for it: a CTA without neurons (more CTAs than warps), and in
-// variant 3 a warp without, read no words and skip the steps. (LIF_DISCRETE N=20000: 6.7 us per step with
-// flags and fences, 4.1 with the exchange and the row slots.) A gather warp
-// starts to poll when its own CTA has published: polled all along, the entries'
-// lines slowed the stores and the history stream (FLIF_GL N=20000, L=128: 5.9
-// us per step, 3.6). The other synapses publish a double per neuron as well
-// and keep the flags and fences.
+// variant 3 a warp without, read no words and skip the steps. (LIF_DISCRETE
+// N=20000: 6.7 us per step with flags and fences, 4.1 with the exchange and the
+// row slots.) A gather warp starts to poll when its own CTA has published:
+// polled all along, the entries' lines slowed the stores and the history stream
+// (FLIF_GL N=20000, L=128: 5.9 us per step, 3.6). The other synapses publish a
+// double per neuron as well and keep the flags and fences.
 //
 // Per micro-step, with a split-phase grid barrier:
 //   history sum of step g      (overlaps the barrier wait)
