@@ -703,8 +703,14 @@ static void default_launch(sp_dev *d)
     // the history sum hides the slower exchange). Column blocks only where
     // they fit the 16 CTAs' shared memory.
     const sp_launch clus = shape(nw >= 16 ? 16 : 8);
+    // PSC_HETEROGENEOUS walks every edge in every step, so that many warps on 16 SMs
+    // wait for one another's loads (small world, 150 steps: N=2000, 4 warps a CTA, 6
+    // edges a row 0.81 ms on the cluster and 0.86 on 63 CTAs, 15 edges 1.9 and 1.7, 50
+    // edges 6.6 and 5.2; N=8000, 50 edges 9.5 on the cluster, 5.8 on 125 CTAs).
+    const bool het = clus.warps_max <= 2 || (clus.warps_max <= 4 && d->nnz <= 12 * (size_t)d->n);
     const bool cluster = nw > 6 && kernel_variant(d, clus) == 3 &&
                          row_plan(d, clus).col_mode != 1 && d->ntype != SP_FLIF_CAPUTO &&
+                         (d->stype != SP_SYN_PSC_HET || het) &&
                          (!gl || (nw >= 64 && clus.warps_max * d->nc.L <= 768));
     if (nw <= 4)
         l = shape(1);  // a warp per scheduler, nothing to exchange

@@ -242,3 +242,17 @@ def test_stages_beside_a_drive_are_few(n, L, syn, prm):
     assert l.variant == 1 and l.stages >= 2
     if 2 * 48 * width * 8 <= 160 * 1024:
         assert l.stages <= 3 and l.stages * l.rows * width * 8 <= 160 * 1024
+
+
+@pytest.mark.parametrize("n,edges,clustered", [(1000, 100, True), (2000, 12, True), (2000, 40, False),
+                                               (4000, 4, False)])
+def test_heterogeneous_synapses_leave_the_cluster(n, edges, clustered):
+    """PSC_HETEROGENEOUS walks every edge in every step: a cluster where its CTAs have few
+    warps and edges, else the wide launch; both as the oracle."""
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=edges / n, dt=1.0,
+                         topo=sp.CONN_SMALL_WORLD, neuron=sp.LIF_DISCRETE,
+                         nparams=O.NEURON_PARAMS[sp.LIF_DISCRETE], synapse=sp.SYN_PSC_HET,
+                         sparams=(1.0, 10.0))
+    r = sp.Reservoir(cfg, seed=11)
+    assert (r.launch().ctas == 16) == clustered
+    run_against_oracle(r, cfg, 12, 11)
