@@ -738,10 +738,14 @@ static void default_launch(sp_dev *d)
         // PSC_HETEROGENEOUS, FRACTIONAL_MULTIEXP: N=20000, L=1024 3 x 48 31.9, 27.7 and
         // 33.0, 3 x 64 34.5, 31.5 and 36.0, 2 x 64 32.2, 29.6 and 34.0; N=12000, L=2000
         // 3 x 64 19.0, 17.5 and 20.0, 5 x 64 20.8, 19.9 and 21.7).
+        // Coefficients that are not staged are read through the L1, which has what the
+        // shared memory leaves: at most 144 KB of stages then (L=9000, N=20 9 x 64 141
+        // us per step, 13 x 64 196; N=2000 142 and 212).
         sp_launch best = l;
         long long best_rows = 0;
         const bool few = d->stype != SP_SYN_SIMPLE && auto_l2_pin(d) > 0;
-        for (int pass = few ? 0 : 1; pass < 2 && best_rows == 0; ++pass)
+        const size_t most = (size_t)(coef_smem_bytes(d) == 0 ? 144 : few ? 160 : 0) * 1024;
+        for (int pass = most > 0 ? 0 : 1; pass < 2 && best_rows == 0; ++pass)
             for (int rows : {64, 48, 32}) {
                 if ((rows > 32) != (d->nc.L >= 512))
                     continue;
@@ -753,7 +757,7 @@ static void default_launch(sp_dev *d)
                 const size_t stage = (size_t)v.rows * nbx * bw * sizeof(double);
                 long long st = pipe_stages(d, v, stage, 2 * 1024);
                 if (pass == 0)
-                    st = std::min({st, 3ll, (long long)(160 * 1024 / stage)});
+                    st = std::min({st, few ? 3ll : 16ll, (long long)(most / stage)});
                 if (st >= 2 && st * rows > best_rows &&
                     encode_ring_map(d, bw, v.rows < d->nc.L ? v.rows : d->nc.L) == SP_OK) {
                     v.stages = (int)st;

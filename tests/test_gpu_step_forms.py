@@ -256,3 +256,16 @@ def test_heterogeneous_synapses_leave_the_cluster(n, edges, clustered):
     r = sp.Reservoir(cfg, seed=11)
     assert (r.launch().ctas == 16) == clustered
     run_against_oracle(r, cfg, 12, 11)
+
+
+def test_stages_leave_the_coefficients_an_l1():
+    """More coefficients than are staged (8192): the stages leave the L1 room for them, and
+    the sums through them are the oracle's."""
+    n = 70
+    cfg = sp.make_config(n, 2, 2, rho=1.3, ei=0.55, gamma=1.2, conn=0.2, dt=1.0,
+                         topo=sp.CONN_RANDOM, neuron=sp.FLIF_GL, nparams=GL(8300))
+    r = sp.Reservoir(cfg, seed=11)
+    l = r.launch()
+    assert l.variant == 1 and 2 <= l.stages
+    assert l.stages * l.rows * 32 * l.warps_max * 8 <= 144 * 1024
+    run_against_oracle(r, cfg, 90, 11)
