@@ -735,9 +735,9 @@ static void default_launch(sp_dev *d)
         // The other synapses read their drive or traces in the serial phase, which a
         // fuller stream slows: beside a ring beyond the L2 they take at most three
         // stages in 160 KB, where that leaves two (scale-free graph, PSC_HOMOGENEOUS,
-        // PSC_HETEROGENEOUS, FRACTIONAL_MULTIEXP: N=20000, L=1024 3 x 48 31.9, 27.7 and
-        // 33.0, 3 x 64 34.5, 31.5 and 36.0, 2 x 64 32.2, 29.6 and 34.0; N=12000, L=2000
-        // 3 x 64 19.0, 17.5 and 20.0, 5 x 64 20.8, 19.9 and 21.7).
+        // PSC_HETEROGENEOUS, FRACTIONAL_MULTIEXP: N=20000, L=1024 3 x 48 29.2, 25.8 and
+        // 30.6, 3 x 64 32.2, 28.1 and 34.5, 2 x 64 29.7, 28.2 and 30.7; N=12000, L=2000
+        // 3 x 64 18.5, 17.1 and 19.4, 5 x 64 19.7, 19.5 and 21.6).
         // Coefficients that are not staged are read through the L1, which has what the
         // shared memory leaves: at most 144 KB of stages then (L=9000, N=20 9 x 64 141
         // us per step, 13 x 64 196; N=2000 142 and 212).

@@ -1376,7 +1376,7 @@ __global__ void __launch_bounds__(Bounds<VAR>::threads, 1) k_run(const __grid_co
     // fit shared memory: the bulk copies keep more bytes in flight than the
     // threads' loads, sixteen each. (N=20000, 512 lags beside a ring of 1024: 86
     // us per step with one load in flight after the update, 69 with sixteen
-    // before the barrier, 46 through the stages; the two histories are 245 MB.)
+    // before the barrier, 43 through the stages; the two histories are 245 MB.)
     double fhist = 0.0;
     int shead = ST == SP_SYN_FRAC ? (int)(p.syn_step0 % p.Ls) : 0;
     int srow = shead;  // its row, counted by empty lanes too
